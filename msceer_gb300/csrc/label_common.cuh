@@ -97,10 +97,10 @@ cudaError_t launch_group_seeds(const int32_t* rep, const int64_t* seed, int n_ex
                                uint8_t* state, int num_sms, cudaStream_t stream);
 int64_t terminal_num_tiles(const VolDims& V);
 // One round of the certain terminal regions' global frontier walk from the vertices
-// qin[0, *n_in) (n_host: the same count on the host, for the grid); vertices beyond a
-// thread's stack go to qout.
+// qin[0, *n_in), dealt out through *cursor; what the blocks hand over goes to qout
+// (*n_out and *cursor are set to zero first).
 cudaError_t launch_terminal_walk(const float* f, int32_t* lab, const VolDims& V, int dir, const int64_t* qin,
-                                 const int* n_in, int n_host, int64_t* qout, int* n_out, int cap, int* err,
+                                 const int* n_in, int* cursor, int64_t* qout, int* n_out, int cap, int* err,
                                  int num_sms, cudaStream_t stream);
 cudaError_t launch_terminal_pass(const float* f, int32_t* lab, const VolDims& V, int dir, const uint8_t* dirty_in,
                                  uint8_t* dirty_out, int* changed, int* err, int num_sms, cudaStream_t stream);

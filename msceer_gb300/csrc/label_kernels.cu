@@ -481,16 +481,29 @@ __global__ void __launch_bounds__(BS) terminal_pass_kernel(const float* __restri
 // region's label (InspectPriorRegions), so its label is a function of its earlier
 // neighbours' labels alone and the regions are the unique fixpoint, whatever the
 // order of the inspections.  Here every newly labelled vertex inspects its later
-// 6-neighbours in global memory, depth-first with a short per-thread stack (what does
-// not fit goes to the next round's frontier); the first round starts from the seeds.
-// A vertex that an inspection finds not yet decided is inspected again when its last
-// earlier neighbour gets its label.  The labels are set by compare-and-swap from -1,
-// so every vertex enters a frontier at most once.
+// 6-neighbours in global memory; the first round starts from the seeds.  A vertex that
+// an inspection finds not yet decided is inspected again when its last earlier
+// neighbour gets its label.  The labels are set by compare-and-swap from -1, so every
+// vertex enters a frontier at most once.
+//
+// The chains are as long as a basin is deep, and what bounds the walk is the latency of
+// one link (two dependent reads and the swap, ~1.5 us through L2), times the links that
+// follow one another.  So a block shares one stack: it takes up to kWalkItems vertices
+// at a time, a thread per (vertex, neighbour), and takes new ones from the frontier
+// while its own stack is short.  (A thread per vertex with a stack of its own walked a
+// whole basin of a smooth field alone, one vertex after another: 265 ms of the 430 ms
+// labels of a 256^3 Gaussian-sum field, where the walk now takes a few ms.)  A block
+// that has worked kWalkTail turns past the frontier's end hands what is on its stack to
+// the next round, which deals it out to all blocks again: one block of a deep basin
+// otherwise worked on while the others had ended.
+constexpr int kWalkThreads = 256;
+constexpr int kWalkItems = 128;   // vertices a turn
+constexpr int kWalkStack = 2048;  // vertices on the block's stack
+constexpr int kWalkTail = 16;
 
-// Comparer::Compare(a, b), "a comes before b": value, then index (ascending labels: the
-// lower value; descending: the higher)
-__device__ __forceinline__ bool walk_before(const float* __restrict__ f, int dir, int64_t a, int64_t b) {
-  const float fa = f[a], fb = f[b];
+// Comparer::Compare(a, b), "a comes before b", on the vertices' values and indices
+// (ascending labels: the lower value; descending: the higher)
+__device__ __forceinline__ bool walk_before(int dir, float fa, int64_t a, float fb, int64_t b) {
   if (dir < 0) {
     if (fb > fa) return true;
     if (fa > fb) return false;
@@ -501,76 +514,138 @@ __device__ __forceinline__ bool walk_before(const float* __restrict__ f, int dir
   return a > b;
 }
 
-__global__ void __launch_bounds__(128) terminal_walk_kernel(const float* __restrict__ f, int32_t* __restrict__ lab,
-                                                            const VolDims V, int dir, const int64_t* __restrict__ qin,
-                                                            const int* __restrict__ n_in, int64_t* __restrict__ qout,
-                                                            int* __restrict__ n_out, int cap, int* __restrict__ err) {
-  constexpr int SD = 16;
-  const int n = *n_in;
-  const int64_t X = V.X, XY = V.X * V.Y;
-  const int64_t E[3] = {V.X, V.Y, V.Z};
-  const int64_t S[3] = {1, V.X, XY};
+// n_in vertices of the frontier qin, dealt out through *cursor (zero at the launch).
+__global__ void __launch_bounds__(kWalkThreads) terminal_walk_kernel(
+    const float* __restrict__ f, int32_t* __restrict__ lab, const VolDims V, int dir, const int64_t* __restrict__ qin,
+    const int* __restrict__ n_in, uint32_t* __restrict__ cursor, int64_t* __restrict__ qout, int* __restrict__ n_out,
+    int cap, int* __restrict__ err) {
+  __shared__ int32_t s_stack[kWalkStack];
+  __shared__ int32_t s_item[kWalkItems];
+  __shared__ int s_top, s_base, s_got;
+  const int tid = threadIdx.x;
+  const int n = *n_in < cap ? *n_in : cap;
+  if (n <= 0) return;
+  // vertices taken from the frontier at a time: a short frontier goes to all blocks
+  const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int fetch = per < 8 ? 8 : (per < kWalkItems ? per : kWalkItems);
+  const uint32_t X = (uint32_t)V.X, Y = (uint32_t)V.Y;  // fewer than 2^31 vertices
+  const int32_t E[3] = {(int32_t)V.X, (int32_t)V.Y, (int32_t)V.Z};
+  const int32_t S[3] = {1, (int32_t)V.X, (int32_t)(V.X * V.Y)};
   volatile int32_t* vl = lab;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    int64_t stack[SD];
-    int sp = 0;
-    stack[sp++] = qin[k];
-    while (sp > 0) {
-      const int64_t v = stack[--sp];
-      const uint32_t u32 = (uint32_t)v, x32 = (uint32_t)X, y32 = (uint32_t)V.Y;  // fewer than 2^31 vertices
-      const uint32_t r = u32 / x32;
-      const int64_t vc[3] = {(int64_t)(u32 - r * x32), (int64_t)(r % y32), (int64_t)(r / y32)};
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-#pragma unroll
-        for (int s = 0; s < 2; s++) {
-          const int64_t wa = vc[a] + (s == 0 ? 1 : -1);
-          if (wa < 0 || wa >= E[a]) continue;
-          const int64_t w = v + (s == 0 ? S[a] : -S[a]);
-          if (vl[w] != -1 || !walk_before(f, dir, v, w)) continue;
-          // InspectPriorRegions of w (gi_extrema_region_builder.h:806-857)
-          int64_t wc[3] = {vc[0], vc[1], vc[2]};
-          wc[a] = wa;
-          int32_t l = -1;
-          bool ok = true;
-#pragma unroll
-          for (int b = 0; b < 3 && ok; b++) {
-#pragma unroll
-            for (int t = 0; t < 2; t++) {
-              const int64_t ua = wc[b] + (t == 0 ? 1 : -1);
-              if (ua < 0 || ua >= E[b]) continue;
-              const int64_t u = w + (t == 0 ? S[b] : -S[b]);
-              if (!walk_before(f, dir, u, w)) continue;
-              const int32_t lu = vl[u];
-              if (lu < 0 || (l >= 0 && lu != l)) {
-                ok = false;
-                break;
-              }
-              l = lu;
-            }
-          }
-          if (!ok || l < 0) continue;
-          if (atomicCAS(&lab[w], -1, l) != -1) continue;
-          if (sp < SD) {
-            stack[sp++] = w;
-          } else {
-            const int slot = atomicAdd(n_out, 1);
-            if (slot < cap) qout[slot] = w; else atomicOr(err, kErrLocalQueue);
-          }
-        }
+  bool more = true;  // the frontier may hold vertices not dealt out yet
+  int tail = 0;
+  if (tid == 0) s_top = 0;
+  __syncthreads();
+  while (true) {
+    const int top = s_top;
+    if (tid == 0) {
+      s_got = 0;
+      if (more && top < kWalkItems) {
+        const uint32_t b = atomicAdd(cursor, (uint32_t)fetch);  // (at most n + fetch * blocks)
+        s_base = (int)b;
+        s_got = b >= (uint32_t)n ? -1 : (n - (int)b < fetch ? n - (int)b : fetch);
       }
     }
+    __syncthreads();
+    const int got = s_got > 0 ? s_got : 0;
+    if (s_got < 0) more = false;
+    if (!more) tail++;
+    if (top + got == 0) {
+      if (!more) break;
+      __syncthreads();  // s_got is rewritten
+      continue;
+    }
+    if (tail > kWalkTail) {  // the rest goes to the next round
+      __shared__ int s_out;
+      if (tid == 0) s_out = atomicAdd(n_out, top);
+      __syncthreads();
+      for (int i = tid; i < top; i += kWalkThreads) {
+        const int slot = s_out + i;
+        if (slot < cap) qout[slot] = s_stack[i]; else atomicOr(err, kErrLocalQueue);
+      }
+      break;
+    }
+    const int take = top < kWalkItems - got ? top : kWalkItems - got;
+    const int m = take + got;
+    if (tid < m) s_item[tid] = tid < take ? s_stack[top - 1 - tid] : (int32_t)qin[s_base + tid - take];
+    if (tid == 0) s_top = top - take;
+    __syncthreads();
+    bool labelled = false;
+    for (int p = tid; p < 6 * m; p += kWalkThreads) {
+      const int k = p / 6, j = p - 6 * k, a = j >> 1;
+      const int32_t v = s_item[k];
+      const uint32_t r = (uint32_t)v / X;
+      int32_t wc[3] = {(int32_t)((uint32_t)v - r * X), (int32_t)(r % Y), (int32_t)(r / Y)};
+      const int sgn = (j & 1) ? -1 : 1;
+      int32_t Sa = S[0];
+      bool in;
+      if (a == 0) {
+        wc[0] += sgn;
+        in = wc[0] >= 0 && wc[0] < E[0];
+      } else if (a == 1) {
+        wc[1] += sgn;
+        Sa = S[1];
+        in = wc[1] >= 0 && wc[1] < E[1];
+      } else {
+        wc[2] += sgn;
+        Sa = S[2];
+        in = wc[2] >= 0 && wc[2] < E[2];
+      }
+      if (!in) continue;
+      const int32_t w = v + sgn * Sa;
+      const int32_t lw = vl[w];
+      const float fv = __ldg(f + v), fw = __ldg(f + w);
+      if (lw != -1 || !walk_before(dir, fv, v, fw, w)) continue;
+      // InspectPriorRegions of w (gi_extrema_region_builder.h:806-857), its neighbours'
+      // values and labels read together
+      float fu[6];
+      int32_t lu[6];
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        const int b = q >> 1, d = (q & 1) ? -1 : 1;
+        const bool has = d > 0 ? wc[b] + 1 < E[b] : wc[b] > 0;
+        const int32_t u = has ? w + d * S[b] : w;
+        fu[q] = __ldg(f + u);
+        lu[q] = vl[u];
+      }
+      int32_t l = -1;
+      bool ok = true;
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        const int b = q >> 1, d = (q & 1) ? -1 : 1;
+        const bool has = d > 0 ? wc[b] + 1 < E[b] : wc[b] > 0;
+        if (!has || !walk_before(dir, fu[q], w + d * S[b], fw, w)) continue;
+        ok = ok && lu[q] >= 0 && (l < 0 || lu[q] == l);
+        l = lu[q];
+      }
+      if (!ok || l < 0) continue;
+      if (atomicCAS(&lab[w], -1, l) != -1) continue;
+      labelled = true;
+      const int slot = atomicAdd(&s_top, 1);
+      if (slot < kWalkStack) {
+        s_stack[slot] = w;
+      } else {
+        const int o = atomicAdd(n_out, 1);
+        if (o < cap) qout[o] = w; else atomicOr(err, kErrLocalQueue);
+      }
+    }
+    // a label is visible before any inspection that follows it reads its neighbours'
+    if (labelled) __threadfence();
+    __syncthreads();
+    if (tid == 0 && s_top > kWalkStack) s_top = kWalkStack;
+    __syncthreads();
   }
 }
 
 cudaError_t launch_terminal_walk(const float* f, int32_t* lab, const VolDims& V, int dir, const int64_t* qin,
-                                 const int* n_in, int n_host, int64_t* qout, int* n_out, int cap, int* err,
+                                 const int* n_in, int* cursor, int64_t* qout, int* n_out, int cap, int* err,
                                  int num_sms, cudaStream_t stream) {
-  if (n_host <= 0) return cudaSuccess;
-  const int blocks = (n_host + 127) / 128;
-  const int grid = blocks < num_sms * 16 ? blocks : num_sms * 16;
+  if (cudaError_t e = cudaMemsetAsync(n_out, 0, sizeof(int), stream)) return e;
+  if (cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(int), stream)) return e;
   ::msc::count_launch();
-  terminal_walk_kernel<<<grid, 128, 0, stream>>>(f, lab, V, dir, qin, n_in, qout, n_out, cap, err);
+  terminal_walk_kernel<<<num_sms * 8, kWalkThreads, 0, stream>>>(f, lab, V, dir, qin, n_in,
+                                                                 reinterpret_cast<uint32_t*>(cursor), qout, n_out, cap,
+                                                                 err);
   return cudaGetLastError();
 }
 

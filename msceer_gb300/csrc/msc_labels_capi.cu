@@ -278,7 +278,7 @@ struct LabelCtx {
   int* counters = nullptr;  // [0] n_ext [1] n_sad [2] n_arcs [3] changed [4] err [5] n_list / wave members
                             // without an end [6] n_next [7] n_amb [8, 10) cleaner [10] long chain
                             // [12] vertices whose ends are computed ahead of the waves
-                            // [13], [14] terminal-walk frontier lengths
+                            // [13], [14] terminal-walk frontier lengths, [15] its cursor
   unsigned long long* work = nullptr;  // [0] claimed fix-up items, [48, 51) advection iterations (first
                                        // pass, FP32, FP64), [56] FP64 claims
   void* hpin = nullptr;                // kPinnedBytes of pinned host memory (pinned_get)
@@ -486,15 +486,19 @@ int prepare_direction(LabelCtx& c, DirLabels& d, int32_t* stage_terminal) {
     LCUDA(cudaMemcpyAsync(c.counters + 13, c.hpin, sizeof(int), cudaMemcpyHostToDevice, st), "write count");
     int* n_cur = c.counters + 13;
     int* n_nxt = c.counters + 14;
-    int rounds = 0;
+    // after the first, rounds go in groups of four between counter reads (a round with
+    // nothing handed over ends at once)
+    int64_t rounds = 0;
     while (n > 0) {
-      if (rounds++ > N) return fail(MSC_ERR_ITER_LIMIT, "terminal regions did not converge");
-      LCUDA(cudaMemsetAsync(n_nxt, 0, sizeof(int), st), "memset");
-      LCUDA(msc::launch_terminal_walk(c.f, d.lab, V, dir, cur, n_cur, n, nxt, n_nxt, (int)N, c.counters + 4, c.sms, st),
-            "regions");
-      if (int rc = read_dev(c, n_nxt, 1, &n)) return rc;
-      std::swap(cur, nxt);
-      std::swap(n_cur, n_nxt);
+      if (rounds > N) return fail(MSC_ERR_ITER_LIMIT, "terminal regions did not converge");
+      for (int q = rounds == 0 ? 1 : 4; q > 0; q--, rounds++) {
+        LCUDA(msc::launch_terminal_walk(c.f, d.lab, V, dir, cur, n_cur, c.counters + 15, nxt, n_nxt, (int)N,
+                                        c.counters + 4, c.sms, st),
+              "regions");
+        std::swap(cur, nxt);
+        std::swap(n_cur, n_nxt);
+      }
+      if (int rc = read_dev(c, n_cur, 1, &n)) return rc;
     }
     trace_mark(st, dir, "terminal walk x" + std::to_string(rounds));
   } else {

@@ -723,73 +723,123 @@ __global__ void __launch_bounds__(256) ldir_check_kernel(const LdirBatch B, cons
   }
 }
 
-// Finish the walks of queued items in global memory, depth first with a short
-// per-thread stack; what does not fit goes to the next round's queue.
-// n_in_dev (when set): the queue length lives in device memory (graph-captured rounds)
+// Finish the walks of queued items in global memory.  The walks of a smooth field are
+// long, and what bounds them is the latency of one step (the cofacet's byte, its
+// compare-and-swap, the partner's: ~1.5 us through L2) times the steps that follow one
+// another.  So a block shares one stack: it takes up to kWalkItems items at a time, a
+// thread per (item, cofacet), and takes new ones from the queue while its own stack is
+// short.  (A thread per item with a stack of its own followed every branch of a walk
+// alone: 6.0 of the 6.3 ms of a 64^3 Gaussian-sum .grad.)  A block that has worked
+// kWalkTail turns past the queue's end hands its stack to the next round, which deals
+// it out to all blocks again.  The queue's length is read on the device (0 after an
+// overflow: the host finishes with tile passes) and it is dealt out through *cursor.
+constexpr int kWalkThreads = 256;
+constexpr int kWalkItems = 128;   // items a turn
+constexpr int kWalkStack = 1024;  // items on the block's stack
+constexpr int kWalkTail = 16;
+
 template <int ND>
-__global__ void __launch_bounds__(128) ldir_walk_kernel(const LdirBatch B, const int64_t* __restrict__ qin, int n_in,
-                                                        const int* __restrict__ n_in_dev, int64_t* __restrict__ qout,
-                                                        int* __restrict__ n_out, int cap, int* lock, int* err) {
-  constexpr int SD = 24;
-  int64_t stack[SD];
-  if (n_in_dev) {
-    n_in = *n_in_dev;
-    if (n_in > cap) n_in = 0;  // overflowed: the host finishes with tile passes
-  }
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_in; k += gridDim.x * blockDim.x) {
-    const int64_t entry = qin[k];
-    const int vi = entry_volume(entry);
-    if (vi >= B.n) {  // not an entry this launch wrote
-      atomicOr(err, kErrPassLimit);
-      continue;
-    }
-    const LdirVol& vol = B.v[vi];
-    const GradDims& D = vol.D;
-    const GradView G = volume_view(vol, lock, err);
-    const int64_t st[3] = {D.cs[0], D.cs[1], D.cs[2]};
-    const int64_t dd[3] = {D.d[0], D.d[1], D.d[2]};
-    int sp = 0;
-    stack[sp++] = entry & kCellMask;
-    while (sp > 0) {
-      const int64_t i = stack[--sp];
-      int64_t l[3];
-      l[0] = i % dd[0];
-      l[1] = (i / dd[0]) % dd[1];
-      l[2] = (ND == 3) ? i / (dd[0] * dd[1]) : 0;
-      const int dim = (int)((l[0] & 1) + (l[1] & 1) + (l[2] & 1));
-      const unsigned value = dim == 1 ? 2u : 1u;  // edges walk the value-2 closure, quads value 1
-#pragma unroll
-      for (int a = 0; a < ND; a++) {
-        if (l[a] & 1) continue;  // cofacets only along even axes, +axis first
-#pragma unroll
-        for (int s = 0; s < 2; s++) {
-          const int sgn = s == 0 ? 1 : -1;
-          const int64_t la = l[a] + sgn;
-          if (la < 0 || la >= dd[a]) continue;
-          const int64_t t = i + sgn * st[a];
-          const uint8_t bt = *reinterpret_cast<volatile uint8_t*>(G.g + t);
-          const unsigned code = (bt >> 2) & 7u;
-          if (!(bt & 1u) || code == 7u) continue;
-          lower_ldir(G, t, value);
-          const int pc = map3(D.dec_map, (int)code);
-          const int pa = pc >> 1;
-          const int64_t tp = t + ((pc & 1) ? -st[pa] : st[pa]);
-          if (tp == i) continue;
-          int64_t lp[3] = {l[0], l[1], l[2]};
-          lp[a] += sgn;
-          lp[pa] += (pc & 1) ? -1 : 1;
-          if (lp[pa] < 0 || lp[pa] >= dd[pa]) continue;  // a pair code pointing out of the complex
-          const int pdim = (int)((lp[0] & 1) + (lp[1] & 1) + (lp[2] & 1));
-          if (value == 2u && pdim != 1) {  // a hex ends the value-2 path
-            lower_ldir(G, tp, 2u);
-            continue;
-          }
-          if (!lower_ldir(G, tp, value)) continue;
-          if (sp < SD) stack[sp++] = tp;
-          else push_item(qout, n_out, cap, err, ((int64_t)vi << kVolShift) | tp);
-        }
+__global__ void __launch_bounds__(kWalkThreads) ldir_walk_kernel(const LdirBatch B, const int64_t* __restrict__ qin,
+                                                                 const int* __restrict__ n_in,
+                                                                 uint32_t* __restrict__ cursor,
+                                                                 int64_t* __restrict__ qout, int* __restrict__ n_out,
+                                                                 int cap, int* lock, int* err) {
+  __shared__ int64_t s_stack[kWalkStack];
+  __shared__ int64_t s_item[kWalkItems];
+  __shared__ int s_top, s_base, s_got, s_out;
+  const int tid = threadIdx.x;
+  const int n = *n_in;
+  if (n <= 0 || n > cap) return;
+  const int per = (n + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int fetch = per < 8 ? 8 : (per < kWalkItems ? per : kWalkItems);
+  bool more = true;
+  int tail = 0;
+  if (tid == 0) s_top = 0;
+  __syncthreads();
+  while (true) {
+    const int top = s_top;
+    if (tid == 0) {
+      s_got = 0;
+      if (more && top < kWalkItems) {
+        const uint32_t b = atomicAdd(cursor, (uint32_t)fetch);
+        s_base = (int)b;
+        s_got = b >= (uint32_t)n ? -1 : (n - (int)b < fetch ? n - (int)b : fetch);
       }
     }
+    __syncthreads();
+    const int got = s_got > 0 ? s_got : 0;
+    if (s_got < 0) more = false;
+    if (!more) tail++;
+    if (top + got == 0) break;  // (with more of the queue left, some of it was taken)
+    if (tail > kWalkTail) {     // the rest goes to the next round
+      if (tid == 0) s_out = atomicAdd(n_out, top);
+      __syncthreads();
+      for (int i = tid; i < top; i += kWalkThreads) {
+        const int slot = s_out + i;
+        if (slot < cap) qout[slot] = s_stack[i]; else atomicOr(err, kErrLocalQueue);
+      }
+      break;
+    }
+    const int take = top < kWalkItems - got ? top : kWalkItems - got;
+    const int m = take + got;
+    if (tid < m) s_item[tid] = tid < take ? s_stack[top - 1 - tid] : qin[s_base + tid - take];
+    if (tid == 0) s_top = top - take;
+    __syncthreads();
+    for (int p = tid; p < 2 * ND * m; p += kWalkThreads) {
+      const int k = p / (2 * ND), j = p - 2 * ND * k, a = j >> 1;
+      const int64_t entry = s_item[k];
+      const int vi = entry_volume(entry);
+      if (vi >= B.n) {  // not an entry this launch wrote
+        atomicOr(err, kErrPassLimit);
+        continue;
+      }
+      const LdirVol& vol = B.v[vi];
+      const GradDims& D = vol.D;
+      const int64_t i = entry & kCellMask;
+      int64_t l[3];
+      if (D.ncells <= (int64_t)0xFFFFFFFF) {
+        const uint32_t u = (uint32_t)i, d0 = (uint32_t)D.d[0], d1 = (uint32_t)D.d[1];
+        const uint32_t r = u / d0;
+        l[0] = u - r * d0;
+        l[1] = ND == 3 ? r % d1 : r;
+        l[2] = ND == 3 ? r / d1 : 0;
+      } else {
+        l[0] = i % D.d[0];
+        l[1] = (i / D.d[0]) % D.d[1];
+        l[2] = ND == 3 ? i / (D.d[0] * D.d[1]) : 0;
+      }
+      const int dim = (int)((l[0] & 1) + (l[1] & 1) + (l[2] & 1));
+      const unsigned value = dim == 1 ? 2u : 1u;  // edges walk the value-2 closure, quads value 1
+      const int64_t ca = a == 0 ? l[0] : (a == 1 ? l[1] : l[2]);
+      if (ca & 1) continue;  // cofacets only along even axes
+      const int sgn = (j & 1) ? -1 : 1;
+      if (ca + sgn < 0 || ca + sgn >= D.d[a]) continue;
+      const int64_t t = i + sgn * D.cs[a];
+      const uint8_t bt = *reinterpret_cast<volatile uint8_t*>(vol.g + t);
+      const unsigned code = (bt >> 2) & 7u;
+      if (!(bt & 1u) || code == 7u) continue;
+      const GradView G = volume_view(vol, lock, err);
+      lower_ldir(G, t, value);
+      const int pc = map3(D.dec_map, (int)code);
+      const int pa = pc >> 1, ps = (pc & 1) ? -1 : 1;
+      const int64_t tp = t + ps * D.cs[pa];
+      if (tp == i) continue;
+      // the partner's coordinate along the pair's axis, and its dimension
+      const int64_t cp = (pa == 0 ? l[0] : (pa == 1 ? l[1] : l[2])) + (pa == a ? sgn : 0) + ps;
+      if (cp < 0 || cp >= D.d[pa]) continue;  // a pair code pointing out of the complex
+      const int pdim = pa == a ? dim : (((cp & 1) != 0) ? dim + 2 : dim);
+      if (value == 2u && pdim != 1) {  // a hex ends the value-2 path
+        lower_ldir(G, tp, 2u);
+        continue;
+      }
+      if (!lower_ldir(G, tp, value)) continue;
+      const int slot = atomicAdd(&s_top, 1);
+      if (slot < kWalkStack) s_stack[slot] = ((int64_t)vi << kVolShift) | tp;
+      else push_item(qout, n_out, cap, err, ((int64_t)vi << kVolShift) | tp);
+    }
+    __syncthreads();
+    if (tid == 0 && s_top > kWalkStack) s_top = kWalkStack;
+    __syncthreads();
   }
 }
 
@@ -877,25 +927,17 @@ cudaError_t launch_ldir_check(int nd, const LdirBatch& B, const uint8_t* rec, in
   return cudaGetLastError();
 }
 
-cudaError_t launch_ldir_walk(int nd, const LdirBatch& B, const int64_t* qin, int n_in, int64_t* qout, int* n_out,
-                             int cap, int* lock, int* err, int num_sms, cudaStream_t stream) {
-  if (n_in <= 0) return cudaSuccess;
-  const int blocks = (n_in + 127) / 128;
-  const int grid = blocks < num_sms * 16 ? blocks : num_sms * 16;
-  if (nd == 3) {
-    ::msc::count_launch();
-    ldir_walk_kernel<3><<<grid, 128, 0, stream>>>(B, qin, n_in, nullptr, qout, n_out, cap, lock, err);
-  } else {
-    ::msc::count_launch();
-    ldir_walk_kernel<2><<<grid, 128, 0, stream>>>(B, qin, n_in, nullptr, qout, n_out, cap, lock, err);
-  }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ldir_walk_dev(const LdirBatch& B, const int64_t* qin, const int* n_in_dev, int64_t* qout, int* n_out,
-                                 int cap, int* lock, int* err, int num_sms, cudaStream_t stream) {
+cudaError_t launch_ldir_walk(int nd, const LdirBatch& B, const int64_t* qin, const int* n_in, int* cursor,
+                             int64_t* qout, int* n_out, int cap, int* lock, int* err, int num_sms,
+                             cudaStream_t stream) {
+  if (cudaError_t e = cudaMemsetAsync(n_out, 0, sizeof(int), stream)) return e;
+  if (cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(int), stream)) return e;
+  uint32_t* cur = reinterpret_cast<uint32_t*>(cursor);
   ::msc::count_launch();
-  ldir_walk_kernel<3><<<num_sms * 16, 128, 0, stream>>>(B, qin, 0, n_in_dev, qout, n_out, cap, lock, err);
+  if (nd == 3)
+    ldir_walk_kernel<3><<<num_sms * 8, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
+  else
+    ldir_walk_kernel<2><<<num_sms * 8, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
   return cudaGetLastError();
 }
 

@@ -178,6 +178,30 @@ int frontier_cap(int64_t ntiles) {
   return cap;
 }
 
+// Walk rounds until the queue is empty: `first` rounds before the counters are read, then
+// groups of four (a round over an empty queue ends at once).  ctr[*cur] is the length of
+// the queue at queues + *cur * cap; *overflow: a queue overflowed, tile passes must finish.
+int walk_rounds(int nd, const msc::LdirBatch& B, int64_t* queues, int* ctr, int cap, int first, int* cur,
+                cudaStream_t stream, int* launches, bool* overflow) {
+  const int sms = num_sms();
+  for (int round = 0, group = first;; group = 4) {
+    for (int q = 0; q < group; q++, round++) {
+      const int in = *cur, out = 1 - *cur;
+      MSC_CUDA(msc::launch_ldir_walk(nd, B, queues + (size_t)in * cap, ctr + in, ctr + 4, queues + (size_t)out * cap,
+                                     ctr + out, cap, ctr + 2, ctr + 3, sms, stream),
+               "ldir walk kernel launch");
+      (*launches)++;
+      *cur = out;
+    }
+    int h[4];
+    MSC_CUDA(cudaMemcpyAsync(h, ctr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream), "read counters");
+    MSC_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+    *overflow = h[3] != 0 || h[0] > cap || h[1] > cap;
+    if (*overflow || h[*cur] == 0) return MSC_OK;
+    if (round > 1 << 20) return fail(MSC_ERR_ITER_LIMIT, "ldir frontier walk did not converge");
+  }
+}
+
 int ldir_batch_impl(int nd, const msc::LdirBatch& B, cudaStream_t stream, Scratch& s, int* passes_out) {
   const int64_t ntiles = B.total_tiles;
   const int64_t box = msc::ldir_halo_bytes(nd);
@@ -185,7 +209,7 @@ int ldir_batch_impl(int nd, const msc::LdirBatch& B, cudaStream_t stream, Scratc
   const int cap = frontier_cap(ntiles);
   uint8_t* saved = nullptr;
   int64_t* queues = nullptr;
-  int* ctr = nullptr;  // [0] queue a [1] queue b [2] lock [3] frontier overflow / CAS limit
+  int* ctr = nullptr;  // [0] queue a [1] queue b [2] lock [3] frontier overflow / CAS limit [4] walk cursor
   MSC_CUDA(msc::scratch_alloc((void**)&saved, (size_t)(ntiles * box), stream), "scratch alloc(halo records)");
   struct FreeAll {
     void* p[3];
@@ -197,36 +221,18 @@ int ldir_batch_impl(int nd, const msc::LdirBatch& B, cudaStream_t stream, Scratc
   } fr{{saved, nullptr, nullptr}, stream};
   MSC_CUDA(msc::scratch_alloc((void**)&queues, (size_t)cap * 2 * sizeof(int64_t), stream), "scratch alloc(queues)");
   fr.p[1] = queues;
-  MSC_CUDA(msc::scratch_alloc((void**)&ctr, 4 * sizeof(int), stream), "scratch alloc(counters)");
+  MSC_CUDA(msc::scratch_alloc((void**)&ctr, 5 * sizeof(int), stream), "scratch alloc(counters)");
   fr.p[2] = ctr;
-  MSC_CUDA(cudaMemsetAsync(ctr, 0, 4 * sizeof(int), stream), "cudaMemsetAsync(counters)");
+  MSC_CUDA(cudaMemsetAsync(ctr, 0, 5 * sizeof(int), stream), "cudaMemsetAsync(counters)");
 
   int launches = 0;
   MSC_CUDA(msc::launch_ldir_tile(nd, B, saved, s.words, sms, stream), "ldir tile kernel launch");
   MSC_CUDA(msc::launch_ldir_check(nd, B, saved, queues, ctr, cap, ctr + 2, ctr + 3, sms, stream),
            "ldir check kernel launch");
   launches += 2;
-  int64_t* qa = queues;
-  int64_t* qb = queues + cap;
   bool overflow = false;
-  for (int round = 0;; round++) {
-    int h[4];
-    MSC_CUDA(cudaMemcpyAsync(h, ctr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream), "read counters");
-    MSC_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    const int n = round % 2 == 0 ? h[0] : h[1];
-    if (h[3] || n > cap) {
-      overflow = true;
-      break;
-    }
-    if (n == 0) break;
-    if (round > 4096) return fail(MSC_ERR_ITER_LIMIT, "ldir frontier walk did not converge");
-    int* n_out = round % 2 == 0 ? ctr + 1 : ctr;
-    MSC_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), stream), "reset queue");
-    MSC_CUDA(msc::launch_ldir_walk(nd, B, qa, n, qb, n_out, cap, ctr + 2, ctr + 3, sms, stream),
-             "ldir walk kernel launch");
-    launches++;
-    std::swap(qa, qb);
-  }
+  int cur = 0;
+  if (int rc = walk_rounds(nd, B, queues, ctr, cap, 1, &cur, stream, &launches, &overflow)) return rc;
   if (overflow) {
     for (int i = 0; i < B.n; i++)
       if (int rc = ldir_passes(nd, B.v[i].g, B.v[i].D, stream, s, &launches)) return rc;
@@ -378,7 +384,7 @@ struct BatchGraph {
   cudaGraphExec_t exec = nullptr;
   uint8_t* saved = nullptr;
   int64_t* queues = nullptr;
-  int* ctr = nullptr;    // [0] [1] queue lengths, [2] lock, [3] overflow / CAS limit
+  int* ctr = nullptr;    // [0] [1] queue lengths, [2] lock, [3] overflow / CAS limit, [4] walk cursor
   int* words = nullptr;  // kernel status words
   int cap = 0;
   void release() {
@@ -409,18 +415,14 @@ int capture_batch_graph(BatchGraph& G, const msc::LstarBatch& LB, const msc::Ldi
   const long long counted = msc::launches_so_far();  // captured launches do not run now
   MSC_CUDA(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   cudaError_t e = cudaMemsetAsync(G.words, 0, 2 * sizeof(int), cs);
-  if (e == cudaSuccess) e = cudaMemsetAsync(G.ctr, 0, 4 * sizeof(int), cs);
+  if (e == cudaSuccess) e = cudaMemsetAsync(G.ctr, 0, 5 * sizeof(int), cs);
   if (e == cudaSuccess) e = msc::launch_lstar_batch(LB, G.words, sms, cs, bps);
   if (e == cudaSuccess) e = msc::launch_ldir_tile(3, B, G.saved, G.words, sms, cs, cps);
   if (e == cudaSuccess) e = msc::launch_ldir_check(3, B, G.saved, G.queues, G.ctr, G.cap, G.ctr + 2, G.ctr + 3, sms, cs);
   for (int r = 0; r < kGraphRounds && e == cudaSuccess; r++) {
-    int* n_in = G.ctr + (r % 2);
-    int* n_out = G.ctr + ((r + 1) % 2);
-    e = cudaMemsetAsync(n_out, 0, sizeof(int), cs);
-    if (e == cudaSuccess)
-      e = msc::launch_ldir_walk_dev(B, G.queues + (size_t)(r % 2) * G.cap, n_in,
-                                    G.queues + (size_t)((r + 1) % 2) * G.cap, n_out, G.cap, G.ctr + 2, G.ctr + 3, sms,
-                                    cs);
+    const int in = r % 2, out = 1 - in;
+    e = msc::launch_ldir_walk(3, B, G.queues + (size_t)in * G.cap, G.ctr + in, G.ctr + 4,
+                              G.queues + (size_t)out * G.cap, G.ctr + out, G.cap, G.ctr + 2, G.ctr + 3, sms, cs);
   }
   cudaGraph_t graph = nullptr;
   const cudaError_t ec = cudaStreamEndCapture(cs, &graph);
@@ -434,27 +436,13 @@ int capture_batch_graph(BatchGraph& G, const msc::LstarBatch& LB, const msc::Ldi
 
 // Finishes what the captured rounds left: more walk rounds, or tile passes on overflow.
 int finish_batch(BatchGraph& G, const msc::LdirBatch& B, cudaStream_t stream, int* launches) {
-  const int sms = num_sms();
   int h[4];
   MSC_CUDA(cudaMemcpyAsync(h, G.ctr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream), "read counters");
   MSC_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
   int cur = kGraphRounds % 2;
-  int n = h[cur];
   bool overflow = h[3] != 0 || h[0] > G.cap || h[1] > G.cap;
-  for (int round = 0; !overflow && n > 0; round++) {
-    if (round > 4096) return fail(MSC_ERR_ITER_LIMIT, "ldir frontier walk did not converge");
-    int* n_out = G.ctr + (1 - cur);
-    MSC_CUDA(cudaMemsetAsync(n_out, 0, sizeof(int), stream), "reset queue");
-    MSC_CUDA(msc::launch_ldir_walk(3, B, G.queues + (size_t)cur * G.cap, n, G.queues + (size_t)(1 - cur) * G.cap, n_out,
-                                   G.cap, G.ctr + 2, G.ctr + 3, sms, stream),
-             "ldir walk kernel launch");
-    (*launches)++;
-    MSC_CUDA(cudaMemcpyAsync(h, G.ctr, 4 * sizeof(int), cudaMemcpyDeviceToHost, stream), "read counters");
-    MSC_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    cur = 1 - cur;
-    n = h[cur];
-    overflow = h[3] != 0 || n > G.cap;
-  }
+  if (!overflow && h[cur] > 0)
+    if (int rc = walk_rounds(3, B, G.queues, G.ctr, G.cap, 4, &cur, stream, launches, &overflow)) return rc;
   if (overflow) {
     Scratch s;
     if (int rc = alloc_scratch(s, stream)) return rc;
@@ -487,7 +475,7 @@ int grad_batch_graph_impl(int n, const float* const* f, const int64_t* dims, uin
     G.cap = cap;
     MSC_CUDA(cudaMalloc((void**)&G.saved, (size_t)B.total_tiles * msc::ldir_halo_bytes(3)), "cudaMalloc(saved halos)");
     MSC_CUDA(cudaMalloc((void**)&G.queues, (size_t)G.cap * 2 * sizeof(int64_t)), "cudaMalloc(queues)");
-    MSC_CUDA(cudaMalloc((void**)&G.ctr, 4 * sizeof(int)), "cudaMalloc(counters)");
+    MSC_CUDA(cudaMalloc((void**)&G.ctr, 5 * sizeof(int)), "cudaMalloc(counters)");
     MSC_CUDA(cudaMalloc((void**)&G.words, 2 * sizeof(int)), "cudaMalloc(status)");
     // launch shapes: tuned once per size class (log2 of the tile count)
     int cls = 0;

@@ -96,13 +96,13 @@ struct LdirBatch {
 cudaError_t make_ldir_batch(int nd, int n, uint8_t* const* g, const GradDims* D, LdirBatch* B);
 cudaError_t launch_ldir_tile(int nd, const LdirBatch& B, uint8_t* saved, int* err, int num_sms, cudaStream_t stream,
                              int ctas_per_sm = 4);
-// one walk round whose input length is read from device memory (for graph capture)
-cudaError_t launch_ldir_walk_dev(const LdirBatch& B, const int64_t* qin, const int* n_in_dev, int64_t* qout, int* n_out,
-                                 int cap, int* lock, int* err, int num_sms, cudaStream_t stream);
 cudaError_t launch_ldir_check(int nd, const LdirBatch& B, const uint8_t* saved, int64_t* queue, int* n_queue, int cap,
                               int* lock, int* err, int num_sms, cudaStream_t stream);
-cudaError_t launch_ldir_walk(int nd, const LdirBatch& B, const int64_t* qin, int n_in, int64_t* qout, int* n_out,
-                             int cap, int* lock, int* err, int num_sms, cudaStream_t stream);
+// one walk round over the queue qin[0, *n_in) (length read on the device); *n_out and
+// *cursor are set to zero first
+cudaError_t launch_ldir_walk(int nd, const LdirBatch& B, const int64_t* qin, const int* n_in, int* cursor,
+                             int64_t* qout, int* n_out, int cap, int* lock, int* err, int num_sms,
+                             cudaStream_t stream);
 cudaError_t launch_ldir_pass(int nd, uint8_t* g, const GradDims& D, const uint8_t* dirty_in, uint8_t* dirty_out,
                              int* changed, int* err, int num_sms, cudaStream_t stream);
 cudaError_t launch_central_diff(int nd, int layout, const float* f, void* out, const GradDims& D, int num_sms,

@@ -387,8 +387,17 @@ __device__ __forceinline__ int batch_volume(const LdirBatch& B, int64_t flat_til
 // walks' items, cofacets and partners never share a dimension, so one frontier and
 // one partner step serve both.  Visiting order does not change a monotone closure, so
 // the marks equal those of the item-by-item walk.  The closures of rough fields are
-// shallow (14 levels for value 2, 12 for value 1 over a whole 128^3 k^-3 volume), so
-// a tile costs a few dozen passes over its rows.
+// shallow (14 levels for value 2, 12 for value 1 over a whole 128^3 k^-3 volume).
+//
+// A lane holds the row at its own y, a register a word of it, so that a warp's
+// registers hold a slab of 32 x 32 cells and a row's y neighbours are one shuffle away.
+// 3D: a box of 32 x 32 x 32, eight warps of four slabs each, one above the other: only
+// the words that cross from warp to warp go through shared memory.  2D: a warp works on
+// a box of 32 x 128 alone.
+// A lane reads its row with three 16-byte loads and turns the 32 bytes into bit planes by
+// 8 x 8 bit transposes (~130 operations a row).  A warp per row with a ballot per
+// property and the word planes in shared memory took 371 K warp instructions a tile, most
+// of them staging: 15.4 ms at 512^3 (ALU pipe 75%).
 constexpr int kBitLX = 32;
 template <int ND, int LY, int LZ>
 struct BitTile {
@@ -400,8 +409,6 @@ struct BitTile {
   // a tile's record: the {value 2, value 1} masks of each halo row's lowered cells,
   // then one byte per inner row (bits 0-3: value 2 at x = 0, 1, 30, 31; 4-7: value 1)
   static constexpr int64_t REC = ((int64_t)NHR * 8 + NIR + 15) / 16 * 16;
-  // shared memory word planes: NC, PC[6] (partner at +x, -x, +y, -y, +z, -z), F, T, M2, M1
-  static constexpr size_t smem_bytes() { return (size_t)11 * R * 4; }
   static_assert(ND == 3 || LZ == 1, "2D boxes have one z row");
   static_assert(LY % 2 == 0 && LZ % 2 == (ND == 3 ? 0 : 1), "tile origins must be even");
 };
@@ -433,23 +440,167 @@ __device__ __forceinline__ void halo_row_of(int h, int& ly, int& lz) {
   ly = q < 2 ? q : LY - 4 + q;
 }
 
-template <int ND, int LY, int LZ, int BS, int MINB>
-__global__ void __launch_bounds__(BS, MINB) ldir_tile_kernel(const LdirBatch B, uint8_t* __restrict__ rec,
-                                                       int* __restrict__ err) {
-  using T = BitTile<ND, LY, LZ>;
-  constexpr int R = T::R;
-  constexpr int NWARP = BS / 32;
-  constexpr int RPT = (R + BS - 1) / BS;  // rows per thread in a level
-  constexpr int KR = 4;                   // rows per warp with loads in flight
-  constexpr uint32_t EVENX = 0x55555555u, ODDX = 0xAAAAAAAAu;
-  extern __shared__ __align__(16) uint32_t s_plane[];
-  uint32_t* sNC = s_plane;
-  uint32_t* sPC = s_plane + R;
-  uint32_t* sF = s_plane + 7 * R;
-  uint32_t* sT = s_plane + 8 * R;
-  uint32_t* sM2 = s_plane + 9 * R;
-  uint32_t* sM1 = s_plane + 10 * R;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+constexpr int kSlabs = 4;        // slabs of 32 x 32 cells per warp
+constexpr int kTileWarps = 8;    // 3D: warps per tile
+constexpr uint32_t kEvenX = 0x55555555u, kOddX = 0xAAAAAAAAu;
+
+// 16 bytes at p (16-byte aligned); bytes outside [lo, hi) read as 0
+__device__ __forceinline__ uint4 load_granule(const uint8_t* p, const uint8_t* lo, const uint8_t* hi) {
+  if (p >= lo && p + 16 <= hi) return *reinterpret_cast<const uint4*>(p);
+  uint32_t w[4] = {0u, 0u, 0u, 0u};
+  for (int k = 0; k < 16; k++)  // the array's first and last bytes
+    if (p + k >= lo && p + k < hi) w[k >> 2] |= (uint32_t)p[k] << (8 * (k & 3));
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// 8 x 8 bit transpose of eight bytes (lo: bytes 0-3): byte b of the result holds bit b of
+// every byte
+__device__ __forceinline__ void transpose8(uint32_t& lo, uint32_t& hi) {
+  uint32_t t = (lo ^ (lo >> 7)) & 0x00AA00AAu;
+  lo ^= t ^ (t << 7);
+  t = (hi ^ (hi >> 7)) & 0x00AA00AAu;
+  hi ^= t ^ (t << 7);
+  t = (lo ^ (lo >> 14)) & 0x0000CCCCu;
+  lo ^= t ^ (t << 14);
+  t = (hi ^ (hi >> 14)) & 0x0000CCCCu;
+  hi ^= t ^ (t << 14);
+  t = (lo & 0x0F0F0F0Fu) | ((hi << 4) & 0xF0F0F0F0u);
+  hi = (hi & 0xF0F0F0F0u) | ((lo >> 4) & 0x0F0F0F0Fu);
+  lo = t;
+}
+// byte k of w[0..3] gathered into p[k]
+__device__ __forceinline__ void gather_bytes(const uint32_t w[4], uint32_t p[4]) {
+  const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+  const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+  p[0] = __byte_perm(a, b, 0x5410);
+  p[1] = __byte_perm(a, b, 0x7632);
+  p[2] = __byte_perm(c, d, 0x5410);
+  p[3] = __byte_perm(c, d, 0x7632);
+}
+
+// The bit planes of the 32 cells at p (which may reach past both ends of the array)
+__device__ __forceinline__ void load_planes(const uint8_t* p, const uint8_t* lo, const uint8_t* hi, uint32_t pl[8]) {
+  const int s = (int)(reinterpret_cast<uintptr_t>(p) & 15u);
+  const uint8_t* q = p - s;
+  const uint4 a = load_granule(q, lo, hi), b = load_granule(q + 16, lo, hi);
+  uint4 c = make_uint4(0u, 0u, 0u, 0u);
+  if (s > 0) c = load_granule(q + 32, lo, hi);
+  uint32_t w[12] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w};
+#pragma unroll
+  for (int i = 0; i < 10; i++) w[i] = (s & 8) ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 9; i++) w[i] = (s & 4) ? w[i + 1] : w[i];
+  const int sh = 8 * (s & 3);
+  uint32_t l[4], h[4];
+#pragma unroll
+  for (int g = 0; g < 4; g++) {
+    l[g] = __funnelshift_r(w[2 * g], w[2 * g + 1], sh);
+    h[g] = __funnelshift_r(w[2 * g + 1], w[2 * g + 2], sh);
+    transpose8(l[g], h[g]);
+  }
+  gather_bytes(l, pl);
+  gather_bytes(h, pl + 4);
+}
+
+// A row's words.
+struct LdirRow {
+  uint32_t nc;        // assigned, not critical
+  uint32_t pc[6];     // paired to +x, -x, +y, -y, +z, -z
+  uint32_t m2, m1;    // marked by the value-2 / value-1 walk
+  uint32_t f;         // frontier
+  uint32_t gt2, gt1;  // assigned, and ldir above 2 / above 1 in the .grad
+};
+// edges, quads, hexes: the row's cells of that dimension
+__device__ __forceinline__ void load_row(LdirRow& R, const uint8_t* p, const uint8_t* lo, const uint8_t* hi,
+                                         uint32_t valid, uint32_t dec_map, uint32_t edges, uint32_t quads) {
+  uint32_t b[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  if (valid) load_planes(p, lo, hi, b);
+  const uint32_t asg = b[0] & valid;
+  const uint32_t c0 = b[2], c1 = b[3], c2 = b[4];
+  R.nc = asg & ~(c0 & c1 & c2);
+  const uint32_t e0 = R.nc & ~c0, e1 = R.nc & c0;
+  R.pc[0] = e0 & ~c1 & ~c2;
+  R.pc[1] = e1 & ~c1 & ~c2;
+  R.pc[2] = e0 & c1 & ~c2;
+  R.pc[3] = e1 & c1 & ~c2;
+  R.pc[4] = e0 & ~c1 & c2;
+  R.pc[5] = e1 & ~c1 & c2;
+  if (dec_map != 0x2C688u) {  // a single-vertex axis: the stored code names another axis
+    uint32_t t[6];
+#pragma unroll
+    for (int c = 0; c < 6; c++) t[c] = R.pc[c];
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+      R.pc[c] = 0;
+#pragma unroll
+      for (int k = 0; k < 6; k++)
+        if (map3(dec_map, k) == c) R.pc[c] |= t[k];
+    }
+  }
+  R.gt2 = asg & (b[7] | (b[6] & b[5]));
+  R.gt1 = asg & (b[7] | b[6]);
+  R.m2 = asg & edges & b[6] & ~b[5] & ~b[7];
+  R.m1 = asg & quads & b[5] & ~b[6] & ~b[7];
+  R.f = R.m2 | R.m1;
+}
+// one level's marks of a row: t the cofacets, p the partners
+__device__ __forceinline__ void mark_row(LdirRow& R, uint32_t t, uint32_t p, uint32_t edges, uint32_t quads,
+                                         uint32_t hexes) {
+  const uint32_t e2 = p & edges & ~R.m2, e1 = p & quads & ~R.m1;
+  R.m2 |= (t & quads) | (p & hexes) | e2;
+  R.m1 |= (t & hexes) | e1;
+  R.f = e2 | e1;
+}
+// The owned cells of 28 rows (lanes 2-29 hold them) that the walks lowered: a lane per
+// cell, four rows in flight.  gp: the slab's first cell of lane 0's row; rows cs1 apart.
+__device__ __forceinline__ void write_rows(uint8_t* gp, int64_t cs1, int lane, uint32_t chg, uint32_t low1, int first,
+                                           int last) {
+#pragma unroll 1
+  for (int r0 = first; r0 < last; r0 += 4) {
+    uint8_t old[4];
+    bool want[4];
+    uint32_t one[4];
+    uint8_t* q = gp + (int64_t)r0 * cs1 + lane;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t c = __shfl_sync(~0u, chg, r0 + k);
+      one[k] = __shfl_sync(~0u, low1, r0 + k);
+      want[k] = (c >> lane) & 1u;
+      old[k] = 0;
+      if (want[k]) old[k] = q[k * cs1];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (want[k]) q[k * cs1] = (uint8_t)((old[k] & 0x1Fu) | (((one[k] >> lane) & 1u) ? 0x20u : 0x40u));
+  }
+}
+// the four halo cells of an inner row, as the record keeps them
+__device__ __forceinline__ uint8_t inner_record(uint32_t low2, uint32_t low1) {
+  const uint32_t q2 = (low2 & 3u) | ((low2 >> 28) & 0xCu), q1 = (low1 & 3u) | ((low1 >> 28) & 0xCu);
+  return (uint8_t)(q2 | (q1 << 4));
+}
+// the cells of a row of 32 from x0 that lie inside the complex
+__device__ __forceinline__ uint32_t valid_cells(int64_t x0, int64_t dX) {
+  const uint32_t below = x0 < 0 ? ~0u << (int)(-x0) : ~0u;
+  const int64_t n = dX - x0;
+  return below & (n >= 32 ? ~0u : (n <= 0 ? 0u : (1u << (int)n) - 1u));
+}
+
+// 3D: a block of eight warps per tile.
+__global__ void __launch_bounds__(32 * kTileWarps, 3) ldir_tile3_kernel(const LdirBatch B, uint8_t* __restrict__ rec,
+                                                                        int* __restrict__ err) {
+  using T = BitTile<3, 32, 32>;
+  __shared__ uint32_t s_f[kTileWarps + 1][32];   // the frontier of each warp's first slab
+  __shared__ uint32_t s_up[kTileWarps + 1][32];  // partners above a warp's last slab (of warp w at w + 1)
+  __shared__ uint32_t s_dn[kTileWarps + 1][32];  // partners below a warp's first slab
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w == 0) {  // beyond the box: nothing
+    s_f[kTileWarps][lane] = 0;
+    s_up[0][lane] = 0;
+    s_dn[kTileWarps][lane] = 0;
+  }
+  const uint32_t yo = (lane & 1) ? ~0u : 0u, n0 = lane > 0 ? ~0u : 0u, n31 = lane < 31 ? ~0u : 0u;
+  const bool yhalo = lane < 2 || lane >= 30;
 
   for (int64_t flat = blockIdx.x; flat < B.total_tiles; flat += gridDim.x) {
     const LdirVol& vol = B.v[batch_volume(B, flat)];
@@ -458,147 +609,159 @@ __global__ void __launch_bounds__(BS, MINB) ldir_tile_kernel(const LdirBatch B, 
     const int64_t dX = D.d[0], dY = D.d[1], dZ = D.d[2];
     const int64_t ntx = (dX + T::TX - 1) / T::TX, nty = (dY + T::TY - 1) / T::TY;
     const int64_t tile = flat - vol.tile0;
-    const int64_t tx = tile % ntx, ty = (tile / ntx) % nty, tz = ND == 3 ? tile / (ntx * nty) : 0;
-    const int64_t o1 = ty * T::TY - 2, o2 = ND == 3 ? tz * T::TZ - 2 : 0;
-    const int64_t gx = tx * T::TX - 2 + lane;
-    const bool xin = gx >= 0 && gx < dX;
+    const int64_t tx = tile % ntx, ty = (tile / ntx) % nty, tz = tile / (ntx * nty);
+    const int64_t x0 = tx * T::TX - 2, y0 = ty * T::TY - 2, z0 = tz * T::TZ - 2 + kSlabs * w;
+    const bool yin = y0 + lane >= 0 && y0 + lane < dY;
+    const uint32_t vx = valid_cells(x0, dX);
+    const int64_t row0 = x0 + (y0 + lane) * D.cs[1] + z0 * D.cs[2];
 
-    // stage: a warp per row, a lane per cell; each property becomes a bit row.  Cells
-    // outside the complex read as 0 (unassigned).  Marked items seed the frontier.  A
-    // warp keeps KR rows' loads in flight before it folds them.
-    for (int r0 = warp; r0 < R; r0 += NWARP * KR) {
-      uint8_t bk[KR];
+    LdirRow R[kSlabs];
 #pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = r0 + k * NWARP;
-        const int ly = r % LY, lz = r / LY;
-        const int64_t gy = o1 + ly, gz = o2 + lz;
-        bk[k] = 0;
-        if (r < R && xin && gy >= 0 && gy < dY && gz >= 0 && gz < dZ) bk[k] = g[gx + gy * D.cs[1] + gz * D.cs[2]];
-      }
-#pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = r0 + k * NWARP;
-        if (r >= R) break;
-        const int ly = r % LY, lz = r / LY;
-        const uint8_t b = bk[k];
-        const unsigned code = (b >> 2) & 7u, ld = b >> 5;
-        const bool asg = b & 1u;
-        const bool nc = asg && code != 7u;
-        const int pc = nc ? map3(D.dec_map, (int)code) : 7;
-        const int dim = (lane & 1) + (ly & 1) + (lz & 1);
-        const uint32_t mnc = __ballot_sync(~0u, nc);
-        const uint32_t m2 = __ballot_sync(~0u, asg && dim == 1 && ld == 2u);
-        const uint32_t m1 = __ballot_sync(~0u, asg && dim == 2 && ld == 1u);
-        uint32_t pcm[6];
-#pragma unroll
-        for (int c = 0; c < 6; c++) pcm[c] = __ballot_sync(~0u, pc == c);
-        if (lane == 0) {
-          sNC[r] = mnc;
-#pragma unroll
-          for (int c = 0; c < 6; c++) sPC[c * R + r] = pcm[c];
-          sF[r] = m2 | m1;
-          sM2[r] = m2;
-          sM1[r] = m1;
-        }
-      }
+    for (int j = 0; j < kSlabs; j++) {
+      const bool in = yin && z0 + j >= 0 && z0 + j < dZ;
+      const uint32_t edges = (j & 1) ? kEvenX & ~yo : kOddX ^ yo, quads = (j & 1) ? kOddX ^ yo : kOddX & yo;
+      load_row(R[j], g + (row0 + j * D.cs[2]), g, g + D.ncells, in ? vx : 0u, D.dec_map, edges, quads);
     }
+    s_f[w][lane] = R[0].f;
     __syncthreads();
 
     // BFS levels until no row gains an item; every level adds an item, so the bound
     // is never reached by a valid gradient
     for (int level = 0;; level++) {
-#pragma unroll 1
-      for (int k = 0; k < RPT; k++) {
-        const int r = tid + k * BS;
-        if (r < R) {
-          const int ly = r % LY, lz = r / LY;
-          const uint32_t f = sF[r] & EVENX;
-          uint32_t c = (f << 1) | (f >> 1);
-          if (ly & 1) c |= sF[r - 1] | (ly + 1 < LY ? sF[r + 1] : 0u);
-          if (ND == 3 && (lz & 1)) c |= sF[r - LY] | (lz + 1 < LZ ? sF[r + LY] : 0u);
-          sT[r] = c & sNC[r];
+      uint32_t t[kSlabs] = {0u, 0u, 0u, 0u};
+      const uint32_t above = s_f[w + 1][lane];
+      const bool act = __any_sync(~0u, (R[0].f | R[1].f | R[2].f | R[3].f | above) != 0u);
+      if (act) {
+#pragma unroll
+        for (int j = 0; j < kSlabs; j++) {
+          const uint32_t f = R[j].f, fe = f & kEvenX;
+          const uint32_t fu = __shfl_up_sync(~0u, f, 1), fd = __shfl_down_sync(~0u, f, 1) & n31;
+          uint32_t c = (fe << 1) | (fe >> 1) | ((fu | fd) & yo);
+          if (j & 1) c |= R[j - 1].f | (j + 1 < kSlabs ? R[j + 1 < kSlabs ? j + 1 : j].f : above);
+          t[j] = c & R[j].nc;
         }
       }
+      s_up[w + 1][lane] = t[kSlabs - 1] & R[kSlabs - 1].pc[4];
+      s_dn[w][lane] = t[0] & R[0].pc[5];
       __syncthreads();
-      int grew = 0;
-#pragma unroll 1
-      for (int k = 0; k < RPT; k++) {
-        const int r = tid + k * BS;
-        if (r < R) {
-          const int ly = r % LY, lz = r / LY;
-          const uint32_t t = sT[r];
-          uint32_t p = ((t & sPC[r]) << 1) | ((t & sPC[R + r]) >> 1);
-          if (ly > 0) p |= sT[r - 1] & sPC[2 * R + r - 1];
-          if (ly + 1 < LY) p |= sT[r + 1] & sPC[3 * R + r + 1];
-          if (ND == 3) {
-            if (lz > 0) p |= sT[r - LY] & sPC[4 * R + r - LY];
-            if (lz + 1 < LZ) p |= sT[r + LY] & sPC[5 * R + r + LY];
-          }
-          const int odd = (ly & 1) + (lz & 1);
-          const uint32_t edges = odd == 0 ? ODDX : (odd == 1 ? EVENX : 0u);
-          const uint32_t quads = odd == 0 ? 0u : (odd == 1 ? ODDX : EVENX);
-          const uint32_t hexes = odd == 2 ? ODDX : 0u;
-          const uint32_t m2 = sM2[r], m1 = sM1[r];
-          const uint32_t e2 = p & edges & ~m2, e1 = p & quads & ~m1;
-          sM2[r] = m2 | (t & quads) | (p & hexes) | e2;
-          sM1[r] = m1 | (t & hexes) | e1;
-          sF[r] = e2 | e1;
-          grew |= (e2 | e1) != 0u;
+      const uint32_t from_up = s_dn[w + 1][lane], from_dn = s_up[w][lane];
+      uint32_t grew = 0;
+      if (act || __any_sync(~0u, (from_up | from_dn) != 0u)) {
+#pragma unroll
+        for (int j = 0; j < kSlabs; j++) {
+          const uint32_t tj = t[j];
+          uint32_t p = ((tj & R[j].pc[0]) << 1) | ((tj & R[j].pc[1]) >> 1);
+          p |= __shfl_up_sync(~0u, tj & R[j].pc[2], 1) & n0;
+          p |= __shfl_down_sync(~0u, tj & R[j].pc[3], 1) & n31;
+          p |= j > 0 ? t[j > 0 ? j - 1 : 0] & R[j > 0 ? j - 1 : 0].pc[4] : from_dn;
+          p |= j + 1 < kSlabs ? t[j + 1 < kSlabs ? j + 1 : j] & R[j + 1 < kSlabs ? j + 1 : j].pc[5] : from_up;
+          const uint32_t edges = (j & 1) ? kEvenX & ~yo : kOddX ^ yo, quads = (j & 1) ? kOddX ^ yo : kOddX & yo;
+          mark_row(R[j], tj, p, edges, quads, (j & 1) ? kOddX & yo : 0u);
+          grew |= R[j].f;
         }
       }
-      if (!__syncthreads_or(grew)) break;
-      if (level > 64 * R) {
-        if (tid == 0) atomicOr(err, kErrPassLimit);
+      s_f[w][lane] = R[0].f;
+      if (!__syncthreads_or(grew != 0u)) break;
+      if (level > 64 * T::R) {
+        if (threadIdx.x == 0) atomicOr(err, kErrPassLimit);
         break;
       }
     }
 
     // write back the owned cells this tile lowered and record the halo cells it holds
-    // lower than the .grad does (their owners may hold them lower by now: the check
-    // compares again)
+    // lower than the .grad did when it was staged (their owners may hold them lower by
+    // now: the check compares again)
     uint8_t* trec = rec + flat * T::REC;
-    for (int r0 = warp; r0 < R; r0 += NWARP * KR) {
-      uint8_t bk[KR];
-      bool m2k[KR], m1k[KR];
 #pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = r0 + k * NWARP;
-        const int ly = r % LY, lz = r / LY;
-        const int64_t gy = o1 + ly, gz = o2 + lz;
-        m2k[k] = r < R && ((sM2[r] >> lane) & 1u);
-        m1k[k] = r < R && ((sM1[r] >> lane) & 1u);
-        bk[k] = 0;
-        if ((m2k[k] || m1k[k]) && xin && gy >= 0 && gy < dY && gz >= 0 && gz < dZ)
-          bk[k] = g[gx + gy * D.cs[1] + gz * D.cs[2]];
-      }
-#pragma unroll
-      for (int k = 0; k < KR; k++) {
-        const int r = r0 + k * NWARP;
-        if (r >= R) break;
-        const int ly = r % LY, lz = r / LY;
-        const int64_t gy = o1 + ly, gz = o2 + lz;
-        const uint8_t b = bk[k];  // 0 (unassigned) outside the complex
-        const bool low2 = m2k[k] && (b & 1u) && (b >> 5) > 2u;
-        const bool low1 = m1k[k] && (b & 1u) && (b >> 5) > 1u;
-        const int slot = halo_row_slot<ND, LY, LZ>(ly, lz);
-        if (slot >= 0) {
-          const uint32_t w2 = __ballot_sync(~0u, low2), w1 = __ballot_sync(~0u, low1);
-          if (lane < 2) reinterpret_cast<uint32_t*>(trec)[2 * slot + lane] = lane == 0 ? w2 : w1;
-        } else {
-          const bool own = lane >= 2 && lane < kBitLX - 2;
-          if (own && (low2 || low1))
-            g[gx + gy * D.cs[1] + gz * D.cs[2]] = (uint8_t)((b & 0x1Fu) | ((low1 ? 1u : 2u) << 5));
-          const uint32_t w2 = __ballot_sync(~0u, low2 && !own), w1 = __ballot_sync(~0u, low1 && !own);
-          if (lane == 0) {
-            const int i = ND == 3 ? (lz - 2) * (LY - 4) + (ly - 2) : ly - 2;
-            const uint32_t q2 = (w2 & 3u) | ((w2 >> 28) & 0xCu), q1 = (w1 & 3u) | ((w1 >> 28) & 0xCu);
-            trec[T::NHR * 8 + i] = (uint8_t)(q2 | (q1 << 4));
-          }
-        }
-      }
+    for (int j = 0; j < kSlabs; j++) {
+      const int lz = kSlabs * w + j;
+      const uint32_t low2 = R[j].m2 & R[j].gt2, low1 = R[j].m1 & R[j].gt1;
+      const bool zhalo = lz < 2 || lz >= 30;
+      if (zhalo || yhalo)
+        reinterpret_cast<uint2*>(trec)[halo_row_slot<3, 32, 32>(lane, lz)] = make_uint2(low2, low1);
+      else
+        trec[T::NHR * 8 + (lz - 2) * T::TY + (lane - 2)] = inner_record(low2, low1);
+      if (!zhalo)
+        write_rows(g + (x0 + y0 * D.cs[1] + (z0 + j) * D.cs[2]), D.cs[1], lane, (low2 | low1) & 0x3FFFFFFCu, low1, 2,
+                   30);
     }
     __syncthreads();
+  }
+}
+
+// 2D: a warp per tile of 32 x 128 cells, its slabs one below the other along y.
+__global__ void __launch_bounds__(256) ldir_tile2_kernel(const LdirBatch B, uint8_t* __restrict__ rec,
+                                                         int* __restrict__ err) {
+  using T = BitTile<2, 32 * kSlabs, 1>;
+  const int lane = threadIdx.x & 31;
+  const uint32_t yo = (lane & 1) ? ~0u : 0u;
+  const uint32_t edges = kOddX ^ yo, quads = kOddX & yo;
+  const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t flat = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); flat < B.total_tiles;
+       flat += nwarp) {
+    const LdirVol& vol = B.v[batch_volume(B, flat)];
+    uint8_t* __restrict__ g = vol.g;
+    const GradDims& D = vol.D;
+    const int64_t dX = D.d[0], dY = D.d[1];
+    const int64_t ntx = (dX + T::TX - 1) / T::TX;
+    const int64_t tile = flat - vol.tile0;
+    const int64_t tx = tile % ntx, ty = tile / ntx;
+    const int64_t x0 = tx * T::TX - 2, y0 = ty * T::TY - 2;
+    const uint32_t vx = valid_cells(x0, dX);
+    LdirRow R[kSlabs];
+#pragma unroll
+    for (int j = 0; j < kSlabs; j++) {
+      const int64_t y = y0 + 32 * j + lane;
+      load_row(R[j], g + (x0 + y * D.cs[1]), g, g + D.ncells, (y >= 0 && y < dY) ? vx : 0u, D.dec_map, edges, quads);
+    }
+    for (int level = 0;; level++) {
+      uint32_t t[kSlabs], up[kSlabs], dn[kSlabs];
+      // the rows above and below: a rotation within the slab, the ends from its neighbours
+#pragma unroll
+      for (int j = 0; j < kSlabs; j++) {
+        up[j] = __shfl_sync(~0u, R[j].f, (lane + 31) & 31);
+        dn[j] = __shfl_sync(~0u, R[j].f, (lane + 1) & 31);
+      }
+#pragma unroll
+      for (int j = 0; j < kSlabs; j++) {
+        const uint32_t fe = R[j].f & kEvenX;
+        const uint32_t fu = lane > 0 ? up[j] : (j > 0 ? up[j > 0 ? j - 1 : 0] : 0u);
+        const uint32_t fd = lane < 31 ? dn[j] : (j + 1 < kSlabs ? dn[j + 1 < kSlabs ? j + 1 : j] : 0u);
+        t[j] = ((fe << 1) | (fe >> 1) | ((fu | fd) & yo)) & R[j].nc;
+      }
+#pragma unroll
+      for (int j = 0; j < kSlabs; j++) {
+        up[j] = __shfl_sync(~0u, t[j] & R[j].pc[2], (lane + 31) & 31);
+        dn[j] = __shfl_sync(~0u, t[j] & R[j].pc[3], (lane + 1) & 31);
+      }
+      uint32_t grew = 0;
+#pragma unroll
+      for (int j = 0; j < kSlabs; j++) {
+        uint32_t p = ((t[j] & R[j].pc[0]) << 1) | ((t[j] & R[j].pc[1]) >> 1);
+        p |= lane > 0 ? up[j] : (j > 0 ? up[j > 0 ? j - 1 : 0] : 0u);
+        p |= lane < 31 ? dn[j] : (j + 1 < kSlabs ? dn[j + 1 < kSlabs ? j + 1 : j] : 0u);
+        mark_row(R[j], t[j], p, edges, quads, 0u);
+        grew |= R[j].f;
+      }
+      if (!__any_sync(~0u, grew != 0u)) break;
+      if (level > 64 * T::R) {
+        if (lane == 0) atomicOr(err, kErrPassLimit);
+        break;
+      }
+    }
+    uint8_t* trec = rec + flat * T::REC;
+#pragma unroll
+    for (int j = 0; j < kSlabs; j++) {
+      const int ly = 32 * j + lane;
+      const uint32_t low2 = R[j].m2 & R[j].gt2, low1 = R[j].m1 & R[j].gt1;
+      const bool halo = ly < 2 || ly >= T::TY + 2;
+      if (halo)
+        reinterpret_cast<uint2*>(trec)[halo_row_slot<2, 32 * kSlabs, 1>(ly, 0)] = make_uint2(low2, low1);
+      else
+        trec[T::NHR * 8 + ly - 2] = inner_record(low2, low1);
+      write_rows(g + (x0 + (y0 + 32 * j) * D.cs[1]), D.cs[1], lane, halo ? 0u : (low2 | low1) & 0x3FFFFFFCu, low1, 0,
+                 32);
+    }
   }
 }
 
@@ -849,11 +1012,12 @@ constexpr int kTX3 = 32, kTY3 = 32, kTZ3 = 16, kBS3 = 512;
 constexpr int kTX2 = 128, kTY2 = 64, kBS2 = 256;
 using Tile3 = LdirTile<3, kTX3, kTY3, kTZ3>;
 using Tile2 = LdirTile<2, kTX2, kTY2, 1>;
-// single-pass bit-row tiles: 28 x 32 x 32 owned cells in 3D, 28 x 252 in 2D
-constexpr int kBitLY3 = 36, kBitLZ3 = 36, kBitBS3 = 512;
-constexpr int kBitLY2 = 256, kBitBS2 = 256;
+// single-pass bit-row tiles: 28 x 28 x 28 owned cells in 3D, 28 x 124 in 2D
+constexpr int kBitLY3 = 32, kBitLZ3 = 32;
+constexpr int kBitLY2 = 32 * kSlabs;
 using Bit3 = BitTile<3, kBitLY3, kBitLZ3>;
 using Bit2 = BitTile<2, kBitLY2, 1>;
+static_assert(kBitLZ3 == kSlabs * kTileWarps, "the block's slabs make the box");
 }  // namespace
 
 int64_t ldir_num_tiles(int nd, const GradDims& D) {
@@ -884,30 +1048,18 @@ cudaError_t make_ldir_batch(int nd, int n, uint8_t* const* g, const GradDims* D,
   return cudaSuccess;
 }
 
-template <class K>
-static cudaError_t launch_bit_tiles(K k, int bs, size_t sm, const LdirBatch& B, uint8_t* rec, int* err, int num_sms,
-                                    cudaStream_t stream, int ctas_per_sm) {
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
-  int fit = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, bs, sm);
-  if (e != cudaSuccess) return e;
-  const int per_sm = ctas_per_sm < fit ? ctas_per_sm : (fit > 0 ? fit : 1);
-  const int64_t cap = (int64_t)num_sms * per_sm;
-  const int grid = (int)(B.total_tiles < cap ? B.total_tiles : cap);
-  if (grid <= 0) return cudaSuccess;
-  ::msc::count_launch();
-  k<<<grid, bs, sm, stream>>>(B, rec, err);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_ldir_tile(int nd, const LdirBatch& B, uint8_t* rec, int* err, int num_sms, cudaStream_t stream,
                              int ctas_per_sm) {
+  const int64_t blocks = nd == 3 ? B.total_tiles : (B.total_tiles + 7) / 8;  // 2D: a warp per tile
+  const int64_t cap = ctas_per_sm > 0 ? (int64_t)num_sms * ctas_per_sm : 0x7FFFFFFF;  // 0: a block per tile
+  const int grid = (int)(blocks < cap ? blocks : cap);
+  if (grid <= 0) return cudaSuccess;
+  ::msc::count_launch();
   if (nd == 3)
-    return launch_bit_tiles(ldir_tile_kernel<3, kBitLY3, kBitLZ3, kBitBS3, 3>, kBitBS3, Bit3::smem_bytes(), B, rec, err,
-                            num_sms, stream, ctas_per_sm);
-  return launch_bit_tiles(ldir_tile_kernel<2, kBitLY2, 1, kBitBS2, 4>, kBitBS2, Bit2::smem_bytes(), B, rec, err, num_sms,
-                          stream, ctas_per_sm);
+    ldir_tile3_kernel<<<grid, 32 * kTileWarps, 0, stream>>>(B, rec, err);
+  else
+    ldir_tile2_kernel<<<grid, 256, 0, stream>>>(B, rec, err);
+  return cudaGetLastError();
 }
 
 static int check_grid(const LdirBatch& B, int num_sms) {

@@ -368,7 +368,7 @@ int host_impl(int nd, const float* fh, const int64_t* dims, uint8_t* gh) {
 // check and kGraphRounds frontier-walk rounds whose queue lengths stay on the device.
 // After a replay the host reads the counters once; a frontier left over after the
 // captured rounds is walked on, an overflow falls back to tile passes.  The launch
-// shapes (K1 blocks per SM, ldir tiles per SM) are picked by timing the candidates on
+// shapes (K1 blocks per SM, ldir tile blocks per SM, 0: one per tile) are picked by timing the candidates on
 // the first batch of a size class; the instantiated graph is kept and replayed while
 // the same buffers come back.
 
@@ -380,7 +380,7 @@ struct BatchGraph {
   std::vector<const float*> f;
   std::vector<uint8_t*> g;
   std::vector<int64_t> dims;
-  int bps = 64, cps = 4;
+  int bps = 64, cps = 0;
   cudaGraphExec_t exec = nullptr;
   uint8_t* saved = nullptr;
   int64_t* queues = nullptr;
@@ -401,7 +401,7 @@ struct BatchGraph {
 };
 thread_local BatchGraph t_bgraph;
 std::mutex g_tune_mu;
-std::map<int, std::pair<int, int>> g_tuned;  // size class -> (K1 blocks per SM, ldir tiles per SM)
+std::map<int, std::pair<int, int>> g_tuned;  // size class -> (K1 blocks per SM, ldir tile blocks per SM, 0: one per tile)
 
 int capture_batch_graph(BatchGraph& G, const msc::LstarBatch& LB, const msc::LdirBatch& B, int bps, int cps,
                         cudaGraphExec_t* out) {
@@ -480,7 +480,7 @@ int grad_batch_graph_impl(int n, const float* const* f, const int64_t* dims, uin
     // launch shapes: tuned once per size class (log2 of the tile count)
     int cls = 0;
     for (int64_t t = B.total_tiles; t > 1; t >>= 1) cls++;
-    std::pair<int, int> best{64, 4};
+    std::pair<int, int> best{64, 0};
     bool tuned = false;
     {
       std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -496,7 +496,7 @@ int grad_batch_graph_impl(int n, const float* const* f, const int64_t* dims, uin
       MSC_CUDA(cudaEventCreate(&e0), "cudaEventCreate");
       MSC_CUDA(cudaEventCreate(&e1), "cudaEventCreate");
       for (int bps : {32, 64, 128})
-        for (int cps : {2, 4}) {
+        for (int cps : {0, 3}) {
           cudaGraphExec_t ex = nullptr;
           if (int rc = capture_batch_graph(G, LB, B, bps, cps, &ex)) return rc;
           cudaGraphLaunch(ex, stream);

@@ -94,8 +94,9 @@ struct LdirBatch {
   LdirVol v[kMaxBatch];
 };
 cudaError_t make_ldir_batch(int nd, int n, uint8_t* const* g, const GradDims* D, LdirBatch* B);
+// ctas_per_sm 0: a block per tile (2D: per eight tiles); above: that many persistent blocks per SM
 cudaError_t launch_ldir_tile(int nd, const LdirBatch& B, uint8_t* saved, int* err, int num_sms, cudaStream_t stream,
-                             int ctas_per_sm = 4);
+                             int ctas_per_sm = 0);
 cudaError_t launch_ldir_check(int nd, const LdirBatch& B, const uint8_t* saved, int64_t* queue, int* n_queue, int cap,
                               int* lock, int* err, int num_sms, cudaStream_t stream);
 // one walk round over the queue qin[0, *n_in) (length read on the device); *n_out and

@@ -58,3 +58,22 @@ def test_terminal_walk_equals_oracle(gpu, oracle, name, shape):
     want = oracle.labels(f, g, 1e-4, 1e-6, 20, 0.25, 0.0)
     for k in ("asc_terminal", "dsc_terminal"):
         assert np.array_equal(got[k].cpu().numpy(), want[k].reshape(-1)), k
+
+
+# cells per axis 2n - 1 around multiples of the tiles' 28 owned cells (3D, and 2D along x)
+# and 124 (2D along y); X = 1 gives the remapped pair codes
+@pytest.mark.parametrize("shape", [(14, 15, 16), (15, 29, 14), (43, 14, 30), (1, 31, 29), (28, 62), (15, 63), (30, 125)],
+                         ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("offset", [0, 1, 7, 14])
+def test_tile_edges_and_byte_alignment(gpu, oracle, shape, offset):
+    """The bit-row tiles at their edges, in a .grad buffer at any byte offset; the bytes
+    around the buffer stay as they were."""
+    import torch
+    from msceer_gb300 import lower_star_grad
+    f = fields.gaussian_sum(shape, 5, seed=6, noise=1e-2)
+    want = oracle.grad(f)
+    buf = torch.full((want.size + 32,), 0xA5, dtype=torch.uint8, device=gpu)
+    out = buf[offset:offset + want.size]
+    lower_star_grad(torch.from_numpy(f).to(gpu), out)
+    assert np.array_equal(out.cpu().numpy(), want)
+    assert bool((buf[:offset] == 0xA5).all()) and bool((buf[offset + want.size:] == 0xA5).all())

@@ -493,11 +493,11 @@ __global__ void __launch_bounds__(BS) terminal_pass_kernel(const float* __restri
 // while its own stack is short.  (A thread per vertex with a stack of its own walked a
 // whole basin of a smooth field alone, one vertex after another: 265 ms of the 430 ms
 // labels of a 256^3 Gaussian-sum field, where the walk now takes a few ms.)  A block
-// that has worked kWalkTail turns past the frontier's end hands what is on its stack to
-// the next round, which deals it out to all blocks again: one block of a deep basin
-// otherwise worked on while the others had ended.
-constexpr int kWalkThreads = 256;
-constexpr int kWalkItems = 128;   // vertices a turn
+// that has worked kWalkTail turns past the frontier's end and still has work for several
+// turns hands its stack to the next round, which deals it out to all blocks again: one
+// block of a deep basin otherwise worked on while the others had ended.
+constexpr int kWalkThreads = 384;
+constexpr int kWalkItems = 128;   // vertices a turn at most: the 64 of a long chain's turn are one pass
 constexpr int kWalkStack = 2048;  // vertices on the block's stack
 constexpr int kWalkTail = 16;
 
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kWalkThreads) terminal_walk_kernel(
       __syncthreads();  // s_got is rewritten
       continue;
     }
-    if (tail > kWalkTail) {  // the rest goes to the next round
+    if (tail > kWalkTail && top > kWalkItems) {  // the rest goes to the next round
       __shared__ int s_out;
       if (tid == 0) s_out = atomicAdd(n_out, top);
       __syncthreads();
@@ -643,7 +643,7 @@ cudaError_t launch_terminal_walk(const float* f, int32_t* lab, const VolDims& V,
   if (cudaError_t e = cudaMemsetAsync(n_out, 0, sizeof(int), stream)) return e;
   if (cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(int), stream)) return e;
   ::msc::count_launch();
-  terminal_walk_kernel<<<num_sms * 8, kWalkThreads, 0, stream>>>(f, lab, V, dir, qin, n_in,
+  terminal_walk_kernel<<<num_sms * 5, kWalkThreads, 0, stream>>>(f, lab, V, dir, qin, n_in,
                                                                  reinterpret_cast<uint32_t*>(cursor), qout, n_out, cap,
                                                                  err);
   return cudaGetLastError();

@@ -365,6 +365,35 @@ __device__ __forceinline__ bool lower_ldir(const GradView& G, int64_t c, unsigne
   return lowered;
 }
 
+// lower_ldir in three steps, so that a thread can have the reads and swaps of two cells
+// in flight: the constructor reads the aligned word, swap() tries the compare-and-swap,
+// finish() tells whether this cell was lowered here (and goes on as lower_ldir after a
+// lost swap, or where the word reaches out of the array).
+struct LdirCell {
+  uint32_t* w;
+  int sh;
+  uint32_t cur, got;
+  bool inside, tried;
+  __device__ __forceinline__ LdirCell(const GradView& G, int64_t c) : got(0), tried(false) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(G.g + c), wa = a & ~uintptr_t(3);
+    inside = wa >= G.lo && wa + 4 <= G.hi;
+    w = reinterpret_cast<uint32_t*>(wa);
+    sh = (int)(a & 3u) * 8;
+    cur = inside ? *reinterpret_cast<volatile uint32_t*>(w)
+                 : (uint32_t)*reinterpret_cast<volatile uint8_t*>(G.g + c) << sh;
+  }
+  __device__ __forceinline__ unsigned byte() const { return (cur >> sh) & 0xFFu; }
+  __device__ __forceinline__ void swap(unsigned val) {
+    const uint32_t b = byte();
+    tried = inside && (b >> 5) > val;
+    if (tried) got = atomicCAS(w, cur, (cur & ~(0xFFu << sh)) | (((b & 0x1Fu) | (val << 5)) << sh));
+  }
+  __device__ __forceinline__ bool finish(const GradView& G, int64_t c, unsigned val) {
+    if (inside && !tried) return false;  // held as low already
+    return (tried && got == cur) || lower_ldir(G, c, val);
+  }
+};
+
 __device__ __forceinline__ int batch_volume(const LdirBatch& B, int64_t flat_tile) {
   int lo = 0, hi = B.n - 1;
   while (lo < hi) {
@@ -813,76 +842,101 @@ __device__ __forceinline__ TileAt tile_at(const LdirBatch& B, int64_t flat) {
   return t;
 }
 
-// Lower one recorded halo cell (box coords lx, ly, lz) in its owner's .grad where the
-// owner holds it higher, and queue it when it became an item.
-__device__ __forceinline__ void check_cell(const LdirBatch& B, const TileAt& t, int lx, int ly, int lz, unsigned v,
-                                           int64_t* queue, int* n_queue, int cap, int* lock, int* err) {
-  const LdirVol& vol = B.v[t.vi];
-  const int64_t gx = t.o[0] + lx, gy = t.o[1] + ly, gz = t.o[2] + lz;
-  const int64_t c = gx + gy * vol.D.cs[1] + gz * vol.D.cs[2];
-  if ((unsigned)(vol.g[c] >> 5) <= v) return;
-  if (!lower_ldir(volume_view(vol, lock, err), c, v)) return;
-  const int dim = (int)((gx & 1) + (gy & 1) + (gz & 1));
-  if ((dim == 1 && v == 2u) || (dim == 2 && v == 1u))
-    push_item(queue, n_queue, cap, err, ((int64_t)t.vi << kVolShift) | c);
-}
-
-// A block per tile: a warp per halo row record (a lane per cell, KU rows' loads in
-// flight), then a thread per inner row byte.
+// A lane per row of a tile's record, 32 rows a warp: a halo row's owner bytes come as bit
+// planes (load_planes), so the few cells that the owner holds higher fall out of two word
+// operations; an inner row's four halo cells are read byte by byte.  (A warp per halo row
+// with a lane per cell spent ~30 warp instructions on a row and waited for one row's
+// bytes at a time; with a lane's cells lowered one after another the warp waited for the
+// row with the most: 2.0 ms at 512^3 either way, 1.2-1.4 ms with the list below.)
 template <int ND, int LY, int LZ>
 __global__ void __launch_bounds__(256) ldir_check_kernel(const LdirBatch B, const uint8_t* __restrict__ rec,
                                                          int64_t* __restrict__ queue, int* __restrict__ n_queue,
                                                          int cap, int* lock, int* err) {
   using T = BitTile<ND, LY, LZ>;
-  constexpr int KU = 4;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  for (int64_t flat = blockIdx.x; flat < B.total_tiles; flat += gridDim.x) {
+  constexpr int UNITS = (T::NHR + T::NIR + 31) / 32;  // warps' rounds per tile
+  __shared__ uint16_t s_cell[8][1024];  // per warp: source lane, x, value 1
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5), total = B.total_tiles * UNITS;
+  for (int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < total; u += nwarp) {
+    const int64_t flat = u / UNITS;
+    const int row = (int)(u - flat * UNITS) * 32 + lane;
     const uint8_t* trec = rec + flat * T::REC;
-    const uint32_t* wrec = reinterpret_cast<const uint32_t*>(trec);
+    uint32_t w2 = 0, w1 = 0;  // cells held at 2 / at 1 by the tile
+    int ly = 0, lz = 0;
+    if (row < T::NHR) {
+      const uint2 w = reinterpret_cast<const uint2*>(trec)[row];
+      w2 = w.x;
+      w1 = w.y;
+      halo_row_of<ND, LY, LZ>(row, ly, lz);
+    } else if (row < T::NHR + T::NIR) {
+      const uint32_t m = trec[T::NHR * 8 + (row - T::NHR)];
+      w2 = (m & 3u) | ((m & 0xCu) << 28);
+      w1 = ((m >> 4) & 3u) | ((m & 0xC0u) << 24);
+      const int i = row - T::NHR;
+      ly = 2 + i % (LY - 4);
+      lz = ND == 3 ? 2 + i / (LY - 4) : 0;
+    }
+    if (!__any_sync(~0u, (w2 | w1) != 0u)) continue;
     const TileAt t = tile_at<ND, LY, LZ>(B, flat);
     const LdirVol& vol = B.v[t.vi];
-    for (int j0 = warp; j0 < T::NHR; j0 += nwarp * KU) {
-      uint32_t w2[KU], w1[KU];
-      uint8_t own[KU];
-      int64_t cell[KU];
+    const int64_t c0 = t.o[0] + (t.o[1] + ly) * vol.D.cs[1] + (t.o[2] + lz) * vol.D.cs[2];
+    uint32_t todo = 0;
+    if ((w2 | w1) && row < T::NHR) {
+      uint32_t b[8];
+      load_planes(vol.g + c0, vol.g, vol.g + vol.D.ncells, b);
+      todo = (w1 & (b[7] | b[6])) | (w2 & (b[7] | (b[6] & b[5])));
+    } else if (w2 | w1) {
+      uint8_t own[4];
 #pragma unroll
-      for (int k = 0; k < KU; k++) {
-        const int j = j0 + k * nwarp;
-        w2[k] = j < T::NHR ? wrec[2 * j] : 0u;
-        w1[k] = j < T::NHR ? wrec[2 * j + 1] : 0u;
-      }
-#pragma unroll
-      for (int k = 0; k < KU; k++) {
-        const int j = j0 + k * nwarp;
-        own[k] = 0;
-        cell[k] = -1;
-        if (((w2[k] | w1[k]) >> lane) & 1u) {
-          int ly, lz;
-          halo_row_of<ND, LY, LZ>(j, ly, lz);
-          cell[k] = (t.o[0] + lane) + (t.o[1] + ly) * vol.D.cs[1] + (t.o[2] + lz) * vol.D.cs[2];
-          own[k] = vol.g[cell[k]];
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < KU; k++) {
-        if (cell[k] < 0) continue;
-        const unsigned v = ((w1[k] >> lane) & 1u) ? 1u : 2u;
-        if ((unsigned)(own[k] >> 5) <= v) continue;
-        int ly, lz;
-        halo_row_of<ND, LY, LZ>(j0 + k * nwarp, ly, lz);
-        check_cell(B, t, lane, ly, lz, v, queue, n_queue, cap, lock, err);
-      }
-    }
-    for (int i = threadIdx.x; i < T::NIR; i += blockDim.x) {
-      const unsigned m = trec[T::NHR * 8 + i];
-      if (!m) continue;
-      const int ly = 2 + i % (LY - 4), lz = ND == 3 ? 2 + i / (LY - 4) : 0;
-#pragma unroll 1
       for (int q = 0; q < 4; q++) {
-        const unsigned a2 = (m >> q) & 1u, a1 = (m >> (4 + q)) & 1u;
-        if (a2 | a1) check_cell(B, t, q < 2 ? q : kBitLX - 4 + q, ly, lz, a1 ? 1u : 2u, queue, n_queue, cap, lock, err);
+        const int lx = q < 2 ? q : kBitLX - 4 + q;
+        own[q] = 0;
+        if (((w2 | w1) >> lx) & 1u) own[q] = vol.g[c0 + lx];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const int lx = q < 2 ? q : kBitLX - 4 + q;
+        if ((unsigned)(own[q] >> 5) > (((w1 >> lx) & 1u) ? 1u : 2u)) todo |= 1u << lx;
       }
     }
+    // the cells of all 32 rows in one list, so that every lane lowers one: most rows have
+    // none and a few have several
+    const int cnt = __popc(todo);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(~0u, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const int n = __shfl_sync(~0u, incl, 31);
+    if (n == 0) continue;
+    for (int slot = incl - cnt; todo; slot++) {
+      const int lx = __ffs(todo) - 1;
+      todo &= todo - 1;
+      s_cell[warp][slot] = (uint16_t)(lane << 5 | lx | ((w1 >> lx) & 1u) << 15);
+    }
+    __syncwarp();
+    const int dim0 = (int)(((t.o[1] + ly) & 1) + ((t.o[2] + lz) & 1));  // (t.o[0] is even)
+    for (int k0 = 0; k0 < n; k0 += 32) {
+      const bool has = k0 + lane < n;
+      const uint32_t e = has ? s_cell[warp][k0 + lane] : 0u;
+      const int src = (int)(e >> 5) & 31, lx = (int)(e & 31u);
+      const int64_t c = __shfl_sync(~0u, c0, src) + lx;
+      const int dim = __shfl_sync(~0u, dim0, src) + (lx & 1);
+      const unsigned v = (e >> 15) ? 1u : 2u;
+      const bool item = has && lower_ldir(volume_view(vol, lock, err), c, v) && dim == 3 - (int)v;
+      // one append per warp: one per item would serialise on the counter in L2
+      const unsigned m = __ballot_sync(~0u, item);
+      if (!m) continue;
+      int base = 0;
+      if (lane == __ffs(m) - 1) base = atomicAdd(n_queue, __popc(m));
+      base = __shfl_sync(~0u, base, __ffs(m) - 1);
+      if (item) {
+        const int slot = base + __popc(m & ((1u << lane) - 1u));
+        if (slot < cap) queue[slot] = ((int64_t)t.vi << kVolShift) | c; else atomicOr(err, kErrLocalQueue);
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -893,11 +947,11 @@ __global__ void __launch_bounds__(256) ldir_check_kernel(const LdirBatch B, cons
 // thread per (item, cofacet), and takes new ones from the queue while its own stack is
 // short.  (A thread per item with a stack of its own followed every branch of a walk
 // alone: 6.0 of the 6.3 ms of a 64^3 Gaussian-sum .grad.)  A block that has worked
-// kWalkTail turns past the queue's end hands its stack to the next round, which deals
-// it out to all blocks again.  The queue's length is read on the device (0 after an
+// kWalkTail turns past the queue's end and still has work for several turns hands its
+// stack to the next round, which deals it out to all blocks again.  The queue's length is read on the device (0 after an
 // overflow: the host finishes with tile passes) and it is dealt out through *cursor.
-constexpr int kWalkThreads = 256;
-constexpr int kWalkItems = 128;   // items a turn
+constexpr int kWalkThreads = 384;
+constexpr int kWalkItems = 128;   // items a turn at most: the 64 of a long chain's turn are one pass in 3D
 constexpr int kWalkStack = 1024;  // items on the block's stack
 constexpr int kWalkTail = 16;
 
@@ -934,7 +988,7 @@ __global__ void __launch_bounds__(kWalkThreads) ldir_walk_kernel(const LdirBatch
     if (s_got < 0) more = false;
     if (!more) tail++;
     if (top + got == 0) break;  // (with more of the queue left, some of it was taken)
-    if (tail > kWalkTail) {     // the rest goes to the next round
+    if (tail > kWalkTail && top > kWalkItems) {  // the rest goes to the next round
       if (tid == 0) s_out = atomicAdd(n_out, top);
       __syncthreads();
       for (int i = tid; i < top; i += kWalkThreads) {
@@ -978,24 +1032,27 @@ __global__ void __launch_bounds__(kWalkThreads) ldir_walk_kernel(const LdirBatch
       const int sgn = (j & 1) ? -1 : 1;
       if (ca + sgn < 0 || ca + sgn >= D.d[a]) continue;
       const int64_t t = i + sgn * D.cs[a];
-      const uint8_t bt = *reinterpret_cast<volatile uint8_t*>(vol.g + t);
-      const unsigned code = (bt >> 2) & 7u;
-      if (!(bt & 1u) || code == 7u) continue;
       const GradView G = volume_view(vol, lock, err);
-      lower_ldir(G, t, value);
+      LdirCell ct(G, t);
+      const unsigned bt = ct.byte(), code = (bt >> 2) & 7u;
+      if (!(bt & 1u) || code == 7u) continue;
       const int pc = map3(D.dec_map, (int)code);
       const int pa = pc >> 1, ps = (pc & 1) ? -1 : 1;
       const int64_t tp = t + ps * D.cs[pa];
-      if (tp == i) continue;
       // the partner's coordinate along the pair's axis, and its dimension
       const int64_t cp = (pa == 0 ? l[0] : (pa == 1 ? l[1] : l[2])) + (pa == a ? sgn : 0) + ps;
-      if (cp < 0 || cp >= D.d[pa]) continue;  // a pair code pointing out of the complex
-      const int pdim = pa == a ? dim : (((cp & 1) != 0) ? dim + 2 : dim);
-      if (value == 2u && pdim != 1) {  // a hex ends the value-2 path
-        lower_ldir(G, tp, 2u);
+      if (tp == i || cp < 0 || cp >= D.d[pa]) {  // (a pair code pointing out of the complex)
+        lower_ldir(G, t, value);
         continue;
       }
-      if (!lower_ldir(G, tp, value)) continue;
+      const int pdim = pa == a ? dim : (((cp & 1) != 0) ? dim + 2 : dim);
+      const bool item = value != 2u || pdim == 1;  // a hex ends the value-2 path
+      // the cofacet's and the partner's swaps go out together
+      LdirCell cq(G, tp);
+      ct.swap(value);
+      cq.swap(value);
+      ct.finish(G, t, value);
+      if (!cq.finish(G, tp, value) || !item) continue;
       const int slot = atomicAdd(&s_top, 1);
       if (slot < kWalkStack) s_stack[slot] = ((int64_t)vi << kVolShift) | tp;
       else push_item(qout, n_out, cap, err, ((int64_t)vi << kVolShift) | tp);
@@ -1062,19 +1119,22 @@ cudaError_t launch_ldir_tile(int nd, const LdirBatch& B, uint8_t* rec, int* err,
   return cudaGetLastError();
 }
 
-static int check_grid(const LdirBatch& B, int num_sms) {
+// eight warps a block, a warp per 32 rows of a tile's record
+static int check_grid(int nd, const LdirBatch& B, int num_sms) {
   const int64_t cap = (int64_t)num_sms * 8;
-  return (int)(B.total_tiles < cap ? (B.total_tiles > 0 ? B.total_tiles : 1) : cap);
+  const int64_t rows = nd == 3 ? Bit3::NHR + Bit3::NIR : Bit2::NHR + Bit2::NIR;
+  const int64_t blocks = (B.total_tiles * ((rows + 31) / 32) + 7) / 8;
+  return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
 cudaError_t launch_ldir_check(int nd, const LdirBatch& B, const uint8_t* rec, int64_t* queue, int* n_queue, int cap,
                               int* lock, int* err, int num_sms, cudaStream_t stream) {
   ::msc::count_launch();
   if (nd == 3)
-    ldir_check_kernel<3, kBitLY3, kBitLZ3><<<check_grid(B, num_sms), 256, 0, stream>>>(B, rec, queue, n_queue, cap,
+    ldir_check_kernel<3, kBitLY3, kBitLZ3><<<check_grid(nd, B, num_sms), 256, 0, stream>>>(B, rec, queue, n_queue, cap,
                                                                                        lock, err);
   else
-    ldir_check_kernel<2, kBitLY2, 1><<<check_grid(B, num_sms), 256, 0, stream>>>(B, rec, queue, n_queue, cap, lock,
+    ldir_check_kernel<2, kBitLY2, 1><<<check_grid(nd, B, num_sms), 256, 0, stream>>>(B, rec, queue, n_queue, cap, lock,
                                                                                  err);
   return cudaGetLastError();
 }
@@ -1087,9 +1147,9 @@ cudaError_t launch_ldir_walk(int nd, const LdirBatch& B, const int64_t* qin, con
   uint32_t* cur = reinterpret_cast<uint32_t*>(cursor);
   ::msc::count_launch();
   if (nd == 3)
-    ldir_walk_kernel<3><<<num_sms * 8, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
+    ldir_walk_kernel<3><<<num_sms * 5, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
   else
-    ldir_walk_kernel<2><<<num_sms * 8, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
+    ldir_walk_kernel<2><<<num_sms * 5, kWalkThreads, 0, stream>>>(B, qin, n_in, cur, qout, n_out, cap, lock, err);
   return cudaGetLastError();
 }
 

@@ -103,16 +103,6 @@ struct Nb {
       if (d(p, a) == val) m |= 1u << p;
     return m;
   }
-  // vertices of cell p
-  MSC_HD static constexpr uint32_t vertex_mask(int p) {
-    uint32_t m = 0;
-    for (int q = 0; q < NPOS; q++) {
-      bool ok = true;
-      for (int a = 0; a < ND; a++) ok = ok && (d(q, a) == 0 || d(q, a) == d(p, a));
-      if (ok) m |= 1u << q;
-    }
-    return m;
-  }
   // AND-fold along axis A: keep bit p only if the bit of p with axis A zeroed is set
   template <int A>
   MSC_HD static uint32_t fold(uint32_t m) {
@@ -120,70 +110,58 @@ struct Nb {
     constexpr uint32_t mp = axis_mask(A, 1), mm = axis_mask(A, -1), m0 = axis_mask(A, 0);
     return m & (((m << s) & mp) | ((m >> s) & mm) | m0);
   }
-  // bit c set when c's facet along axis A (the one toward the centre) is in m
-  template <int A>
-  MSC_HD static uint32_t facet_in(uint32_t m) {
-    constexpr int s = stride(A);
-    constexpr uint32_t mp = axis_mask(A, 1), mm = axis_mask(A, -1);
-    return ((m << s) & mp) | ((m >> s) & mm);
-  }
-  // facets along axis A of the cells in r whose A-facet is flagged in f
-  template <int A>
-  MSC_HD static uint32_t facet_of(uint32_t r, uint32_t f) {
-    constexpr int s = stride(A);
-    constexpr uint32_t mp = axis_mask(A, 1), mm = axis_mask(A, -1);
-    return ((r & f & mp) >> s) | ((r & f & mm) << s);
-  }
 };
 
 // Per-cell key of the cell's lowest vertex (order_key), indexed by neighbourhood
-// position.  Device: a per-thread column in shared memory; host: a plain array.
+// position.  Device: a per-thread column; host: a plain array.
 struct KeyCol {
+  using Key = uint64_t;
   uint64_t* base;
   int stride;
   MSC_HD uint64_t operator()(int p) const { return base[p * stride]; }
+  // the key one step along axis a from position p
+  MSC_HD uint64_t next(int p, int a, bool up) const {
+    const int s = a == 0 ? 1 : (a == 1 ? 3 : 9);
+    return base[(up ? p + s : p - s) * stride];
+  }
+  MSC_HD static uint64_t last() { return ~0ull; }  // after every key
+  MSC_HD static bool less(uint64_t a, uint64_t b) { return a < b; }
 };
 
-template <int ND, class Keys>
-struct LowerStarState {
-  using N = Nb<ND>;
-  Keys lk;             // lowest-vertex key per cell
-  uint32_t P = 0;      // processed cells
-  uint32_t K = 0;      // critical cells
+// The pairing kept as bit planes over the neighbourhood's cells.
+struct PlaneSink {
+  uint32_t K = 0;                   // critical cells
   uint32_t C0 = 0, C1 = 0, C2 = 0;  // pair-direction code bit-planes
+  // cell q (bit qb) and cell r (bit rb), one step along `axis` from q (up: in its
+  // positive direction); codes 0..5 = +x,-x,+y,-y,+z,-z name each one's partner
+  MSC_HD void pair(int, uint32_t qb, uint32_t rb, int axis, bool up) {
+    const uint32_t pm = qb | rb;
+    C0 |= up ? rb : qb;  // the one whose partner lies in the negative direction
+    if (axis == 1) C1 |= pm;
+    if (axis == 2) C2 |= pm;
+  }
+  MSC_HD void critical(int, uint32_t qb, int) { K |= qb; }
+};
 
-  MSC_HD explicit LowerStarState(Keys k) : lk(k) {}
+template <int ND, class Keys, class Sink>
+struct LowerStarExpand {
+  using N = Nb<ND>;
+  using Key = typename Keys::Key;
+  Keys lk;  // lowest-vertex key per cell
+  Sink& out;
 
-  MSC_HD void set_code(int q, int code) {
-    C0 |= (uint32_t)(code & 1) << q;
-    C1 |= (uint32_t)((code >> 1) & 1) << q;
-    C2 |= (uint32_t)((code >> 2) & 1) << q;
-  }
-  // direction code of the pair partner at delta = partner - cell: +x,-x,+y,-y,+z,-z
-  MSC_HD static int dir_code(int delta) {
-    const int ad = delta < 0 ? -delta : delta;
-    return (delta < 0 ? 1 : 0) | (ad == 3 ? 2 : (ad == 9 ? 4 : 0));
-  }
-  MSC_HD void make_pair(int q, int r) {
-    P |= (1u << q) | (1u << r);
-    set_code(q, dir_code(r - q));
-    set_code(r, dir_code(q - r));
-  }
-  MSC_HD void make_critical(int q) {
-    P |= 1u << q;
-    K |= 1u << q;
-  }
+  MSC_HD LowerStarExpand(Keys k, Sink& s) : lk(k), out(s) {}
 
   // the cell of U whose lowest vertex comes first (first in star order wins ties)
   MSC_HD int lowest_of(uint32_t U) const {
     int q = ffs32(U) - 1;
-    uint64_t kb = lk(q);
+    Key kb = lk(q);
     uint32_t W = U & (U - 1);
     while (W) {
       const int o = ffs32(W) - 1;
       W &= W - 1;
-      const uint64_t ko = lk(o);
-      if (ko < kb) {
+      const Key ko = lk(o);
+      if (Keys::less(ko, kb)) {
         q = o;
         kb = ko;
       }
@@ -195,63 +173,90 @@ struct LowerStarState {
   MSC_HD void expand(uint32_t S) {
     constexpr int C = N::CENTER;
     constexpr uint32_t EDGES = N::dim_mask(1);
+    uint32_t A = S;  // unprocessed cells of the class
     if (S & (1u << C)) {
-      // the vertex pairs with the edge to its lowest neighbour (steepest descent)
-      const uint32_t E = S & EDGES;
-      if (!E) make_critical(C);
-      else make_pair(C, lowest_of(E));  // an edge's lowest vertex is its other end
-    }
-    constexpr uint32_t DM1 = N::dim_mask(1), DM2 = N::dim_mask(2), DM3 = N::dim_mask(3);
-    constexpr uint32_t AX0 = N::axis_mask(0, 0), AX1 = N::axis_mask(1, 0), AX2 = N::axis_mask(2, 0);
-    // One step per iteration, always in the lowest dimension that still has
-    // unprocessed cells -- the order of the reference's per-dimension loops -- so the
-    // loop body is the same straight-line set algebra for every thread of a warp.
-    for (int guard = 0; guard < N::NPOS; guard++) {
-      const uint32_t A = S & ~P;  // unprocessed cells of the class
-      if (!A) break;
-      const bool d1 = (A & DM1) != 0u, d2 = !d1 && (A & DM2) != 0u;
-      const uint32_t DMd = d1 ? DM1 : (d2 ? DM2 : DM3);
-      const uint32_t DMu = d1 ? DM2 : (d2 ? DM3 : 0u);
-      const uint32_t F0 = N::template facet_in<0>(A);
-      const uint32_t F1 = N::template facet_in<1>(A);
-      const uint32_t F2 = (ND == 3) ? N::template facet_in<2>(A) : 0u;
-      const uint32_t one = (F0 ^ F1 ^ F2) & ~(F0 & F1 & F2);  // exactly one unprocessed facet
-      const uint32_t R = A & DMu & one;                       // ready (d+1)-cells
-      uint32_t Q = N::template facet_of<0>(R, F0) | N::template facet_of<1>(R, F1);
-      if (ND == 3) Q |= N::template facet_of<2>(R, F2);
-      if (Q) {
-        const int q = ffs32(Q) - 1;
-        // ready cofacets of q, i.e. its candidates
-        uint32_t cm = 0;
+      A &= ~(1u << C);
+      // the vertex pairs with the edge to its lowest neighbour (steepest descent; an
+      // edge's lowest vertex is its other end, so no two keys are equal)
+      if (!(S & EDGES)) {
+        out.critical(C, 1u << C, 0);
+      } else {
+        Key kb = Keys::last();
+        uint32_t rb = 0;
+        int axis = 0;
+        bool up = false;
 #pragma unroll
         for (int a = 0; a < ND; a++) {
-          const uint32_t even = a == 0 ? AX0 : (a == 1 ? AX1 : AX2);
-          if ((even >> q) & 1u) cm |= (1u << (q + N::stride(a))) | (1u << (q - N::stride(a)));
-        }
-        cm &= R;
-        int best = ffs32(cm) - 1;
-        if (cm & (cm - 1)) {
-          // several: the first in cofacet order (+x,-x,+y,-y,+z,-z) whose lowest
-          // vertex comes first wins (PickLowestCandidate)
-          best = -1;
-          uint64_t kb = ~0ull;
 #pragma unroll
-          for (int a = 0; a < ND; a++) {
-#pragma unroll
-            for (int sgn = 0; sgn < 2; sgn++) {
-              const int c = q + (sgn == 0 ? N::stride(a) : -N::stride(a));
-              if (c < 0 || c >= N::NPOS || !((cm >> c) & 1u)) continue;
-              const uint64_t kc = lk(c);
-              if (best < 0 || kc < kb) {
-                best = c;
-                kb = kc;
-              }
+          for (int s = 0; s < 2; s++) {
+            const uint32_t eb = 1u << (C + (s == 0 ? N::stride(a) : -N::stride(a)));
+            if (!(S & eb)) continue;
+            const Key k = lk.next(C, a, s == 0);
+            if (Keys::less(k, kb)) {
+              kb = k;
+              rb = eb;
+              axis = a;
+              up = s == 0;
             }
           }
         }
-        make_pair(q, best);
+        A &= ~rb;
+        out.pair(C, 1u << C, rb, axis, up);
+      }
+    }
+    constexpr uint32_t DM1 = N::dim_mask(1), DM2 = N::dim_mask(2), DM3 = N::dim_mask(3);
+    constexpr uint32_t M0 = N::axis_mask(0, 0), M1 = N::axis_mask(1, 0), M2 = N::axis_mask(2, 0);
+    constexpr int S1 = N::stride(1), S2 = N::stride(2);
+    // One step per iteration, always in the lowest dimension that still has
+    // unprocessed cells -- the order of the reference's per-dimension loops -- so the
+    // loop body is the same straight-line set algebra for every thread of a warp.
+    // Within the neighbourhood a cell with offset 0 along an axis has its two cofacets
+    // there one stride away on either side, so facets and cofacets along an axis are the
+    // set shifted both ways, of the cells (before) or kept on the cells (after) of
+    // offset 0.
+    for (int guard = 0; guard < N::NPOS && A; guard++) {
+      const uint32_t A1 = A & DM1, A2 = A & DM2;
+      const uint32_t D = A1 ? A1 : (A2 ? A2 : A);        // the dimension worked on
+      const uint32_t U = A1 ? A2 : (A2 ? A & DM3 : 0u);  // and the next one
+      const int dim = A1 ? 1 : (A2 ? 2 : 3);
+      const uint32_t Z0 = D & M0, Z1 = D & M1, Z2 = ND == 3 ? D & M2 : 0u;
+      const uint32_t F0 = (Z0 << 1) | (Z0 >> 1), F1 = (Z1 << S1) | (Z1 >> S1), F2 = (Z2 << S2) | (Z2 >> S2);
+      const uint32_t one = (F0 ^ F1 ^ F2) & ~(F0 & F1 & F2);  // exactly one unprocessed facet
+      const uint32_t R = U & one;                             // ready (d+1)-cells
+      const uint32_t W0 = R & F0, W1 = R & F1, W2 = R & F2;
+      uint32_t Q = (((W0 << 1) | (W0 >> 1)) & M0) | (((W1 << S1) | (W1 >> S1)) & M1);
+      if (ND == 3) Q |= ((W2 << S2) | (W2 >> S2)) & M2;
+      if (Q) {
+        const uint32_t qb = Q & (0u - Q);
+        const int q = ffs32(Q) - 1;
+        // ready cofacets of q, i.e. its candidates
+        const uint32_t q0 = qb & M0, q1 = qb & M1, q2 = ND == 3 ? qb & M2 : 0u;
+        const uint32_t u0 = R & (q0 << 1), d0 = R & (q0 >> 1), u1 = R & (q1 << S1), d1 = R & (q1 >> S1);
+        const uint32_t u2 = R & (q2 << S2), d2 = R & (q2 >> S2);
+        const uint32_t c1 = u1 | d1, c2 = u2 | d2, cm = u0 | d0 | c1 | c2;
+        uint32_t rb = cm;
+        if (cm & (cm - 1)) {
+          // several: the first in cofacet order (+x,-x,+y,-y,+z,-z) whose lowest
+          // vertex comes first wins (PickLowestCandidate)
+          Key kb = Keys::last();
+          rb = 0;
+          const uint32_t cand[6] = {u0, d0, u1, d1, u2, d2};
+#pragma unroll
+          for (int j = 0; j < 2 * ND; j++) {
+            if (!cand[j]) continue;
+            const Key k = lk.next(q, j >> 1, (j & 1) == 0);
+            if (Keys::less(k, kb)) {
+              kb = k;
+              rb = cand[j];
+            }
+          }
+        }
+        A &= ~(qb | rb);
+        out.pair(q, qb, rb, (rb & c1) ? 1 : ((rb & c2) ? 2 : 0), rb > qb);
       } else {
-        make_critical(lowest_of(A & DMd));
+        const int q = lowest_of(D);
+        A &= ~(1u << q);
+        out.critical(q, 1u << q, dim);
       }
     }
   }
@@ -295,23 +300,6 @@ MSC_HD uint32_t run_classes(State& st, uint32_t L, bool bx, bool by, bool bz) {
     if ((c = L & all3)) st.expand(c);
   }
   return Bany;
-}
-
-// Final .grad byte of the cell at position p of a processed lower star.
-//   code: 7 if critical, else the (axis-remapped) pair direction
-//   ldir: roots of the ascending-manifold closure -- critical 1-cells 2, critical
-//         2-cells 1, critical 3-cells 0 (gi_topological_gradient_using_algorithms.h:
-//         460-477) -- and 3 everywhere else
-//   flag: cell on the boundary (outputToFile, gi_discrete_gradient_labeling.h:206-211)
-template <int ND, class State>
-MSC_HD uint8_t cell_byte(const State& st, int p, uint32_t Bany, uint32_t enc_map) {
-  const bool crit = (st.K >> p) & 1u;
-  const int lc = (int)(((st.C0 >> p) & 1u) | (((st.C1 >> p) & 1u) << 1) | (((st.C2 >> p) & 1u) << 2));
-  const int code = crit ? 7 : (int)((enc_map >> (3 * lc)) & 7u);
-  const int dimp = Nb<ND>::dim(p);
-  const int ldir = crit ? (dimp == 1 ? 2 : (dimp == 2 ? 1 : (dimp == 3 ? 0 : 3))) : 3;
-  const int flag = (Bany >> p) & 1u;
-  return (uint8_t)(1 | (flag << 1) | (code << 2) | (ldir << 5));
 }
 
 // First half of one vertex's work: gather its 3^ND neighbourhood through `load(p)`,
@@ -424,12 +412,13 @@ MSC_HD void store_cells(const State& st, uint32_t L, uint32_t Bany, uint32_t enc
 template <int ND, class Store>
 MSC_HD void expand_and_store(uint32_t L, uint64_t* col, int cs, bool interior, bool bx, bool by, bool bz,
                              uint32_t enc_map, const Store& store) {
-  LowerStarState<ND, KeyCol> st(KeyCol{col, cs});
+  PlaneSink st;
+  LowerStarExpand<ND, KeyCol, PlaneSink> ex(KeyCol{col, cs}, st);
   uint32_t Bany = 0;
   if (interior)
-    st.expand(L);
+    ex.expand(L);
   else
-    Bany = run_classes<ND>(st, L, bx, by, ND == 3 && bz);
+    Bany = run_classes<ND>(ex, L, bx, by, ND == 3 && bz);
   store_cells<ND>(st, L, Bany, enc_map, store);
 }
 
@@ -444,7 +433,8 @@ MSC_HD void expand_and_store_keyed(uint32_t L, uint64_t* col, int cs, const uint
                                    uint32_t enc_map, const Store& store) {
   using N = Nb<ND>;
   constexpr int NPOS = N::NPOS;
-  LowerStarState<ND, KeyCol> st(KeyCol{col, cs});
+  PlaneSink st;
+  LowerStarExpand<ND, KeyCol, PlaneSink> ex(KeyCol{col, cs}, st);
   const uint32_t B0 = bx ? N::axis_mask(0, 0) : 0u;
   const uint32_t B1 = by ? N::axis_mask(1, 0) : 0u;
   const uint32_t B2 = (ND == 3 && bz) ? N::axis_mask(2, 0) : 0u;
@@ -460,7 +450,7 @@ MSC_HD void expand_and_store_keyed(uint32_t L, uint64_t* col, int cs, const uint
     cls[key] |= 1u << p;
   }
   for (int k = 0; k < kClasses; k++)
-    if (cls[k]) st.expand(cls[k]);
+    if (cls[k]) ex.expand(cls[k]);
   store_cells<ND>(st, L, B0 | B1 | B2, enc_map, store);
 }
 

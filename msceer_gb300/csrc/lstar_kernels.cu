@@ -12,105 +12,167 @@
 // cell: the boundary flag and the ldir value of critical cells (the roots of the
 // ascending-manifold closure, finished by ldir_kernels.cu).
 //
-// The max/min vertex labeling is never materialised: the per-vertex work
-// (lstar_core.cuh) derives the lower star from the neighbours below the vertex and
-// expands it on bitmasks.  The lowest-vertex key of every cell of the neighbourhood
-// lives in a per-thread shared-memory column so the comparisons can index it.  Each
-// cell is owned by exactly one vertex (its highest), so its final byte is written
-// once with a plain store; for one neighbour position the 32 stores of a warp fall in
-// one 64-byte span.
-#include "lstar_core.cuh"
+// The max/min vertex labeling is never materialised.  A block takes a tile of 32 x 4 x 4
+// vertices (2D: 32 x 16): f with one neighbour around it goes to shared memory, the
+// lowest vertex of every cell of the tile is computed there once (lstar_tile.cuh), every
+// vertex gets its lower star, and the expansions (lstar_core.cuh) are handed out in order
+// of the lower star's size, since their loop runs once per pairing step: the lanes of a
+// warp run loops of similar length (one thread per vertex left half the lanes idle).  The
+// pairing puts the cells' bytes into shared memory, and they leave it row by row: a
+// byte stored from its own thread cost an L2 write of its own.
+// What bounds it is integer issue: 52.7 warp instructions per vertex of a 64^3 Gaussian-sum
+// field (24 of 32 lanes active), 88.4 with a key per vertex and neighbouring cell; 13.0 ->
+// 7.2 ms at 512^3 (k^-3), 2.06 -> 1.35 ms for an 8192^2 image.
+#include <cstddef>
+
+#include "lstar_tile.cuh"
 #include "msc_device.cuh"
 
 namespace msc {
 
-// One block's work: 32 consecutive x by BS/32 consecutive y at one z of volume (f, g,
-// D).  Neighbour and cell offsets are 32-bit; only the per-vertex base addresses are
-// 64-bit.  Every thread first builds its own vertex's keys and lower star; the
-// expansions -- whose loop runs once per pairing step, so its length follows the
-// lower star's size -- are then handed out in order of that size, so that the lanes
-// of a warp run loops of similar length (one thread per vertex otherwise left half the
-// lanes idle).  Every thread of the block must call this (it synchronises the block).
-template <int ND, int BS>
-__device__ __forceinline__ bool lstar_block(const float* __restrict__ f, uint8_t* __restrict__ g, const GradDims& D,
-                                            int64_t bx, int64_t by, int64_t z, uint64_t* s_key, uint32_t* s_L,
-                                            int* s_order, int* s_hist) {
+namespace {
+constexpr int kLstarBS = 256;
+constexpr int kLstarWarps = kLstarBS / 32;
+bool lstar_dims_ok(const GradDims& D) {
+  // a z-plane of cells must be addressable with 32-bit offsets
+  return !(D.v[0] > (int64_t)1 << 30 || D.v[1] > (int64_t)1 << 30 || D.v[0] * D.v[1] > ((int64_t)1 << 31) - 1 ||
+           D.cs[2] > ((int64_t)1 << 31) - 1);
+}
+template <int ND>
+struct LstarSmem {
+  using T = LstarTile<ND>;
+  LatKey lat[T::NL];
+  float f[T::NF];
+  uint32_t L[T::NV];
+  alignas(16) uint8_t bytes[(T::NL + 15) / 16 * 16];  // cleared 16 bytes at a time
+  uint16_t order[T::NV];
+  int16_t off[32];
+  int hist[32];
+};
+static_assert(offsetof(LstarSmem<3>, bytes) % 16 == 0 && offsetof(LstarSmem<2>, bytes) % 16 == 0, "uint4 stores");
+}  // namespace
+
+// One tile of volume (f, g, D); its first vertex is (x0, y0, z0).  Every thread of the
+// block calls this.
+template <int ND>
+__device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t* __restrict__ g, const GradDims& D,
+                                           int64_t x0, int64_t y0, int64_t z0, LstarSmem<ND>& S) {
+  using T = LstarTile<ND>;
   using N = Nb<ND>;
-  constexpr int ROWS = BS / 32;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t X = D.v[0], Y = D.v[1], Z = D.v[2];
-  const int sX = (int)X, sXY = (int)(X * Y);
-  const int c1 = (int)D.cs[1], c2 = (int)D.cs[2];
-  auto vertex = [&](int t, int64_t& x, int64_t& y) {
-    x = bx * 32 + (t & 31);
-    y = by * ROWS + (t >> 5);
-    return x < X && y < Y;
-  };
-  auto is_interior = [&](int64_t x, int64_t y) {
-    return x > 0 && x < X - 1 && y > 0 && y < Y - 1 && (ND == 2 || (z > 0 && z < Z - 1));
-  };
-  if (tid < 32) s_hist[tid] = 0;
-  __syncthreads();
-  int64_t x, y;
-  bool nan = false;
-  int size = -1;  // popcount of the lower star; -1: no vertex here
-  if (vertex(tid, x, y)) {
-    const float* fv = f + (x + X * (y + Y * z));
-    auto load = [&](int p, float& v) {
-      v = __ldg(fv + (N::d(p, 0) + N::d(p, 1) * sX + (ND == 3 ? N::d(p, 2) : 0) * sXY));
-    };
-    const uint32_t L = lower_star_keys<ND>(x, y, z, X, Y, Z, is_interior(x, y), load, s_key + tid, BS, nan);
-    s_L[tid] = L;
-    size = __popc(L);
+  const bool rim = x0 == 0 || y0 == 0 || x0 + T::BX >= X || y0 + T::BY >= Y ||
+                   (ND == 3 && (z0 == 0 || z0 + T::BZ >= Z));
+  if (tid < 32) {
+    S.hist[tid] = 0;
+    S.off[tid] = (int16_t)(tid < N::NPOS ? T::off(tid) : 0);
   }
-  // counting sort of the block's vertices by lower-star size (28 sizes)
-  const int bin = size < 0 ? 31 : size;
-  const int rank = atomicAdd(&s_hist[bin], 1);
+  for (int i = tid; i < (int)sizeof(S.bytes) / 16; i += kLstarBS)
+    reinterpret_cast<uint4*>(S.bytes)[i] = make_uint4(0u, 0u, 0u, 0u);
+  // f, a warp per row (values outside the volume read as 0: no cell that holds one is in
+  // a lower star)
+  bool nan = false;
+  for (int r = warp; r < T::FY * T::FZ; r += kLstarWarps) {
+    const int64_t y = y0 - 1 + r % T::FY, z = ND == 3 ? z0 - 1 + r / T::FY : 0;
+    const bool row = y >= 0 && y < Y && z >= 0 && z < Z;
+    const float* fr = f + (x0 - 1 + X * (y + Y * z));
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int lx = lane + 32 * h;
+      if (lx >= T::FX) break;
+      const int64_t x = x0 - 1 + lx;
+      float v = 0.f;
+      if (row && x >= 0 && x < X) v = __ldg(fr + lx);
+      nan |= v != v;
+      S.f[r * T::FX + lx] = plain_zero(v);
+    }
+  }
+  __syncthreads();
+  // the cells' keys, a thread per base vertex
+  constexpr int CX = T::BX + 1, CY = T::BY + 1, CZ = ND == 3 ? T::BZ + 1 : 1;
+  for (int i = tid; i < CX * CY * CZ; i += kLstarBS) {
+    const int z = i / (CX * CY), r = i - z * (CX * CY), y = r / CX, x = r - y * CX;
+    tile_cell_keys<ND>(S.f, S.lat, x - 1, y - 1, ND == 3 ? z - 1 : 0);
+  }
+  // lower stars, and a counting sort of the vertices by their size (28 sizes; 31: no vertex)
+  int bin[T::NV / kLstarBS], rank[T::NV / kLstarBS];
+#pragma unroll
+  for (int h = 0; h < T::NV / kLstarBS; h++) {
+    const int t = tid + h * kLstarBS;
+    int x, y, z;
+    T::vertex(t, x, y, z);
+    bin[h] = 31;
+    if (x0 + x < X && y0 + y < Y && (ND == 2 || z0 + z < Z)) {
+      uint32_t lower = tile_lower_mask<ND>(S.f, x, y, z);
+      if (rim) lower &= inside_mask<ND>(x0 + x, y0 + y, z0 + z, D.v);
+      const uint32_t L = lower_star_mask<ND>(lower);
+      S.L[t] = L;
+      bin[h] = __popc(L);
+    }
+    rank[h] = atomicAdd(&S.hist[bin[h]], 1);
+  }
   __syncthreads();
   if (tid < 32) {
-    const int c = s_hist[tid];
+    const int c = S.hist[tid];
     int incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, incl, o);
       if (tid >= o) incl += u;
     }
-    s_hist[tid] = incl - c;  // exclusive start of each bin
+    S.hist[tid] = incl - c;  // exclusive start of each bin
   }
   __syncthreads();
-  s_order[s_hist[bin] + rank] = tid;
+#pragma unroll
+  for (int h = 0; h < T::NV / kLstarBS; h++)
+    S.order[S.hist[bin[h]] + rank[h]] = (uint16_t)(bin[h] == 31 ? 0xFFFF : tid + h * kLstarBS);
   __syncthreads();
-  const int t = s_order[tid];
-  if (vertex(t, x, y)) {
-    uint8_t* gc = g + (2 * x + 2 * y * D.cs[1] + 2 * z * D.cs[2]);
-    auto store = [&](int p, uint8_t b) { gc[N::d(p, 0) + N::d(p, 1) * c1 + (ND == 3 ? N::d(p, 2) : 0) * c2] = b; };
-    expand_and_store<ND>(s_L[t], s_key + t, BS, is_interior(x, y), x == 0 || x == X - 1, y == 0 || y == Y - 1,
-                         z == 0 || z == Z - 1, D.enc_map, store);
+  // a warp takes small stars first time and large ones the second, so that all have the
+  // same work
+#pragma unroll 1
+  for (int h = 0; h < T::NV / kLstarBS; h++) {
+    const int t = S.order[(h & 1) ? T::NV - 1 - tid - (h - 1) / 2 * kLstarBS : tid + h / 2 * kLstarBS];
+    if (t == 0xFFFF) continue;
+    int x, y, z;
+    T::vertex(t, x, y, z);
+    tile_expand<ND>(S.L[t], t, rim, x0 + x, y0 + y, z0 + z, D.v, S.lat, S.bytes, S.off, D.enc_map);
   }
-  __syncthreads();  // the keys and masks are reused for the next z
+  __syncthreads();
+  // the bytes, a warp per lattice row
+  uint8_t* g0 = g + (2 * x0 - 1) + (2 * y0 - 1) * D.cs[1] + (ND == 3 ? (2 * z0 - 1) * D.cs[2] : 0);
+  for (int r = warp; r < T::ROWS; r += kLstarWarps) {
+    const int cy = r % T::LY, cz = r / T::LY;
+    uint8_t* gr = g0 + cy * D.cs[1] + cz * D.cs[2];
+    const uint8_t* b = S.bytes + r * T::LX;
+    const uint8_t b0 = b[lane], b1 = b[lane + 32];
+    if (b0) gr[lane] = b0;
+    if (b1) gr[lane + 32] = b1;
+    if (lane == 0 && b[64]) gr[64] = b[64];
+  }
   return nan;
 }
 
-// One volume: grid (x-blocks, y-blocks, z), looping over z when Z exceeds the grid.
-template <int ND, int BS>
-__global__ void __launch_bounds__(BS) lstar_kernel(const float* __restrict__ f, uint8_t* __restrict__ g,
-                                                   const GradDims D, int* __restrict__ err) {
-  __shared__ uint64_t s_key[Nb<ND>::NPOS * BS];
-  __shared__ uint32_t s_L[BS];
-  __shared__ int s_order[BS], s_hist[32];
+// One volume: grid (x-tiles, y-tiles, z-tiles), looping over z when they exceed the grid.
+template <int ND>
+__global__ void __launch_bounds__(kLstarBS, 4) lstar_kernel(const float* __restrict__ f, uint8_t* __restrict__ g,
+                                                            const GradDims D, int* __restrict__ err) {
+  using T = LstarTile<ND>;
+  extern __shared__ __align__(16) unsigned char s_tile[];
+  LstarSmem<ND>& S = *reinterpret_cast<LstarSmem<ND>*>(s_tile);
   bool nan = false;
-  for (int64_t z = blockIdx.z; z < D.v[2]; z += gridDim.z)
-    nan |= lstar_block<ND, BS>(f, g, D, blockIdx.x, blockIdx.y, z, s_key, s_L, s_order, s_hist);
+  for (int64_t z = blockIdx.z; z * T::BZ < D.v[2]; z += gridDim.z) {
+    nan |= lstar_tile<ND>(f, g, D, (int64_t)blockIdx.x * T::BX, (int64_t)blockIdx.y * T::BY, z * T::BZ, S);
+    __syncthreads();  // the next tile reuses the shared memory
+  }
   if (nan) atomicOr(err, kErrNaN);
 }
 
-// Many volumes in one launch: a flat grid over every volume's (x-block, y-block, z)
-// triples; a block finds its volume by binary search over the volumes' first blocks.
-template <int BS>
-__global__ void __launch_bounds__(BS) lstar_batch_kernel(const LstarBatch B, int* __restrict__ err) {
-  __shared__ uint64_t s_key[27 * BS];
-  __shared__ uint32_t s_L[BS];
-  __shared__ int s_order[BS], s_hist[32];
+// Many volumes in one launch: a flat grid over every volume's tiles; a block finds its
+// volume by binary search over the volumes' first tiles.
+__global__ void __launch_bounds__(kLstarBS, 4) lstar_batch_kernel(const LstarBatch B, int* __restrict__ err) {
+  using T = LstarTile<3>;
+  extern __shared__ __align__(16) unsigned char s_tile[];
+  LstarSmem<3>& S = *reinterpret_cast<LstarSmem<3>*>(s_tile);
   bool nan = false;
   for (int64_t blk = blockIdx.x; blk < B.total_blocks; blk += gridDim.x) {
     int lo = 0, hi = B.n - 1;
@@ -120,37 +182,36 @@ __global__ void __launch_bounds__(BS) lstar_batch_kernel(const LstarBatch B, int
     }
     const LstarVol& V = B.v[lo];
     const int64_t r = blk - V.block0;
-    const int64_t bx = r % V.gx, by = (r / V.gx) % V.gy, z = r / ((int64_t)V.gx * V.gy);
-    nan |= lstar_block<3, BS>(V.f, V.g, V.D, bx, by, z, s_key, s_L, s_order, s_hist);
+    const int64_t bx = r % V.gx, by = (r / V.gx) % V.gy, bz = r / ((int64_t)V.gx * V.gy);
+    nan |= lstar_tile<3>(V.f, V.g, V.D, bx * T::BX, by * T::BY, bz * T::BZ, S);
+    __syncthreads();
   }
   if (nan) atomicOr(err, kErrNaN);
 }
 
 namespace {
-constexpr int kLstarBS = 128;
-bool lstar_dims_ok(const GradDims& D) {
-  // a z-plane of cells must be addressable with 32-bit offsets
-  return !(D.v[0] > (int64_t)1 << 30 || D.v[1] > (int64_t)1 << 30 || D.v[0] * D.v[1] > ((int64_t)1 << 31) - 1 ||
-           D.cs[2] > ((int64_t)1 << 31) - 1);
+template <class K>
+cudaError_t allow_smem(K k, size_t bytes) {
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+template <int ND>
+cudaError_t launch_lstar_nd(const float* f, uint8_t* g, const GradDims& D, int* err, cudaStream_t stream) {
+  using T = LstarTile<ND>;
+  const int64_t gy = (D.v[1] + T::BY - 1) / T::BY, gz = (D.v[2] + T::BZ - 1) / T::BZ;
+  if (gy > 65535) return cudaErrorInvalidValue;
+  const dim3 grid((unsigned)((D.v[0] + T::BX - 1) / T::BX), (unsigned)gy, (unsigned)(gz < 65535 ? gz : 65535));
+  if (cudaError_t e = allow_smem(lstar_kernel<ND>, sizeof(LstarSmem<ND>))) return e;
+  ::msc::count_launch();
+  lstar_kernel<ND><<<grid, kLstarBS, sizeof(LstarSmem<ND>), stream>>>(f, g, D, err);
+  return cudaGetLastError();
 }
 }  // namespace
 
 cudaError_t launch_lstar(int nd, const float* f, uint8_t* g, const GradDims& D, int* err, int num_sms,
                          cudaStream_t stream) {
   (void)num_sms;
-  constexpr int BS = kLstarBS;
   if (!lstar_dims_ok(D)) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)((D.v[0] + 31) / 32), (unsigned)((D.v[1] + BS / 32 - 1) / (BS / 32)),
-                  (unsigned)(D.v[2] < 65535 ? D.v[2] : 65535));
-  if (grid.y > 65535u) return cudaErrorInvalidValue;
-  if (nd == 3) {
-    ::msc::count_launch();
-    lstar_kernel<3, BS><<<grid, BS, 0, stream>>>(f, g, D, err);
-  } else {
-    ::msc::count_launch();
-    lstar_kernel<2, BS><<<grid, BS, 0, stream>>>(f, g, D, err);
-  }
-  return cudaGetLastError();
+  return nd == 3 ? launch_lstar_nd<3>(f, g, D, err, stream) : launch_lstar_nd<2>(f, g, D, err, stream);
 }
 
 cudaError_t make_lstar_batch(int n, const float* const* f, uint8_t* const* g, const GradDims* D, LstarBatch* B) {
@@ -163,10 +224,11 @@ cudaError_t make_lstar_batch(int n, const float* const* f, uint8_t* const* g, co
     v.f = f[i];
     v.g = g[i];
     v.D = D[i];
-    v.gx = (int)((D[i].v[0] + 31) / 32);
-    v.gy = (int)((D[i].v[1] + kLstarBS / 32 - 1) / (kLstarBS / 32));
+    using T = LstarTile<3>;
+    v.gx = (int)((D[i].v[0] + T::BX - 1) / T::BX);
+    v.gy = (int)((D[i].v[1] + T::BY - 1) / T::BY);
     v.block0 = off;
-    off += (int64_t)v.gx * v.gy * D[i].v[2];
+    off += (int64_t)v.gx * v.gy * ((D[i].v[2] + T::BZ - 1) / T::BZ);
   }
   B->total_blocks = off;
   return cudaSuccess;
@@ -176,8 +238,9 @@ cudaError_t launch_lstar_batch(const LstarBatch& B, int* err, int num_sms, cudaS
   const int64_t cap = (int64_t)num_sms * blocks_per_sm;
   const int grid = (int)(B.total_blocks < cap ? B.total_blocks : cap);
   if (grid <= 0) return cudaSuccess;
+  if (cudaError_t e = allow_smem(lstar_batch_kernel, sizeof(LstarSmem<3>))) return e;
   ::msc::count_launch();
-  lstar_batch_kernel<kLstarBS><<<grid, kLstarBS, 0, stream>>>(B, err);
+  lstar_batch_kernel<<<grid, kLstarBS, sizeof(LstarSmem<3>), stream>>>(B, err);
   return cudaGetLastError();
 }
 

@@ -77,3 +77,15 @@ def test_tile_edges_and_byte_alignment(gpu, oracle, shape, offset):
     lower_star_grad(torch.from_numpy(f).to(gpu), out)
     assert np.array_equal(out.cpu().numpy(), want)
     assert bool((buf[:offset] == 0xA5).all()) and bool((buf[offset + want.size:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("shape", [(33, 9, 10), (67, 40)], ids=lambda s: "x".join(map(str, s)))
+def test_zeros_and_infinities(gpu, oracle, shape):
+    """Both zeros, infinities, a denormal and the largest values, many of them equal: the
+    order is by value, then index."""
+    import torch
+    from msceer_gb300 import lower_star_grad
+    rng = np.random.default_rng(7)
+    vals = np.array([0.0, -0.0, np.inf, -np.inf, 1.0, -1e-42, 3e38, -3e38], dtype=np.float32)
+    f = rng.choice(vals, size=shape[::-1])
+    assert np.array_equal(lower_star_grad(torch.from_numpy(f).to(gpu)).cpu().numpy(), oracle.grad(f))

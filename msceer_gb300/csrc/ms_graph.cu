@@ -17,12 +17,15 @@
 //          an arc twice.  persistence = value(upper) - value(lower) (createArcFromNodeIDs).
 //
 // GPU form: an ordered compaction of the critical cells (block counts, one scan, an
-// ordered write), one thread per node for the attributes, and two depth-first passes
-// per node thread -- one counts its arcs, a scan places them, one writes them -- with
-// an explicit task stack: a visited cell pushes its children (arc ends and cells to
-// visit) in reverse facet order, so a path without branches keeps the stack flat.
+// ordered write, and a bitmap with the rank of every 32 cells, so that the node of a cell
+// is one load and a popcount), one thread per node for the attributes, and one
+// depth-first trace per node thread that counts its arcs and keeps them; a scan places
+// them and a copy puts them there.  The trace has an explicit task stack: a visited cell
+// goes on with its first child in a register and pushes the others (arc ends and cells
+// to visit) in reverse facet order, so a path without branches leaves the stack alone.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -159,13 +162,19 @@ __global__ void __launch_bounds__(kScanThreads) chunk_scan_kernel(T* __restrict_
   if (i < n) a[i] = offs[blockIdx.x] + off;
 }
 
+// The nodes in cell order, and for every 32 cells their critical bits and the number of
+// critical cells before them.
 __global__ void __launch_bounds__(kCritThreads) crit_write_kernel(const uint8_t* __restrict__ g, int64_t ncells,
                                                                   const int64_t* __restrict__ offsets,
-                                                                  int64_t* __restrict__ node_cell) {
+                                                                  int64_t* __restrict__ node_cell,
+                                                                  uint2* __restrict__ index) {
   __shared__ int64_t s_warp[32];
   const int64_t base = (int64_t)blockIdx.x * kCritChunk + (int64_t)threadIdx.x * kCritPerThread;
   uint32_t m = crit_bits(g, ncells, base);
   int64_t o = offsets[blockIdx.x] + block_excl_scan<int64_t>(__popc(m), s_warp, nullptr);
+  // two threads' cells make a word (the index is as long as the blocks' cells)
+  const uint32_t hi = __shfl_down_sync(0xffffffffu, m, 1);
+  if ((threadIdx.x & 1) == 0) index[base >> 5] = make_uint2(m | (hi << 16), (uint32_t)o);
   while (m) {
     const int k = __ffs(m) - 1;
     m &= m - 1;
@@ -204,128 +213,196 @@ __global__ void node_attr_kernel(const MsMesh M, const int64_t* __restrict__ nod
   }
 }
 
-__device__ __forceinline__ int64_t node_of(const int64_t* __restrict__ node_cell, int64_t n, int64_t cell) {
-  int64_t lo = 0, hi = n - 1;
-  while (lo <= hi) {
-    const int64_t mid = (lo + hi) >> 1;
-    const int64_t v = node_cell[mid];
-    if (v == cell) return mid;
-    if (v < cell) lo = mid + 1; else hi = mid - 1;
-  }
-  return -1;
+// the node of a critical cell (fewer than 2^31 nodes)
+__device__ __forceinline__ int32_t node_of(const uint2* __restrict__ index, int64_t cell) {
+  const uint2 w = __ldg(index + (cell >> 5));
+  return (int32_t)(w.y + (uint32_t)__popc(w.x & ((1u << (cell & 31)) - 1u)));
 }
 
-// One node's trace (rec_tdcr_candidates): counts its arcs, or writes them from `out`.
-// Returns 0, kErrLocalQueue if the task stack overflowed, kErrIterLimit past kMaxVisits.
-template <bool WRITE>
-__device__ int trace_node(const MsMesh& M, const int64_t* __restrict__ node_cell, int64_t n, int64_t node,
-                           int64_t* count, int64_t out, const float* __restrict__ value, int32_t* __restrict__ lower,
-                           int32_t* __restrict__ upper, float* __restrict__ pers) {
-  const int64_t start = node_cell[node];
+// One node's trace (rec_tdcr_candidates): calls emit(critical cell) for every arc in
+// order.  Returns 0, kErrLocalQueue if the task stack overflowed, kErrIterLimit past
+// kMaxVisits.
+template <class Emit>
+__device__ __forceinline__ int trace_node(const MsMesh& M, int64_t start, const Emit& emit) {
   const int temp_dim = ldir(M.g[start]) + 1;
-  int64_t stack[kStack];
+  int64_t stack[kStack + 6];  // a visit's children are pushed before they are counted
   int sp = 0;
-  stack[sp++] = start;
-  int64_t k = 0, visits = 0;
-  while (sp > 0) {
-    const int64_t t = stack[--sp];
-    if (t & kEmit) {
-      if (WRITE) {
-        const int64_t lo = node_of(node_cell, n, t & ~kEmit);
-        lower[out + k] = (int32_t)lo;
-        upper[out + k] = (int32_t)node;
-        if (pers) pers[out + k] = value[node] - value[lo];
-      }
-      k++;
-      continue;
-    }
+  int64_t t = start, visits = 0;
+  while (true) {
     if (++visits > kMaxVisits) return kErrIterLimit;
     int64_t c[3];
     coords(M, t, c);
     const int dim = dim_of(c);
-    int64_t child[6];
-    int nc = 0;
+    // the facets' bytes together
+    uint8_t fb[6];
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
+    for (int j = 0; j < 6; j++) {
+      const int a = j >> 1;
+      fb[j] = 0;
+      if (c[a] & 1) fb[j] = M.g[(j & 1) ? t - M.cs[a] : t + M.cs[a]];
+    }
+    // the children, last facet first: the first one stays in `next`
+    int64_t next = -1;
+    int pending = sp;
+#pragma unroll
+    for (int j = 5; j >= 0; j--) {
+      const int a = j >> 1;
       if (!(c[a] & 1)) continue;
-#pragma unroll
-      for (int s = 0; s < 2; s++) {
-        const int64_t fc = s == 0 ? t + M.cs[a] : t - M.cs[a];
-        const uint8_t b = M.g[fc];
-        const unsigned code = (b >> 2) & 7u;
-        if (code == 7u) {
-          child[nc++] = fc | kEmit;
-        } else if (code < 6u && ldir(b) == temp_dim) {
-          // the pair: the cell at the code's stride (UncompressByteTo6NeighborOffset;
-          // with a single-vertex axis two axes share a stride and the code names the
-          // first), inside the array for any byte
-          const int64_t p = (code & 1u) ? fc - M.cs[code >> 1] : fc + M.cs[code >> 1];
-          if (p == t || p < 0 || p >= M.ncells) continue;
+      const int64_t fc = (j & 1) ? t - M.cs[a] : t + M.cs[a];
+      const unsigned code = (fb[j] >> 2) & 7u;
+      int64_t child = -1;
+      if (code == 7u) {
+        child = fc | kEmit;
+      } else if (code < 6u && ldir(fb[j]) == temp_dim) {
+        // the pair: the cell at the code's stride (UncompressByteTo6NeighborOffset;
+        // with a single-vertex axis two axes share a stride and the code names the
+        // first), inside the array for any byte
+        const int64_t st = code < 2u ? M.cs[0] : (code < 4u ? M.cs[1] : M.cs[2]);
+        const int64_t p = (code & 1u) ? fc - st : fc + st;
+        if (p != t && p >= 0 && p < M.ncells) {
           int64_t pc[3];
           coords(M, p, pc);
-          if (dim_of(pc) == dim) child[nc++] = p;
+          if (dim_of(pc) == dim) child = p;
         }
       }
+      if (child < 0) continue;
+      pending++;
+      if (next >= 0) stack[sp++] = next;
+      next = child;
     }
-    if (sp + nc > kStack) return kErrLocalQueue;
-    for (int i = nc - 1; i >= 0; i--) stack[sp++] = child[i];
+    if (pending > kStack) return kErrLocalQueue;
+    // arcs end here; go on at the first cell
+    while (true) {
+      if (next < 0) {
+        if (sp == 0) return 0;
+        next = stack[--sp];
+      }
+      if (!(next & kEmit)) break;
+      emit(next & ~kEmit);
+      next = -1;
+    }
+    t = next;
   }
-  *count = k;
-  return 0;
 }
 
 // The nodes whose arcs are traced (dimension d >= 1 with build bit d - 1), listed so
-// that the tracing threads of a warp all trace (in cell order a warp's nodes mix all
-// four dimensions, and minima and unbuilt dimensions left most lanes idle).
+// that the tracing threads of a warp all trace, and trace alike: in cell order a warp's
+// nodes mix all four dimensions, minima and unbuilt dimensions left most lanes idle, and
+// a saddle's two paths waited for a maximum's tree of them.  Maxima go into list[0, n)
+// from the back (n_list[1] of them), the others from the front (n_list[0]).
 __global__ void traced_list_kernel(const MsMesh M, const int64_t* __restrict__ node_cell, int64_t n, int build,
                                    int32_t* __restrict__ list, unsigned long long* __restrict__ n_list) {
   const int lane = threadIdx.x & 31;
   for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = i0 + threadIdx.x;
-    bool want = false;
+    int d = 0;
     if (i < n) {
       int64_t c[3];
       coords(M, node_cell[i], c);
-      const int d = dim_of(c);
-      want = d > 0 && ((build >> (d - 1)) & 1);
+      d = dim_of(c);
+      if (d > 0 && !((build >> (d - 1)) & 1)) d = 0;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, want);
-    if (!m) continue;
-    const int leader = __ffs(m) - 1;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const bool want = q == 0 ? d == 1 || d == 2 : d == 3;
+      const unsigned m = __ballot_sync(0xffffffffu, want);
+      if (!m) continue;
+      const int leader = __ffs(m) - 1;
+      unsigned long long base = 0;
+      if (lane == leader) base = atomicAdd(&n_list[q], (unsigned long long)__popc(m));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      const int64_t at = (int64_t)base + __popc(m & ((1u << lane) - 1u));
+      if (want) list[q == 0 ? at : n - 1 - at] = (int32_t)i;
+    }
+  }
+}
+// the j-th node to trace: maxima first (their traces are the longest)
+__device__ __forceinline__ int64_t traced_node(const int32_t* __restrict__ list, int64_t n, int64_t n_max, int64_t j) {
+  return j < n_max ? list[n - 1 - j] : list[j - n_max];
+}
+
+// Counts every traced node's arcs; with `store` set, also keeps them (lower node ids):
+// the arcs of a warp's nodes in one stretch of store[0, store_cap), place[j] the first of
+// list entry j's.  A node with more arcs than its thread keeps, or whose warp found the
+// store full, gets place -1 and is traced again by the write.
+constexpr int kKeep = 64;  // arcs a thread keeps
+template <bool STORE>
+__global__ void __launch_bounds__(128) arc_trace_kernel(const MsMesh M, const int64_t* __restrict__ node_cell,
+                                                        int64_t n, const uint2* __restrict__ index,
+                                                        const int32_t* __restrict__ list,
+                                                        const unsigned long long* __restrict__ n_list,
+                                                        int64_t* __restrict__ counts, int32_t* __restrict__ store,
+                                                        unsigned long long* __restrict__ n_store,
+                                                        unsigned long long store_cap, int64_t* __restrict__ place,
+                                                        int* __restrict__ err) {
+  const int64_t n_max = (int64_t)n_list[1], nl = (int64_t)n_list[0] + n_max;
+  const int lane = threadIdx.x & 31;
+  for (int64_t j0 = blockIdx.x * (int64_t)blockDim.x; j0 < nl; j0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = j0 + threadIdx.x;
+    int32_t keep[STORE ? kKeep : 1];
+    int k = 0;
+    if (j < nl) {
+      const int64_t i = traced_node(list, n, n_max, j);
+      const int e = trace_node(M, node_cell[i], [&](int64_t cell) {
+        if (STORE && k < kKeep) keep[k] = node_of(index, cell);
+        k++;
+      });
+      if (e) {
+        atomicOr(err, e);
+        k = 0;
+      }
+      counts[i] = k;
+    }
+    if (!STORE) continue;
+    const int mine = k <= kKeep ? k : 0;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
     unsigned long long base = 0;
-    if (lane == leader) base = atomicAdd(n_list, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    if (want) list[base + __popc(m & ((1u << lane) - 1u))] = (int32_t)i;
+    if (lane == 31 && total > 0) base = atomicAdd(n_store, (unsigned long long)total);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (j >= nl) continue;
+    const bool fits = k <= kKeep && base + (unsigned long long)total <= store_cap;
+    const int64_t at = (int64_t)base + incl - mine;
+    place[j] = fits ? at : -1;
+    if (fits)
+      for (int q = 0; q < k; q++) store[at + q] = keep[q];
   }
 }
 
-__global__ void arc_count_kernel(const MsMesh M, const int64_t* __restrict__ node_cell, int64_t n,
-                                 const int32_t* __restrict__ list, const unsigned long long* __restrict__ n_list,
-                                 int64_t* __restrict__ counts, int* __restrict__ err) {
-  const int64_t nl = (int64_t)*n_list;
+// The kept arcs to their places.
+__global__ void __launch_bounds__(128) arc_write_kernel(const MsMesh M, const int64_t* __restrict__ node_cell,
+                                                        const uint2* __restrict__ index,
+                                                        const int32_t* __restrict__ list,
+                                                        const unsigned long long* __restrict__ n_list,
+                                                        const int64_t* __restrict__ offsets, int64_t n, int64_t n_arcs,
+                                                        const int32_t* __restrict__ store,
+                                                        const int64_t* __restrict__ place,
+                                                        const float* __restrict__ value, int32_t* __restrict__ lower,
+                                                        int32_t* __restrict__ upper, float* __restrict__ pers,
+                                                        int* __restrict__ err) {
+  const int64_t n_max = (int64_t)n_list[1], nl = (int64_t)n_list[0] + n_max;
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nl; j += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = list[j];
-    int64_t k = 0;
-    const int e = trace_node<false>(M, node_cell, n, i, &k, 0, nullptr, nullptr, nullptr, nullptr);
-    if (e) {
-      atomicOr(err, e);
-      k = 0;
+    const int64_t i = traced_node(list, n, n_max, j);
+    const int64_t out = offsets[i], at = place[j];
+    const float v = value[i];
+    auto put = [&](int64_t o, int32_t lo) {
+      lower[o] = lo;
+      upper[o] = (int32_t)i;
+      if (pers) pers[o] = v - value[lo];
+    };
+    if (at >= 0) {
+      const int64_t end = i + 1 < n ? offsets[i + 1] : n_arcs;
+      for (int64_t o = out; o < end; o++) put(o, store[at + (o - out)]);
+    } else {
+      int64_t o = out;
+      const int e = trace_node(M, node_cell[i], [&](int64_t cell) { put(o++, node_of(index, cell)); });
+      if (e) atomicOr(err, e);
     }
-    counts[i] = k;
-  }
-}
-
-__global__ void arc_write_kernel(const MsMesh M, const int64_t* __restrict__ node_cell, int64_t n,
-                                 const int32_t* __restrict__ list, const unsigned long long* __restrict__ n_list,
-                                 const int64_t* __restrict__ offsets, const float* __restrict__ value,
-                                 int32_t* __restrict__ lower, int32_t* __restrict__ upper, float* __restrict__ pers,
-                                 int* __restrict__ err) {
-  const int64_t nl = (int64_t)*n_list;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nl; j += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = list[j];
-    int64_t k = 0;
-    const int e = trace_node<true>(M, node_cell, n, i, &k, offsets[i], value, lower, upper, pers);
-    if (e) atomicOr(err, e);
   }
 }
 
@@ -426,21 +503,39 @@ int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const i
     GCUDA(P.get((void**)&cells, (size_t)n * sizeof(int64_t)), "scratch alloc(node cells)");
     GCUDA(P.get((void**)&vals, (size_t)n * sizeof(float)), "scratch alloc(node values)");
   }
+  uint2* index = nullptr;  // (a whole number of words for every block)
+  GCUDA(P.get((void**)&index, (size_t)nblk * (kCritChunk / 32) * sizeof(uint2)), "scratch alloc(node index)");
   count_launch();
-  crit_write_kernel<<<(unsigned)nblk, kCritThreads, 0, stream>>>(g, D.ncells, blk, cells);
+  crit_write_kernel<<<(unsigned)nblk, kCritThreads, 0, stream>>>(g, D.ncells, blk, cells, index);
   int64_t* acnt = nullptr;
   int32_t* tlist = nullptr;
   unsigned long long* n_tlist = nullptr;
   GCUDA(P.get((void**)&acnt, (size_t)n * sizeof(int64_t)), "scratch alloc(arc counts)");
   GCUDA(P.get((void**)&tlist, (size_t)n * sizeof(int32_t)), "scratch alloc(traced nodes)");
-  GCUDA(P.get((void**)&n_tlist, sizeof(unsigned long long)), "scratch alloc(traced count)");
+  GCUDA(P.get((void**)&n_tlist, 3 * sizeof(unsigned long long)), "scratch alloc(traced and kept counts)");
+  // room for two arcs a node of any dimension (rough fields have 1.5 with extractmsc's
+  // flags; what does not fit is traced again)
+  const bool want_arcs = arc_lower && arc_upper && arc_cap > 0;
+  const int64_t store_cap = want_arcs ? std::min<int64_t>(arc_cap, 2 * n + 4096) : 0;
+  int32_t* store = nullptr;
+  int64_t* place = nullptr;
+  if (want_arcs) {
+    GCUDA(P.get((void**)&store, (size_t)store_cap * sizeof(int32_t)), "scratch alloc(kept arcs)");
+    GCUDA(P.get((void**)&place, (size_t)n * sizeof(int64_t)), "scratch alloc(arc places)");
+  }
   GCUDA(cudaMemsetAsync(acnt, 0, (size_t)n * sizeof(int64_t), stream), "cudaMemsetAsync(arc counts)");
-  GCUDA(cudaMemsetAsync(n_tlist, 0, sizeof(unsigned long long), stream), "cudaMemsetAsync(traced count)");
+  GCUDA(cudaMemsetAsync(n_tlist, 0, 3 * sizeof(unsigned long long), stream), "cudaMemsetAsync(traced count)");
   if (n > 0) {
     count_launch();
     traced_list_kernel<<<grid_for(n, 256), 256, 0, stream>>>(M, cells, n, bmask, tlist, n_tlist);
     count_launch();
-    arc_count_kernel<<<grid_for(n, 128), 128, 0, stream>>>(M, cells, n, tlist, n_tlist, acnt, err);
+    if (want_arcs)
+      arc_trace_kernel<true><<<grid_for(n, 128), 128, 0, stream>>>(M, cells, n, index, tlist, n_tlist, acnt, store,
+                                                                  n_tlist + 2, (unsigned long long)store_cap, place,
+                                                                  err);
+    else
+      arc_trace_kernel<false><<<grid_for(n, 128), 128, 0, stream>>>(M, cells, n, index, tlist, n_tlist, acnt, nullptr,
+                                                                   nullptr, 0ull, nullptr, err);
   }
   if (int rc = scan_in_place(P, acnt, n, sums + 1, stream)) return rc;
   GCUDA(cudaGetLastError(), "arc count launch");
@@ -466,10 +561,10 @@ int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const i
     count_launch();
     node_attr_kernel<<<grid_for(n, 256), 256, 0, stream>>>(M, cells, n, vals, dims_b, bnd_b);
   }
-  if (arcs_out && n > 0) {
+  if (arcs_out && na > 0) {
     count_launch();
-    arc_write_kernel<<<grid_for(n, 128), 128, 0, stream>>>(M, cells, n, tlist, n_tlist, acnt, vals, arc_lower,
-                                                           arc_upper, arc_pers, err);
+    arc_write_kernel<<<grid_for(n, 128), 128, 0, stream>>>(M, cells, index, tlist, n_tlist, acnt, n, na, store, place,
+                                                           vals, arc_lower, arc_upper, arc_pers, err);
   }
   GCUDA(cudaGetLastError(), "node / arc write launch");
   GCUDA(cudaMemcpyAsync(&st, err, sizeof(int), cudaMemcpyDeviceToHost, stream), "read status");

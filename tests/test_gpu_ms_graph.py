@@ -89,3 +89,19 @@ def test_ms_graph_counts_only_then_fill(gpu):
     # every arc joins a node to one a dimension lower
     assert bool((dim[lo.long()].int() + 1 == dim[up.long()].int()).all())
     assert num_cells(f.shape[::-1]) == g.numel()
+
+
+@pytest.mark.parametrize("noise", [0.0, 8.0, 60.0])
+@pytest.mark.parametrize("shape", [(2, 2, 2), (17, 9, 16), (1, 40, 33), (40, 33, 30)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_ms_graph_one_peak_vs_oracle(gpu, oracle, shape, noise):
+    """Cell counts around the words and blocks of the node index, and one peak under noise:
+    nodes with far more arcs than a tracing thread keeps (up to 1,647 at 40x33x30), and more
+    arcs than the room for kept ones."""
+    z, y, x = np.meshgrid(*[np.arange(n, dtype=np.float64) for n in shape[::-1]], indexing="ij")
+    f = -((x - 0.5 * shape[0]) ** 2 + (y - 0.5 * shape[1]) ** 2 + (z - 0.5 * shape[2]) ** 2).astype(np.float32)
+    f += np.random.default_rng(3).uniform(-noise, noise, size=f.shape).astype(np.float32)
+    g, got = _device_graph(gpu, f, (1, 1, 1))
+    want = oracle.ms_graph(f, g.cpu().numpy(), (1, 1, 1))
+    for k, v in want.items():
+        assert np.array_equal(got[k].cpu().numpy(), v), k

@@ -456,28 +456,32 @@ __global__ void __launch_bounds__(kCompactThreads) spread_write_kernel(const Spr
     if (vx[j] >= 0) items[o++] = (int32_t)vx[j];
 }
 
-// Walks an item's entries in order.
-struct SeqWalk {
-  const SpecSet& Q;
-  int64_t k;
-  uint32_t seg = 0;
-  int i = 0;
-  __device__ __forceinline__ SeqWalk(const SpecSet& q, int64_t item) : Q(q), k(item) {}
-  __device__ __forceinline__ uint32_t next() {
-    const int j = i++;
-    if (j == 0) return (uint32_t)Q.vtx[k] | kRec;
-    if (j == 1) return Q.e1[k];
-    const int p = j - 2;
-    if (p == 0) seg = Q.head[k];
-    else if ((p & (kSeg - 1)) == 0) seg = Q.pool[seg + kSeg];
-    return Q.pool[seg + (p & (kSeg - 1))];
-  }
-};
+// An item's entries.  The first kNear are read at once (the pool reads do not wait for one
+// another); farther ones lie in segments, reached by their links.
+constexpr int kNear = 8;
+__device__ __forceinline__ void near_entries(const SpecSet& Q, int64_t k, int n, uint32_t u[kNear]) {
+  const uint32_t seg = n > 2 ? Q.head[k] : 0u;
+  u[0] = (uint32_t)Q.vtx[k] | kRec;
+  u[1] = n > 1 ? Q.e1[k] : 0u;
+#pragma unroll
+  for (int e = 2; e < kNear; e++) u[e] = e < n ? Q.pool[seg + (e - 2)] : 0u;
+}
+// word offset of the segment that holds entry e >= 2
+__device__ __forceinline__ uint32_t segment_of(const SpecSet& Q, int64_t k, int e) {
+  uint32_t seg = Q.head[k];
+  for (int s = (e - 2) / kSeg; s > 0; s--) seg = Q.pool[seg + kSeg];
+  return seg;
+}
+__device__ __forceinline__ uint32_t entry_of(const SpecSet& Q, int64_t k, int e) {
+  if (e == 0) return (uint32_t)Q.vtx[k] | kRec;
+  if (e == 1) return Q.e1[k];
+  return Q.pool[segment_of(Q, k, e) + ((e - 2) & (kSeg - 1))];
+}
 
 // Speculative streamlines of items [k0, k1) of the ordered list: they stop only at
-// vertices labelled before this batch (lvl < A.level), record their entries with a
-// holder node per entry, and make the first round's claims (every item alive, its
-// whole path effective).
+// vertices labelled before this batch (lvl < A.level), record their entries, count them
+// at their vertices, and make the first round's claims (every item alive, its whole path
+// effective).
 template <int K>
 __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const SpecSet Q, int64_t k0, int64_t k1,
                                                            const int32_t* __restrict__ lab,
@@ -523,6 +527,7 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
           if (A.lvl[i] < level) {  // labelled by an earlier batch of this group
             Q.alive[k] = 0;
             Q.len[k] = 0;
+            Q.ext[k] = 0;
           } else {
             split_index(V, i, x, y, z);
             cur = {(float)x, (float)y, (float)z};
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
       }
     }
     // flush: an ended streamline writes the rest of its entries, a long one a full
-    // segment (+ its link word); one pool and one holder-node allocation per warp and
+    // segment (+ its link word); one pool allocation and one count of the entries per warp and
     // turn.  A segment is flushed early only with an entry to spare (an ending marks the
     // last entry).
     const bool ending = phase == kLaneEnd;
@@ -607,14 +612,11 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
         continue;
       }
     }
-    // a recorded entry: its holder node (and, for a path vertex, the first round's claim)
-    int32_t node = (int32_t)(nbase + (unsigned long long)(nincl - nodes));
-    auto hold = [&](uint32_t u, int idx) {
+    // a recorded entry: counted at its vertex (and, for a path vertex, the first round's
+    // claim)
+    auto hold = [&](uint32_t u) {
       const uint32_t v = u & ~kRec;
-      Q.hitem[node] = (int32_t)k;
-      Q.hidx[node] = (uint32_t)idx | (u & kRec);
-      Q.hnext[node] = atomicExch(&Q.hhead[v], node);
-      node++;
+      atomicAdd(&Q.hcount[v], 1);
       if (u & kRec) atomicMin(&claim[v], (uint32_t)k);
     };
     if (words > 0) {
@@ -624,14 +626,14 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
       const int seg = nb > kSeg ? kSeg : nb;  // entries of the segment written now
       for (int e = 0; e < seg; e++) {
         Q.pool[off + e] = buf[e];
-        hold(buf[e], 2 + flushed + e);
+        hold(buf[e]);
       }
       if (ending) {
         if (nb > kSeg) {  // the rest follows the full segment's link word
           Q.pool[off + kSeg] = off + kSeg + 1;
           for (int e = kSeg; e < nb; e++) {
             Q.pool[off + 1 + e] = buf[e];
-            hold(buf[e], 2 + flushed + e);
+            hold(buf[e]);
           }
         }
       } else {
@@ -642,15 +644,70 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
       }
     }
     if (ending) {
-      hold((uint32_t)Q.vtx[k] | kRec, 0);
-      if (cnt >= 2) hold(e1, 1);
+      hold((uint32_t)Q.vtx[k] | kRec);
+      if (cnt >= 2) hold(e1);
       Q.e1[k] = e1;
       Q.len[k] = cnt;
       Q.endlab[k] = endlab;
       Q.alive[k] = 1;
       Q.cut[k] = -1;
+      Q.ext[k] = cnt;
       nb = 0;
       phase = kLaneIdle;
+    }
+  }
+}
+
+// The batch's holders by vertex: every counted vertex gets a range of Q.holders
+// (spec_range_kernel), and every item's entries are put into their vertices' ranges in
+// whatever order they come (spec_fill_kernel), which counts the vertices' counts down to
+// zero again.
+__global__ void __launch_bounds__(256) spec_range_kernel(const int32_t* __restrict__ count, int64_t N,
+                                                         int2* __restrict__ range, int* __restrict__ cursor) {
+  __shared__ int s_part[kAppendWarps + 1];
+  const int64_t n4 = (N + 3) / 4;  // (count holds a multiple of four)
+  for (int64_t b0 = blockIdx.x * (int64_t)blockDim.x; b0 < n4; b0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = b0 + threadIdx.x;  // (block-uniform trips: block_append)
+    const int4 c = i < n4 ? reinterpret_cast<const int4*>(count)[i] : make_int4(0, 0, 0, 0);
+    int at = block_append(c.x + c.y + c.z + c.w, cursor, s_part);
+    const int cc[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (cc[q] == 0) continue;
+      range[4 * i + q] = make_int2(at, cc[q]);
+      at += cc[q];
+    }
+  }
+}
+__global__ void __launch_bounds__(256) spec_fill_kernel(const SpecSet Q, int64_t k0, int64_t k1) {
+  const int lane = threadIdx.x & 31;
+  auto put = [&](uint32_t u, int64_t k, int e) {
+    const uint32_t v = u & ~kRec;
+    const int at = Q.hrange[v].x + atomicSub(&Q.hcount[v], 1) - 1;
+    Q.holders[at] = make_int2((int32_t)k, (int32_t)((uint32_t)e | (u & kRec)));
+  };
+  for (int64_t b0 = k0 + blockIdx.x * (int64_t)blockDim.x; b0 < k1; b0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = b0 + threadIdx.x;  // (warp-uniform trips)
+    const int n = k < k1 ? Q.len[k] : 0;
+    if (n > 0) {
+      uint32_t u[kNear];
+      near_entries(Q, k, n, u);
+#pragma unroll
+      for (int e = 0; e < kNear; e++)
+        if (e < n) put(u[e], k, e);
+    }
+    unsigned far = __ballot_sync(kFullMask, n > kNear);
+    while (far) {  // the rest of the long sequences, a segment at a time
+      const int src = __ffs(far) - 1;
+      far &= far - 1;
+      const int64_t fk = __shfl_sync(kFullMask, k, src);
+      const int fn = __shfl_sync(kFullMask, n, src);
+      uint32_t seg = Q.head[fk];
+      for (int e0 = 2; e0 < fn; e0 += kSeg) {
+        const int e = e0 + lane;
+        if (e >= kNear && e < fn) put(Q.pool[seg + lane], fk, e);
+        if (e0 + kSeg < fn) seg = Q.pool[seg + kSeg];
+      }
     }
   }
 }
@@ -688,46 +745,81 @@ __device__ __forceinline__ void mark_dirty(bool want, uint32_t v, uint32_t* __re
 // New alive / cut of item t of the batch (t < 0: none; every lane of the warp calls it)
 // from the claims.  A changed item marks the path vertices between its old and new
 // extent in nxt: their claims are recomputed next round.
+// A lane looks at its item's first kNear entries, read together; what is left of the long
+// ones the warp takes up together, a segment of 32 entries at a time.  (A lane that
+// walked its sequence alone waited for two dependent reads per entry, and its warp and
+// round with it: ~150 us a round on Gaussian-sum fields, whose sequences run to hundreds
+// of entries; 90 of the 300 ms that the kernels of 64^3 labels took one after another.)
 __device__ __forceinline__ void check_item(const SpecSet& Q, int64_t k0, int64_t t, const uint32_t* __restrict__ claim,
                                            uint32_t* __restrict__ nxt, uint32_t* __restrict__ nxt_list,
                                            unsigned long long* __restrict__ n_nxt) {
+  const int lane = threadIdx.x & 31;
   const int64_t k = k0 + (t >= 0 ? t : 0);
   const int n = t >= 0 ? Q.len[k] : 0;
-  const bool look = n > 0;
   uint8_t oa = 0, na = 0;
-  int oc = -1, nc = -1;
-  bool changed = false;
-  if (look) {
+  int oc = -1, nc = -1, old_ext = 0;
+  uint32_t u[kNear];
+  if (n > 0) {
     const uint32_t kk = (uint32_t)k;
     oa = Q.alive[k];
     oc = Q.cut[k];
-    na = claim[Q.vtx[k]] < kk ? 0 : 1;
-    SeqWalk w(Q, k);
-    w.next();
-    for (int e = 1; e < n; e++) {
-      const uint32_t v = w.next() & ~kRec;
-      if (claim[v] < kk) {
-        nc = e;
+    old_ext = Q.ext[k];
+    near_entries(Q, k, n, u);
+    uint32_t cl[kNear];
+#pragma unroll
+    for (int e = 0; e < kNear; e++) cl[e] = e < n ? claim[u[e] & ~kRec] : kNoClaim;
+    na = cl[0] < kk ? 0 : 1;
+#pragma unroll
+    for (int e = kNear - 1; e >= 1; e--)
+      if (cl[e] < kk) nc = e;
+  }
+  // the rest of the long sequences
+  unsigned far = __ballot_sync(kFullMask, n > kNear && nc < 0);
+  while (far) {
+    const int src = __ffs(far) - 1;
+    far &= far - 1;
+    const int64_t fk = __shfl_sync(kFullMask, k, src);
+    const int fn = __shfl_sync(kFullMask, n, src);
+    uint32_t seg = Q.head[fk];
+    int hit = -1;
+    for (int e0 = 2; e0 < fn; e0 += kSeg) {  // entries e0 .. e0 + 31 (the first kNear again)
+      const int e = e0 + lane;
+      const uint32_t w = e < fn ? Q.pool[seg + lane] : 0u;
+      if (e0 + kSeg < fn) seg = Q.pool[seg + kSeg];
+      const unsigned m = __ballot_sync(kFullMask, e < fn && claim[w & ~kRec] < (uint32_t)fk);
+      if (m) {
+        hit = e0 + __ffs(m) - 1;
         break;
       }
     }
-    changed = na != oa || nc != oc;
-    if (changed) {
-      Q.alive[k] = na;
-      Q.cut[k] = nc;
-    }
+    if (lane == src) nc = hit;
+  }
+  const bool changed = n > 0 && (na != oa || nc != oc);
+  const int xo = changed ? old_ext : 0, xn = changed ? spec_extent(na, nc, n) : 0;
+  if (changed) {
+    Q.alive[k] = na;
+    Q.cut[k] = nc;
+    Q.ext[k] = xn;
   }
   // the path vertices between the old and the new extent
-  const int xo = changed ? spec_extent(oa, oc, n) : 0, xn = changed ? spec_extent(na, nc, n) : 0;
   const int lo = xo < xn ? xo : xn, hi = xo < xn ? xn : xo;
-  int trips = hi;
+  if (!__any_sync(kFullMask, hi > lo)) return;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) trips = max(trips, __shfl_xor_sync(kFullMask, trips, o));
-  SeqWalk w(Q, k);
-  for (int e = 0; e < trips; e++) {
-    uint32_t u = 0;
-    if (e < hi) u = w.next();
-    mark_dirty(e >= lo && e < hi && (u & kRec), u & ~kRec, nxt, nxt_list, n_nxt);
+  for (int e = 0; e < kNear; e++)
+    mark_dirty(e >= lo && e < hi && (u[e] & kRec), u[e] & ~kRec, nxt, nxt_list, n_nxt);
+  far = __ballot_sync(kFullMask, hi > lo && hi > kNear);
+  while (far) {
+    const int src = __ffs(far) - 1;
+    far &= far - 1;
+    const int64_t fk = __shfl_sync(kFullMask, k, src);
+    const int flo = max(__shfl_sync(kFullMask, lo, src), kNear), fhi = __shfl_sync(kFullMask, hi, src);
+    int e0 = 2 + (flo - 2) / kSeg * kSeg;
+    for (uint32_t seg = segment_of(Q, fk, flo); e0 < fhi; e0 += kSeg) {
+      const int e = e0 + lane;
+      const uint32_t w = e >= flo && e < fhi ? Q.pool[seg + lane] : 0u;
+      if (e0 + kSeg < fhi) seg = Q.pool[seg + kSeg];
+      mark_dirty((w & kRec) != 0u, w & ~kRec, nxt, nxt_list, n_nxt);
+    }
   }
 }
 
@@ -735,7 +827,8 @@ __device__ __forceinline__ void check_item(const SpecSet& Q, int64_t k0, int64_t
 // round), or those whose bit is set in ibits (a bit per item from k0, ibits_words
 // words), each bit cleared as it is taken so that the bitmap is clear again after the
 // round.
-__global__ void spec_check_kernel(const SpecSet Q, int64_t k0, int64_t k1, const uint32_t* __restrict__ claim,
+__global__ void __launch_bounds__(256) spec_check_kernel(const SpecSet Q, int64_t k0, int64_t k1,
+                                  const uint32_t* __restrict__ claim,
                                   uint32_t* __restrict__ ibits, int64_t ibits_words, uint32_t* __restrict__ nxt,
                                   uint32_t* __restrict__ nxt_list, unsigned long long* __restrict__ n_nxt) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -748,45 +841,107 @@ __global__ void spec_check_kernel(const SpecSet Q, int64_t k0, int64_t k1, const
     }
     return;
   }
-  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x; w0 < ibits_words; w0 += stride) {
-    const int64_t wd = w0 + threadIdx.x;
+  // A warp takes a window of the bitmap, of as few words as gives every warp one, 32 at
+  // most.  Its lanes take a word each and the items set there one after another, or all a
+  // word's items at once, whichever are fewer turns: a small batch has few words, full of
+  // items.  (No shared memory for a list of them: a block that asks for some waits for an
+  // SM whose blocks of the other launches, which run on for the whole call, have ended --
+  // 392 -> 535 ms for the 512^3 labels.)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t nwarp = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t per = (ibits_words + nwarp - 1) / nwarp;
+  const int W = per < 1 ? 1 : (per < 32 ? (int)per : 32);
+  for (int64_t w0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + warp) * W; w0 < ibits_words; w0 += nwarp * W) {
     uint32_t m = 0;
-    if (wd < ibits_words) {
-      m = ibits[wd];
-      if (m) ibits[wd] = 0;
+    if (lane < W && w0 + lane < ibits_words) {
+      m = ibits[w0 + lane];
+      if (m) ibits[w0 + lane] = 0;
     }
-    while (__any_sync(kFullMask, m != 0)) {
-      int64_t t = -1;
-      if (m) {
-        t = wd * 32 + (__ffs(m) - 1);
-        m &= m - 1;
+    unsigned words = __ballot_sync(kFullMask, m != 0u);
+    int most = __popc(m);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(kFullMask, most, o));
+    if (__popc(words) < most) {
+      while (words) {
+        const int src = __ffs(words) - 1;
+        words &= words - 1;
+        const uint32_t all = __shfl_sync(kFullMask, m, src);
+        check_item(Q, k0, (all >> lane) & 1u ? (w0 + src) * 32 + lane : -1, claim, nxt, nxt_list, n_nxt);
       }
-      check_item(Q, k0, t, claim, nxt, nxt_list, n_nxt);
+    } else {
+      for (int j = 0; j < most; j++) {
+        int64_t t = -1;
+        if (m) {
+          t = (w0 + lane) * 32 + (__ffs(m) - 1);
+          m &= m - 1;
+        }
+        check_item(Q, k0, t, claim, nxt, nxt_list, n_nxt);
+      }
     }
   }
 }
 
-// The claims of a round's dirty vertices from their holders' current extents, the
-// holders marked in ibits for the round's check, and the vertices' dirty bits cleared
-// (the bitmap takes the next-but-one round's marks).
-__global__ void spec_reclaim_kernel(const SpecSet Q, int64_t k0, const uint32_t* __restrict__ list,
-                                    const unsigned long long* __restrict__ n_list, uint32_t* __restrict__ bits,
-                                    uint32_t* __restrict__ claim, uint32_t* __restrict__ ibits) {
-  const unsigned long long n = *n_list;
-  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n;
-       i += (unsigned long long)gridDim.x * blockDim.x) {
-    const uint32_t v = list[i];
-    atomicAnd(&bits[v >> 5], ~(1u << (v & 31)));
-    uint32_t m = kNoClaim;
-    for (int32_t h = Q.hhead[v]; h >= 0; h = Q.hnext[h]) {
-      const int32_t k = Q.hitem[h];
-      const int64_t t = k - k0;
-      atomicOr(&ibits[t >> 5], 1u << (t & 31));
-      const uint32_t ix = Q.hidx[h];
-      if (!(ix & kRec)) continue;
-      if ((int)(ix & ~kRec) < spec_extent(Q.alive[k], Q.cut[k], Q.len[k]) && (uint32_t)k < m) m = (uint32_t)k;
+// The claims of a round's dirty vertices from their holders' current extents, and the
+// vertices' dirty bits cleared (the bitmap takes the next-but-one round's marks).  An item
+// asks of a vertex only whether an earlier item claims it, so of a claim that moved from
+// one item to another only the holders after the earlier and up to the later one of the
+// two see a difference: those are marked in ibits for the round's check.
+// Eight lanes take a vertex, the whole warp one with a long list: on smooth fields
+// hundreds of streamlines run through a vertex, and following them as a linked list, a
+// read after a read, made a round of ~100 us.
+constexpr int kFewHolders = 64;
+__device__ __forceinline__ uint32_t claim_of(const SpecSet& Q, int at, int len, int lane, int step) {
+  uint32_t m = kNoClaim;
+  for (int j = lane; j < len; j += step) {
+    const int2 h = Q.holders[at + j];
+    const uint32_t ix = (uint32_t)h.y;
+    if ((ix & kRec) && (int)(ix & ~kRec) < Q.ext[h.x]) m = min(m, (uint32_t)h.x);
+  }
+  for (int o = step >> 1; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(kFullMask, m, o));
+  return m;
+}
+__device__ __forceinline__ void mark_holders(const SpecSet& Q, int at, int len, int lane, int step, uint32_t a,
+                                             uint32_t b, int64_t k0, uint32_t* __restrict__ ibits) {
+  const uint32_t lo = min(a, b), hi = max(a, b);
+  for (int j = lane; j < len; j += step) {
+    const uint32_t k = (uint32_t)Q.holders[at + j].x;
+    if (k <= lo || k > hi) continue;
+    const int64_t t = (int64_t)k - k0;
+    atomicOr(&ibits[t >> 5], 1u << (t & 31));
+  }
+}
+__global__ void __launch_bounds__(256) spec_reclaim_kernel(const SpecSet Q, int64_t k0,
+                                                           const uint32_t* __restrict__ list,
+                                                           const unsigned long long* __restrict__ n_list,
+                                                           uint32_t* __restrict__ bits, uint32_t* __restrict__ claim,
+                                                           uint32_t* __restrict__ ibits) {
+  const int64_t n = (int64_t)*n_list;
+  const int lane = threadIdx.x & 31, sub = lane & 7;
+  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 3);
+  // every lane of a warp makes the same trips
+  for (int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) >> 3; i0 < n; i0 += stride) {
+    const int64_t i = i0 + (lane >> 3);
+    const bool have = i < n;
+    const uint32_t v = have ? list[i] : 0u;
+    const int2 r = have ? Q.hrange[v] : make_int2(0, 0);
+    const uint32_t old = have ? claim[v] : 0u;
+    if (have && sub == 0) atomicAnd(&bits[v >> 5], ~(1u << (v & 31)));
+    const bool few = r.y <= kFewHolders;
+    const uint32_t m = claim_of(Q, r.x, few ? r.y : 0, sub, 8);
+    if (have && few) {
+      if (m != old) mark_holders(Q, r.x, r.y, sub, 8, old, m, k0, ibits);
+      if (sub == 0) claim[v] = m;
     }
-    claim[v] = m;
+    unsigned far = __ballot_sync(kFullMask, !few && sub == 0);
+    while (far) {
+      const int src = __ffs(far) - 1;
+      far &= far - 1;
+      const uint32_t fv = __shfl_sync(kFullMask, v, src), fo = __shfl_sync(kFullMask, old, src);
+      const int at = __shfl_sync(kFullMask, r.x, src), len = __shfl_sync(kFullMask, r.y, src);
+      const uint32_t fm = claim_of(Q, at, len, lane, 32);
+      if (fm != fo) mark_holders(Q, at, len, lane, 32, fo, fm, k0, ibits);
+      if (lane == 0) claim[fv] = fm;
+    }
   }
 }
 
@@ -796,12 +951,7 @@ __global__ void spec_ptr_kernel(const SpecSet Q, int64_t k0, int64_t k1, const u
     if (!Q.alive[k]) continue;
     const int ct = Q.cut[k];
     int32_t p = (int32_t)k;
-    if (ct >= 0) {
-      SeqWalk w(Q, k);
-      uint32_t u = 0;
-      for (int e = 0; e <= ct; e++) u = w.next();
-      p = (int32_t)claim[u & ~kRec];
-    }
+    if (ct >= 0) p = (int32_t)claim[entry_of(Q, k, ct) & ~kRec];
     Q.ptr[k] = p;
   }
 }
@@ -819,28 +969,56 @@ constexpr int kChainSteps = 64;
 __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8_t* __restrict__ lvl, int level,
                                   const uint32_t* __restrict__ claim, int32_t* __restrict__ lab,
                                   int* __restrict__ long_chain) {
-  for (int64_t k = k0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < k1; k += (int64_t)gridDim.x * blockDim.x) {
-    if (!Q.alive[k]) continue;
-    int32_t p = Q.ptr[k];
-    for (int s = 0; s < kChainSteps; s++) {
-      const int32_t q = Q.ptr[p];
-      if (q == p) break;
-      p = q;
+  const int lane = threadIdx.x & 31;
+  for (int64_t b0 = k0 + blockIdx.x * (int64_t)blockDim.x; b0 < k1; b0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = b0 + threadIdx.x;  // (warp-uniform trips)
+    int n = 0;
+    int32_t d = 0;
+    if (k < k1 && Q.alive[k]) {
+      int32_t p = Q.ptr[k];
+      for (int s = 0; s < kChainSteps; s++) {
+        const int32_t q = Q.ptr[p];
+        if (q == p) break;
+        p = q;
+      }
+      if (Q.ptr[p] != p) {
+        atomicExch(long_chain, 1);
+      } else {
+        d = Q.endlab[p];
+        n = Q.ext[k];
+      }
     }
-    if (Q.ptr[p] != p) {
-      atomicExch(long_chain, 1);
-      continue;
+    if (n > 0) {
+      uint32_t u[kNear], cl[kNear];
+      near_entries(Q, k, n, u);
+#pragma unroll
+      for (int e = 0; e < kNear; e++) cl[e] = e < n && (u[e] & kRec) ? claim[u[e] & ~kRec] : kNoClaim;
+#pragma unroll
+      for (int e = 0; e < kNear; e++)
+        if (cl[e] == (uint32_t)k) {
+          lab[u[e] & ~kRec] = d;
+          lvl[u[e] & ~kRec] = (uint8_t)level;
+        }
     }
-    const int32_t d = Q.endlab[p];
-    const int n = Q.cut[k] >= 0 ? Q.cut[k] : Q.len[k];
-    SeqWalk w(Q, k);
-    for (int e = 0; e < n; e++) {
-      const uint32_t u = w.next();
-      if (!(u & kRec)) continue;
-      const uint32_t v = u & ~kRec;
-      if (claim[v] == (uint32_t)k) {
-        lab[v] = d;
-        lvl[v] = (uint8_t)level;
+    // the rest of the long sequences, a segment at a time (as check_item)
+    unsigned far = __ballot_sync(kFullMask, n > kNear);
+    while (far) {
+      const int src = __ffs(far) - 1;
+      far &= far - 1;
+      const int64_t fk = __shfl_sync(kFullMask, k, src);
+      const int fn = __shfl_sync(kFullMask, n, src);
+      const int32_t fd = __shfl_sync(kFullMask, d, src);
+      uint32_t seg = Q.head[fk];
+      for (int e0 = 2; e0 < fn; e0 += kSeg) {
+        const int e = e0 + lane;
+        const uint32_t w = e >= kNear && e < fn ? Q.pool[seg + lane] : 0u;
+        if (e0 + kSeg < fn) seg = Q.pool[seg + kSeg];
+        if (!(w & kRec)) continue;
+        const uint32_t v = w & ~kRec;
+        if (claim[v] == (uint32_t)fk) {
+          lab[v] = fd;
+          lvl[v] = (uint8_t)level;
+        }
       }
     }
   }
@@ -1650,8 +1828,20 @@ cudaError_t launch_spec_round(const SpecSet& Q, int64_t k0, int64_t k1, uint32_t
   ::msc::count_launch();
   spec_reclaim_kernel<<<num_sms * 8, 256, 0, stream>>>(Q, k0, cur->list, cur->n, cur->bits, claim, ibits);
   ::msc::count_launch();
-  spec_check_kernel<<<grid_for(ibits_words, num_sms), 256, 0, stream>>>(Q, k0, k1, claim, ibits, ibits_words,
+  const int64_t blocks = (ibits_words + 7) / 8;  // a warp per word while there are fewer words than warps
+  const int grid = (int)(blocks < (int64_t)num_sms * 8 ? blocks : (int64_t)num_sms * 8);
+  spec_check_kernel<<<grid, 256, 0, stream>>>(Q, k0, k1, claim, ibits, ibits_words,
                                                                         nxt.bits, nxt.list, nxt.n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_spec_holders(const SpecSet& Q, int64_t k0, int64_t k1, int64_t N, int* cursor, int num_sms,
+                                cudaStream_t stream) {
+  if (cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(int), stream)) return e;
+  ::msc::count_launch();
+  spec_range_kernel<<<grid_for((N + 3) / 4, num_sms), 256, 0, stream>>>(Q.hcount, N, Q.hrange, cursor);
+  ::msc::count_launch();
+  spec_fill_kernel<<<grid_for(k1 - k0, num_sms), 256, 0, stream>>>(Q, k0, k1);
   return cudaGetLastError();
 }
 

@@ -137,19 +137,20 @@ struct SpecSet {
   int32_t* len;        // recorded entries (0: the item was skipped)
   int32_t* endlab;     // label where the streamline stopped, if labelled before the batch
   int32_t* cut;        // -1, or the entry where an earlier item's path stops it
+  int32_t* ext;        // effective extent: 0 if skipped, the cut, or len
   int32_t* ptr;        // the item whose label it takes
   uint8_t* alive;      // runs (no earlier item labelled its vertex)
   uint32_t* pool;      // entry segments
   unsigned long long pool_words;
   unsigned long long* cursor;  // next free pool word
   int* overflow;               // set when the pool or the holder nodes ran out (the batch is redone smaller)
-  // holders: for every vertex the list of (item, entry index) that recorded it
-  int32_t* hhead;              // per vertex: its first holder node, -1 for none
-  int32_t* hitem;              // per node: the item
-  uint32_t* hidx;              // per node: the entry index, kRec-flagged for path vertices
-  int32_t* hnext;              // per node: the vertex's next node
+  // holders: for every vertex the (item, entry index) that recorded it
+  int32_t* hcount;             // per vertex: its holders not placed yet (0 between batches; room for
+                               // a multiple of four)
+  int2* hrange;                // per vertex with holders: the first one in `holders`, and their number
+  int2* holders;               // the item, the entry index (kRec-flagged for path vertices)
   unsigned long long node_cap;
-  unsigned long long* ncursor;  // next free node
+  unsigned long long* ncursor;  // entries recorded
 };
 // lvl: 0 for labelled vertices, 255 for the rest
 cudaError_t launch_init_levels(const int32_t* lab, uint8_t* lvl, int64_t N, int num_sms, cudaStream_t stream);
@@ -161,7 +162,7 @@ cudaError_t launch_count_unlabelled(const uint8_t* lvl, int64_t N, unsigned long
 cudaError_t launch_spread_compact(const SpreadOrder& S, int64_t u0, int64_t u1, const uint8_t* lvl, int stamp,
                                   int* counts, int32_t* items, unsigned long long* n_items, cudaStream_t stream);
 // Speculative streamlines of items [k0, k1) (stopping at lvl < stamp); they build the
-// holder lists (hhead all -1 at launch) and make the first resolution round's claims.
+// holder counts (hcount all 0 at launch) and make the first resolution round's claims.
 // `work`: a device counter, zero at launch; `trips`: advection iterations are added to it.
 cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParams& P, const SpecSet& Q, int64_t k0,
                              int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, uint32_t* claim,
@@ -184,6 +185,9 @@ struct SpecDirty {
 // between rounds).  An item whose alive / cut changed marks the path vertices between
 // its old and new extent in nxt (whose bitmap must be clear).  The rounds end when a
 // round marks nothing; a round after that one finds no items and marks nothing.
+// The holder lists of the batch's recorded entries (hcount goes back to 0).
+cudaError_t launch_spec_holders(const SpecSet& Q, int64_t k0, int64_t k1, int64_t N, int* cursor, int num_sms,
+                                cudaStream_t stream);
 cudaError_t launch_spec_round(const SpecSet& Q, int64_t k0, int64_t k1, uint32_t* claim, const SpecDirty* cur,
                               const SpecDirty& nxt, uint32_t* ibits, int64_t ibits_words, int num_sms,
                               cudaStream_t stream);

@@ -580,7 +580,7 @@ int first_pass(LabelCtx& c, DirLabels& d) {
   int32_t* vtx;
   uint32_t* ibits;
   unsigned long long* sc;  // [0] pool cursor [1] items [3] claimed items [4, 6) dirty-list lengths
-                           // [6] holder-node cursor
+                           // [6] entries recorded
   msc::SpecSet Q{};
   const int64_t max_items = std::min<int64_t>(N, S.offset[S.nlev]);
   const int64_t ibits_cap = max_items / 32 + 1;
@@ -595,13 +595,14 @@ int first_pass(LabelCtx& c, DirLabels& d) {
   LCUDA(c.pool.get(&Q.len, max_items), "alloc");
   LCUDA(c.pool.get(&Q.endlab, max_items), "alloc");
   LCUDA(c.pool.get(&Q.cut, max_items), "alloc");
+  LCUDA(c.pool.get(&Q.ext, max_items), "alloc");
   LCUDA(c.pool.get(&Q.ptr, max_items), "alloc");
   LCUDA(c.pool.get(&Q.alive, max_items), "alloc");
   LCUDA(c.pool.get(&Q.pool, Q.pool_words), "alloc");
-  LCUDA(c.pool.get(&Q.hhead, N), "alloc");
-  LCUDA(c.pool.get(&Q.hitem, Q.node_cap), "alloc");
-  LCUDA(c.pool.get(&Q.hidx, Q.node_cap), "alloc");
-  LCUDA(c.pool.get(&Q.hnext, Q.node_cap), "alloc");
+  LCUDA(c.pool.get(&Q.hcount, (N + 3) / 4 * 4), "alloc");
+  LCUDA(c.pool.get(&Q.hrange, N), "alloc");
+  LCUDA(c.pool.get(&Q.holders, Q.node_cap), "alloc");
+  LCUDA(cudaMemsetAsync(Q.hcount, 0, (size_t)((N + 3) / 4 * 4) * sizeof(int32_t), st), "memset");  // (0 between batches)
   LCUDA(c.pool.get(&ibits, ibits_cap), "alloc");
   LCUDA(cudaMemsetAsync(ibits, 0, (size_t)ibits_cap * sizeof(uint32_t), st), "memset");  // (clear between rounds)
   LCUDA(c.pool.get(&sc, 8), "alloc");
@@ -661,7 +662,6 @@ int first_pass(LabelCtx& c, DirLabels& d) {
         LCUDA(cudaMemsetAsync(sc, 0, sizeof(unsigned long long), st), "memset");
         LCUDA(cudaMemsetAsync(sc + 3, 0, sizeof(unsigned long long), st), "memset");
         LCUDA(cudaMemsetAsync(sc + 6, 0, sizeof(unsigned long long), st), "memset");
-        LCUDA(cudaMemsetAsync(Q.hhead, 0xFF, (size_t)N * sizeof(int32_t), st), "memset");
         LCUDA(cudaMemsetAsync(Q.overflow, 0, sizeof(int), st), "memset");
         LCUDA(msc::launch_speculate(c.g32, c.V, P, Q, k0, k1, d.lab, lvl, stamp, claim, sc + 3, c.work + 48, c.sms,
                                     st),
@@ -670,10 +670,12 @@ int first_pass(LabelCtx& c, DirLabels& d) {
         if (int rc = read_dev(c, Q.overflow, 1, &ovf)) return rc;
         if (!ovf) break;
         LCUDA(msc::launch_spec_unclaim_all(lvl, stamp, claim, N, c.sms, st), "unclaim");
+        LCUDA(cudaMemsetAsync(Q.hcount, 0, (size_t)N * sizeof(int32_t), st), "memset");
         if (k1 - k0 <= 1) return fail(MSC_ERR_OOM, "first pass: one streamline's record exceeds its pool");
         k1 = k0 + (k1 - k0) / 2;
       }
       trace_mark(st, d.dir, "  speculated " + std::to_string(k1 - k0));
+      LCUDA(msc::launch_spec_holders(Q, k0, k1, N, Q.overflow, c.sms, st), "holders");
       // resolution rounds: the first looks at every item, a later one at the items that
       // hold a vertex whose claim may have changed; they end when a round changes no
       // claim.  After the first two, rounds go in groups of four between counter reads

@@ -23,6 +23,7 @@
 //   another region; chains resolve by pointer jumping.
 #include <cstdio>
 #include <cstdlib>
+#include <string>
 
 #include "label_common.cuh"
 
@@ -48,11 +49,38 @@ __device__ __forceinline__ float clampf_ext(float v, float fn) {
 // Streamlines differ in length by orders of magnitude (most end within a few dozen
 // iterations, a few run to the iteration limit circling a sink on a boundary face), so
 // a warp that integrated 32 fixed streamlines would idle most of its lanes behind the
-// longest one.  Instead every lane runs its streamline one iteration per turn of the
-// warp's loop and takes the next work item as soon as its own streamline ends; the
-// items are handed out by one warp-aggregated atomicAdd per turn.
+// longest one.  Instead every lane runs its streamline one iteration per round of the
+// warp's loop and takes the next work item as soon as its own streamline ends
+// (WarpItems).
 enum : int { kLaneIdle = 0, kLaneEnter, kLaneStep, kLaneEnd, kLaneDone };
 
+// The state of a lane's streamline.
+struct Lane32 {
+  F3 cur = {0.f, 0.f, 0.f};
+  float b[3] = {0.f, 0.f, 0.f};  // the voxel's base corner
+  F3 c[8];                       // its corner gradients (Adv32::load_voxel)
+  float step = 0.f;
+  int iters = 0;
+  int32_t base = 0;              // vertex of the base corner
+  uint32_t stop = 0;             // corners that stop the streamline (bit x + 2y + 4z)
+  int32_t nv = -1;               // nearest vertex, as the stop test last passed it
+  bool nb = false;               // the voxel was entered next to the grid's boundary
+  float gm_end = 0.f;            // gradient magnitude at a low-gradient stop (0 where there was none)
+  F3 anchor = {0.f, 0.f, 0.f};   // trapped-streamline test
+  int t_iters = 0, t_n = 0;
+};
+
+// SHORT: a step moves less than half a voxel along any axis (P.max_step at most
+// kShortStep: an accepted step differs from the full Euler step, of length max_step at
+// most, by less than sqrt(ethresh)).  Then the nearest vertex of a position in a voxel, or
+// just stepped out of it, is one of the voxel's corners, and whether it stops the
+// streamline was read with the corner gradients, from their fourth component
+// (kStopTerminal / kStopLabelled): a step reads no memory and converts nothing to an
+// integer.  The longer steps that a caller may ask for read the vertex's state.
+constexpr float kShortStep = 0.45f;
+constexpr float kShortThresh = 1e-3f;  // sqrt: 0.032
+
+template <bool SHORT>
 struct Adv32 {
   const float4* G;
   VolDims V;
@@ -64,9 +92,8 @@ struct Adv32 {
   // (float)V.X .. and (float)(V.X - 2) ..  (a double-to-float or 64-bit integer
   // conversion per iteration would run on the slow FP64 pipe)
   float ms = 0.f, sgn = 0.f;
-  float ext[3] = {0.f, 0.f, 0.f}, ext2[3] = {0.f, 0.f, 0.f};
-  int64_t XY = 0;    // vertices per z-plane
-  bool i32 = false;  // vertex ids fit 32 bits
+  float ext[3] = {0.f, 0.f, 0.f}, ext1[3] = {0.f, 0.f, 0.f}, ext2[3] = {0.f, 0.f, 0.f};
+  int32_t X = 0, XY = 0;  // vertices per row and z-plane (fewer than 2^31 vertices)
 
   static Adv32 make(const float4* G, const VolDims& V, const IntegParams& P, const uint8_t* lvl, int level,
                     const uint8_t* state) {
@@ -76,43 +103,45 @@ struct Adv32 {
     const int64_t e[3] = {V.X, V.Y, V.Z};
     for (int a = 0; a < 3; a++) {
       A.ext[a] = (float)e[a];
+      A.ext1[a] = (float)(e[a] - 1);
       A.ext2[a] = (float)(e[a] - 2);
     }
-    A.XY = V.X * V.Y;
-    A.i32 = V.X * V.Y * V.Z <= (int64_t)0xFFFFFFFF;
+    A.X = (int32_t)V.X;
+    A.XY = (int32_t)(V.X * V.Y);
     return A;
   }
 
-  // Vertex id of (x, y, z) in 32-bit arithmetic while the grid's ids fit 32 bits
-  __device__ __forceinline__ int64_t index(int x, int y, int z) const {
-    if (i32) return (int64_t)((uint32_t)x + (uint32_t)V.X * ((uint32_t)y + (uint32_t)V.Y * (uint32_t)z));
-    return vid(V, x, y, z);
-  }
-  // The voxel that holds `cur` (clamped into the grid near its boundary): its base
-  // corner as floats and its corner gradients, c[n] for the corners n = x + 2y + 4z,
-  // stored for trilin() as c[2k] and c[2k + 1] - c[2k] (the difference along x).  A
-  // voxel clamped onto the grid's last plane along an axis repeats that plane's
-  // corners there.
-  __device__ __forceinline__ void load_voxel(const F3& cur, bool nearb, float bf[3], F3 c[8]) const {
-    const float p[3] = {cur.x, cur.y, cur.z};
+  __device__ __forceinline__ int32_t index(int x, int y, int z) const { return x + X * y + XY * z; }
+
+  // The voxel that holds the position (clamped into the grid near its boundary): its base
+  // corner and its corner gradients, c[n] for the corners n = x + 2y + 4z, stored for
+  // trilin() as c[2k] and c[2k + 1] - c[2k] (the difference along x).  A voxel clamped
+  // onto the grid's last plane along an axis repeats that plane's corners there.
+  __device__ __forceinline__ void load_voxel(Lane32& L) const {
+    const float p[3] = {L.cur.x, L.cur.y, L.cur.z};
     int b[3];
-    int64_t o[3] = {1, V.X, XY};
+    int o[3] = {1, X, XY};
     const int E[3] = {(int)V.X, (int)V.Y, (int)V.Z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      b[a] = nearb ? (int)clampf_ext(p[a], ext[a]) : (int)fminf(fmaxf(p[a], 0.f), ext2[a]);
-      b[a] = max(b[a], 0);
-      if (nearb && b[a] >= E[a] - 1) o[a] = 0;
-      bf[a] = (float)b[a];
+      // (short steps never leave the grid: away from its boundary they cannot reach it, and
+      // next to it they are clamped)
+      if (SHORT) b[a] = (int)p[a];
+      else b[a] = max(L.nb ? (int)clampf_ext(p[a], ext[a]) : (int)fminf(fmaxf(p[a], 0.f), ext2[a]), 0);
+      if (L.nb && b[a] >= E[a] - 1) o[a] = 0;
+      L.b[a] = (float)b[a];
     }
-    const float4* q = G + index(b[0], b[1], b[2]);
+    L.base = index(b[0], b[1], b[2]);
+    uint32_t stop = 0;
 #pragma unroll
     for (int n = 0; n < 8; n++) {
-      const float4 v = __ldg(q + ((n & 1) ? o[0] : 0) + ((n & 2) ? o[1] : 0) + ((n & 4) ? o[2] : 0));
-      c[n] = {v.x, v.y, v.z};
+      const float4 v = __ldg(G + (L.base + ((n & 1) ? o[0] : 0) + ((n & 2) ? o[1] : 0) + ((n & 4) ? o[2] : 0)));
+      L.c[n] = {v.x, v.y, v.z};
+      if (SHORT) stop |= __float_as_uint(v.w) & ((state ? 1u : 0x100u) << n);
     }
+    if (SHORT) L.stop = state ? stop : stop >> 8;
 #pragma unroll
-    for (int n = 1; n < 8; n += 2) c[n] = {c[n].x - c[n - 1].x, c[n].y - c[n - 1].y, c[n].z - c[n - 1].z};
+    for (int n = 1; n < 8; n += 2) L.c[n] = {L.c[n].x - L.c[n - 1].x, L.c[n].y - L.c[n - 1].y, L.c[n].z - L.c[n - 1].z};
   }
   // Trilinear interpolation of the corner gradients at s (bf: the base corner as
   // floats; c as load_voxel() stores it), each linear interpolation as a + t (b - a)
@@ -133,32 +162,127 @@ struct Adv32 {
     iy = (int)clampf_ext(p.y + 0.5f, ext[1]);
     iz = (int)clampf_ext(p.z + 0.5f, ext[2]);
   }
-  __device__ __forceinline__ int64_t nearest(F3 p) const {
-    int ix, iy, iz;
-    nearest3(p, ix, iy, iz);
-    return index(ix, iy, iz);
+  // A streamline from vertex (x, y, z) of index v
+  __device__ __forceinline__ void start(Lane32& L, int x, int y, int z, int32_t nv) const {
+    L.cur = {(float)x, (float)y, (float)z};
+    L.nb = near_boundary(x, y, z);
+    L.iters = P.iteration_limit;
+    L.anchor = L.cur;
+    L.t_iters = L.iters;
+    L.t_n = 0;
+    L.nv = nv;
   }
-  // The trapped-streamline test (IntegParams::trap_window): compares `cur` with the
-  // anchor set trap_window iterations before, moves the anchor, counts the
-  // consecutive tight windows in `n`; true once there are two.
-  __device__ __forceinline__ bool trapped(const F3& cur, F3& anchor, int& n) const {
-    const float d = fmaxf(fabsf(cur.x - anchor.x), fmaxf(fabsf(cur.y - anchor.y), fabsf(cur.z - anchor.z)));
-    n = d < P.trap_radius ? n + 1 : 0;
-    anchor = cur;
-    return n >= 2;
+  __device__ __forceinline__ bool near_boundary(int x, int y, int z) const {
+    const int dx = min(x, (int)V.X - 1 - x), dy = min(y, (int)V.Y - 1 - y), dz = min(z, (int)V.Z - 1 - z);
+    return min(min(dx, dy), dz) <= 1;
+  }
+  // The trapped-streamline test (IntegParams::trap_window), due every trap_window
+  // iterations, at multiples of kTrapEvery of a streamline's iterations: compares the
+  // position with the anchor set at the test before, moves the anchor, counts the
+  // consecutive tight windows; true once there are two.
+  static constexpr int kTrapEvery = 16;
+  __device__ __forceinline__ bool trapped(Lane32& L) const {
+    if (P.trap_window <= 0 || ((P.iteration_limit - L.iters) & (kTrapEvery - 1)) != 0 ||
+        L.t_iters - L.iters < P.trap_window)
+      return false;
+    L.t_iters = L.iters;
+    const float d = fmaxf(fabsf(L.cur.x - L.anchor.x),
+                          fmaxf(fabsf(L.cur.y - L.anchor.y), fabsf(L.cur.z - L.anchor.z)));
+    L.t_n = d < P.trap_radius ? L.t_n + 1 : 0;
+    L.anchor = L.cur;
+    return L.t_n >= 2;
   }
   // One round of a lane's streamline (phase kLaneEnter or kLaneStep): the loop body of
-  // AdvectThroughVoxel{NoCheck,NearBoundary}, one `iters` decrement, with the entry
-  // into a voxel folded in (x, y, z: the entering lane's nearest vertex).  Written
-  // without branches between its outcomes (moved or not, step accepted or rejected):
-  // every stepping lane of a warp runs the same instructions, so that the warp issues
-  // one iteration's instructions per round rather than one per outcome.  A lane whose
-  // last step was rejected evaluates the gradient at its unchanged position again (the
-  // same value).  slim caches max_step / |g|.  EV_NONE to go on; gm_end: the gradient
-  // magnitude at a low-gradient stop (0 where there was none).
-  __device__ __forceinline__ int advance(int& phase, int x, int y, int z, F3& cur, F3& old, int& iters, bool& nb,
-                                         float b[3], F3 c[8], F3& g, float& gm, float& step, float& slim,
-                                         float& gm_end, int64_t& last_nv, unsigned long long& ntrips) const;
+  // AdvectThroughVoxel{NoCheck,NearBoundary}, with the entry into a voxel folded in, and
+  // the iteration that finds the voxel left.  Written without branches between a step's
+  // outcomes (moved or not, accepted or rejected): every stepping lane of a warp runs the
+  // same instructions, so that the warp issues one iteration's instructions per round
+  // rather than one per outcome.  A lane whose last step was rejected evaluates the
+  // gradient at its unchanged position again (the same value).  EV_NONE to go on; `out`:
+  // the step left the voxel (phase kLaneEnter).
+  __device__ __forceinline__ int advance(int& phase, Lane32& L, bool& out) const {
+    const bool ent = phase == kLaneEnter;
+    out = false;
+    if (ent) {
+      load_voxel(L);
+      L.gm_end = 0.f;
+      phase = kLaneStep;
+    }
+    const F3 g = trilin(L.cur, L.b, L.c);
+    const float gm = sqrtf(g.x * g.x + g.y * g.y + g.z * g.z);
+    const bool bad = !(gm > 0.f) || !isfinite(gm);
+    // in the reference's order: an entering lane stops on a vanishing gradient before it
+    // takes an iteration; a stepping lane checks the iteration count, then the gradient
+    if (ent && bad) return EV_LOW_GRADIENT;
+    if (L.iters-- <= 0) return EV_OVER_MAX_ITERATIONS;
+    if (bad) return EV_LOW_GRADIENT;
+    const float sl = ms / gm;
+    float step = L.step;
+    if (ent || gm * step > ms) step = sl;
+    if (gm < P.gthresh) {
+      L.gm_end = gm;
+      return EV_LOW_GRADIENT;
+    }
+    // the adaptive Euler step: a full step and two half steps, accepted (the step grows)
+    // when they agree within ethresh, otherwise halved
+    const F3 cur = L.cur;
+    const float sm = sgn * step;
+    const F3 e1 = {g.x * sm, g.y * sm, g.z * sm};
+    const float hs = sm * 0.5f;
+    const F3 hd = {g.x * hs, g.y * hs, g.z * hs};
+    const F3 hg = trilin({cur.x + hd.x, cur.y + hd.y, cur.z + hd.z}, L.b, L.c);
+    const F3 e2 = {hg.x * hs + hd.x, hg.y * hs + hd.y, hg.z * hs + hd.z};
+    const float dx = e2.x - e1.x, dy = e2.y - e1.y, dz = e2.z - e1.z;
+    const bool acc = dx * dx + dy * dy + dz * dz < P.ethresh;
+    F3 np = {cur.x + e2.x, cur.y + e2.y, cur.z + e2.z};
+    if (L.nb) {
+      np.x = clampf_ext(np.x, ext[0]);
+      np.y = clampf_ext(np.y, ext[1]);
+      np.z = clampf_ext(np.z, ext[2]);
+    }
+    L.step = acc ? fminf(step * 1.8f, sl) : step * 0.5f;
+    if (acc) L.cur = np;
+    bool left, near;
+    if (SHORT) {
+      // the voxel's next corner planes; nearest corner by comparison (p + 0.5 rounded as
+      // the conversion to an integer would see it, and clamped into the grid)
+      const float b1x = L.b[0] + 1.f, b1y = L.b[1] + 1.f, b1z = L.b[2] + 1.f;
+      const bool ux = fminf(np.x + 0.5f, ext1[0]) >= b1x, uy = fminf(np.y + 0.5f, ext1[1]) >= b1y,
+                 uz = fminf(np.z + 0.5f, ext1[2]) >= b1z;
+      const int corner = (ux ? 1 : 0) + (uy ? 2 : 0) + (uz ? 4 : 0);
+      if (acc && ((L.stop >> corner) & 1u)) return EV_HIT_PREASSIGNED;
+      if (acc) L.nv = L.base + (ux ? 1 : 0) + (uy ? X : 0) + (uz ? XY : 0);
+      left = acc && !(np.x >= L.b[0] && np.x < b1x && np.y >= L.b[1] && np.y < b1y && np.z >= L.b[2] && np.z < b1z);
+      // (the nearest vertex, for the entry into the next voxel)
+      const float vx = ux ? b1x : L.b[0], vy = uy ? b1y : L.b[1], vz = uz ? b1z : L.b[2];
+      near = fminf(fminf(fminf(vx, ext1[0] - vx), fminf(vy, ext1[1] - vy)), fminf(vz, ext1[2] - vz)) <= 1.f;
+    } else {
+      // the stop test reads memory only when an accepted step changed the nearest vertex:
+      // what it reads (certain terminals in the fix-up, earlier levels in the first pass)
+      // does not change while the kernel runs, and a vertex it passed once does not stop
+      // the streamline later
+      int ix, iy, iz;
+      nearest3(np, ix, iy, iz);
+      const int32_t nv = index(ix, iy, iz);
+      if (acc && nv != L.nv) {
+        const uint8_t st = state ? state[nv] : lvl[nv];
+        const bool hit = state ? (st == kStSeed || st == kStTerminal) : st < level;
+        if (hit) return EV_HIT_PREASSIGNED;
+        L.nv = nv;
+      }
+      left = acc && ((int)np.x != (int)cur.x || (int)np.y != (int)cur.y || (int)np.z != (int)cur.z);
+      near = near_boundary(ix, iy, iz);
+    }
+    if (trapped(L)) return EV_OVER_MAX_ITERATIONS;  // ends where the iteration limit would have
+    if (left) {
+      // the iteration that finds the voxel left (the iteration count is checked first)
+      if (L.iters-- <= 0) return EV_OVER_MAX_ITERATIONS;
+      L.nb = near;
+      out = true;
+      phase = kLaneEnter;
+    }
+    return EV_NONE;
+  }
 };
 
 // Distance of vertex (x, y, z) to the grid's nearest face, in vertices
@@ -166,77 +290,6 @@ __device__ __forceinline__ int dist_to_boundary(const VolDims& V, int x, int y, 
   const int X = (int)V.X, Y = (int)V.Y, Z = (int)V.Z;
   return min(min(min(x, X - 1 - x), min(y, Y - 1 - y)), min(z, Z - 1 - z));
 }
-
-__device__ __forceinline__ int Adv32::advance(int& phase, int x, int y, int z, F3& cur, F3& old, int& iters, bool& nb,
-                                              float b[3], F3 c[8], F3& g, float& gm, float& step, float& slim,
-                                              float& gm_end, int64_t& last_nv, unsigned long long& ntrips) const {
-  const bool ent = phase == kLaneEnter;
-  if (ent) {
-    nb = dist_to_boundary(V, x, y, z) <= 1;
-    load_voxel(cur, nb, b, c);
-    gm_end = 0.f;
-    phase = kLaneStep;
-  }
-  const bool moved = !ent && !(old.x == cur.x && old.y == cur.y && old.z == cur.z);
-  const bool left = moved && ((int)cur.x != (int)old.x || (int)cur.y != (int)old.y || (int)cur.z != (int)old.z);
-  const F3 gc = trilin(cur, b, c);
-  const float gmc = sqrtf(gc.x * gc.x + gc.y * gc.y + gc.z * gc.z);
-  const bool bad = !(gmc > 0.f) || !isfinite(gmc);
-  // events before the step, in the reference's order: an entering lane stops on a
-  // vanishing gradient before it takes an iteration; a stepping lane checks the
-  // iteration count, then whether it left its voxel, then the gradient
-  const bool counts = !(ent && bad);
-  ntrips += counts;
-  const bool spent = counts && !(iters > 0);
-  iters -= counts;
-  int ev = spent ? EV_OVER_MAX_ITERATIONS : EV_NONE;
-  if (ent && bad) ev = EV_LOW_GRADIENT;
-  if (!spent && left) ev = EV_OUT_OF_VOXEL;
-  if (!spent && !left && moved && bad) ev = EV_LOW_GRADIENT;
-  if (ev != EV_NONE) return ev;
-  const float sl = ms / gmc;
-  if (ent || gmc * step > ms) step = sl;
-  g = gc;
-  gm = gmc;
-  slim = sl;
-  old = cur;
-  if (gm < P.gthresh) {
-    gm_end = gm;
-    return EV_LOW_GRADIENT;
-  }
-  // the adaptive Euler step: a full step and two half steps, accepted (the step grows)
-  // when they agree within ethresh, otherwise halved
-  const float sm = sgn * step;
-  const F3 e1 = {g.x * sm, g.y * sm, g.z * sm};
-  const float hs = sm * 0.5f;
-  const F3 hd = {g.x * hs, g.y * hs, g.z * hs};
-  const F3 hg = trilin({cur.x + hd.x, cur.y + hd.y, cur.z + hd.z}, b, c);
-  const F3 e2 = {hg.x * hs + hd.x, hg.y * hs + hd.y, hg.z * hs + hd.z};
-  const float dx = e2.x - e1.x, dy = e2.y - e1.y, dz = e2.z - e1.z;
-  const bool acc = dx * dx + dy * dy + dz * dz < P.ethresh;
-  F3 np = {cur.x + e2.x, cur.y + e2.y, cur.z + e2.z};
-  if (nb) {
-    np.x = clampf_ext(np.x, ext[0]);
-    np.y = clampf_ext(np.y, ext[1]);
-    np.z = clampf_ext(np.z, ext[2]);
-  }
-  step = acc ? fminf(step * 1.8f, sl) : step * 0.5f;
-  if (acc) cur = np;
-  // the stop test reads memory only when an accepted step changed the nearest vertex:
-  // what it reads (certain terminals in the fix-up, earlier levels in the first pass)
-  // does not change while the kernel runs, and a vertex it passed once does not stop
-  // the streamline later
-  const int64_t nv = nearest(np);
-  if (acc && nv != last_nv) {
-    const uint8_t st = state ? state[nv] : lvl[nv];
-    const bool hit = state ? (st == kStSeed || st == kStTerminal) : st < level;
-    if (hit) return EV_HIT_PREASSIGNED;
-    last_nv = nv;
-  }
-  return EV_NONE;
-}
-
-
 
 // Vertex coordinates of index v; 32-bit division while the grid's indices fit 32 bits.
 __device__ __forceinline__ void split_index(const VolDims& V, int64_t v, int& x, int& y, int& z) {
@@ -253,11 +306,15 @@ __device__ __forceinline__ void split_index(const VolDims& V, int64_t v, int& x,
   }
 }
 
-constexpr int kPathCap = 48;
+// Rounds between the hand-outs of new work items: a hand-out costs about half a round, a
+// lane whose streamline ends waits for it (512^3 k^-3 / 256^3 Gaussian labels: 368 / 97 ms
+// with 4, 342 / 91 with 8, 336 / 90 with 16, 361 / 91 with 32).
+constexpr int kRoundsPerTurn = 16;
 constexpr unsigned kFullMask = 0xffffffffu;
 
 // CTAs of 128 threads per SM launched for the lane-refilling FP32 kernels (their
-// registers allow 7 resident per SM); MSC_LANE_CTAS_PER_SM overrides it for tuning.
+// registers allow 6 resident per SM: 80 without spills; 7 and 72 with them measured
+// the same at 512^3 and 5% slower at 256^3); MSC_LANE_CTAS_PER_SM overrides it for tuning.
 int lane_ctas_per_sm();
 
 // Claims a work item for every lane of the warp that asks for one (`want`); returns
@@ -272,6 +329,51 @@ __device__ __forceinline__ unsigned long long claim_item(bool want, unsigned lon
   base = __shfl_sync(kFullMask, base, leader);
   return base + (unsigned long long)__popc(ask & ((1u << lane) - 1u));
 }
+
+// The work items of a warp: taken 32 at a time from *work (one atomic and one coalesced
+// read of the list per 32 streamlines instead of one each per turn), a lane holds one in
+// reserve, and idle lanes get theirs by a shuffle.
+struct WarpItems {
+  unsigned long long base = 0;  // first item of the reserve
+  int32_t held = 0;             // this lane's reserve item's vertex
+  int next = 0, have = 0;       // the reserve: items base + [next, have)
+  bool more = true;
+  // Every lane of the warp calls it.  Where `want`: true with the item and its vertex, or
+  // false when there are no more.  fetch(k): the vertex of item k < n.
+  template <class Fetch>
+  __device__ __forceinline__ bool take(bool want, unsigned long long n, unsigned long long* work, const Fetch& fetch,
+                                       unsigned long long& k, int32_t& v) {
+    const int lane = threadIdx.x & 31;
+    bool got = false;
+    unsigned ask = __ballot_sync(kFullMask, want);
+    while (ask) {
+      if (next == have) {
+        if (!more) break;
+        unsigned long long b = 0;
+        if (lane == 0) b = atomicAdd(work, 32ull);
+        base = __shfl_sync(kFullMask, b, 0);
+        next = 0;
+        have = base >= n ? 0 : (n - base < 32ull ? (int)(n - base) : 32);
+        more = have == 32;
+        if (lane < have) held = fetch(base + lane);
+        if (have == 0) break;
+      }
+      // the i-th asking lane gets the i-th item of the reserve
+      const int src = next + __popc(ask & ((1u << lane) - 1u));
+      const bool mine = ((ask >> lane) & 1u) && src < have;
+      const int32_t hv = __shfl_sync(kFullMask, held, src & 31);
+      if (mine) {
+        k = base + src;
+        v = hv;
+        got = true;
+      }
+      const unsigned served = __ballot_sync(kFullMask, mine);
+      next += __popc(served);
+      ask &= ~served;
+    }
+    return got;
+  }
+};
 
 // Adds the warp's trip counts to *trips (one atomic per warp; every lane calls it).
 __device__ __forceinline__ void add_trips(unsigned long long n, unsigned long long* trips) {
@@ -342,7 +444,7 @@ __device__ __forceinline__ int block_append(int cnt, int* __restrict__ n, int* s
 
 constexpr uint32_t kRec = 0x80000000u;
 constexpr int kSeg = 32;
-constexpr int kSpecBuf = 48;  // a lane holds <= kSeg entries at a turn's start, + at most K <= 16 in the turn
+constexpr int kSpecBuf = kSeg + kRoundsPerTurn;  // a lane holds <= kSeg entries at a turn's start
 constexpr uint32_t kNoClaim = 0xFFFFFFFFu;
 
 __device__ __forceinline__ int64_t spread_vertex(const SpreadOrder& S, int64_t u) {
@@ -482,12 +584,13 @@ __device__ __forceinline__ uint32_t entry_of(const SpecSet& Q, int64_t k, int e)
 // vertices labelled before this batch (lvl < A.level), record their entries, count them
 // at their vertices, and make the first round's claims (every item alive, its whole path
 // effective).
-template <int K>
-__global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const SpecSet Q, int64_t k0, int64_t k1,
-                                                           const int32_t* __restrict__ lab,
+template <bool SHORT>
+__global__ void __launch_bounds__(128, 6) speculate_kernel(const Adv32<SHORT> A, const SpecSet Q, int64_t k0,
+                                                           int64_t k1, const int32_t* __restrict__ lab,
                                                            uint32_t* __restrict__ claim,
                                                            unsigned long long* __restrict__ work,
                                                            unsigned long long* __restrict__ trips) {
+  constexpr int K = kRoundsPerTurn;
   const VolDims& V = A.V;
   const int level = A.level;
   const int lane = threadIdx.x & 31;
@@ -495,21 +598,13 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
   int nb = 0;
   int cnt = 0;             // entries so far
   uint32_t e1 = 0;         // entry 1
-  int64_t k = -1;          // the lane's item
+  int32_t k = -1;          // the lane's item
   int flushed = 0;         // pool entries written
   uint32_t link = 0;       // word offset of the last full segment's link slot
   int phase = kLaneIdle;
   unsigned long long ntrips = 0;
-  int x = 0, y = 0, z = 0;
-  F3 cur = {0.f, 0.f, 0.f}, old = cur, g = cur;
-  float gm = 0.f, step = 0.f, slim = 0.f, gm_end = 0.f;
-  int iters = 0;
-  bool nb_near = false;
-  float b[3] = {0.f, 0.f, 0.f};
-  F3 c[8];
-  F3 anchor = cur;
-  int t_iters = 0, t_n = 0;
-  int64_t last_nv = -1;
+  Lane32 L;
+  WarpItems items;
   int32_t endlab = kLabelNone;
   auto mark_rec = [&]() {  // the reference pushes its nearest vertex: the last one passed
     if (cnt == 2) e1 |= kRec;
@@ -517,25 +612,23 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
   };
   while (true) {
     {
-      const unsigned long long t = claim_item(phase == kLaneIdle, work);
+      unsigned long long t = 0;
+      int32_t v = 0;
+      const bool got = items.take(phase == kLaneIdle, (unsigned long long)(k1 - k0), work,
+                                  [&](unsigned long long j) { return Q.vtx[k0 + (int64_t)j]; }, t, v);
       if (phase == kLaneIdle) {
-        k = k0 + (int64_t)t;
-        if (k >= k1 || *(volatile int*)Q.overflow) {
+        if (!got || *(volatile int*)Q.overflow) {
           phase = kLaneDone;
         } else {
-          const int64_t i = Q.vtx[k];
-          if (A.lvl[i] < level) {  // labelled by an earlier batch of this group
+          k = (int32_t)(k0 + (int64_t)t);
+          if (A.lvl[v] < level) {  // labelled by an earlier batch of this group
             Q.alive[k] = 0;
             Q.len[k] = 0;
             Q.ext[k] = 0;
           } else {
-            split_index(V, i, x, y, z);
-            cur = {(float)x, (float)y, (float)z};
-            iters = A.P.iteration_limit;
-            anchor = cur;
-            t_iters = iters;
-            t_n = 0;
-            last_nv = i;
+            int x, y, z;
+            split_index(V, v, x, y, z);
+            A.start(L, x, y, z, v);
             nb = 0;
             cnt = 1;
             e1 = 0;
@@ -552,34 +645,29 @@ __global__ void __launch_bounds__(128, 7) speculate_kernel(const Adv32 A, const 
     }
     for (int r = 0; r < K; r++) {
       if (phase != kLaneEnter && phase != kLaneStep) continue;
-      const int64_t seen = last_nv;
-      const int ev = A.advance(phase, x, y, z, cur, old, iters, nb_near, b, c, g, gm, step, slim, gm_end, last_nv,
-                               ntrips);
-      if (last_nv != seen) {  // the stop test passed a new vertex
-        if (cnt == 1) e1 = (uint32_t)last_nv;
-        else buf[nb++] = (uint32_t)last_nv;
+      const int32_t seen = L.nv;
+      bool out;
+      const int ev = A.advance(phase, L, out);
+      if (L.nv != seen) {  // the stop test passed a new vertex
+        if (cnt == 1) e1 = (uint32_t)L.nv;
+        else buf[nb++] = (uint32_t)L.nv;
         cnt++;
       }
-      if (ev == EV_NONE) continue;
-      A.nearest3(cur, x, y, z);
+      if (ev == EV_NONE && !out) continue;
       if (ev == EV_HIT_PREASSIGNED) {
         // stopped by a vertex labelled before the batch: its label is the streamline's
         // (the vertex itself is not recorded, so every entry is a vertex unlabelled
         // before the batch)
-        const int32_t l = lab[vid(V, x, y, z)];
+        int x, y, z;
+        A.nearest3(L.cur, x, y, z);
+        const int32_t l = lab[A.index(x, y, z)];
         endlab = l == -1 ? kLabelNone : l;
       } else {
         mark_rec();
       }
-      phase = ev == EV_OUT_OF_VOXEL ? kLaneEnter : kLaneEnd;
+      if (ev != EV_NONE) phase = kLaneEnd;
     }
-    if (phase == kLaneStep && A.P.trap_window > 0 && t_iters - iters >= A.P.trap_window) {
-      t_iters = iters;
-      if (A.trapped(cur, anchor, t_n)) {  // ends where the iteration limit would have
-        mark_rec();
-        phase = kLaneEnd;
-      }
-    }
+    if (phase == kLaneEnd) ntrips += (unsigned long long)(A.P.iteration_limit - L.iters);
     // flush: an ended streamline writes the rest of its entries, a long one a full
     // segment (+ its link word); one pool allocation and one count of the entries per warp and
     // turn.  A segment is flushed early only with an entry to spare (an ending marks the
@@ -968,8 +1056,13 @@ __global__ void spec_jump_kernel(const SpecSet Q, int64_t k0, int64_t k1) {
 constexpr int kChainSteps = 64;
 __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8_t* __restrict__ lvl, int level,
                                   const uint32_t* __restrict__ claim, int32_t* __restrict__ lab,
-                                  int* __restrict__ long_chain) {
+                                  float4* __restrict__ g32, int* __restrict__ long_chain) {
   const int lane = threadIdx.x & 31;
+  auto put = [&](uint32_t v, int32_t l) {
+    lab[v] = l;
+    lvl[v] = (uint8_t)level;
+    reinterpret_cast<uint32_t*>(g32 + v)[3] = kStopLabelled;
+  };
   for (int64_t b0 = k0 + blockIdx.x * (int64_t)blockDim.x; b0 < k1; b0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = b0 + threadIdx.x;  // (warp-uniform trips)
     int n = 0;
@@ -995,10 +1088,7 @@ __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8
       for (int e = 0; e < kNear; e++) cl[e] = e < n && (u[e] & kRec) ? claim[u[e] & ~kRec] : kNoClaim;
 #pragma unroll
       for (int e = 0; e < kNear; e++)
-        if (cl[e] == (uint32_t)k) {
-          lab[u[e] & ~kRec] = d;
-          lvl[u[e] & ~kRec] = (uint8_t)level;
-        }
+        if (cl[e] == (uint32_t)k) put(u[e] & ~kRec, d);
     }
     // the rest of the long sequences, a segment at a time (as check_item)
     unsigned far = __ballot_sync(kFullMask, n > kNear);
@@ -1015,12 +1105,35 @@ __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8
         if (e0 + kSeg < fn) seg = Q.pool[seg + kSeg];
         if (!(w & kRec)) continue;
         const uint32_t v = w & ~kRec;
-        if (claim[v] == (uint32_t)fk) {
-          lab[v] = fd;
-          lvl[v] = (uint8_t)level;
-        }
+        if (claim[v] == (uint32_t)fk) put(v, fd);
       }
     }
+  }
+}
+
+// The gradient of every vertex for the FP32 passes (central differences as
+// central_diff_kernel's xyzw form; zero where a bit of `zeroed` is set), with what stops a
+// streamline there as the fourth component, and the vertex's state, from the certain
+// terminal regions.  (The first pass adds kStopLabelled to the vertices it labels while
+// the ends beside it run; those look at kStopTerminal's bits alone, which stay.)
+__global__ void __launch_bounds__(256) label_gradient_kernel(const float* __restrict__ f,
+                                                             const int32_t* __restrict__ lab,
+                                                             const uint32_t* __restrict__ zeroed, const VolDims V,
+                                                             uint8_t* __restrict__ state, float4* __restrict__ g32) {
+  const int64_t N = V.X * V.Y * V.Z, X = V.X, XY = V.X * V.Y;
+  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < N; v += (int64_t)gridDim.x * blockDim.x) {
+    int x, y, z;
+    split_index(V, v, x, y, z);
+    const float* p = f + v;
+    const bool ix = x > 0 && x < V.X - 1, iy = y > 0 && y < V.Y - 1, iz = z > 0 && z < V.Z - 1;
+    float gx = ix ? 0.5f * (__ldg(p + 1) - __ldg(p - 1)) : 0.f;
+    float gy = iy ? 0.5f * (__ldg(p + X) - __ldg(p - X)) : 0.f;
+    float gz = iz ? 0.5f * (__ldg(p + XY) - __ldg(p - XY)) : 0.f;
+    if ((zeroed[v >> 5] >> (v & 31)) & 1u) gx = gy = gz = 0.f;
+    uint8_t st = state[v];
+    const bool seed = st == kStSeed;
+    if (!seed) state[v] = st = lab[v] >= 0 ? kStTerminal : kStUnassigned;
+    g32[v] = make_float4(gx, gy, gz, __uint_as_float(st == kStUnassigned ? 0u : kStopTerminal | kStopLabelled));
   }
 }
 
@@ -1316,8 +1429,8 @@ __global__ void __launch_bounds__(32) fixup_end64_kernel(const Adv64 A, const in
 //     different certain region (FP32 rounding may have picked the wrong side);
 //   amb_mode 2: its final voxel touches two different certain regions (any ending
 //     within half a voxel of a basin boundary).
-template <int K>
-__global__ void __launch_bounds__(128, 7) fixup_end32_kernel(const Adv32 A, const int32_t* __restrict__ lab,
+template <bool SHORT>
+__global__ void __launch_bounds__(128, 6) fixup_end32_kernel(const Adv32<SHORT> A, const int32_t* __restrict__ lab,
                                                           const uint8_t* __restrict__ state,
                                                           const int64_t* __restrict__ list, int n,
                                                           const int* __restrict__ n_dev,
@@ -1325,36 +1438,29 @@ __global__ void __launch_bounds__(128, 7) fixup_end32_kernel(const Adv32 A, cons
                                                           int* __restrict__ n_amb, int amb_mode,
                                                           unsigned long long* __restrict__ work,
                                                           unsigned long long* __restrict__ trips) {
+  constexpr int K = kRoundsPerTurn;
   const VolDims& V = A.V;
   if (n_dev) n = *n_dev;  // a list whose length the stream wrote before this launch
   int phase = kLaneIdle;
   unsigned long long ntrips = 0;
-  int64_t v = 0;
-  int x = 0, y = 0, z = 0;
-  F3 cur = {0.f, 0.f, 0.f}, old = cur, g = cur;
-  float gm = 0.f, step = 0.f, slim = 0.f, gm_end = 0.f;
-  int iters = 0, ev = EV_NONE;
-  bool nb = false;
-  float b[3] = {0.f, 0.f, 0.f};
-  F3 c[8];
-  F3 anchor = cur;  // trapped-streamline test
-  int t_iters = 0, t_n = 0;
-  int64_t last_nv = -1;  // nearest vertex the stop test last passed
+  int32_t v = 0;
+  int ev = EV_NONE;
+  Lane32 L;
+  WarpItems items;
   while (true) {
-    const unsigned long long k = claim_item(phase == kLaneIdle, work);
-    if (phase == kLaneIdle) {
-      if (k >= (unsigned long long)n) {
-        phase = kLaneDone;
-      } else {
-        v = list[k];
-        split_index(V, v, x, y, z);
-        cur = {(float)x, (float)y, (float)z};
-        iters = A.P.iteration_limit;
-        anchor = cur;
-        t_iters = iters;
-        t_n = 0;
-        last_nv = -1;
-        phase = kLaneEnter;
+    {
+      unsigned long long t = 0;
+      const bool got = items.take(phase == kLaneIdle, (unsigned long long)n, work,
+                                  [&](unsigned long long j) { return (int32_t)list[j]; }, t, v);
+      if (phase == kLaneIdle) {
+        if (!got) {
+          phase = kLaneDone;
+        } else {
+          int x, y, z;
+          split_index(V, v, x, y, z);
+          A.start(L, x, y, z, -1);
+          phase = kLaneEnter;
+        }
       }
     }
     if (__all_sync(kFullMask, phase == kLaneDone)) {
@@ -1363,31 +1469,23 @@ __global__ void __launch_bounds__(128, 7) fixup_end32_kernel(const Adv32 A, cons
     }
     for (int r = 0; r < K; r++) {
       if (phase != kLaneEnter && phase != kLaneStep) continue;
-      ev = A.advance(phase, x, y, z, cur, old, iters, nb, b, c, g, gm, step, slim, gm_end, last_nv, ntrips);
-      if (ev == EV_NONE) continue;
-      A.nearest3(cur, x, y, z);
-      phase = ev == EV_OUT_OF_VOXEL ? kLaneEnter : kLaneEnd;
-    }
-    {
-      if (phase == kLaneStep && A.P.trap_window > 0 && t_iters - iters >= A.P.trap_window) {
-        t_iters = iters;
-        if (A.trapped(cur, anchor, t_n)) {  // ends where the iteration limit would have
-          ev = EV_OVER_MAX_ITERATIONS;
-          A.nearest3(cur, x, y, z);
-          phase = kLaneEnd;
-        }
-      }
+      bool out;
+      ev = A.advance(phase, L, out);
+      if (ev != EV_NONE) phase = kLaneEnd;
     }
     if (phase != kLaneEnd) continue;
     phase = kLaneIdle;
-    const int64_t end = vid(V, x, y, z);
+    ntrips += (unsigned long long)(A.P.iteration_limit - L.iters);
+    int x, y, z;
+    A.nearest3(L.cur, x, y, z);
+    const int64_t end = A.index(x, y, z);
     // a low-gradient stop whose FP32 magnitude lies within 2^-8 (relative) of the
     // threshold: FP32 rounding could have taken the other side of the stop test.  A
     // streamline that decelerates into an extremum crosses the threshold well inside
     // that test's FP32 accuracy otherwise, and FP64 would stop it at the same step.
-    bool ambiguous = ev == EV_LOW_GRADIENT && gm_end >= A.P.gthresh * (1.f - 1.f / 256.f);
+    bool ambiguous = ev == EV_LOW_GRADIENT && L.gm_end >= A.P.gthresh * (1.f - 1.f / 256.f);
     if (!ambiguous && ev == EV_HIT_PREASSIGNED && amb_mode == 0) {
-      const float pc[3] = {cur.x, cur.y, cur.z};
+      const float pc[3] = {L.cur.x, L.cur.y, L.cur.z};
       const int64_t ext[3] = {V.X, V.Y, V.Z};
       const int64_t ev3[3] = {x, y, z};
       // the end is a certain terminal here, whose label no pass changes (the ends can
@@ -1407,8 +1505,8 @@ __global__ void __launch_bounds__(128, 7) fixup_end32_kernel(const Adv32 A, cons
         if ((st == kStSeed || st == kStTerminal) && lab[u] != le) ambiguous = true;
       }
     } else if (!ambiguous && ev == EV_HIT_PREASSIGNED) {
-      const int64_t bb[3] = {(int)fminf(fmaxf(cur.x, 0.f), A.ext2[0]), (int)fminf(fmaxf(cur.y, 0.f), A.ext2[1]),
-                             (int)fminf(fmaxf(cur.z, 0.f), A.ext2[2])};
+      const int64_t bb[3] = {(int)fminf(fmaxf(L.cur.x, 0.f), A.ext2[0]), (int)fminf(fmaxf(L.cur.y, 0.f), A.ext2[1]),
+                             (int)fminf(fmaxf(L.cur.z, 0.f), A.ext2[2])};
       int32_t seen = kLabelNone;
 #pragma unroll
       for (int q = 0; q < 8; q++) {
@@ -1728,11 +1826,8 @@ __global__ void clean_resolve_kernel(const int32_t* __restrict__ lab, const VolD
 
 // ---- launchers ---------------------------------------------------------------------------
 
-// Stepping iterations per turn of the lane-refilling loops: more amortise the turn's
-// hand-out and voxel-entry work, fewer leave less idle time after a lane's event.
-// MSC_TRIPS_PER_TURN (2, 4, 8 or 16) overrides the default for tuning (512^3 k^-3
-// labels, both stages alike: 0.44 / 0.43 / 0.42 s for 4 / 8 / 16).
-// MSC_TRIPS_PER_TURN_PASS1 sets the first pass's apart from the fix-up's.
+// MSC_TRIPS_PER_TURN_FP64 (2, 4, 8 or 16): stepping iterations per turn of the FP64 loop,
+// for tuning.
 static int trips_env(const char* name, int dflt) {
   const char* e = std::getenv(name);
   const int v = e ? std::atoi(e) : dflt;
@@ -1746,9 +1841,14 @@ int lane_ctas_per_sm() {
   }();
   return k;
 }
-int trips_per_turn() {
-  static const int k = trips_env("MSC_TRIPS_PER_TURN", 16);
-  return k;
+// The corner test of Adv32<true> holds for these parameters (MSC_STOP_TEST=memory: the
+// general path all the same, for the test that compares the two).
+static bool short_steps(const IntegParams& P) {
+  static const bool memory = [] {
+    const char* e = std::getenv("MSC_STOP_TEST");
+    return e && std::string(e) == "memory";
+  }();
+  return !memory && P.max_step >= 0.0 && P.max_step <= (double)kShortStep && P.ethresh <= kShortThresh;
 }
 namespace {
 int grid_for(int64_t n, int num_sms) {
@@ -1757,16 +1857,18 @@ int grid_for(int64_t n, int num_sms) {
 }
 }  // namespace
 
-static int trips_per_turn_pass1() {
-  static const int k = trips_env("MSC_TRIPS_PER_TURN_PASS1", trips_per_turn());
-  return k;
-}
-
 cudaError_t launch_count_unlabelled(const uint8_t* lvl, int64_t N, unsigned long long* n, int num_sms,
                                     cudaStream_t stream) {
   if (cudaError_t e = cudaMemsetAsync(n, 0, sizeof(unsigned long long), stream)) return e;
   ::msc::count_launch();
   count_unlabelled_kernel<<<num_sms * 4, 256, 0, stream>>>(lvl, N, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_label_gradient(const float* f, const int32_t* lab, const uint32_t* zeroed, const VolDims& V,
+                                  uint8_t* state, float4* g32, int num_sms, cudaStream_t stream) {
+  ::msc::count_launch();
+  label_gradient_kernel<<<num_sms * 8, 256, 0, stream>>>(f, lab, zeroed, V, state, g32);
   return cudaGetLastError();
 }
 
@@ -1793,24 +1895,16 @@ cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParam
                              int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, uint32_t* claim,
                              unsigned long long* work, unsigned long long* trips, int num_sms, cudaStream_t stream) {
   if (k1 <= k0) return cudaSuccess;
-  const Adv32 A = Adv32::make(G, V, P, lvl, stamp, nullptr);
   const int64_t blocks = (k1 - k0 + 127) / 128;
   const int cap = num_sms * lane_ctas_per_sm();
   const int grid = (int)(blocks < cap ? blocks : cap);
   ::msc::count_launch();
-  switch (trips_per_turn_pass1()) {
-    case 2:
-      speculate_kernel<2><<<grid, 128, 0, stream>>>(A, Q, k0, k1, lab, claim, work, trips);
-      break;
-    case 4:
-      speculate_kernel<4><<<grid, 128, 0, stream>>>(A, Q, k0, k1, lab, claim, work, trips);
-      break;
-    case 8:
-      speculate_kernel<8><<<grid, 128, 0, stream>>>(A, Q, k0, k1, lab, claim, work, trips);
-      break;
-    default:
-      speculate_kernel<16><<<grid, 128, 0, stream>>>(A, Q, k0, k1, lab, claim, work, trips);
-  }
+  if (short_steps(P))
+    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr), Q, k0, k1, lab,
+                                                     claim, work, trips);
+  else
+    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr), Q, k0, k1, lab,
+                                                      claim, work, trips);
   return cudaGetLastError();
 }
 
@@ -1871,9 +1965,10 @@ cudaError_t launch_spec_jumps(const SpecSet& Q, int64_t k0, int64_t k1, int num_
 }
 
 cudaError_t launch_spec_write(const SpecSet& Q, int64_t k0, int64_t k1, uint8_t* lvl, int stamp, const uint32_t* claim,
-                              int32_t* lab, int* long_chain, int num_sms, cudaStream_t stream) {
+                              int32_t* lab, float4* g32, int* long_chain, int num_sms, cudaStream_t stream) {
   ::msc::count_launch();
-  spec_write_kernel<<<grid_for(k1 - k0, num_sms), 256, 0, stream>>>(Q, k0, k1, lvl, stamp, claim, lab, long_chain);
+  spec_write_kernel<<<grid_for(k1 - k0, num_sms), 256, 0, stream>>>(Q, k0, k1, lvl, stamp, claim, lab, g32,
+                                                                    long_chain);
   return cudaGetLastError();
 }
 
@@ -1928,7 +2023,6 @@ cudaError_t launch_fixup_end32(const float4* G, const VolDims& V, const IntegPar
                                int* n_amb, int amb_mode, unsigned long long* work, unsigned long long* trips,
                                int num_sms, cudaStream_t stream, const int* n_dev) {
   if (n <= 0) return cudaSuccess;
-  const Adv32 A = Adv32::make(G, V, P, nullptr, 0, state);
   const int blocks = (n + 127) / 128;
   if (cudaError_t e = cudaMemsetAsync(work, 0, sizeof(unsigned long long), stream)) return e;
   ::msc::count_launch();
@@ -1942,23 +2036,12 @@ cudaError_t launch_fixup_end32(const float4* G, const VolDims& V, const IntegPar
   }();
   const int cap = num_sms * (n_dev ? early_ctas : lane_ctas_per_sm());
   const int grid = blocks < cap ? blocks : cap;
-  switch (trips_per_turn()) {
-    case 16:
-      fixup_end32_kernel<16><<<grid, 128, 0, stream>>>(A, lab, state, list, n, n_dev, endv, amb, n_amb, amb_mode, work,
-                                                          trips);
-      break;
-    case 2:
-      fixup_end32_kernel<2><<<grid, 128, 0, stream>>>(A, lab, state, list, n, n_dev, endv, amb, n_amb, amb_mode, work,
-                                                          trips);
-      break;
-    case 4:
-      fixup_end32_kernel<4><<<grid, 128, 0, stream>>>(A, lab, state, list, n, n_dev, endv, amb, n_amb, amb_mode, work,
-                                                          trips);
-      break;
-    default:
-      fixup_end32_kernel<8><<<grid, 128, 0, stream>>>(A, lab, state, list, n, n_dev, endv, amb, n_amb, amb_mode, work,
-                                                          trips);
-  }
+  if (short_steps(P))
+    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state), lab, state, list,
+                                                       n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
+  else
+    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state), lab, state,
+                                                        list, n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
   return cudaGetLastError();
 }
 

@@ -111,10 +111,6 @@ __global__ void iota_kernel(int32_t* a, int n) {
 __global__ void fill_i32_kernel(int32_t* a, int64_t n, int32_t v) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) a[i] = v;
 }
-__global__ void terminal_state_kernel(const int32_t* lab, uint8_t* state, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    if (state[i] != msc::kStSeed) state[i] = lab[i] >= 0 ? msc::kStTerminal : msc::kStUnassigned;
-}
 // caller labels into the internal form: the reference's -1 ("none") reads as kLabelNone
 __global__ void none_in_kernel(const int32_t* in, int32_t* lab, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -135,7 +131,8 @@ __global__ void scatter_rep_kernel(const int32_t* pairs, int m, int32_t* rep) {
 __global__ void zero_seed_grad_kernel(const int64_t* seed, int n, float4* g32, uint32_t* zeroed) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int64_t s = seed[e];
-    g32[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float* g = reinterpret_cast<float*>(g32 + s);  // (the fourth component: what stops a streamline)
+    g[0] = g[1] = g[2] = 0.f;
     atomicOr(&zeroed[s >> 5], 1u << (s & 31));
   }
 }
@@ -355,12 +352,6 @@ int setup_ctx(LabelCtx& c, const float* f, const uint8_t* grad, const int64_t* d
   LCUDA(c.pool.get(&c.counters, 16), "alloc");
   LCUDA(c.pool.get(&c.work, 64), "alloc");
   LCUDA(cudaMemsetAsync(c.counters, 0, 16 * sizeof(int), c.st), "memset");
-  msc::GradDims GD{};
-  for (int a = 0; a < 3; a++) {
-    GD.v[a] = dims[a];
-    GD.d[a] = 2 * dims[a] - 1;
-  }
-  LCUDA(msc::launch_central_diff(3, 1, f, c.g32, GD, c.sms, c.st), "gradient f32");
   LCUDA(cudaMemsetAsync(c.zeroed, 0, (size_t)(N / 32 + 1) * sizeof(uint32_t), c.st), "memset");
   return MSC_OK;
 }
@@ -524,8 +515,7 @@ int prepare_direction(LabelCtx& c, DirLabels& d, int32_t* stage_terminal) {
     ::msc::count_launch();
     snapshot_kernel<<<c.grid, 256, 0, st>>>(d.lab, stage_terminal, N);
   }
-  ::msc::count_launch();
-  terminal_state_kernel<<<c.grid, 256, 0, st>>>(d.lab, d.state, N);
+  LCUDA(msc::launch_label_gradient(c.f, d.lab, c.zeroed, V, d.state, c.g32, c.sms, st), "gradient f32");
   if (d.before_integration)
     if (int rc = d.before_integration()) return rc;
   return MSC_OK;
@@ -696,12 +686,12 @@ int first_pass(LabelCtx& c, DirLabels& d) {
       trace_mark(st, d.dir, "  resolved");
       LCUDA(msc::launch_spec_ptr(Q, k0, k1, claim, c.sms, st), "label");
       LCUDA(cudaMemsetAsync(Q.overflow, 0, sizeof(int), st), "memset");
-      LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, Q.overflow, c.sms, st), "label");
+      LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, c.g32, Q.overflow, c.sms, st), "label");
       int long_chain = 0;
       if (int rc = read_dev(c, Q.overflow, 1, &long_chain)) return rc;
       if (long_chain) {  // a few long chains of cut items: jump, then write again
         LCUDA(msc::launch_spec_jumps(Q, k0, k1, c.sms, st), "label");
-        LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, Q.overflow, c.sms, st), "label");
+        LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, c.g32, Q.overflow, c.sms, st), "label");
       }
       batches++;
       trace_mark(st, d.dir, "batch " + std::to_string(g0) + "-" + std::to_string(L1 - 1) + " items " +

@@ -193,6 +193,23 @@ int msc_ms_graph_3d(const uint8_t* grad, const float* f, const int64_t dims[3], 
                     uint8_t* node_boundary, int64_t arc_cap, int32_t* arc_lower, int32_t* arc_upper,
                     float* arc_persistence, int64_t counts[2], msc_stream_t stream);
 
+/* The same in one call for callers that allocate on demand: alloc(ctx, array, count) is
+ * called once per output array when its length is known (the four node arrays, then the
+ * three arc arrays), on the calling thread, and returns device memory for `count`
+ * elements of the array's type (NULL or anything for count 0; NULL otherwise ends the call
+ * with MSC_ERR_OOM).  The library writes the arrays on `stream` and never frees them.
+ * Sizing the arrays with a first call of msc_ms_graph_3d traces every V-path twice. */
+#define MSC_GRAPH_NODE_CELL 0       /* int64 */
+#define MSC_GRAPH_NODE_VALUE 1      /* float */
+#define MSC_GRAPH_NODE_DIM 2        /* uint8 */
+#define MSC_GRAPH_NODE_BOUNDARY 3   /* uint8 */
+#define MSC_GRAPH_ARC_LOWER 4       /* int32 */
+#define MSC_GRAPH_ARC_UPPER 5       /* int32 */
+#define MSC_GRAPH_ARC_PERSISTENCE 6 /* float */
+typedef void* (*msc_graph_alloc_fn)(void* ctx, int array, int64_t count);
+int msc_ms_graph_alloc_3d(const uint8_t* grad, const float* f, const int64_t dims[3], const int build_arcs[3],
+                          msc_graph_alloc_fn alloc, void* ctx, int64_t counts[2], msc_stream_t stream);
+
 /* The saddle streamline digitizers of ondemandaccurate's needASC1 / needDSC1 modes
  * (ReIntegrateUpFrom2Saddles / ReIntegrateDownFrom1Saddles, ondemandaccurate.cxx:254-505,
  * with DigitizingNumericStreamlineIntegrator3dASC / 3dDSC,

@@ -22,6 +22,7 @@ ERRORS = {
 # every symbol include/msc_gpu.h declares: (restype, argtypes)
 _I64P = ctypes.POINTER(ctypes.c_int64)
 _VP = ctypes.c_void_p
+GRAPH_ALLOC = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64)  # msc_graph_alloc_fn
 SIGNATURES = {
     "msc_version": (ctypes.c_int, []),
     "msc_last_error_string": (ctypes.c_char_p, []),
@@ -61,6 +62,8 @@ SIGNATURES = {
     # grad f dims build node_cap cell value dim boundary arc_cap lower upper persistence counts stream
     "msc_ms_graph_3d": (ctypes.c_int, [_VP, _VP, _I64P, _VP, ctypes.c_int64, _VP, _VP, _VP, _VP, ctypes.c_int64, _VP,
                                        _VP, _VP, _I64P, _VP]),
+    # grad f dims build alloc ctx counts stream
+    "msc_ms_graph_alloc_3d": (ctypes.c_int, [_VP, _VP, _I64P, _VP, GRAPH_ALLOC, _VP, _I64P, _VP]),
     # f grad zeroed dims which params cells stats stream
     "msc_saddle_lines_3d": (ctypes.c_int, [_VP, _VP, _VP, _I64P, ctypes.c_int, _VP, _VP, _I64P, _VP]),
 }

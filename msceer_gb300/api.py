@@ -221,7 +221,7 @@ def conforming_grad(f, grad, labels_asc=None, labels_dsc=None, restriction=False
 
 def ms_graph(grad, f, build_arcs=(1, 0, 1)):
     """MorseSmaleComplexBasic::ComputeFromGrad without arc geometry on a device .grad
-    (msc_ms_graph_3d): the critical cells as nodes and the traced V-paths as arcs.
+    (msc_ms_graph_alloc_3d): the critical cells as nodes and the traced V-paths as arcs.
     ``grad``: CUDA uint8 .grad of ``f`` (CUDA float32 (Z, Y, X)); ``build_arcs``: the
     reference's SetBuildArcs flags (arcs from 1-saddles, 2-saddles, maxima; extractmsc
     uses (1, 0, 1)).  Returns a dict of CUDA tensors: node_cell (int64), node_value
@@ -239,23 +239,26 @@ def ms_graph(grad, f, build_arcs=(1, 0, 1)):
     b = (ctypes.c_int * 3)(*[int(x) for x in build_arcs])
     counts = (ctypes.c_int64 * 2)()
     ptr = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    arrays = (("node_cell", torch.int64), ("node_value", torch.float32), ("node_dim", torch.uint8),
+              ("node_boundary", torch.uint8), ("arc_lower", torch.int32), ("arc_upper", torch.int32),
+              ("arc_persistence", torch.float32))
+    out, failed = {}, []
+
+    def alloc(_, array, count):
+        try:
+            name, dtype = arrays[array]
+            out[name] = torch.empty(count, dtype=dtype, device=dev)
+            return out[name].data_ptr()
+        except Exception as e:  # nothing may be raised through the library
+            failed.append(e)
+            return None
+
     with torch.cuda.device(dev):
-        rc = lib.msc_ms_graph_3d(ptr(grad), ptr(f), _lib.dims_arg(dims), b, 0, None, None, None, None, 0, None, None,
-                                 None, counts, ctypes.c_void_p(stream))
-        _lib.check(rc, "msc_ms_graph_3d")
-        nn, na = counts[0], counts[1]
-        out = {"node_cell": torch.empty(nn, dtype=torch.int64, device=dev),
-               "node_value": torch.empty(nn, dtype=torch.float32, device=dev),
-               "node_dim": torch.empty(nn, dtype=torch.uint8, device=dev),
-               "node_boundary": torch.empty(nn, dtype=torch.uint8, device=dev),
-               "arc_lower": torch.empty(na, dtype=torch.int32, device=dev),
-               "arc_upper": torch.empty(na, dtype=torch.int32, device=dev),
-               "arc_persistence": torch.empty(na, dtype=torch.float32, device=dev)}
-        rc = lib.msc_ms_graph_3d(ptr(grad), ptr(f), _lib.dims_arg(dims), b, nn, ptr(out["node_cell"]),
-                                 ptr(out["node_value"]), ptr(out["node_dim"]), ptr(out["node_boundary"]), na,
-                                 ptr(out["arc_lower"]), ptr(out["arc_upper"]), ptr(out["arc_persistence"]), counts,
-                                 ctypes.c_void_p(stream))
-        _lib.check(rc, "msc_ms_graph_3d")
+        rc = lib.msc_ms_graph_alloc_3d(ptr(grad), ptr(f), _lib.dims_arg(dims), b, _lib.GRAPH_ALLOC(alloc), None, counts,
+                                       ctypes.c_void_p(stream))
+        if failed:
+            raise failed[0]
+        _lib.check(rc, "msc_ms_graph_alloc_3d")
     return out
 
 

@@ -455,10 +455,12 @@ int scan_in_place(Pool& P, int64_t* a, int64_t n, int64_t* sum, cudaStream_t str
   return MSC_OK;
 }
 
+// alloc (when set) supplies every output array once its length is known; the arrays passed
+// are then ignored.
 int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const int* build, int64_t node_cap,
                   int64_t* node_cell, float* node_value, uint8_t* node_dim, uint8_t* node_boundary, int64_t arc_cap,
-                  int32_t* arc_lower, int32_t* arc_upper, float* arc_pers, int64_t* counts_out,
-                  cudaStream_t stream) {
+                  int32_t* arc_lower, int32_t* arc_upper, float* arc_pers, int64_t* counts_out, msc_graph_alloc_fn alloc,
+                  void* alloc_ctx, cudaStream_t stream) {
   if (!dims || !build || !counts_out) return fail(MSC_ERR_NULL_POINTER, "null argument");
   GradDims D;
   if (!make_grad_dims(3, dims, &D)) return fail(MSC_ERR_BAD_DIMS, "invalid dims");
@@ -496,6 +498,15 @@ int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const i
   const int64_t n = h[0];
   if (n >= ((int64_t)1 << 31)) return fail(MSC_ERR_BAD_DIMS, "more than 2^31 - 1 critical cells");
 
+  if (alloc) {
+    node_cell = static_cast<int64_t*>(alloc(alloc_ctx, MSC_GRAPH_NODE_CELL, n));
+    node_value = static_cast<float*>(alloc(alloc_ctx, MSC_GRAPH_NODE_VALUE, n));
+    node_dim = static_cast<uint8_t*>(alloc(alloc_ctx, MSC_GRAPH_NODE_DIM, n));
+    node_boundary = static_cast<uint8_t*>(alloc(alloc_ctx, MSC_GRAPH_NODE_BOUNDARY, n));
+    node_cap = n;
+    if (n > 0 && !(node_cell && node_value && node_dim && node_boundary))
+      return fail(MSC_ERR_OOM, "the node arrays were not allocated");
+  }
   const bool nodes_out = node_cell && node_value && node_dim && node_boundary && node_cap >= n;
   int64_t* cells = node_cell;
   float* vals = node_value;
@@ -515,8 +526,8 @@ int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const i
   GCUDA(P.get((void**)&n_tlist, 3 * sizeof(unsigned long long)), "scratch alloc(traced and kept counts)");
   // room for two arcs a node of any dimension (rough fields have 1.5 with extractmsc's
   // flags; what does not fit is traced again)
-  const bool want_arcs = arc_lower && arc_upper && arc_cap > 0;
-  const int64_t store_cap = want_arcs ? std::min<int64_t>(arc_cap, 2 * n + 4096) : 0;
+  const bool want_arcs = alloc || (arc_lower && arc_upper && arc_cap > 0);
+  const int64_t store_cap = !want_arcs ? 0 : (alloc ? 2 * n + 4096 : std::min<int64_t>(arc_cap, 2 * n + 4096));
   int32_t* store = nullptr;
   int64_t* place = nullptr;
   if (want_arcs) {
@@ -549,6 +560,13 @@ int ms_graph_impl(const uint8_t* g, const float* f, const int64_t* dims, const i
   counts_out[0] = n;
   counts_out[1] = na;
 
+  if (alloc) {
+    arc_lower = static_cast<int32_t*>(alloc(alloc_ctx, MSC_GRAPH_ARC_LOWER, na));
+    arc_upper = static_cast<int32_t*>(alloc(alloc_ctx, MSC_GRAPH_ARC_UPPER, na));
+    arc_pers = static_cast<float*>(alloc(alloc_ctx, MSC_GRAPH_ARC_PERSISTENCE, na));
+    arc_cap = na;
+    if (na > 0 && !(arc_lower && arc_upper && arc_pers)) return fail(MSC_ERR_OOM, "the arc arrays were not allocated");
+  }
   const bool arcs_out = arc_lower && arc_upper && arc_cap >= na;
   if (!nodes_out && !arcs_out) return MSC_OK;
   uint8_t* dims_b = node_dim;
@@ -584,8 +602,15 @@ int msc_ms_graph_3d(const uint8_t* grad, const float* f, const int64_t dims[3], 
                     uint8_t* node_boundary, int64_t arc_cap, int32_t* arc_lower, int32_t* arc_upper,
                     float* arc_persistence, int64_t counts[2], msc_stream_t stream) {
   return msc::ms_graph_impl(grad, f, dims, build_arcs, node_cap, node_cell, node_value, node_dim, node_boundary,
-                            arc_cap, arc_lower, arc_upper, arc_persistence, counts,
+                            arc_cap, arc_lower, arc_upper, arc_persistence, counts, nullptr, nullptr,
                             reinterpret_cast<cudaStream_t>(stream));
+}
+
+int msc_ms_graph_alloc_3d(const uint8_t* grad, const float* f, const int64_t dims[3], const int build_arcs[3],
+                          msc_graph_alloc_fn alloc, void* ctx, int64_t counts[2], msc_stream_t stream) {
+  if (!alloc) return msc::fail(MSC_ERR_NULL_POINTER, "null allocator");
+  return msc::ms_graph_impl(grad, f, dims, build_arcs, 0, nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr,
+                            nullptr, counts, alloc, ctx, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

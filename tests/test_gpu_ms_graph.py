@@ -105,3 +105,27 @@ def test_ms_graph_one_peak_vs_oracle(gpu, oracle, shape, noise):
     want = oracle.ms_graph(f, g.cpu().numpy(), (1, 1, 1))
     for k, v in want.items():
         assert np.array_equal(got[k].cpu().numpy(), v), k
+
+
+def test_ms_graph_allocator(gpu):
+    """The one-call form: each array asked for once with its final length, the result that of
+    the sized call, an allocator that fails ends the call."""
+    import torch
+    from msceer_gb300 import _lib, lower_star_grad, ms_graph
+    f = torch.from_numpy(fields.power_law_field((30, 27, 25), seed=2)).to(gpu)
+    g = lower_star_grad(f)
+    want = ms_graph(g, f, (1, 1, 1))
+    lib, p = _lib.load(), lambda x: ctypes.c_void_p(x.data_ptr())  # noqa: E731
+    s = ctypes.c_void_p(torch.cuda.current_stream(gpu).cuda_stream)
+    counts, build, asked = (ctypes.c_int64 * 2)(), (ctypes.c_int * 3)(1, 1, 1), []
+    fail = _lib.GRAPH_ALLOC(lambda ctx, array, count: asked.append((array, count)))
+    assert lib.msc_ms_graph_alloc_3d(p(g), p(f), _lib.dims_arg((30, 27, 25)), build, fail, None, counts, s) == -4
+    assert asked == [(a, want["node_cell"].numel()) for a in range(4)]
+    assert lib.msc_ms_graph_alloc_3d(p(g), p(f), _lib.dims_arg((30, 27, 25)), build, _lib.GRAPH_ALLOC(), None, counts, s) == -2
+    nn, na = want["node_cell"].numel(), want["arc_lower"].numel()
+    got = {k: torch.empty_like(v) for k, v in want.items()}
+    rc = lib.msc_ms_graph_3d(p(g), p(f), _lib.dims_arg((30, 27, 25)), build, nn, *[p(got[k]) for k in list(got)[:4]], na,
+                             *[p(got[k]) for k in list(got)[4:]], counts, s)
+    assert rc == 0 and (counts[0], counts[1]) == (nn, na)
+    for k in want:
+        assert torch.equal(got[k], want[k]), k

@@ -9,22 +9,29 @@
 #include "../../include/msc_triage.h"
 #include "triage.cuh"
 
+namespace {
+int sm_count() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 1;
+}
+}  // namespace
+
 namespace msc {
 
 cudaError_t triage_forward(const __nv_bfloat16* feat, const ConvDims& D, const float* params, uint8_t* blobs,
                            __nv_bfloat16* act1, __nv_bfloat16* act2, float* logits, int* err, cudaStream_t st) {
   cudaError_t e = launch_pack_weights(params, blobs, st);
   if (e != cudaSuccess) return e;
-  CUtensorMap m0, m1, m2;
-  if ((e = make_act_map(feat, D, &m0)) != cudaSuccess) return e;
-  if ((e = make_act_map(act1, D, &m1)) != cudaSuccess) return e;
-  if ((e = make_act_map(act2, D, &m2)) != cudaSuccess) return e;
   const float* bias = params + 3 * kTriageW;
-  if ((e = launch_conv3_tc(kEpiReluBf16, m0, blobs, bias, D, act1, nullptr, nullptr, err, st)) != cudaSuccess) return e;
-  if ((e = launch_conv3_tc(kEpiReluBf16, m1, blobs + 27 * 512, bias + 16, D, act2, nullptr, nullptr, err, st)) !=
+  const int sms = sm_count();
+  if ((e = launch_conv3_tc(kEpiReluBf16, feat, blobs, bias, D, act1, nullptr, nullptr, err, sms, st)) != cudaSuccess)
+    return e;
+  if ((e = launch_conv3_tc(kEpiReluBf16, act1, blobs + 27 * 512, bias + 16, D, act2, nullptr, nullptr, err, sms, st)) !=
       cudaSuccess)
     return e;
-  return launch_conv3_tc(kEpiLogits, m2, blobs + 2 * 27 * 512, bias + 32, D, nullptr, logits, nullptr, err, st);
+  return launch_conv3_tc(kEpiLogits, act2, blobs + 2 * 27 * 512, bias + 32, D, nullptr, logits, nullptr, err, sms, st);
 }
 
 }  // namespace msc
@@ -44,13 +51,6 @@ int fail(int code, const std::string& m) {
     if (e_ != cudaSuccess) return fail(MSC_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
-int sm_count() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 1;
-}
-
 bool conv_dims(const int64_t* dims, msc::ConvDims* D) {
   if (!dims || dims[0] < 1 || dims[1] < 1 || dims[2] < 1) return false;
   if (dims[0] > (1 << 24) || dims[1] > (1 << 24) || dims[2] > 65535) return false;
@@ -58,7 +58,8 @@ bool conv_dims(const int64_t* dims, msc::ConvDims* D) {
   return true;
 }
 
-// device scratch of one call, freed in stream order
+// device scratch of one call, from the library's pool (memory of the default pool is
+// mapped afresh by every call), freed in stream order
 struct Scratch {
   cudaStream_t st;
   std::vector<void*> p;
@@ -69,7 +70,7 @@ struct Scratch {
   template <class T>
   cudaError_t get(T** out, size_t bytes) {
     void* q = nullptr;
-    cudaError_t e = cudaMallocAsync(&q, bytes, st);
+    cudaError_t e = msc::scratch_alloc(&q, bytes, st);
     if (e == cudaSuccess) {
       p.push_back(q);
       *out = reinterpret_cast<T*>(q);
@@ -156,18 +157,15 @@ int msc_triage_backward_3d(const uint16_t* features, const uint16_t* act1, const
   float* gW = grads;
   float* gb = grads + 3 * msc::kTriageW;
   // layer 3
-  TCUDA(msc::launch_conv_wgrad(a2, dy3, D, gW + 2 * msc::kTriageW, gb + 32, sms, st), "weight gradient 3");
-  CUtensorMap m3, m2;
-  TCUDA(msc::make_act_map(dy3, D, &m3), "tensor map");
-  TCUDA(msc::launch_conv3_tc(msc::kEpiMaskBf16, m3, blobs + 4 * 27 * 512, nullptr, D, dy2, nullptr, a2, err, st),
+  TCUDA(msc::launch_conv_wgrad(a2, dy3, D, gW + 2 * msc::kTriageW, gb + 32, err, sms, st), "weight gradient 3");
+  TCUDA(msc::launch_conv3_tc(msc::kEpiMaskBf16, dy3, blobs + 4 * 27 * 512, nullptr, D, dy2, nullptr, a2, err, sms, st),
         "input gradient 3");
   // layer 2
-  TCUDA(msc::launch_conv_wgrad(a1, dy2, D, gW + msc::kTriageW, gb + 16, sms, st), "weight gradient 2");
-  TCUDA(msc::make_act_map(dy2, D, &m2), "tensor map");
-  TCUDA(msc::launch_conv3_tc(msc::kEpiMaskBf16, m2, blobs + 3 * 27 * 512, nullptr, D, dy1, nullptr, a1, err, st),
+  TCUDA(msc::launch_conv_wgrad(a1, dy2, D, gW + msc::kTriageW, gb + 16, err, sms, st), "weight gradient 2");
+  TCUDA(msc::launch_conv3_tc(msc::kEpiMaskBf16, dy2, blobs + 3 * 27 * 512, nullptr, D, dy1, nullptr, a1, err, sms, st),
         "input gradient 2");
   // layer 1
-  TCUDA(msc::launch_conv_wgrad(feat, dy1, D, gW, gb, sms, st), "weight gradient 1");
+  TCUDA(msc::launch_conv_wgrad(feat, dy1, D, gW, gb, err, sms, st), "weight gradient 1");
   return read_err(err, st);
 }
 

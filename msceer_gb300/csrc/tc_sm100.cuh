@@ -27,6 +27,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // bounded wait for the phase with the given parity to complete
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = 1u << 22) {
   for (uint32_t i = 0; i < limit; i++)
@@ -59,10 +62,11 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ---- descriptors ---------------------------------------------------------------------------
-// Shared-memory matrix descriptor, no swizzle, K-major canonical layout: 8-row x 16-byte
-// core matrices whose rows are 16 bytes apart; `kstride` = bytes between core matrices
-// adjacent along K (leading dimension), `mstride` = bytes between core matrices
-// adjacent along M/N (stride dimension).
+// Shared-memory matrix descriptor, no swizzle: 8-row x 16-byte core matrices whose rows
+// are 16 bytes apart.  K-major: a row is one M/N index with 8 BF16 along K; MN-major (a
+// transposed operand, see idesc_bf16_f32): a row is one K index with 8 along M/N.
+// `kstride` = bytes between core matrices adjacent along K (leading dimension), `mstride`
+// = bytes between core matrices adjacent along M/N (stride dimension).
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t kstride, uint32_t mstride) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
@@ -72,11 +76,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t kstride, 
   // base offset 0, absolute LBO mode 0, layout type 0 = no swizzle
   return d;
 }
-// Instruction descriptor of kind::f16: BF16 A and B (both K-major), FP32 accumulator.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
+// Instruction descriptor of kind::f16: BF16 A and B (both K-major, or both MN-major), FP32
+// accumulator.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool mn_major = false) {
   return (1u << 4)                         // D format: F32
          | (1u << 7)                       // A format: BF16
          | (1u << 10)                      // B format: BF16
+         | (mn_major ? 3u << 15 : 0u)      // A and B transposed
          | ((uint32_t)(N >> 3) << 17)      // N / 8
          | ((uint32_t)(M >> 4) << 24);     // M / 16
 }

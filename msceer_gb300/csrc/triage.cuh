@@ -1,7 +1,6 @@
 // Learned triage: shared declarations of the network kernels (triage_kernels.cu,
 // triage_train.cu) and the labeling glue (msc_triage_capi.cu).
 #pragma once
-#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -10,6 +9,7 @@
 namespace msc {
 
 void count_launch();  // msc_capi.cu
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t stream);
 
 struct ConvDims {
   int64_t X, Y, Z, N;  // vertices per axis, N = X*Y*Z
@@ -27,10 +27,12 @@ constexpr int kTriageParams = 3 * kTriageW + 3 * 16;
 
 constexpr int kTriageBlobBytes = 5 * 27 * 512;  // forward W1..W3, input-gradient W2, W3
 
-cudaError_t make_act_map(const __nv_bfloat16* act, const ConvDims& D, CUtensorMap* map);
-cudaError_t launch_conv3_tc(int epi, const CUtensorMap& in_map, const uint8_t* wblob, const float* bias,
+cudaError_t launch_conv3_tc(int epi, const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias,
                             const ConvDims& D, __nv_bfloat16* out_act, float* out_logits,
-                            const __nv_bfloat16* mask_act, int* err, cudaStream_t st);
+                            const __nv_bfloat16* mask_act, int* err, int num_sms, cudaStream_t st);
+// dW, db accumulate (zero before the first call); err: a device status word
+cudaError_t launch_conv_wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, const ConvDims& D, float* dW, float* db,
+                              int* err, int num_sms, cudaStream_t st);
 
 struct VolDims;
 cudaError_t launch_features(const float* f, const float4* g, const int32_t* lab, const uint8_t* state, const VolDims& V,
@@ -45,8 +47,6 @@ cudaError_t launch_change_targets(const int32_t* lab, const int32_t* first, int6
 cudaError_t launch_pack_weights(const float* params, uint8_t* blobs, cudaStream_t st);
 cudaError_t launch_bce_loss(const float* logits, const uint8_t* target, const ConvDims& D, float pos_weight,
                             float scale, __nv_bfloat16* dY, double* loss, int num_sms, cudaStream_t st);
-cudaError_t launch_conv_wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, const ConvDims& D, float* dW,
-                              float* db, int num_sms, cudaStream_t st);
 cudaError_t launch_adam(float* p, const float* g, float* m, float* v, int n, float lr, int step, const uint8_t* mask,
                         cudaStream_t st);
 

@@ -11,14 +11,18 @@
 // row: output vertices x0..x0+127 under tap (dx, dy, dz) read the staged row of
 // (y+dy, z+dz) starting at x0+dx.
 //
-// One CTA computes a 128 (x) x 4 (y) block of output rows at one z: a single TMA
-// load stages the 130 x 6 x 3 input rows (zero fill outside the volume = zero
-// padding), a bulk copy stages the 27 weight taps, one thread issues the 4 x 27
-// MMAs (M=128 vertices, N=16 output channels, K=16 input channels each) into four
-// TMEM accumulators, and four warps read them back for the epilogue.
-#include <cuda.h>
+// A tile is a 128 (x) x 4 (y) block of output rows at one z: its 130 x 6 x 3 input rows are
+// staged by bulk copies, one per 8-channel plane of a row (zeros outside the volume), one
+// thread issues the 4 x 27 MMAs (M=128 vertices, N=16 output channels, K=16 input channels
+// each) into four TMEM accumulators, and four warps read them back for the epilogue.  One
+// CTA per SM keeps the 27 weight taps in shared memory and works through its tiles with two
+// stages and two sets of accumulators, so that the load of a tile, the MMAs of the one
+// before and the epilogue of the one before that run side by side.
+// (A CTA per tile did the three one after another, with a TMEM allocation and the weights'
+// load for each: 181-217 us a layer at 128^3; so 152-159 us.  Tensor-map loads instead of
+// the bulk copies come to the same within a tenth.  The MMAs bound it, at 95 cycles each
+// whatever their N; a layer's activations in and out take 20 us of HBM time.)
 #include <cuda_bf16.h>
-#include <cudaTypedefs.h>
 
 #include "tc_sm100.cuh"
 #include "triage.cuh"
@@ -28,26 +32,21 @@ namespace msc {
 namespace {
 constexpr int kBX = 128;  // output vertices per row (MMA M)
 constexpr int kBY = 4;    // output rows per CTA (along y)
-constexpr int kInY = kBY + 2, kInZ = 3;
+constexpr int kInX = kBX + 2, kInY = kBY + 2, kInZ = 3;
 constexpr int kPlaneB = (kBX + 2) * 16;             // one staged 8-channel plane
 constexpr int kRowB = 2 * kPlaneB;                  // one staged row
 constexpr int kStageB = kRowB * kInY * kInZ;        // the TMA box
 constexpr int kTapB = 512;                          // 16 x 16 BF16 weights of one tap
 constexpr int kWeightB = 27 * kTapB;
-constexpr int kSmemConv = 1024 + kStageB + kWeightB + 64;
-constexpr uint32_t kTmemCols = 64;                  // 4 accumulators of 16 columns
+constexpr int kStages = 2;
+constexpr int kSmemConv = 1024 + kStages * kStageB + kWeightB + 128;
+constexpr uint32_t kSetCols = 64;                   // 4 accumulators of 16 columns
+constexpr uint32_t kTmemCols = kStages * kSetCols;
+constexpr int kConvThreads = 192;                   // four epilogue warps, the MMAs', the loads'
 static_assert(kStageB % 16 == 0 && kWeightB % 16 == 0, "bulk copy sizes");
-static_assert(kBY * 16 <= (int)kTmemCols, "accumulators fit the allocation");
+static_assert(kBY * 16 <= (int)kSetCols, "accumulators fit the allocation");
 }  // namespace
 
-__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2,
-                                            int c3, int c4) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
-      "[%7];" ::"r"(tc::smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(tc::smem_u32(bar))
-      : "memory");
-}
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    tc::smem_u32(dst)),
@@ -63,169 +62,410 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 //   kEpiReluBf16  out = bf16(relu(acc + bias))                         (hidden layers)
 //   kEpiLogits    logits[c][v] = acc[c] + bias[c], c < 2, FP32 planar  (output layer)
 //   kEpiMaskBf16  out = bf16(acc * (mask_act > 0))                     (input gradient)
+// Stages NX x NY x NZ vertices of a row-planar activation from (xs, ys, zs) on, both planes
+// of a row one after the other, zeros outside the volume; `bar` gets one arrival with the
+// bytes to come (and `more` bytes besides).  One whole warp calls it, after the stage's
+// last reader is done.
+template <int NX, int NY, int NZ>
+__device__ __forceinline__ void stage_rows(unsigned char* dst, const __nv_bfloat16* __restrict__ act, const ConvDims& D,
+                                           int xs, int ys, int zs, uint32_t more, uint64_t* bar) {
+  constexpr int ROWS = NY * NZ * 2, PLANE = NX * 16;
+  const int lane = threadIdx.x & 31;
+  const int xa = max(xs, 0), xb = (int)min((int64_t)(xs + NX), D.X);
+  auto row_of = [&](int p, int& y, int& z) {
+    y = ys + (p >> 1) % NY;
+    z = zs + (p >> 1) / NY;
+    return y >= 0 && y < D.Y && z >= 0 && z < D.Z;
+  };
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  int y, z;
+  if (xa > xs || xb < xs + NX)
+    for (int p = lane; p < ROWS; p += 32) {
+      uint4* r = reinterpret_cast<uint4*>(dst + p * PLANE);
+      for (int x = 0; x < xa - xs; x++) r[x] = zero;
+      for (int x = xb - xs; x < NX; x++) r[x] = zero;
+    }
+  if (ys < 0 || ys + NY > D.Y || zs < 0 || zs + NZ > D.Z)
+    for (int p = 0; p < ROWS; p++) {
+      if (row_of(p, y, z)) continue;
+      for (int x = lane; x < NX; x += 32) reinterpret_cast<uint4*>(dst + p * PLANE)[x] = zero;
+    }
+  tc::fence_proxy_async_smem();
+  __syncwarp();
+  const int ny = (int)min((int64_t)(ys + NY), D.Y) - max(ys, 0), nz = (int)min((int64_t)(zs + NZ), D.Z) - max(zs, 0);
+  const uint32_t bytes = (uint32_t)(xb - xa) * 16u;
+  if (lane == 0) mbar_expect_tx(bar, (uint32_t)(ny * nz * 2) * bytes + more);
+  __syncwarp();
+  for (int p = lane; p < ROWS; p += 32)
+    if (row_of(p, y, z))
+      bulk_load(dst + p * PLANE + (xa - xs) * 16,
+                act + ((((int64_t)z * D.Y + y) * 2 + (p & 1)) * D.X + xa) * 8, bytes, bar);
+}
+
+struct ConvTiles {
+  int nx, ny;
+  int64_t n;
+  __device__ __forceinline__ void at(int64_t t, int& x0, int& y0, int& z) const {
+    const int64_t r = t / nx;
+    x0 = (int)(t - r * nx) * kBX;
+    y0 = (int)(r % ny) * kBY;
+    z = (int)(r / ny);
+  }
+};
+
 template <int EPI>
-__global__ void __launch_bounds__(128) conv3_tc_kernel(const __grid_constant__ CUtensorMap in_map,
-                                                       const uint8_t* __restrict__ wblob, const float* __restrict__ bias,
-                                                       const ConvDims D, __nv_bfloat16* __restrict__ out_act,
-                                                       float* __restrict__ out_logits,
-                                                       const __nv_bfloat16* __restrict__ mask_act, int* __restrict__ err) {
+__device__ __forceinline__ void conv_epilogue(uint32_t tl, int x, int y0, int z, const float* __restrict__ bias,
+                                              const ConvDims& D, __nv_bfloat16* __restrict__ out_act,
+                                              float* __restrict__ out_logits,
+                                              const __nv_bfloat16* __restrict__ mask_act, uint64_t* done) {
+#pragma unroll 1
+  for (int j = 0; j < kBY; j++) {
+    float v[16];
+    tc::tmem_ld16(tl + 16 * j, v);
+    if (j == kBY - 1) {  // the accumulators are free for the next tile but one
+      tc::fence_before_sync();
+      __syncwarp();
+      if ((threadIdx.x & 31) == 0) tc::mbar_arrive(done);
+    }
+    const int y = y0 + j;
+    if (x >= D.X || y >= D.Y) continue;
+    const int64_t row = (int64_t)z * D.Y + y;
+    if (EPI == kEpiLogits) {
+      const int64_t vid = row * D.X + x;
+      out_logits[vid] = v[0] + bias[0];
+      out_logits[D.N + vid] = v[1] + bias[1];
+    } else {
+      __nv_bfloat16* o = out_act + row * 2 * D.X * 8;  // row base, plane 0
+      float m[16];
+      if (EPI == kEpiMaskBf16) {
+        const __nv_bfloat16* mk = mask_act + row * 2 * D.X * 8;
+        const uint4 q0 = *reinterpret_cast<const uint4*>(mk + (int64_t)x * 8);
+        const uint4 q1 = *reinterpret_cast<const uint4*>(mk + (int64_t)(D.X + x) * 8);
+        const __nv_bfloat16* h0 = reinterpret_cast<const __nv_bfloat16*>(&q0);
+        const __nv_bfloat16* h1 = reinterpret_cast<const __nv_bfloat16*>(&q1);
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+          m[c] = __bfloat162float(h0[c]) > 0.f ? 1.f : 0.f;
+          m[8 + c] = __bfloat162float(h1[c]) > 0.f ? 1.f : 0.f;
+        }
+      }
+      __align__(16) __nv_bfloat16 r[16];
+#pragma unroll
+      for (int c = 0; c < 16; c++) {
+        float a = v[c];
+        if (EPI == kEpiReluBf16) a = fmaxf(a + bias[c], 0.f);
+        else a = a * m[c];
+        r[c] = __float2bfloat16_rn(a);
+      }
+      *reinterpret_cast<uint4*>(o + (int64_t)x * 8) = *reinterpret_cast<const uint4*>(&r[0]);
+      *reinterpret_cast<uint4*>(o + (int64_t)(D.X + x) * 8) = *reinterpret_cast<const uint4*>(&r[8]);
+    }
+  }
+}
+
+// Every wait is bounded; a role whose wait runs out reports it in err and ends, and the
+// others' waits run out after it.
+template <int EPI>
+__global__ void __launch_bounds__(kConvThreads) conv3_tc_kernel(const __nv_bfloat16* __restrict__ in_act,
+                                                                const uint8_t* __restrict__ wblob,
+                                                                const float* __restrict__ bias, const ConvDims D,
+                                                                const ConvTiles T, __nv_bfloat16* __restrict__ out_act,
+                                                                float* __restrict__ out_logits,
+                                                                const __nv_bfloat16* __restrict__ mask_act,
+                                                                int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_in = sm;
-  unsigned char* s_w = sm + kStageB;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + kWeightB);  // [0] loads, [1] mma
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 2);
+  unsigned char* s_w = sm + kStages * kStageB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + kWeightB);
+  uint64_t* full = bars;                   // a stage's input rows (and, first of all, the weights) have come
+  uint64_t* empty = bars + kStages;        // its MMAs are done
+  uint64_t* tfull = bars + 2 * kStages;    // a set of accumulators is ready
+  uint64_t* tempty = bars + 3 * kStages;   // and read
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 4 * kStages);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int x0 = blockIdx.x * kBX, y0 = blockIdx.y * kBY, z = blockIdx.z;
-
   if (tid == 0) {
-    tc::mbar_init(&bars[0], 1);
-    tc::mbar_init(&bars[1], 1);
+    for (int q = 0; q < kStages; q++) {
+      tc::mbar_init(&full[q], 1);
+      tc::mbar_init(&empty[q], 1);
+      tc::mbar_init(&tfull[q], 1);
+      tc::mbar_init(&tempty[q], 4);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tc::tmem_alloc<kTmemCols>(s_tmem);
+  if (warp == 4) tc::tmem_alloc<kTmemCols>(s_tmem);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *s_tmem;
 
-  if (tid == 0) {
-    mbar_expect_tx(&bars[0], (uint32_t)(kStageB + kWeightB));
-    tma_load_5d(s_in, &in_map, &bars[0], 0, x0 - 1, 0, y0 - 1, z - 1);
-    bulk_load(s_w, wblob, (uint32_t)kWeightB, &bars[0]);
-  }
-  bool ok = tc::mbar_wait(&bars[0], 0);
-  if (tid == 0 && ok) {
-    tc::fence_after_sync();
-    constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 16);
-    const uint32_t a0 = tc::smem_u32(s_in), b0 = tc::smem_u32(s_w);
-#pragma unroll 1
-    for (int j = 0; j < kBY; j++) {
-#pragma unroll 1
-      for (int t = 0; t < 27; t++) {
-        const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;  // 0..2 = offset -1..+1
-        const uint32_t a = a0 + (uint32_t)((dz * kInY + j + dy) * kRowB + dx * 16);
-        tc::mma_bf16(tbase + 16 * j, tc::smem_desc(a, kPlaneB, 128), tc::smem_desc(b0 + t * kTapB, 256, 128), idesc,
-                     t > 0);
+  if (warp == 5) {  // loads
+    int64_t i = 0;
+    for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
+      const int q = (int)(i % kStages);
+      const bool ok = i < kStages || tc::mbar_wait(&empty[q], (uint32_t)(i / kStages - 1) & 1u);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) atomicOr(err, 1);
+        break;
       }
+      int x0, y0, z;
+      T.at(t, x0, y0, z);
+      if (i == 0 && lane == 0) bulk_load(s_w, wblob, (uint32_t)kWeightB, &full[q]);
+      stage_rows<kInX, kInY, kInZ>(s_in + q * kStageB, in_act, D, x0 - 1, y0 - 1, z - 1,
+                                   i == 0 ? (uint32_t)kWeightB : 0u, &full[q]);
     }
-    tc::mma_commit(&bars[1]);
-  }
-  if (!ok) {
-    if (tid == 0) atomicOr(err, 1);
-  } else {
-    ok = tc::mbar_wait(&bars[1], 0);
-    if (!ok && lane == 0) atomicOr(err, 2);
-  }
-  tc::fence_after_sync();
-  if (__all_sync(0xffffffffu, ok)) {
-    const int x = x0 + 32 * warp + lane;  // TMEM lane = output vertex
-    const uint32_t tl = tbase + ((uint32_t)(32 * warp) << 16);
+    // every load has landed before the block ends, also where the MMAs gave up on it
+    for (int64_t k = i > kStages ? i - kStages : 0; k < i; k++)
+      if (!tc::mbar_wait(&full[k % kStages], (uint32_t)(k / kStages) & 1u) && lane == 0) atomicOr(err, 1);
+  } else if (warp == 4) {  // MMAs
+    if (lane == 0) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 16);
+      const uint32_t b0 = tc::smem_u32(s_w);
+      int64_t i = 0;
+      for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
+        const int q = (int)(i % kStages);
+        if (!tc::mbar_wait(&full[q], (uint32_t)(i / kStages) & 1u) ||
+            (i >= kStages && !tc::mbar_wait(&tempty[q], (uint32_t)(i / kStages - 1) & 1u))) {
+          atomicOr(err, 1);
+          break;
+        }
+        tc::fence_after_sync();
+        const uint32_t a0 = tc::smem_u32(s_in + q * kStageB), d0 = tbase + q * kSetCols;
 #pragma unroll 1
-    for (int j = 0; j < kBY; j++) {
-      float v[16];
-      tc::tmem_ld16(tl + 16 * j, v);
-      const int y = y0 + j;
-      if (x >= D.X || y >= D.Y) continue;
-      const int64_t row = (int64_t)z * D.Y + y;
-      if (EPI == kEpiLogits) {
-        const int64_t vid = row * D.X + x;
-        out_logits[vid] = v[0] + bias[0];
-        out_logits[D.N + vid] = v[1] + bias[1];
-      } else {
-        __nv_bfloat16* o = out_act + row * 2 * D.X * 8;  // row base, plane 0
-        float m[16];
-        if (EPI == kEpiMaskBf16) {
-          const __nv_bfloat16* mk = mask_act + row * 2 * D.X * 8;
-          const uint4 q0 = *reinterpret_cast<const uint4*>(mk + (int64_t)x * 8);
-          const uint4 q1 = *reinterpret_cast<const uint4*>(mk + (int64_t)(D.X + x) * 8);
-          const __nv_bfloat16* h0 = reinterpret_cast<const __nv_bfloat16*>(&q0);
-          const __nv_bfloat16* h1 = reinterpret_cast<const __nv_bfloat16*>(&q1);
+        for (int tap = 0; tap < 27; tap++) {
+          const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;  // 0..2 = offset -1..+1
+          const uint64_t bd = tc::smem_desc(b0 + tap * kTapB, 256, 128);
 #pragma unroll
-          for (int c = 0; c < 8; c++) {
-            m[c] = __bfloat162float(h0[c]) > 0.f ? 1.f : 0.f;
-            m[8 + c] = __bfloat162float(h1[c]) > 0.f ? 1.f : 0.f;
+          for (int j = 0; j < kBY; j++) {  // (four accumulators in turn: no MMA waits for the one before)
+            const uint32_t a = a0 + (uint32_t)((dz * kInY + j + dy) * kRowB + dx * 16);
+            tc::mma_bf16(d0 + 16 * j, tc::smem_desc(a, kPlaneB, 128), bd, idesc, tap > 0);
           }
         }
-        __align__(16) __nv_bfloat16 r[16];
-#pragma unroll
-        for (int c = 0; c < 16; c++) {
-          float a = v[c];
-          if (EPI == kEpiReluBf16) a = fmaxf(a + bias[c], 0.f);
-          else a = a * m[c];
-          r[c] = __float2bfloat16_rn(a);
-        }
-        *reinterpret_cast<uint4*>(o + (int64_t)x * 8) = *reinterpret_cast<const uint4*>(&r[0]);
-        *reinterpret_cast<uint4*>(o + (int64_t)(D.X + x) * 8) = *reinterpret_cast<const uint4*>(&r[8]);
+        tc::mma_commit(&empty[q]);
+        tc::mma_commit(&tfull[q]);
       }
     }
+  } else {  // epilogue
+    int64_t i = 0;
+    for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
+      const int q = (int)(i % kStages);
+      const bool ok = tc::mbar_wait(&tfull[q], (uint32_t)(i / kStages) & 1u);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) atomicOr(err, 2);
+        break;
+      }
+      tc::fence_after_sync();
+      int x0, y0, z;
+      T.at(t, x0, y0, z);
+      // TMEM lane = output vertex
+      conv_epilogue<EPI>(tbase + q * kSetCols + ((uint32_t)(32 * warp) << 16), x0 + 32 * warp + lane, y0, z, bias, D,
+                         out_act, out_logits, mask_act, &tempty[q]);
+    }
   }
+  __syncwarp();
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 0) tc::tmem_dealloc<kTmemCols>(tbase);
+  tc::fence_after_sync();
+  if (warp == 4) tc::tmem_dealloc<kTmemCols>(tbase);
 }
 
-// ---- tensor map of a row-planar activation ----------------------------------------------
-namespace {
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+// ---- weight gradient ----------------------------------------------------------------------
+//
+// dW[tap][cin][cout] = sum over the vertices v of X[v + tap][cin] * dY[v][cout], db[cout] =
+// sum dY[v][cout]: the vertices are the MMA's K, so both operands are MN-major as the
+// row-planar rows lie (a core matrix is 8 channels x 8 vertices).  A tile's staged X is 18
+// rows (3 z x 6 y) of two 8-channel planes, all planes kPlaneB apart, so one M = 128
+// operand spans eight consecutive rows: for output row j the rows from j on hold the taps
+// (dy, dz) = (0..2, 0) and, six rows on, (0..1, 1); the rows from j + 8 on (2, 1) and, four
+// rows on, (0..2, 2).  With dx as a shift of 16 bytes, two MMAs per dx and 16 vertices
+// cover all 27 taps; the products of the other rows are not read.  The tensor core's FP32
+// accumulation loses up to an ulp per MMA, so its six accumulators (dx, which of the two)
+// run over one output row only, eight MMAs, and are added to FP32 registers; two sets take
+// turns, so that a row's MMAs run while the one before is read.  Against 64 bits the
+// layer-3 gradient at 128^3 is off by 2.9e-7 (4.4e-7 with FP32 FMAs, 4.3e-6 with the
+// accumulators kept in TMEM over all tiles).
+// The CUDA-core form (27 x 2 accumulators per thread, X and dY staged as FP32) took 1.0 ms
+// a layer at 128^3; this one 197-211 us.
+constexpr int kDyB = kBY * 2 * kBX * 16;  // staged dY rows
+constexpr int kSmemWgrad = 1024 + kStageB + kDyB + 64;
+constexpr uint32_t kWgradSet = 96;        // 6 x 16 columns
+constexpr uint32_t kWgradCols = 256;      // two sets
+static_assert(18 * kRowB == kStageB && kRowB <= kDyB, "the row after the last staged one lies in shared memory");
+
+__global__ void __launch_bounds__(128, 2) conv_wgrad_tc_kernel(const __nv_bfloat16* __restrict__ X,
+                                                               const __nv_bfloat16* __restrict__ dY, const ConvDims D,
+                                                               const ConvTiles T, float* __restrict__ dW,
+                                                               float* __restrict__ db, int* __restrict__ err) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* s_x = sm;
+  unsigned char* s_dy = sm + kStageB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dy + kDyB);  // [0] loads, [1] [2] the MMAs of a set
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 3);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int q = 0; q < 3; q++) tc::mbar_init(&bars[q], q == 0 ? 2 : 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  return fn;
-}
-}  // namespace
+  if (warp == 0) tc::tmem_alloc<kWgradCols>(s_tmem);
+  // the row after the last staged one is read for products that are not used
+  for (int i = tid; i < kDyB / 16; i += 128) reinterpret_cast<uint4*>(s_dy)[i] = make_uint4(0u, 0u, 0u, 0u);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tbase = *s_tmem, tlane = tbase + ((uint32_t)(32 * warp) << 16);
+  constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 16, true);
+  const uint32_t a0 = tc::smem_u32(s_x), b0 = tc::smem_u32(s_dy);
 
-cudaError_t make_act_map(const __nv_bfloat16* act, const ConvDims& D, CUtensorMap* map) {
-  auto fn = encode_fn();
-  if (!fn) return cudaErrorNotSupported;
-  if ((reinterpret_cast<uintptr_t>(act) & 15u) != 0) return cudaErrorInvalidValue;
-  const cuuint64_t dims[5] = {8, (cuuint64_t)D.X, 2, (cuuint64_t)D.Y, (cuuint64_t)D.Z};
-  const cuuint64_t strides[4] = {16, (cuuint64_t)D.X * 16, (cuuint64_t)D.X * 32, (cuuint64_t)D.X * D.Y * 32};
-  const cuuint32_t box[5] = {8, kBX + 2, 2, kInY, kInZ};
-  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(act), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+  float acc[6][16], bsum[16];
+#pragma unroll
+  for (int c = 0; c < 16; c++) bsum[c] = 0.f;
+#pragma unroll
+  for (int q = 0; q < 6; q++)
+#pragma unroll
+    for (int c = 0; c < 16; c++) acc[q][c] = 0.f;
+  uint32_t parity = 0;
+  bool ok = true;
+  for (int64_t t = blockIdx.x; t < T.n && ok; t += gridDim.x, parity ^= 1u) {
+    int x0, y0, z;
+    T.at(t, x0, y0, z);
+    if (warp == 0) {
+      stage_rows<kBX, kBY, 1>(s_dy, dY, D, x0, y0, z, 0u, &bars[0]);
+      stage_rows<kInX, kInY, kInZ>(s_x, X, D, x0 - 1, y0 - 1, z - 1, 0u, &bars[0]);
+    }
+    ok = tc::mbar_wait(&bars[0], parity);
+    if (!ok && lane == 0) atomicOr(err, 1);
+    ok = __syncthreads_and(ok);
+    // row j's MMAs go out, then row j - 1's accumulators are read; a set's barrier
+    // completes twice a tile
+#pragma unroll 1
+    for (int j = 0; j <= kBY && ok; j++) {
+      if (tid == 0 && j < kBY) {
+        tc::fence_after_sync();
+        const uint32_t d0 = tbase + (j & 1) * kWgradSet;
+#pragma unroll 1
+        for (int k = 0; k < kBX; k += 16) {
+          const uint64_t bd = tc::smem_desc(b0 + (uint32_t)(j * 2 * kBX * 16 + k * 16), 128, kBX * 16);
+#pragma unroll
+          for (int q = 0; q < 6; q++) {
+            const uint32_t a = a0 + (uint32_t)((j + 8 * (q & 1)) * kRowB + (k + (q >> 1)) * 16);
+            tc::mma_bf16(d0 + 16 * q, tc::smem_desc(a, 128, kPlaneB), bd, idesc, k > 0);
+          }
+        }
+        tc::mma_commit(&bars[1 + (j & 1)]);
+      }
+      if (j < kBY) {  // the bias gradient while the MMAs run: thread = vertex along x
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+          const uint4 q = *reinterpret_cast<const uint4*>(s_dy + ((j * 2 + p) * kBX + tid) * 16);
+          const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&q);
+#pragma unroll
+          for (int c = 0; c < 8; c++) bsum[8 * p + c] += __bfloat162float(h[c]);
+        }
+      }
+      __syncwarp();
+      if (j > 0) {
+        const int i = j - 1;
+        ok = tc::mbar_wait(&bars[1 + (i & 1)], (uint32_t)(i >> 1) & 1u);
+        if (!ok && lane == 0) atomicOr(err, 2);
+        if (__all_sync(0xffffffffu, ok)) {
+          tc::fence_after_sync();
+#pragma unroll
+          for (int q = 0; q < 6; q++) {
+            float v[16];
+            tc::tmem_ld16(tlane + (i & 1) * kWgradSet + 16 * q, v);
+#pragma unroll
+            for (int c = 0; c < 16; c++) acc[q][c] += v[c];
+          }
+        }
+        tc::fence_before_sync();
+        ok = __syncthreads_and(ok);  // the set is free, and after the last row the buffers
+      }
+    }
+    if (!ok && tid == 0) {  // nothing in flight when the block ends
+      tc::mbar_wait(&bars[0], parity);
+      tc::mbar_wait(&bars[1], 1);
+      tc::mbar_wait(&bars[2], 1);
+    }
+  }
+  if (ok) {
+    // TMEM lane = row of the operand: 16 r + channel of the r-th of its eight rows
+    const int r = 2 * warp + (lane >> 4), ci = lane & 15;
+#pragma unroll
+    for (int q = 0; q < 6; q++) {
+      const int dx = q >> 1;
+      int dy, dz;
+      if ((q & 1) == 0) {
+        dz = r >= 6 ? 1 : 0;
+        dy = r >= 6 ? r - 6 : r;
+      } else {
+        dz = r >= 4 ? 2 : 1;
+        dy = r >= 4 ? r - 4 : (r == 0 ? 2 : 3);
+      }
+      if (dy > 2) continue;
+      float* w = dW + (dx + 3 * dy + 9 * dz) * 256 + ci * 16;
+#pragma unroll
+      for (int c = 0; c < 16; c++) atomicAdd(&w[c], acc[q][c]);
+    }
+#pragma unroll
+    for (int c = 0; c < 16; c++) {
+      float b = bsum[c];
+#pragma unroll
+      for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+      if (lane == 0) atomicAdd(&db[c], b);
+    }
+  }
+  __syncwarp();
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (warp == 0) tc::tmem_dealloc<kWgradCols>(tbase);
 }
 
-cudaError_t launch_conv3_tc(int epi, const CUtensorMap& in_map, const uint8_t* wblob, const float* bias,
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+static ConvTiles conv_tiles(const ConvDims& D) {
+  ConvTiles T;
+  T.nx = (int)((D.X + kBX - 1) / kBX);
+  T.ny = (int)((D.Y + kBY - 1) / kBY);
+  T.n = (int64_t)T.nx * T.ny * D.Z;
+  return T;
+}
+
+template <int EPI>
+static cudaError_t launch_conv(const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias, const ConvDims& D,
+                               __nv_bfloat16* out_act, float* out_logits, const __nv_bfloat16* mask_act, int* err,
+                               int num_sms, cudaStream_t st) {
+  const ConvTiles T = conv_tiles(D);
+  cudaError_t e = cudaFuncSetAttribute(conv3_tc_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemConv);
+  if (e != cudaSuccess) return e;
+  ::msc::count_launch();
+  conv3_tc_kernel<EPI><<<(unsigned)(T.n < num_sms ? T.n : num_sms), kConvThreads, kSmemConv, st>>>(
+      in_act, wblob, bias, D, T, out_act, out_logits, mask_act, err);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_conv3_tc(int epi, const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias,
                             const ConvDims& D, __nv_bfloat16* out_act, float* out_logits,
-                            const __nv_bfloat16* mask_act, int* err, cudaStream_t st) {
-  if ((reinterpret_cast<uintptr_t>(wblob) & 15u) != 0) return cudaErrorInvalidValue;
-  const dim3 grid((unsigned)((D.X + kBX - 1) / kBX), (unsigned)((D.Y + kBY - 1) / kBY), (unsigned)D.Z);
-  cudaError_t e;
-  switch (epi) {
-    case kEpiReluBf16:
-      e = cudaFuncSetAttribute(conv3_tc_kernel<kEpiReluBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemConv);
-      if (e != cudaSuccess) return e;
-      ::msc::count_launch();
-      conv3_tc_kernel<kEpiReluBf16><<<grid, 128, kSmemConv, st>>>(in_map, wblob, bias, D, out_act, out_logits,
-                                                                   mask_act, err);
-      break;
-    case kEpiLogits:
-      e = cudaFuncSetAttribute(conv3_tc_kernel<kEpiLogits>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemConv);
-      if (e != cudaSuccess) return e;
-      ::msc::count_launch();
-      conv3_tc_kernel<kEpiLogits><<<grid, 128, kSmemConv, st>>>(in_map, wblob, bias, D, out_act, out_logits, mask_act,
-                                                                 err);
-      break;
-    default:
-      e = cudaFuncSetAttribute(conv3_tc_kernel<kEpiMaskBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemConv);
-      if (e != cudaSuccess) return e;
-      ::msc::count_launch();
-      conv3_tc_kernel<kEpiMaskBf16><<<grid, 128, kSmemConv, st>>>(in_map, wblob, bias, D, out_act, out_logits,
-                                                                   mask_act, err);
-      break;
-  }
+                            const __nv_bfloat16* mask_act, int* err, int num_sms, cudaStream_t st) {
+  if (!aligned16(in_act) || !aligned16(wblob)) return cudaErrorInvalidValue;  // bulk copies
+  if (epi == kEpiReluBf16)
+    return launch_conv<kEpiReluBf16>(in_act, wblob, bias, D, out_act, out_logits, mask_act, err, num_sms, st);
+  if (epi == kEpiLogits)
+    return launch_conv<kEpiLogits>(in_act, wblob, bias, D, out_act, out_logits, mask_act, err, num_sms, st);
+  return launch_conv<kEpiMaskBf16>(in_act, wblob, bias, D, out_act, out_logits, mask_act, err, num_sms, st);
+}
+
+cudaError_t launch_conv_wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, const ConvDims& D, float* dW, float* db,
+                              int* err, int num_sms, cudaStream_t st) {
+  if (!aligned16(X) || !aligned16(dY)) return cudaErrorInvalidValue;  // bulk copies
+  const ConvTiles T = conv_tiles(D);
+  cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemWgrad);
+  if (e != cudaSuccess) return e;
+  ::msc::count_launch();
+  conv_wgrad_tc_kernel<<<(unsigned)(T.n < 2 * num_sms ? T.n : 2 * num_sms), 128, kSmemWgrad, st>>>(X, dY, D, T, dW, db,
+                                                                                                   err);
   return cudaGetLastError();
 }
 

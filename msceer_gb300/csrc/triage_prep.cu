@@ -246,86 +246,6 @@ __global__ void bce_loss_kernel(const float* __restrict__ logits, const uint8_t*
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
 }
 
-// dW[tap][cin][cout] += sum_v X[v + tap][cin] * dY[v][cout] and db[cout] += sum_v dY[v][cout]
-// over a block of 32 (x) x 4 (y) output vertices at one z.  Thread (cin, cout pair)
-// keeps 27 x 2 accumulators; X (with its halo) and dY are staged as FP32.
-constexpr int kGWX = 32, kGWY = 4;
-__global__ void __launch_bounds__(128) conv_wgrad_kernel(const __nv_bfloat16* __restrict__ X,
-                                                         const __nv_bfloat16* __restrict__ dY, const ConvDims D,
-                                                         float* __restrict__ dW, float* __restrict__ db) {
-  __shared__ float sx[3][kGWY + 2][kGWX + 2][16];
-  __shared__ float sy[kGWY][kGWX][16];
-  const int tid = threadIdx.x;
-  const int cin = tid >> 3, cp = (tid & 7) * 2;
-  float acc[27][2];
-#pragma unroll
-  for (int t = 0; t < 27; t++) acc[t][0] = acc[t][1] = 0.f;
-  float bacc[2] = {0.f, 0.f};
-  const int64_t ntx = (D.X + kGWX - 1) / kGWX, nty = (D.Y + kGWY - 1) / kGWY;
-  const int64_t nblk = ntx * nty * D.Z;
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    const int64_t bx = blk % ntx, by = (blk / ntx) % nty, bz = blk / (ntx * nty);
-    const int64_t x0 = bx * kGWX, y0 = by * kGWY;
-    __syncthreads();
-    // X with a one-vertex halo (zero outside), 16 channels
-    for (int i = tid; i < 3 * (kGWY + 2) * (kGWX + 2) * 2; i += 128) {
-      const int half = i & 1, p = i >> 1;
-      const int lx = p % (kGWX + 2), ly = (p / (kGWX + 2)) % (kGWY + 2), lz = p / ((kGWX + 2) * (kGWY + 2));
-      const int64_t gx = x0 + lx - 1, gy = y0 + ly - 1, gz = bz + lz - 1;
-      float* dst = &sx[lz][ly][lx][half * 8];
-      if (gx < 0 || gy < 0 || gz < 0 || gx >= D.X || gy >= D.Y || gz >= D.Z) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) dst[c] = 0.f;
-      } else {
-        const uint4 q = *reinterpret_cast<const uint4*>(X + ((gz * D.Y + gy) * 2 + half) * D.X * 8 + gx * 8);
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&q);
-#pragma unroll
-        for (int c = 0; c < 8; c++) dst[c] = __bfloat162float(h[c]);
-      }
-    }
-    for (int i = tid; i < kGWY * kGWX * 2; i += 128) {
-      const int half = i & 1, p = i >> 1;
-      const int lx = p % kGWX, ly = p / kGWX;
-      const int64_t gx = x0 + lx, gy = y0 + ly;
-      float* dst = &sy[ly][lx][half * 8];
-      if (gx >= D.X || gy >= D.Y) {
-#pragma unroll
-        for (int c = 0; c < 8; c++) dst[c] = 0.f;
-      } else {
-        const uint4 q = *reinterpret_cast<const uint4*>(dY + ((bz * D.Y + gy) * 2 + half) * D.X * 8 + gx * 8);
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&q);
-#pragma unroll
-        for (int c = 0; c < 8; c++) dst[c] = __bfloat162float(h[c]);
-      }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int ly = 0; ly < kGWY; ly++) {
-#pragma unroll 1
-      for (int lx = 0; lx < kGWX; lx++) {
-        const float g0 = sy[ly][lx][cp], g1 = sy[ly][lx][cp + 1];
-        bacc[0] += g0;
-        bacc[1] += g1;
-#pragma unroll
-        for (int t = 0; t < 27; t++) {
-          const float xv = sx[t / 9][ly + (t / 3) % 3][lx + t % 3][cin];
-          acc[t][0] = fmaf(xv, g0, acc[t][0]);
-          acc[t][1] = fmaf(xv, g1, acc[t][1]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 27; t++) {
-    atomicAdd(&dW[t * 256 + cin * 16 + cp], acc[t][0]);
-    atomicAdd(&dW[t * 256 + cin * 16 + cp + 1], acc[t][1]);
-  }
-  if (cin == 0) {
-    atomicAdd(&db[cp], bacc[0]);
-    atomicAdd(&db[cp + 1], bacc[1]);
-  }
-}
-
 // Adam on the FP32 master parameters; `mask` zeroes the padded channels' updates.
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float bc1, float bc2,
@@ -392,13 +312,6 @@ cudaError_t launch_bce_loss(const float* logits, const uint8_t* target, const Co
                             float scale, __nv_bfloat16* dY, double* loss, int num_sms, cudaStream_t st) {
   ::msc::count_launch();
   bce_loss_kernel<<<num_sms * 8, 256, 0, st>>>(logits, target, D, pos_weight, scale, dY, loss);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_conv_wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, const ConvDims& D, float* dW,
-                              float* db, int num_sms, cudaStream_t st) {
-  ::msc::count_launch();
-  conv_wgrad_kernel<<<num_sms * 4, 128, 0, st>>>(X, dY, D, dW, db);
   return cudaGetLastError();
 }
 

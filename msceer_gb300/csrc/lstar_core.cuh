@@ -169,8 +169,8 @@ struct LowerStarExpand {
     return q;
   }
 
-  // HomotopyExpand of one boundary class S of the lower star.
-  MSC_HD void expand(uint32_t S) {
+  // The vertex's own step in its class S; returns the cells of S left to process.
+  MSC_HD uint32_t center(uint32_t S) {
     constexpr int C = N::CENTER;
     constexpr uint32_t EDGES = N::dim_mask(1);
     uint32_t A = S;  // unprocessed cells of the class
@@ -204,60 +204,92 @@ struct LowerStarExpand {
         out.pair(C, 1u << C, rb, axis, up);
       }
     }
+    return A;
+  }
+
+  // One step of HomotopyExpand on the cells A of a class that are left, always in the
+  // lowest dimension that still has unprocessed cells -- the order of the reference's
+  // per-dimension loops -- so the loop body is the same straight-line set algebra for
+  // every thread of a warp.
+  // Within the neighbourhood a cell with offset 0 along an axis has its two cofacets
+  // there one stride away on either side, so facets and cofacets along an axis are the
+  // set shifted both ways, of the cells (before) or kept on the cells (after) of
+  // offset 0.
+  MSC_HD void step(uint32_t& A) {
     constexpr uint32_t DM1 = N::dim_mask(1), DM2 = N::dim_mask(2), DM3 = N::dim_mask(3);
     constexpr uint32_t M0 = N::axis_mask(0, 0), M1 = N::axis_mask(1, 0), M2 = N::axis_mask(2, 0);
     constexpr int S1 = N::stride(1), S2 = N::stride(2);
-    // One step per iteration, always in the lowest dimension that still has
-    // unprocessed cells -- the order of the reference's per-dimension loops -- so the
-    // loop body is the same straight-line set algebra for every thread of a warp.
-    // Within the neighbourhood a cell with offset 0 along an axis has its two cofacets
-    // there one stride away on either side, so facets and cofacets along an axis are the
-    // set shifted both ways, of the cells (before) or kept on the cells (after) of
-    // offset 0.
-    for (int guard = 0; guard < N::NPOS && A; guard++) {
-      const uint32_t A1 = A & DM1, A2 = A & DM2;
-      const uint32_t D = A1 ? A1 : (A2 ? A2 : A);        // the dimension worked on
-      const uint32_t U = A1 ? A2 : (A2 ? A & DM3 : 0u);  // and the next one
-      const int dim = A1 ? 1 : (A2 ? 2 : 3);
-      const uint32_t Z0 = D & M0, Z1 = D & M1, Z2 = ND == 3 ? D & M2 : 0u;
-      const uint32_t F0 = (Z0 << 1) | (Z0 >> 1), F1 = (Z1 << S1) | (Z1 >> S1), F2 = (Z2 << S2) | (Z2 >> S2);
-      const uint32_t one = (F0 ^ F1 ^ F2) & ~(F0 & F1 & F2);  // exactly one unprocessed facet
-      const uint32_t R = U & one;                             // ready (d+1)-cells
-      const uint32_t W0 = R & F0, W1 = R & F1, W2 = R & F2;
-      uint32_t Q = (((W0 << 1) | (W0 >> 1)) & M0) | (((W1 << S1) | (W1 >> S1)) & M1);
-      if (ND == 3) Q |= ((W2 << S2) | (W2 >> S2)) & M2;
-      if (Q) {
-        const uint32_t qb = Q & (0u - Q);
-        const int q = ffs32(Q) - 1;
-        // ready cofacets of q, i.e. its candidates
-        const uint32_t q0 = qb & M0, q1 = qb & M1, q2 = ND == 3 ? qb & M2 : 0u;
-        const uint32_t u0 = R & (q0 << 1), d0 = R & (q0 >> 1), u1 = R & (q1 << S1), d1 = R & (q1 >> S1);
-        const uint32_t u2 = R & (q2 << S2), d2 = R & (q2 >> S2);
-        const uint32_t c1 = u1 | d1, c2 = u2 | d2, cm = u0 | d0 | c1 | c2;
-        uint32_t rb = cm;
-        if (cm & (cm - 1)) {
-          // several: the first in cofacet order (+x,-x,+y,-y,+z,-z) whose lowest
-          // vertex comes first wins (PickLowestCandidate)
-          Key kb = Keys::last();
-          rb = 0;
-          const uint32_t cand[6] = {u0, d0, u1, d1, u2, d2};
+    const uint32_t A1 = A & DM1, A2 = A & DM2;
+    const uint32_t D = A1 ? A1 : (A2 ? A2 : A);        // the dimension worked on
+    const uint32_t U = A1 ? A2 : (A2 ? A & DM3 : 0u);  // and the next one
+    const int dim = A1 ? 1 : (A2 ? 2 : 3);
+    const uint32_t Z0 = D & M0, Z1 = D & M1, Z2 = ND == 3 ? D & M2 : 0u;
+    const uint32_t F0 = (Z0 << 1) | (Z0 >> 1), F1 = (Z1 << S1) | (Z1 >> S1), F2 = (Z2 << S2) | (Z2 >> S2);
+    const uint32_t one = (F0 ^ F1 ^ F2) & ~(F0 & F1 & F2);  // exactly one unprocessed facet
+    const uint32_t R = U & one;                             // ready (d+1)-cells
+    const uint32_t W0 = R & F0, W1 = R & F1, W2 = R & F2;
+    uint32_t Q = (((W0 << 1) | (W0 >> 1)) & M0) | (((W1 << S1) | (W1 >> S1)) & M1);
+    if (ND == 3) Q |= ((W2 << S2) | (W2 >> S2)) & M2;
+    if (Q) {
+      const uint32_t qb = Q & (0u - Q);
+      const int q = ffs32(Q) - 1;
+      // ready cofacets of q, i.e. its candidates
+      const uint32_t q0 = qb & M0, q1 = qb & M1, q2 = ND == 3 ? qb & M2 : 0u;
+      const uint32_t u0 = R & (q0 << 1), d0 = R & (q0 >> 1), u1 = R & (q1 << S1), d1 = R & (q1 >> S1);
+      const uint32_t u2 = R & (q2 << S2), d2 = R & (q2 >> S2);
+      const uint32_t c1 = u1 | d1, c2 = u2 | d2, cm = u0 | d0 | c1 | c2;
+      uint32_t rb = cm;
+      if (cm & (cm - 1)) {
+        // several: the first in cofacet order (+x,-x,+y,-y,+z,-z) whose lowest
+        // vertex comes first wins (PickLowestCandidate)
+        Key kb = Keys::last();
+        rb = 0;
+        const uint32_t cand[6] = {u0, d0, u1, d1, u2, d2};
 #pragma unroll
-          for (int j = 0; j < 2 * ND; j++) {
-            if (!cand[j]) continue;
-            const Key k = lk.next(q, j >> 1, (j & 1) == 0);
-            if (Keys::less(k, kb)) {
-              kb = k;
-              rb = cand[j];
-            }
+        for (int j = 0; j < 2 * ND; j++) {
+          if (!cand[j]) continue;
+          const Key k = lk.next(q, j >> 1, (j & 1) == 0);
+          if (Keys::less(k, kb)) {
+            kb = k;
+            rb = cand[j];
           }
         }
-        A &= ~(qb | rb);
-        out.pair(q, qb, rb, (rb & c1) ? 1 : ((rb & c2) ? 2 : 0), rb > qb);
-      } else {
-        const int q = lowest_of(D);
-        A &= ~(1u << q);
-        out.critical(q, 1u << q, dim);
       }
+      A &= ~(qb | rb);
+      out.pair(q, qb, rb, (rb & c1) ? 1 : ((rb & c2) ? 2 : 0), rb > qb);
+    } else {
+      const int q = lowest_of(D);
+      A &= ~(1u << q);
+      out.critical(q, 1u << q, dim);
+    }
+  }
+
+  // HomotopyExpand of one boundary class S of the lower star.
+  MSC_HD void expand(uint32_t S) {
+    uint32_t A = center(S);
+    for (int guard = 0; guard < N::NPOS && A; guard++) step(A);
+  }
+
+  // HomotopyExpand of every class of the lower star L: two cells are of one class if
+  // they agree in all planes of k.  The classes know nothing of one another, so their
+  // order is free, and one loop takes them all: the lanes of a warp meet in it, whatever
+  // the number of their classes.
+  template <int NK>
+  MSC_HD void expand_classes(uint32_t L, const uint32_t (&k)[NK]) {
+    auto same = [&](int q) {
+      uint32_t m = ~0u;
+#pragma unroll
+      for (int i = 0; i < NK; i++) m &= ((k[i] >> q) & 1u) ? k[i] : ~k[i];
+      return m;
+    };
+    const uint32_t S = L & same(N::CENTER);
+    uint32_t rest = L & ~S, A = center(S);
+    for (int guard = 0; guard < N::NPOS && (A | rest); guard++) {
+      if (!A) {
+        A = rest & same(ffs32(rest) - 1);
+        rest &= ~A;
+      }
+      step(A);
     }
   }
 };
@@ -425,67 +457,61 @@ MSC_HD void expand_and_store(uint32_t L, uint64_t* col, int cs, bool interior, b
 // The constrained re-pairing of ondemandaccurate's accurate 3-manifolds
 // (MyRobinsNoalloc<...,4,6>::ComputeLowerStar with a restriction map,
 // gi_modified_robins.h:1281-1343): the lower star L split by class
-// restriction_label * maxDim + boundaryValue (maxDim = 3; at most 24 classes, the last
-// taking every larger one), the classes expanded in increasing order.  rl[p]: the
-// restriction label of the cell at position p.
-template <int ND, class Store>
-MSC_HD void expand_and_store_keyed(uint32_t L, uint64_t* col, int cs, const uint8_t* rl, bool bx, bool by, bool bz,
-                                   uint32_t enc_map, const Store& store) {
+// restriction_label * maxDim + boundaryValue (maxDim = 3).  A restriction label is 0 to
+// 3: bit p of r1 / r2 is the low / high bit of the label of the cell at position p.
+// Away from the boundary the label is the class.
+template <int ND, class Expand>
+MSC_HD uint32_t run_restricted(Expand& ex, uint32_t L, uint32_t r1, uint32_t r2, bool bx, bool by, bool bz) {
   using N = Nb<ND>;
-  constexpr int NPOS = N::NPOS;
-  PlaneSink st;
-  LowerStarExpand<ND, KeyCol, PlaneSink> ex(KeyCol{col, cs}, st);
+  if (!(bx || by || (ND == 3 && bz))) {
+    const uint32_t k[2] = {r1, r2};
+    ex.expand_classes(L, k);
+    return 0u;
+  }
   const uint32_t B0 = bx ? N::axis_mask(0, 0) : 0u;
   const uint32_t B1 = by ? N::axis_mask(1, 0) : 0u;
   const uint32_t B2 = (ND == 3 && bz) ? N::axis_mask(2, 0) : 0u;
-  constexpr int kClasses = 24;
-  uint32_t cls[kClasses];
-#pragma unroll
-  for (int k = 0; k < kClasses; k++) cls[k] = 0u;
-  for (int p = 0; p < NPOS; p++) {
-    if (!((L >> p) & 1u)) continue;
-    const int bv = (int)((B0 >> p) & 1u) + (int)((B1 >> p) & 1u) + (int)((B2 >> p) & 1u);
-    int key = 3 * (int)rl[p] + bv;
-    if (key > kClasses - 1) key = kClasses - 1;
-    cls[key] |= 1u << p;
-  }
-  for (int k = 0; k < kClasses; k++)
-    if (cls[k]) ex.expand(cls[k]);
-  store_cells<ND>(st, L, B0 | B1 | B2, enc_map, store);
+  // boundary value 3 with label r is value 0 with label r + 1
+  const uint32_t all3 = B0 & B1 & B2, carry = r1 & all3;
+  const uint32_t k[5] = {(B0 ^ B1 ^ B2) & ~all3, ((B0 & B1) | (B0 & B2) | (B1 & B2)) & ~all3, r1 ^ all3, r2 ^ carry,
+                         r2 & carry};
+  ex.expand_classes(L, k);
+  return B0 | B1 | B2;
 }
 
 // One vertex of the conforming re-pairing of ondemandaccurate's accurate 3-manifolds
 // (ondemandaccurate.cxx:1000-1063): a vertex whose own cell, or a cell of whose lower
-// star, carries a restriction label recomputes its lower star split by label
-// (expand_and_store_keyed); every other vertex keeps its pairs.  rlab(p, r): the
-// restriction label of the cell at position p (called for positions inside the
-// complex only).  Returns true if the vertex recomputed its lower star.
+// star, carries a restriction label recomputes its lower star split by label; every other
+// vertex keeps its pairs.  rlab(p, r): the restriction label of the cell at position p
+// (called for positions inside the complex only).  Returns true if the vertex recomputed
+// its lower star.  The kernel's form works on a tile (lstar_tile.cuh).
 template <int ND, class Load, class Restrict, class Store>
 MSC_HD bool conform_vertex(int64_t x, int64_t y, int64_t z, int64_t X, int64_t Y, int64_t Z, bool interior,
                            const Load& load, const Restrict& rlab, uint64_t* col, int cs, uint32_t enc_map,
                            const Store& store) {
   using N = Nb<ND>;
-  constexpr int NPOS = N::NPOS;
   const uint32_t okx = (x > 0 ? N::axis_mask(0, -1) : 0u) | N::axis_mask(0, 0) | (x < X - 1 ? N::axis_mask(0, 1) : 0u);
   const uint32_t oky = (y > 0 ? N::axis_mask(1, -1) : 0u) | N::axis_mask(1, 0) | (y < Y - 1 ? N::axis_mask(1, 1) : 0u);
   const uint32_t okz = (ND == 2) ? ~0u
                                  : ((z > 0 ? N::axis_mask(2, -1) : 0u) | N::axis_mask(2, 0) |
                                     (z < Z - 1 ? N::axis_mask(2, 1) : 0u));
   const uint32_t ok = okx & oky & okz;
-  uint8_t rl[NPOS];
-  uint32_t R = 0;
-  for (int p = 0; p < NPOS; p++) {
+  uint32_t r1 = 0, r2 = 0;
+  for (int p = 0; p < N::NPOS; p++) {
     uint8_t r = 0;
     if ((ok >> p) & 1u) rlab(p, r);
-    rl[p] = r;
-    if (r) R |= 1u << p;
+    r1 |= (uint32_t)(r & 1u) << p;
+    r2 |= (uint32_t)((r >> 1) & 1u) << p;
   }
-  if (!R) return false;
+  if (!(r1 | r2)) return false;
   bool nan = false;
   const uint32_t L = lower_star_keys<ND>(x, y, z, X, Y, Z, interior, load, col, cs, nan);
-  if (!(R & L)) return false;  // (L holds the vertex itself)
-  expand_and_store_keyed<ND>(L, col, cs, rl, x == 0 || x == X - 1, y == 0 || y == Y - 1, z == 0 || z == Z - 1,
-                             enc_map, store);
+  if (!((r1 | r2) & L)) return false;  // (L holds the vertex itself)
+  PlaneSink st;
+  LowerStarExpand<ND, KeyCol, PlaneSink> ex(KeyCol{col, cs}, st);
+  const uint32_t Bany =
+      run_restricted<ND>(ex, L, r1, r2, x == 0 || x == X - 1, y == 0 || y == Y - 1, z == 0 || z == Z - 1);
+  store_cells<ND>(st, L, Bany, enc_map, store);
   return true;
 }
 

@@ -53,10 +53,13 @@ static_assert(offsetof(LstarSmem<3>, bytes) % 16 == 0 && offsetof(LstarSmem<2>, 
 }  // namespace
 
 // One tile of volume (f, g, D); its first vertex is (x0, y0, z0).  Every thread of the
-// block calls this.
-template <int ND>
+// block calls this.  RESTRICTED: the vertices with a restricted cell in their lower star
+// (`bits`, conform_kernels.cu) are paired again, counted in `touched`, and the others left
+// as they are.
+template <int ND, bool RESTRICTED = false>
 __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t* __restrict__ g, const GradDims& D,
-                                           int64_t x0, int64_t y0, int64_t z0, LstarSmem<ND>& S) {
+                                           int64_t x0, int64_t y0, int64_t z0, LstarSmem<ND>& S,
+                                           const uint16_t* __restrict__ bits = nullptr, int* touched = nullptr) {
   using T = LstarTile<ND>;
   using N = Nb<ND>;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -67,8 +70,9 @@ __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t*
     S.hist[tid] = 0;
     S.off[tid] = (int16_t)(tid < N::NPOS ? T::off(tid) : 0);
   }
-  for (int i = tid; i < (int)sizeof(S.bytes) / 16; i += kLstarBS)
-    reinterpret_cast<uint4*>(S.bytes)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (!RESTRICTED)
+    for (int i = tid; i < (int)sizeof(S.bytes) / 16; i += kLstarBS)
+      reinterpret_cast<uint4*>(S.bytes)[i] = make_uint4(0u, 0u, 0u, 0u);
   // f, a warp per row (values outside the volume read as 0: no cell that holds one is in
   // a lower star)
   bool nan = false;
@@ -93,7 +97,13 @@ __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t*
   for (int i = tid; i < CX * CY * CZ; i += kLstarBS) {
     const int z = i / (CX * CY), r = i - z * (CX * CY), y = r / CX, x = r - y * CX;
     tile_cell_keys<ND>(S.f, S.lat, x - 1, y - 1, ND == 3 ? z - 1 : 0);
+    if (RESTRICTED) {
+      const int64_t vx = x0 - 1 + x, vy = y0 - 1 + y, vz = z0 - 1 + z;
+      const bool in = vx >= 0 && vx < X && vy >= 0 && vy < Y && vz >= 0 && vz < Z;
+      tile_restrict(in ? bits[vx + X * (vy + Y * vz)] : 0u, S.bytes, x - 1, y - 1, z - 1);
+    }
   }
+  if (RESTRICTED) __syncthreads();  // the labels are read next
   // lower stars, and a counting sort of the vertices by their size (28 sizes; 31: no vertex)
   int bin[T::NV / kLstarBS], rank[T::NV / kLstarBS];
 #pragma unroll
@@ -108,6 +118,11 @@ __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t*
       const uint32_t L = lower_star_mask<ND>(lower);
       S.L[t] = L;
       bin[h] = __popc(L);
+      if (RESTRICTED) {
+        uint32_t r1, r2;
+        if (tile_labels(L, t, S.bytes, S.off, r1, r2)) (*touched)++;
+        else bin[h] = 31;
+      }
     }
     rank[h] = atomicAdd(&S.hist[bin[h]], 1);
   }
@@ -135,7 +150,14 @@ __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t*
     if (t == 0xFFFF) continue;
     int x, y, z;
     T::vertex(t, x, y, z);
-    tile_expand<ND>(S.L[t], t, rim, x0 + x, y0 + y, z0 + z, D.v, S.lat, S.bytes, S.off, D.enc_map);
+    if (RESTRICTED) {
+      uint32_t r1, r2;
+      tile_labels(S.L[t], t, S.bytes, S.off, r1, r2);
+      tile_expand_restricted(S.L[t], r1, r2, t, rim, x0 + x, y0 + y, z0 + z, D.v,
+                             reinterpret_cast<const LatKey*>(S.lat), S.bytes, S.off, D.enc_map);
+    } else {
+      tile_expand<ND>(S.L[t], t, rim, x0 + x, y0 + y, z0 + z, D.v, S.lat, S.bytes, S.off, D.enc_map);
+    }
   }
   __syncthreads();
   // the bytes, a warp per lattice row
@@ -145,9 +167,9 @@ __device__ __forceinline__ bool lstar_tile(const float* __restrict__ f, uint8_t*
     uint8_t* gr = g0 + cy * D.cs[1] + cz * D.cs[2];
     const uint8_t* b = S.bytes + r * T::LX;
     const uint8_t b0 = b[lane], b1 = b[lane + 32];
-    if (b0) gr[lane] = b0;
-    if (b1) gr[lane + 32] = b1;
-    if (lane == 0 && b[64]) gr[64] = b[64];
+    if (b0 & 1u) gr[lane] = b0;
+    if (b1 & 1u) gr[lane + 32] = b1;
+    if (lane == 0 && (b[64] & 1u)) gr[64] = b[64];
   }
   return nan;
 }
@@ -189,6 +211,33 @@ __global__ void __launch_bounds__(kLstarBS, 4) lstar_batch_kernel(const LstarBat
   if (nan) atomicOr(err, kErrNaN);
 }
 
+// The conforming re-pairing of one volume: a flat grid over its tiles.  Between patches of
+// labels as small as the labels of noise make them most vertices are touched (8.6 of 10.0 M
+// at 223 x 187 x 241), so it is the lower star's pass with classes, bound by integer issue
+// like it.  A thread per vertex with its 27 keys in local memory, its classes one after the
+// other, took 2.6 ms there, with lists of the touched vertices 2.3 ms (13 of 32 lanes
+// active); the tiles and one loop over all classes take 1.07 ms.
+__global__ void __launch_bounds__(kLstarBS, 4) conform_kernel(const float* __restrict__ f,
+                                                              const uint16_t* __restrict__ bits,
+                                                              uint8_t* __restrict__ g, const GradDims D,
+                                                              unsigned long long* __restrict__ touched) {
+  using T = LstarTile<3>;
+  extern __shared__ __align__(16) unsigned char s_tile[];
+  LstarSmem<3>& S = *reinterpret_cast<LstarSmem<3>*>(s_tile);
+  const int64_t gx = (D.v[0] + T::BX - 1) / T::BX, gy = (D.v[1] + T::BY - 1) / T::BY;
+  const int64_t n = gx * gy * ((D.v[2] + T::BZ - 1) / T::BZ);
+  int mine = 0;
+  for (int64_t b = blockIdx.x; b < n; b += gridDim.x) {
+    const int64_t q = b / gx;
+    lstar_tile<3, true>(f, g, D, (b - q * gx) * T::BX, (q % gy) * T::BY, (q / gy) * T::BZ, S, bits, &mine);
+    __syncthreads();  // the next tile reuses the shared memory
+  }
+  unsigned long long sum = (unsigned long long)mine;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0 && sum) atomicAdd(touched, sum);
+}
+
 namespace {
 template <class K>
 cudaError_t allow_smem(K k, size_t bytes) {
@@ -212,6 +261,17 @@ cudaError_t launch_lstar(int nd, const float* f, uint8_t* g, const GradDims& D, 
   (void)num_sms;
   if (!lstar_dims_ok(D)) return cudaErrorInvalidValue;
   return nd == 3 ? launch_lstar_nd<3>(f, g, D, err, stream) : launch_lstar_nd<2>(f, g, D, err, stream);
+}
+
+cudaError_t launch_conform(const float* f, const uint16_t* bits, uint8_t* g, const GradDims& D,
+                           unsigned long long* touched, int num_sms, cudaStream_t stream) {
+  using T = LstarTile<3>;
+  const int64_t n = ((D.v[0] + T::BX - 1) / T::BX) * ((D.v[1] + T::BY - 1) / T::BY) * ((D.v[2] + T::BZ - 1) / T::BZ);
+  if (cudaError_t e = allow_smem(conform_kernel, sizeof(LstarSmem<3>))) return e;
+  const int64_t grid = (int64_t)num_sms * 64;  // the last tiles even out over the blocks' turns
+  ::msc::count_launch();
+  conform_kernel<<<(unsigned)(n < grid ? n : grid), kLstarBS, sizeof(LstarSmem<3>), stream>>>(f, bits, g, D, touched);
+  return cudaGetLastError();
 }
 
 cudaError_t make_lstar_batch(int n, const float* const* f, uint8_t* const* g, const GradDims* D, LstarBatch* B) {

@@ -173,6 +173,38 @@ MSC_HD uint32_t inside_mask(int64_t x, int64_t y, int64_t z, const int64_t v[3])
   return ok;
 }
 
+// The restriction labels of the cells that tile vertex (x, y, z) owns, -1 <= x < BX and so
+// on, into the byte lattice: bit s of `word` is the low bit of the label of cell 2v + s
+// (s = sx + 2 sy + 4 sz), bit 8 + s the high bit.  They lie there as 2 * label, a value
+// that no pairing writes (bit 0 of an assigned byte is set), until the cell is paired:
+// only the vertex that owns a cell reads its label.
+MSC_HD void tile_restrict(uint32_t word, uint8_t* bytes, int x, int y, int z) {
+  using T = LstarTile<3>;
+  uint8_t* c = bytes + T::center(x, y, z);
+#pragma unroll
+  for (int s = 0; s < 8; s++) {
+    if ((!(s & 1) && x < 0) || (!(s & 2) && y < 0) || (!(s & 4) && z < 0)) continue;  // not in the lattice
+    c[(s & 1) + ((s >> 1) & 1) * T::LX + (s >> 2) * T::LX * T::LY] =
+        (uint8_t)((((word >> s) & 1u) << 1) | (((word >> (8 + s)) & 1u) << 2));
+  }
+}
+// The labels of the cells of lower star L of tile vertex t as bit planes; false if all are 0
+MSC_HD bool tile_labels(uint32_t L, int t, const uint8_t* bytes, const int16_t* off, uint32_t& r1, uint32_t& r2) {
+  using T = LstarTile<3>;
+  int x, y, z;
+  T::vertex(t, x, y, z);
+  const uint8_t* c = bytes + T::center(x, y, z);
+  r1 = r2 = 0;
+  while (L) {
+    const int p = ffs32(L) - 1;
+    const uint32_t pb = L & (0u - L), r = c[off[p]];
+    L ^= pb;
+    if (r & 2u) r1 |= pb;
+    if (r & 4u) r2 |= pb;
+  }
+  return (r1 | r2) != 0;
+}
+
 // The pairing of tile vertex t with lower star L (vertex (x, y, z) of the volume; rim:
 // the tile touches the volume's boundary)
 template <int ND>
@@ -192,6 +224,23 @@ MSC_HD void tile_expand(uint32_t L, int t, bool rim, int64_t x, int64_t y, int64
   const bool bx = x == 0 || x == v[0] - 1, by = y == 0 || y == v[1] - 1, bz = ND == 3 && (z == 0 || z == v[2] - 1);
   out.bany = (bx ? N::axis_mask(0, 0) : 0u) | (by ? N::axis_mask(1, 0) : 0u) | (bz ? N::axis_mask(2, 0) : 0u);
   run_classes<ND>(ex, L, bx, by, bz);
+}
+
+// The same with the lower star split by restriction label (r1, r2 of tile_labels) too
+MSC_HD void tile_expand_restricted(uint32_t L, uint32_t r1, uint32_t r2, int t, bool rim, int64_t x, int64_t y,
+                                   int64_t z, const int64_t v[3], const LatKey* lat, uint8_t* bytes,
+                                   const int16_t* off, uint32_t enc_map) {
+  using T = LstarTile<3>;
+  using N = Nb<3>;
+  int lx, ly, lz;
+  T::vertex(t, lx, ly, lz);
+  const int c = T::center(lx, ly, lz);
+  ByteSink out{bytes + c, off, T::LX, T::LX * T::LY, 0u, enc_map};
+  LowerStarExpand<3, LatKeys, ByteSink> ex(LatKeys{lat + c, off, T::LX, T::LX * T::LY}, out);
+  const bool bx = rim && (x == 0 || x == v[0] - 1), by = rim && (y == 0 || y == v[1] - 1);
+  const bool bz = rim && (z == 0 || z == v[2] - 1);
+  out.bany = (bx ? N::axis_mask(0, 0) : 0u) | (by ? N::axis_mask(1, 0) : 0u) | (bz ? N::axis_mask(2, 0) : 0u);
+  run_restricted<3>(ex, L, r1, r2, bx, by, bz);
 }
 
 }  // namespace msc

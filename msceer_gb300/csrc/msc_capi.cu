@@ -279,7 +279,8 @@ int conform_impl(const float* f, const int32_t* asc, const int32_t* dsc, const i
   if (!f || !g) return fail(MSC_ERR_NULL_POINTER, "null buffer");
   Scratch s;
   if (int rc = alloc_scratch(s, stream)) return rc;
-  uint8_t* rl = restrict_out;
+  // the hexes' descending labels, then 16 restriction bits per vertex
+  int32_t* hex = nullptr;
   unsigned long long* touched = nullptr;
   struct Free {
     void* a;
@@ -290,16 +291,17 @@ int conform_impl(const float* f, const int32_t* asc, const int32_t* dsc, const i
       if (b) cudaFreeAsync(b, st);
     }
   } fr{nullptr, nullptr, stream};
-  if (!rl) {
-    MSC_CUDA(msc::scratch_alloc((void**)&rl, (size_t)D.ncells, stream), "scratch alloc(restriction labels)");
-    fr.a = rl;
-  }
+  const size_t nv = (size_t)(D.v[0] * D.v[1] * D.v[2]);
+  MSC_CUDA(msc::scratch_alloc((void**)&hex, nv * 6, stream), "scratch alloc(restriction labels)");
+  fr.a = hex;
+  uint16_t* bits = reinterpret_cast<uint16_t*>(hex + nv);
   MSC_CUDA(msc::scratch_alloc((void**)&touched, sizeof(unsigned long long), stream), "scratch alloc(counter)");
   fr.b = touched;
   MSC_CUDA(cudaMemsetAsync(touched, 0, sizeof(unsigned long long), stream), "cudaMemsetAsync");
   const int sms = num_sms();
-  MSC_CUDA(msc::launch_restriction_labels(asc, dsc, f, D, rl, sms, stream), "restriction labels");
-  MSC_CUDA(msc::launch_conform(f, rl, g, D, touched, sms, stream), "conforming re-pairing");
+  MSC_CUDA(msc::launch_restriction_labels(asc, dsc, f, D, hex, bits, restrict_out, sms, stream), "restriction labels");
+  MSC_CUDA(msc::launch_conform(f, bits, g, D, touched, sms, stream), "conforming re-pairing");
+  MSC_CUDA(msc::launch_ldir_roots(g, D, sms, stream), "ldir roots");
   if (int rc = ldir_impl(3, g, dims, stream, s, nullptr)) return rc;
   if (touched_out) {
     unsigned long long h = 0;

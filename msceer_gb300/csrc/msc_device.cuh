@@ -112,7 +112,8 @@ cudaError_t launch_central_diff(int nd, int layout, const float* f, void* out, c
 // ascending / descending labels (either may be null), then the re-pairing of the
 // touched vertices (`touched` counts them) and every cell's ldir back to its roots.
 cudaError_t launch_restriction_labels(const int32_t* asc, const int32_t* dsc, const float* f, const GradDims& D,
-                                      uint8_t* out, int num_sms, cudaStream_t stream);
-cudaError_t launch_conform(const float* f, const uint8_t* rlab, uint8_t* g, const GradDims& D,
+                                      int32_t* hex, uint16_t* bits, uint8_t* out, int num_sms, cudaStream_t stream);
+cudaError_t launch_conform(const float* f, const uint16_t* bits, uint8_t* g, const GradDims& D,
                            unsigned long long* touched, int num_sms, cudaStream_t stream);
+cudaError_t launch_ldir_roots(uint8_t* g, const GradDims& D, int num_sms, cudaStream_t stream);
 }  // namespace msc

@@ -82,3 +82,37 @@ def test_conforming_grad_end_to_end(gpu, oracle, name):
     cell_diff = int((got != want).sum())
     print(name, "label differences", lab_diff, "cell differences", cell_diff)
     assert cell_diff <= 64 * lab_diff
+
+
+@pytest.mark.parametrize("shape,which", [((2, 2, 2), "both"), ((3, 2, 9), "both"), ((1, 7, 6), "both"),
+                                         ((5, 9, 33), "both"), ((17, 13, 41), "dsc"), ((13, 31, 16), "asc"),
+                                         ((40, 37, 29), "both")])
+def test_restriction_and_re_pairing_of_any_labels(gpu, oracle, shape, which):
+    """Labels in random patches, -1 among them, so that every kind of cell gets every
+    restriction label, on the faces too; the .grad buffer starts at any byte."""
+    import torch
+    from msceer_gb300 import conforming_grad, lower_star_grad
+    rng = np.random.default_rng(sum(shape))
+    f = rng.standard_normal(shape).astype(np.float32)
+    base = oracle.grad(f)
+
+    def patches():
+        l = rng.integers(-1, 4, size=tuple((n + 2) // 3 for n in shape))
+        for a in range(3):
+            l = l.repeat(3, a)
+        return np.ascontiguousarray(l[:shape[0], :shape[1], :shape[2]]).astype(np.int32).reshape(-1)
+
+    asc = patches() if which != "dsc" else None
+    dsc = patches() if which != "asc" else None
+    restrict = oracle.boundary_labels(f, asc, dsc)
+    want = oracle.conform(f, restrict, base)
+    t = torch.from_numpy(f).to(gpu)
+    dev = lambda a: None if a is None else torch.from_numpy(a).to(gpu)  # noqa: E731
+    assert np.array_equal(lower_star_grad(t).cpu().numpy(), base)
+    for shift in (0, 1, 15):
+        g = torch.empty(base.size + shift, dtype=torch.uint8, device=gpu)[shift:]
+        g.copy_(torch.from_numpy(base.reshape(-1)))
+        _, rl = conforming_grad(t, g, dev(asc), dev(dsc), restriction=True)
+        assert np.array_equal(rl.cpu().numpy(), restrict.reshape(-1))
+        assert np.array_equal(g.cpu().numpy(), want.reshape(-1)), oracle_lib.describe_mismatch(
+            g.cpu().numpy(), want, f.shape[::-1])

@@ -46,3 +46,23 @@ def test_tile_equals_oracle(tile, oracle, kind, shape):
     want = oracle.grad(f)
     assert (g & 1).all()
     assert np.array_equal(g & 0x1F, want & 0x1F)  # assigned, flag and pairs; the closure sets the rest
+
+
+@pytest.mark.parametrize("labels", ["random", "slab"])
+@pytest.mark.parametrize("shape", [(32, 4, 4), (33, 5, 5), (70, 13, 6), (1, 7, 9), (2, 2, 2), (31, 3, 9)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_restricted_tile_equals_oracle(tile, oracle, shape, labels):
+    f = np.ascontiguousarray(make("ties", shape))
+    tile.tile_conform.argtypes = [ctypes.c_void_p] + [ctypes.c_int64] * 3 + [ctypes.c_void_p, ctypes.c_void_p,
+                                                                             ctypes.c_uint32]
+    tile.tile_conform.restype = ctypes.c_int64
+    base = oracle.grad(f)
+    rng = np.random.default_rng(3)
+    if labels == "random":
+        r = rng.integers(0, 4, size=base.size).astype(np.uint8)
+    else:  # few restricted cells, so that some lower stars keep their pairs
+        r = (rng.random(base.size) < 0.02).astype(np.uint8) * rng.integers(1, 4, size=base.size).astype(np.uint8)
+    want = oracle.conform(f, r, base)
+    g = base.copy().reshape(-1)
+    assert tile.tile_conform(f.ctypes.data, *shape, r.ctypes.data, g.ctypes.data, enc_map(shape)) > 0
+    assert np.array_equal(g & 0x1F, want.reshape(-1) & 0x1F)

@@ -1168,17 +1168,9 @@ __global__ void count_unlabelled_kernel(const uint8_t* __restrict__ lvl, int64_t
 
 // ---- FP64 advector (fix-up), the reference's arithmetic --------------------------------
 
-struct D3 {
-  double x, y, z;
-};
 __device__ __forceinline__ double dm(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double da(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double ds(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ D3 dlerp(D3 a, D3 b, double t) {
-  const double u = ds(1.0, t);
-  return {da(dm(a.x, u), dm(b.x, t)), da(dm(a.y, u), dm(b.y, t)), da(dm(a.z, u), dm(b.z, t))};
-}
-__device__ __forceinline__ double magsq(D3 a) { return da(da(dm(a.x, a.x), dm(a.y, a.y)), dm(a.z, a.z)); }
 __device__ __forceinline__ double clampd_ext(double v, int64_t n) {
   if (v < 0) v = 0;
   if (v >= (double)n) v = (double)n - 1;
@@ -1196,135 +1188,6 @@ struct Adv64 {
   VolDims V;
   IntegParams P;
   const uint8_t* state;  // fix-up stop: certain terminal
-
-  __device__ __forceinline__ D3 corner(int64_t x, int64_t y, int64_t z) const {
-    const int64_t v = vid(V, x, y, z);
-    if ((zeroed[v >> 5] >> (v & 31)) & 1u) return {0.0, 0.0, 0.0};
-    const float c = __ldg(f + v);
-    // 0 + (-0.5f * f[-1]) + (0.0f * f[0]) + (0.5f * f[+1]), each product a float, summed
-    // in double; 0 + (0.0f * f[0]) on a first or last plane
-    auto comp = [&](bool inside, int64_t s) -> double {
-      if (!inside) return 0.0 + (double)(0.0f * c);
-      const float a = __ldg(f + v - s), b = __ldg(f + v + s);
-      double r = 0.0;
-      r += (double)(-0.5f * a);
-      r += (double)(0.0f * c);
-      r += (double)(0.5f * b);
-      return r;
-    };
-    return {comp(x > 0 && x < V.X - 1, 1), comp(y > 0 && y < V.Y - 1, V.X), comp(z > 0 && z < V.Z - 1, V.X * V.Y)};
-  }
-  __device__ __forceinline__ void surround(const int64_t b[3], bool clamp, D3 c[8]) const {
-    int64_t vv[3][2];
-    const int64_t ext[3] = {V.X, V.Y, V.Z};
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-      vv[a][0] = b[a];
-      vv[a][1] = b[a] + 1;
-      if (clamp) {
-        if (b[a] < 0) vv[a][0] = 0;
-        if (b[a] >= ext[a] - 1) vv[a][0] = vv[a][1] = ext[a] - 1;
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < 8; n++) c[n] = corner(vv[0][n & 1], vv[1][(n >> 1) & 1], vv[2][n >> 2]);
-  }
-  // bf: the base corner as doubles
-  __device__ __forceinline__ static D3 trilin(D3 s, const double bf[3], const D3 c[8]) {
-    const double fx = ds(s.x, bf[0]), fy = ds(s.y, bf[1]), fz = ds(s.z, bf[2]);
-    const D3 x0 = dlerp(c[0], c[1], fx), x1 = dlerp(c[2], c[3], fx), x2 = dlerp(c[4], c[5], fx), x3 = dlerp(c[6], c[7], fx);
-    return dlerp(dlerp(x0, x1, fy), dlerp(x2, x3, fy), fz);
-  }
-  __device__ __forceinline__ void nearest3(D3 p, int& ix, int& iy, int& iz) const {
-    ix = (int)(int64_t)clampd_ext(da(p.x, 0.5), V.X);
-    iy = (int)(int64_t)clampd_ext(da(p.y, 0.5), V.Y);
-    iz = (int)(int64_t)clampd_ext(da(p.z, 0.5), V.Z);
-  }
-  __device__ __forceinline__ int64_t nearest(D3 p, bool) const {
-    int ix, iy, iz;
-    nearest3(p, ix, iy, iz);
-    return vid(V, ix, iy, iz);
-  }
-  // The FP32 advector's trapped-streamline test on FP64 positions.
-  __device__ __forceinline__ bool trapped(const D3& cur, D3& anchor, int& n) const {
-    const double d = fmax(fabs(cur.x - anchor.x), fmax(fabs(cur.y - anchor.y), fabs(cur.z - anchor.z)));
-    n = d < (double)P.trap_radius ? n + 1 : 0;
-    anchor = cur;
-    return n >= 2;
-  }
-  // The voxel that holds `cur` and its eight corner gradients (as the FP32 advector's)
-  __device__ __forceinline__ void load_voxel(const D3& cur, bool nearb, double bf[3], D3 c[8]) const {
-    int64_t b[3];
-    if (nearb) {
-      b[0] = (int64_t)clampd_ext(cur.x, V.X);
-      b[1] = (int64_t)clampd_ext(cur.y, V.Y);
-      b[2] = (int64_t)clampd_ext(cur.z, V.Z);
-    } else {
-      b[0] = (int64_t)fmin(fmax(cur.x, 0.0), (double)(V.X - 2));
-      b[1] = (int64_t)fmin(fmax(cur.y, 0.0), (double)(V.Y - 2));
-      b[2] = (int64_t)fmin(fmax(cur.z, 0.0), (double)(V.Z - 2));
-    }
-    surround(b, nearb, c);
-    bf[0] = (double)b[0];
-    bf[1] = (double)b[1];
-    bf[2] = (double)b[2];
-  }
-  // The FP32 advector's round (Adv32::advance: one uniform iteration for every stepping
-  // lane, the voxel entry folded in) in the reference's FP64 arithmetic.
-  __device__ __forceinline__ int advance(int& phase, int x, int y, int z, D3& cur, D3& old, int& iters, bool& nb,
-                                         double bf[3], D3 c[8], D3& g, float& gm, float& step,
-                                         unsigned long long& ntrips) const {
-    const bool ent = phase == kLaneEnter;
-    if (ent) {
-      nb = dist_to_boundary(V, x, y, z) <= 1;
-      load_voxel(cur, nb, bf, c);
-      phase = kLaneStep;
-    }
-    const bool moved = !ent && !(old.x == cur.x && old.y == cur.y && old.z == cur.z);
-    const bool left = moved && ((int)cur.x != (int)old.x || (int)cur.y != (int)old.y || (int)cur.z != (int)old.z);
-    const D3 gc = trilin(cur, bf, c);
-    const float gmc = __double2float_rn(__dsqrt_rn(magsq(gc)));
-    const bool bad = !(gmc > 0.f) || !isfinite(gmc);  // no direction to follow
-    const bool counts = !(ent && bad);
-    ntrips += counts;
-    const bool spent = counts && !(iters > 0);
-    iters -= counts;
-    int ev = spent ? EV_OVER_MAX_ITERATIONS : EV_NONE;
-    if (ent && bad) ev = EV_LOW_GRADIENT;
-    if (!spent && left) ev = EV_OUT_OF_VOXEL;
-    if (!spent && !left && moved && bad) ev = EV_LOW_GRADIENT;
-    if (ev != EV_NONE) return ev;
-    const float sl = __double2float_rn(__ddiv_rn(P.max_step, (double)gmc));
-    if (ent || (double)__fmul_rn(gmc, step) > P.max_step) step = sl;
-    g = gc;
-    gm = gmc;
-    old = cur;
-    if (gm < P.gthresh) return EV_LOW_GRADIENT;
-    // full step: Vec3d * float multiplies in float (gi_vectors.h:250)
-    const float sm = __fmul_rn((float)P.step_mult, step);
-    const D3 e1 = {(double)__fmul_rn(__double2float_rn(g.x), sm), (double)__fmul_rn(__double2float_rn(g.y), sm),
-                   (double)__fmul_rn(__double2float_rn(g.z), sm)};
-    const double hs = dm((double)step, (double)P.step_mult * 0.5);
-    const D3 hd = {dm(g.x, hs), dm(g.y, hs), dm(g.z, hs)};
-    const D3 hg = trilin({da(cur.x, hd.x), da(cur.y, hd.y), da(cur.z, hd.z)}, bf, c);
-    const D3 e2 = {da(dm(hg.x, hs), hd.x), da(dm(hg.y, hs), hd.y), da(dm(hg.z, hs), hd.z)};
-    const D3 df = {ds(e2.x, e1.x), ds(e2.y, e1.y), ds(e2.z, e1.z)};
-    const bool acc = __double2float_rn(magsq(df)) < P.ethresh;
-    D3 np = {da(cur.x, e2.x), da(cur.y, e2.y), da(cur.z, e2.z)};
-    if (nb) {
-      np.x = clampd_ext(np.x, V.X);
-      np.y = clampd_ext(np.y, V.Y);
-      np.z = clampd_ext(np.z, V.Z);
-    }
-    const float grown = __double2float_rn(dm((double)step, 1.8));
-    step = acc ? (grown < sl ? grown : sl) : __double2float_rn(dm((double)step, 0.5));
-    if (acc) {
-      cur = np;
-      const uint8_t st = state[nearest(cur, nb)];
-      if (st == kStSeed || st == kStTerminal) return EV_HIT_PREASSIGNED;
-    }
-    return EV_NONE;
-  }
 };
 
 // Vertices assigned in pass 1 with a differently labelled 6-neighbour (:279-307).
@@ -1361,36 +1224,174 @@ __global__ void boundary_set_kernel(const int32_t* __restrict__ lab, const uint8
 // vertex, integrate until a certain terminal region (or a low gradient / the iteration
 // limit); the streamline's final nearest vertex goes to endv.  The integration reads no
 // labels, so where a vertex's streamline ends does not depend on the wave order.
+//
+// Three lanes per streamline, one per component: ten streamlines a warp.  The FP64 pipe
+// bounds it: it takes a warp instruction some 16 cycles whatever its active lanes, and a
+// streamline of thousands of iterations cannot be split, so what a list takes is mostly one
+// iteration's instructions times the iterations of its longest streamlines.  A lane
+// interpolates its own component only, and the fractions and squares that all three need
+// come by shuffle.  Where a double operation has operands that are floats and its result is
+// rounded to float, the float operation gives the same bits (a product by 0.5, a
+// comparison, and the quotient, since 53 >= 2 * 24 + 2), and takes its place.  With a lane
+// per streamline and everything in double, labels wholly in FP64 took 48 / 381 / 567 ms on
+// 40^3 and 64^3 Gaussian sums and a 128^3 k^-3 volume; so 25 / 177 / 421 ms.
+struct Lane64 {
+  double cur, old, bf, c[8];  // own component
+  int icur, iold, near;       // cur and old truncated, cur's nearest vertex
+};
+__device__ __forceinline__ double shfl_d(double v, int src) { return __shfl_sync(kFullMask, v, src); }
+
+struct Adv64x3 {
+  Adv64 A;
+  int a, l0;              // component, first lane of the streamline
+  int ext, own;           // extent and vertex stride along the component
+  __device__ __forceinline__ bool any3(bool p) const {
+    return ((__ballot_sync(kFullMask, p) >> l0) & 7u) != 0;
+  }
+  __device__ __forceinline__ double sq3(double v) const {
+    const double q = dm(v, v);
+    return da(da(shfl_d(q, l0), shfl_d(q, l0 + 1)), shfl_d(q, l0 + 2));
+  }
+  // The component of the corner gradient at vertex v: 0 + (-0.5f * f[-1]) + (0.0f * f[0]) +
+  // (0.5f * f[+1]), each product a float, summed in double; 0 + (0.0f * f[0]) on a first or
+  // last plane.  i: the vertex's
+  // coordinate along the component
+  __device__ __forceinline__ double corner(int64_t v, int i) const {
+    if ((A.zeroed[v >> 5] >> (v & 31)) & 1u) return 0.0;
+    const float m = __fmul_rn(0.0f, __ldg(A.f + v));
+    if (!(i > 0 && i < ext - 1)) return (double)__fadd_rn(0.0f, m);
+    // (adding a zero, or a NaN that stays one, is exact in float)
+    const float lo = __fadd_rn(__fadd_rn(0.0f, __fmul_rn(-0.5f, __ldg(A.f + v - own))), m);
+    return da((double)lo, (double)__fmul_rn(0.5f, __ldg(A.f + v + own)));
+  }
+  __device__ __forceinline__ static double lerp(double p, double q, double t, double u) { return da(dm(p, u), dm(q, t)); }
+  __device__ __forceinline__ double trilin(double pos, double bf, const double c[8]) const {
+    const double f = ds(pos, bf), u = ds(1.0, f);
+    const double fx = shfl_d(f, l0), fy = shfl_d(f, l0 + 1), fz = shfl_d(f, l0 + 2);
+    const double ux = shfl_d(u, l0), uy = shfl_d(u, l0 + 1), uz = shfl_d(u, l0 + 2);
+    const double x0 = lerp(c[0], c[1], fx, ux), x1 = lerp(c[2], c[3], fx, ux);
+    const double x2 = lerp(c[4], c[5], fx, ux), x3 = lerp(c[6], c[7], fx, ux);
+    return lerp(lerp(x0, x1, fy, uy), lerp(x2, x3, fy, uy), fz, uz);
+  }
+  __device__ __forceinline__ int nearest(double cur) const { return (int)(int64_t)clampd_ext(da(cur, 0.5), ext); }
+  __device__ __forceinline__ int64_t vertex(int i) const {
+    const int64_t x = __shfl_sync(kFullMask, i, l0), y = __shfl_sync(kFullMask, i, l0 + 1);
+    const int64_t z = __shfl_sync(kFullMask, i, l0 + 2);
+    return vid(A.V, x, y, z);
+  }
+  // The FP32 advector's round (Adv32::advance: one uniform iteration for every stepping
+  // lane, the voxel entry folded in).  Every lane of the warp calls it; the lanes of a streamline agree in
+  // everything but their component.
+  __device__ __forceinline__ int advance(int& phase, Lane64& L, int& iters, bool& nb, float& step,
+                                         unsigned long long& ntrips) const {
+    const IntegParams& P = A.P;
+    const bool ent = phase == kLaneEnter, act = ent || phase == kLaneStep;
+    if (__any_sync(kFullMask, ent)) {
+      const bool close = any3(min(L.near, ext - 1 - L.near) <= 1);
+      int b;
+      if (close) b = (int)(int64_t)clampd_ext(L.cur, ext);
+      else b = (int)fmin(fmax(L.cur, 0.0), (double)(ext - 2));
+      int lo = b, hi = b + 1;
+      if (close) {
+        if (b < 0) lo = 0;
+        if (b >= ext - 1) lo = hi = ext - 1;
+      }
+      int at[3][2];
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        at[k][0] = __shfl_sync(kFullMask, lo, l0 + k);
+        at[k][1] = __shfl_sync(kFullMask, hi, l0 + k);
+      }
+      if (ent) {
+        nb = close;
+#pragma unroll
+        for (int n = 0; n < 8; n++)
+          L.c[n] = corner(vid(A.V, at[0][n & 1], at[1][(n >> 1) & 1], at[2][n >> 2]),
+                          (a == 0 ? n & 1 : (a == 1 ? (n >> 1) & 1 : n >> 2)) ? hi : lo);
+        L.bf = (double)b;
+        phase = kLaneStep;
+      }
+    }
+    const bool moved = any3(!(L.old == L.cur)) && !ent, left = any3(L.icur != L.iold) && moved;
+    const double gc = trilin(L.cur, L.bf, L.c);
+    const float gmc = __double2float_rn(__dsqrt_rn(sq3(gc)));
+    const bool bad = !(gmc > 0.f) || !isfinite(gmc);  // no direction to follow
+    const bool counts = act && !(ent && bad);
+    ntrips += counts && a == 0;
+    const bool spent = counts && !(iters > 0);
+    iters -= counts;
+    int ev = spent ? EV_OVER_MAX_ITERATIONS : EV_NONE;
+    if (ent && bad) ev = EV_LOW_GRADIENT;
+    if (!spent && left) ev = EV_OUT_OF_VOXEL;
+    if (!spent && !left && moved && bad) ev = EV_LOW_GRADIENT;
+    const float ms = (float)P.max_step;  // exact: it came as a float
+    const float sl = __fdiv_rn(ms, gmc);
+    const bool go = act && ev == EV_NONE;
+    if (go) {
+      if (ent || __fmul_rn(gmc, step) > ms) step = sl;
+      L.old = L.cur;
+      L.iold = L.icur;
+      if (gmc < P.gthresh) ev = EV_LOW_GRADIENT;
+    }
+    // full step: Vec3d * float multiplies in float (gi_vectors.h:250)
+    const double e1 = (double)__fmul_rn(__double2float_rn(gc), __fmul_rn((float)P.step_mult, step));
+    const double dstep = (double)step;
+    const double hs = dm(dstep, (double)P.step_mult * 0.5), hd = dm(gc, hs);
+    const double hg = trilin(da(L.cur, hd), L.bf, L.c);
+    const double e2 = da(dm(hg, hs), hd);
+    const bool ok = __double2float_rn(sq3(ds(e2, e1))) < P.ethresh;
+    double np = da(L.cur, e2);
+    if (nb) np = clampd_ext(np, ext);
+    const float grown = __double2float_rn(dm(dstep, 1.8));
+    const bool acc = go && ev == EV_NONE && ok;
+    if (go && ev == EV_NONE) step = ok ? (grown < sl ? grown : sl) : __fmul_rn(step, 0.5f);
+    if (acc) {
+      L.cur = np;
+      L.icur = (int)np;
+      L.near = nearest(np);
+    }
+    const int64_t v = vertex(L.near);
+    if (acc) {
+      const uint8_t st = A.state[v];
+      if (st == kStSeed || st == kStTerminal) ev = EV_HIT_PREASSIGNED;
+    }
+    return ev;
+  }
+};
+
 template <int K>
-__global__ void __launch_bounds__(32) fixup_end64_kernel(const Adv64 A, const int64_t* __restrict__ list, int n,
-                                                         const int* __restrict__ n_dev, int32_t* __restrict__ endv,
-                                                         unsigned long long* __restrict__ work,
-                                                         unsigned long long* __restrict__ trips) {
-  const VolDims& V = A.V;
+__global__ void __launch_bounds__(32) fixup_end64_kernel(const Adv64 A64, const int64_t* __restrict__ list, int n,
+                                                           const int* __restrict__ n_dev, int32_t* __restrict__ endv,
+                                                           unsigned long long* __restrict__ work,
+                                                           unsigned long long* __restrict__ trips) {
   if (n_dev) n = *n_dev;  // a list whose length the stream wrote before this launch
-  int phase = kLaneIdle;
+  const int lane = threadIdx.x & 31;
+  Adv64x3 A{A64, lane % 3, lane < 30 ? lane - lane % 3 : 0, 0, 0};
+  const VolDims& V = A64.V;
+  A.ext = (int)(A.a == 0 ? V.X : (A.a == 1 ? V.Y : V.Z));
+  A.own = (int)(A.a == 0 ? 1 : (A.a == 1 ? V.X : V.X * V.Y));
+  int phase = lane < 30 ? kLaneIdle : kLaneDone;  // the last two lanes only take part in the shuffles
   unsigned long long ntrips = 0;
   int64_t v = 0;
-  int x = 0, y = 0, z = 0;
-  D3 cur = {0.0, 0.0, 0.0}, old = cur, g = cur;
-  float gm = 0.f, step = 0.f;
-  int iters = 0;
+  Lane64 L = {};
+  float step = 0.f;
+  int iters = 0, t_iters = 0, t_n = 0;
   bool nb = false;
-  double b[3] = {0.0, 0.0, 0.0};
-  D3 c[8];
-  D3 anchor = cur;  // trapped-streamline test (off in the all-FP64 mode)
-  int t_iters = 0, t_n = 0;
+  double anchor = 0.0;  // trapped-streamline test (off in the all-FP64 mode)
   while (true) {
-    const unsigned long long k = claim_item(phase == kLaneIdle, work);
+    const unsigned long long mine = claim_item(phase == kLaneIdle && A.a == 0, work);
+    const unsigned long long k = __shfl_sync(kFullMask, mine, A.l0);
     if (phase == kLaneIdle) {
       if (k >= (unsigned long long)n) {
         phase = kLaneDone;
       } else {
         v = list[k];
+        int x, y, z;
         split_index(V, v, x, y, z);
-        cur = {(double)x, (double)y, (double)z};
-        iters = A.P.iteration_limit;
-        anchor = cur;
+        L.near = L.icur = A.a == 0 ? x : (A.a == 1 ? y : z);
+        L.cur = (double)L.near;
+        iters = A64.P.iteration_limit;
+        anchor = L.cur;
         t_iters = iters;
         t_n = 0;
         phase = kLaneEnter;
@@ -1401,22 +1402,24 @@ __global__ void __launch_bounds__(32) fixup_end64_kernel(const Adv64 A, const in
       break;
     }
     for (int r = 0; r < K; r++) {
-      if (phase != kLaneEnter && phase != kLaneStep) continue;
-      const int ev = A.advance(phase, x, y, z, cur, old, iters, nb, b, c, g, gm, step, ntrips);
-      if (ev == EV_NONE) continue;
-      A.nearest3(cur, x, y, z);
-      phase = ev == EV_OUT_OF_VOXEL ? kLaneEnter : kLaneEnd;
+      const bool on = phase == kLaneEnter || phase == kLaneStep;
+      const int ev = A.advance(phase, L, iters, nb, step, ntrips);
+      if (on && ev != EV_NONE) phase = ev == EV_OUT_OF_VOXEL ? kLaneEnter : kLaneEnd;
     }
-    if (phase == kLaneStep && A.P.trap_window > 0 && t_iters - iters >= A.P.trap_window) {
-      t_iters = iters;
-      if (A.trapped(cur, anchor, t_n)) {  // ends where the iteration limit would have
-        A.nearest3(cur, x, y, z);
-        phase = kLaneEnd;
+    const bool check = phase == kLaneStep && A64.P.trap_window > 0 && t_iters - iters >= A64.P.trap_window;
+    if (__any_sync(kFullMask, check)) {
+      const bool far = A.any3(fabs(L.cur - anchor) >= (double)A64.P.trap_radius);
+      if (check) {
+        t_iters = iters;
+        t_n = far ? 0 : t_n + 1;
+        anchor = L.cur;
+        if (t_n >= 2) phase = kLaneEnd;  // ends where the iteration limit would have
       }
     }
+    const int64_t e = A.vertex(L.near);
     if (phase != kLaneEnd) continue;
     phase = kLaneIdle;
-    endv[v] = (int32_t)vid(V, x, y, z);
+    if (A.a == 0) endv[v] = (int32_t)e;
   }
 }
 
@@ -1985,15 +1988,15 @@ cudaError_t launch_fixup_end64(const float* f, const uint32_t* zeroed, const Vol
                                unsigned long long* trips, int num_sms, cudaStream_t stream, const int* n_dev) {
   if (n <= 0) return cudaSuccess;
   Adv64 A{f, zeroed, V, P, state};
-  const int blocks = (n + 31) / 32;
   if (cudaError_t e = cudaMemsetAsync(work, 0, sizeof(unsigned long long), stream)) return e;
   ::msc::count_launch();
   // one-warp CTAs, at most four per SM: the FP64 re-decisions are few (~0.1% of the
-  // re-decisions) and bound by each SM's FP64 pipe, which executes every warp
-  // instruction in full however few lanes are active -- so a small wave is spread over
-  // as many SMs as it has warps, and a large one keeps a few items per lane
+  // re-decisions) and bound by each SM's FP64 pipe, so a small wave is spread over as many
+  // SMs as it has warps, and a large one keeps several items per lane (2 / 4 / 8 / 16 per SM:
+  // 538 / 412 / 386 / 421 ms at 128^3, 186 / 175 / 185 / 190 ms at 64^3)
   // iterations per turn: MSC_TRIPS_PER_TURN_FP64 (2, 4, 8 or 16) overrides the default
   static const int k = trips_env("MSC_TRIPS_PER_TURN_FP64", 2);
+  const int blocks = (n + 9) / 10;
   const int grid = (blocks < num_sms * 4 && !n_dev) ? blocks : num_sms * 4;
   switch (k) {
     case 4:

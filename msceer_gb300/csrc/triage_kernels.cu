@@ -1,27 +1,33 @@
 // Learned triage: a 3x3x3 convolutional network (Cin -> 16 -> 16 -> 2 channels) that
 // flags the vertices whose integrated destination differs from their combinatorial
 // steepest-path destination.  Forward and input-gradient convolutions are BF16
-// implicit GEMMs on the tcgen05 tensor cores with FP32 accumulation in TMEM; the
-// weight gradient, loss and optimiser run on the CUDA cores in FP32.
+// implicit GEMMs on the tcgen05 tensor cores with FP32 accumulation in TMEM, and so is the
+// weight gradient; loss and optimiser run on the CUDA cores in FP32.
 //
 // Activation layout ("row-planar"): [Z][Y][2][X][8] BF16.  Each (y, z) row of the
 // volume holds two planes, channels 0-7 and channels 8-15, each X x 16 bytes.  That
 // is the K-major, no-swizzle operand layout of the MMA (8-row x 16-byte core
-// matrices, rows 16 bytes apart), so an A operand is a plain address into a staged
+// matrices, rows 16 bytes apart), so an operand is a plain address into a staged
 // row: output vertices x0..x0+127 under tap (dx, dy, dz) read the staged row of
 // (y+dy, z+dz) starting at x0+dx.
 //
-// A tile is a 128 (x) x 4 (y) block of output rows at one z: its 130 x 6 x 3 input rows are
-// staged by bulk copies, one per 8-channel plane of a row (zeros outside the volume), one
-// thread issues the 4 x 27 MMAs (M=128 vertices, N=16 output channels, K=16 input channels
-// each) into four TMEM accumulators, and four warps read them back for the epilogue.  One
-// CTA per SM keeps the 27 weight taps in shared memory and works through its tiles with two
-// stages and two sets of accumulators, so that the load of a tile, the MMAs of the one
-// before and the epilogue of the one before that run side by side.
-// (A CTA per tile did the three one after another, with a TMEM allocation and the weights'
-// load for each: 181-217 us a layer at 128^3; so 152-159 us.  Tensor-map loads instead of
-// the bulk copies come to the same within a tenth.  The MMAs bound it, at 95 cycles each
-// whatever their N; a layer's activations in and out take 20 us of HBM time.)
+// A convolution's tile is 128 (x) x 8 (y) output vertices at one z, and its accumulator 128
+// x 128: a TMEM lane is an output row and one of 16 output channels, a column a vertex.  An
+// input row belongs to up to three of the eight output rows, at dy = -1, 0, +1, so one MMA
+// (M = eight rows x 16 channels, N = 128 vertices, K = 16 input channels) takes it to all of
+// them: the weights of dy = +1, 0, -1 lie one after the other, so that the operand of input
+// row yy, at the block of dy = yy, holds for output row j the weights of dy = yy - j; the
+// lanes of the other rows are switched off.  90 MMAs for a tile's 8 x 27 taps, each output
+// row's in the order dz, dy, dx, all of one shape on one accumulator and so in order.
+// One CTA per SM keeps the weights in shared memory and works through a run of tiles along
+// z, each with one new plane of input rows (10 x 130, staged by bulk copies, one per
+// 8-channel plane of a row, zeros outside the volume) in a ring of four, and two
+// accumulators, so that the load of a plane, the MMAs of a tile and the epilogue of the one
+// before run side by side.  The epilogue turns lanes of channels into rows of vertices in
+// shared memory.
+// (One MMA per tap and output row, M = 128 vertices and N = 16 channels, took the same 95
+// cycles, 108 of them for 4 x 128 vertices: 152-159 us a layer at 128^3, and with a CTA per
+// tile 181-217 us; so 80-87 us.  A layer's activations in and out take 20 us of HBM time.)
 #include <cuda_bf16.h>
 
 #include "tc_sm100.cuh"
@@ -30,21 +36,27 @@
 namespace msc {
 
 namespace {
-constexpr int kBX = 128;  // output vertices per row (MMA M)
-constexpr int kBY = 4;    // output rows per CTA (along y)
-constexpr int kInX = kBX + 2, kInY = kBY + 2, kInZ = 3;
-constexpr int kPlaneB = (kBX + 2) * 16;             // one staged 8-channel plane
+constexpr int kBX = 128;                            // vertices of a tile along x
+constexpr int kInX = kBX + 2, kInZ = 3;
+constexpr int kPlaneB = kInX * 16;                  // one staged 8-channel plane of a row
 constexpr int kRowB = 2 * kPlaneB;                  // one staged row
-constexpr int kStageB = kRowB * kInY * kInZ;        // the TMA box
-constexpr int kTapB = 512;                          // 16 x 16 BF16 weights of one tap
-constexpr int kWeightB = 27 * kTapB;
-constexpr int kStages = 2;
-constexpr int kSmemConv = 1024 + kStages * kStageB + kWeightB + 128;
-constexpr uint32_t kSetCols = 64;                   // 4 accumulators of 16 columns
-constexpr uint32_t kTmemCols = kStages * kSetCols;
+// convolution
+constexpr int kCY = 8, kCInY = kCY + 2;             // output rows, input rows per z
+constexpr int kSlotB = kCInY * kRowB;               // a ring slot: the input rows of one z
+constexpr int kSlots = 4;
+constexpr int kTapB = 256;                          // 16 rows (output channels) x 8 BF16 of a tap
+constexpr int kHalfB = 27 * kTapB;                  // of one 8-channel half of K
+constexpr int kWeightB = 2 * kHalfB;
+constexpr int kWPadB = (kCY - 1) * kTapB;           // the operands reach so far to either side of the weights
+constexpr int kOutPlaneB = kBX * 16 + 32;           // epilogue: a row's 8-channel plane, clear of the others' banks
+constexpr int kOutB = 4 * kOutPlaneB;               // of one warp: two rows
+constexpr int kSmemConv = 1024 + kSlots * kSlotB + 2 * kWPadB + kWeightB + 4 * kOutB + 128;
+constexpr uint32_t kSetCols = kBX;                  // columns of an accumulator
+constexpr uint32_t kTmemCols = 2 * kSetCols;
 constexpr int kConvThreads = 192;                   // four epilogue warps, the MMAs', the loads'
-static_assert(kStageB % 16 == 0 && kWeightB % 16 == 0, "bulk copy sizes");
-static_assert(kBY * 16 <= (int)kSetCols, "accumulators fit the allocation");
+static_assert(kSlotB % 16 == 0 && kWPadB % 16 == 0 && kWeightB % 16 == 0 && kOutB % 16 == 0, "16-byte copies");
+static_assert(kSmemConv <= 227 * 1024, "shared memory of a block");
+static_assert(2 * kBX * 2 * 4 <= kOutB, "two rows' logits fit a warp's staging");
 }  // namespace
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -102,63 +114,98 @@ __device__ __forceinline__ void stage_rows(unsigned char* dst, const __nv_bfloat
                 act + ((((int64_t)z * D.Y + y) * 2 + (p & 1)) * D.X + xa) * 8, bytes, bar);
 }
 
-struct ConvTiles {
+// Tiles of a convolution, z fastest.
+struct ConvColumns {
   int nx, ny;
-  int64_t n;
+  int64_t Z, n;
   __device__ __forceinline__ void at(int64_t t, int& x0, int& y0, int& z) const {
-    const int64_t r = t / nx;
-    x0 = (int)(t - r * nx) * kBX;
-    y0 = (int)(r % ny) * kBY;
-    z = (int)(r / ny);
+    const int64_t c = t / Z, r = c / nx;
+    z = (int)(t - c * Z);
+    x0 = (int)(c - r * nx) * kBX;
+    y0 = (int)r * kCY;
   }
+  // tiles of block b of g
+  __device__ __forceinline__ int64_t first(int b, int g) const { return n / g * b + (n % g * b) / g; }
 };
 
+// The mask's values for one warp's share of a tile, as conv_epilogue writes it.  They are
+// asked for before the wait for the tile's MMAs: loaded where they are used, the mask held
+// up the epilogue (164 us a layer at 128^3 instead of 87).
+__device__ __forceinline__ void load_mask(uint4 (&m)[16], const __nv_bfloat16* __restrict__ mask_act, int x0, int y,
+                                          int z, const ConvDims& D) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const int q = i >> 2, x = x0 + lane + 32 * (i & 3);  // q: row, plane
+    m[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (y + (q >> 1) < D.Y && x < D.X)
+      m[i] = *reinterpret_cast<const uint4*>(mask_act +
+                                             ((((int64_t)z * D.Y + y + (q >> 1)) * 2 + (q & 1)) * D.X + x) * 8);
+  }
+}
+
+// One warp's share of a tile: the accumulator lanes of output rows 2 w and 2 w + 1.
+// `done` gets an arrival when they have been read.
 template <int EPI>
-__device__ __forceinline__ void conv_epilogue(uint32_t tl, int x, int y0, int z, const float* __restrict__ bias,
+__device__ __forceinline__ void conv_epilogue(uint32_t tl, unsigned char* s_out, int x0, int y, int z, float bias,
                                               const ConvDims& D, __nv_bfloat16* __restrict__ out_act,
                                               float* __restrict__ out_logits,
-                                              const __nv_bfloat16* __restrict__ mask_act, uint64_t* done) {
+                                              const uint4 (&mask)[16], uint64_t* done) {
+  const int lane = threadIdx.x & 31, row = lane >> 4, ch = lane & 15;
+  const bool odd = lane & 1;
+  unsigned char* mine = s_out + (2 * row + (ch >> 3)) * kOutPlaneB + (odd ? 16 : 0) + (ch & 6) * 2;
+  __syncwarp();  // the tile before has left the staging
 #pragma unroll 1
-  for (int j = 0; j < kBY; j++) {
+  for (int c = 0; c < kBX; c += 16) {
     float v[16];
-    tc::tmem_ld16(tl + 16 * j, v);
-    if (j == kBY - 1) {  // the accumulators are free for the next tile but one
-      tc::fence_before_sync();
-      __syncwarp();
-      if ((threadIdx.x & 31) == 0) tc::mbar_arrive(done);
-    }
-    const int y = y0 + j;
-    if (x >= D.X || y >= D.Y) continue;
-    const int64_t row = (int64_t)z * D.Y + y;
+    tc::tmem_ld16(tl + c, v);
     if (EPI == kEpiLogits) {
-      const int64_t vid = row * D.X + x;
-      out_logits[vid] = v[0] + bias[0];
-      out_logits[D.N + vid] = v[1] + bias[1];
+      if (ch < 2) {
+        float4* o = reinterpret_cast<float4*>(s_out + (2 * row + ch) * kBX * 4 + c * 4);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          o[k] = make_float4(v[4 * k] + bias, v[4 * k + 1] + bias, v[4 * k + 2] + bias, v[4 * k + 3] + bias);
+      }
     } else {
-      __nv_bfloat16* o = out_act + row * 2 * D.X * 8;  // row base, plane 0
-      float m[16];
+      uint32_t h[16];
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        const float a = EPI == kEpiReluBf16 ? fmaxf(v[k] + bias, 0.f) : v[k];
+        h[k] = __bfloat16_as_ushort(__float2bfloat16_rn(a));
+      }
+      // two channels to a word: the even lane of a pair takes the even vertices
+#pragma unroll
+      for (int k = 0; k < 16; k += 2) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? h[k] : h[k + 1], 1);
+        *reinterpret_cast<uint32_t*>(mine + (c + k) * 16) = odd ? (got | (h[k + 1] << 16)) : (h[k] | (got << 16));
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncwarp();
+  if (lane == 0) tc::mbar_arrive(done);
+  if constexpr (EPI == kEpiLogits) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {  // row, channel
+      if (y + (q >> 1) >= D.Y) continue;
+      const float* sv = reinterpret_cast<const float*>(s_out) + q * kBX;
+      float* o = out_logits + (q & 1) * D.N + ((int64_t)z * D.Y + y + (q >> 1)) * D.X + x0;
+      for (int x = lane; x < kBX && x0 + x < D.X; x += 32) o[x] = sv[x];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int q = i >> 2, x = lane + 32 * (i & 3);  // q: row, plane
+      if (y + (q >> 1) >= D.Y || x0 + x >= D.X) continue;
+      uint4 r = *reinterpret_cast<const uint4*>(s_out + q * kOutPlaneB + x * 16);
       if (EPI == kEpiMaskBf16) {
-        const __nv_bfloat16* mk = mask_act + row * 2 * D.X * 8;
-        const uint4 q0 = *reinterpret_cast<const uint4*>(mk + (int64_t)x * 8);
-        const uint4 q1 = *reinterpret_cast<const uint4*>(mk + (int64_t)(D.X + x) * 8);
-        const __nv_bfloat16* h0 = reinterpret_cast<const __nv_bfloat16*>(&q0);
-        const __nv_bfloat16* h1 = reinterpret_cast<const __nv_bfloat16*>(&q1);
+        const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&mask[i]);
+        __nv_bfloat16* rh = reinterpret_cast<__nv_bfloat16*>(&r);
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-          m[c] = __bfloat162float(h0[c]) > 0.f ? 1.f : 0.f;
-          m[8 + c] = __bfloat162float(h1[c]) > 0.f ? 1.f : 0.f;
-        }
+        for (int c = 0; c < 8; c++)
+          rh[c] = __float2bfloat16_rn(__bfloat162float(rh[c]) * (__bfloat162float(mh[c]) > 0.f ? 1.f : 0.f));
       }
-      __align__(16) __nv_bfloat16 r[16];
-#pragma unroll
-      for (int c = 0; c < 16; c++) {
-        float a = v[c];
-        if (EPI == kEpiReluBf16) a = fmaxf(a + bias[c], 0.f);
-        else a = a * m[c];
-        r[c] = __float2bfloat16_rn(a);
-      }
-      *reinterpret_cast<uint4*>(o + (int64_t)x * 8) = *reinterpret_cast<const uint4*>(&r[0]);
-      *reinterpret_cast<uint4*>(o + (int64_t)(D.X + x) * 8) = *reinterpret_cast<const uint4*>(&r[8]);
+      *reinterpret_cast<uint4*>(out_act + ((((int64_t)z * D.Y + y + (q >> 1)) * 2 + (q & 1)) * D.X + x0 + x) * 8) = r;
     }
   }
 }
@@ -166,29 +213,33 @@ __device__ __forceinline__ void conv_epilogue(uint32_t tl, int x, int y0, int z,
 // Every wait is bounded; a role whose wait runs out reports it in err and ends, and the
 // others' waits run out after it.
 template <int EPI>
-__global__ void __launch_bounds__(kConvThreads) conv3_tc_kernel(const __nv_bfloat16* __restrict__ in_act,
+__global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __nv_bfloat16* __restrict__ in_act,
                                                                 const uint8_t* __restrict__ wblob,
                                                                 const float* __restrict__ bias, const ConvDims D,
-                                                                const ConvTiles T, __nv_bfloat16* __restrict__ out_act,
+                                                                const ConvColumns T,
+                                                                __nv_bfloat16* __restrict__ out_act,
                                                                 float* __restrict__ out_logits,
                                                                 const __nv_bfloat16* __restrict__ mask_act,
                                                                 int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* s_in = sm;
-  unsigned char* s_w = sm + kStages * kStageB;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + kWeightB);
-  uint64_t* full = bars;                   // a stage's input rows (and, first of all, the weights) have come
-  uint64_t* empty = bars + kStages;        // its MMAs are done
-  uint64_t* tfull = bars + 2 * kStages;    // a set of accumulators is ready
-  uint64_t* tempty = bars + 3 * kStages;   // and read
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 4 * kStages);
+  unsigned char* s_w = sm + kSlots * kSlotB + kWPadB;
+  unsigned char* s_out = s_w + kWeightB + kWPadB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_out + 4 * kOutB);
+  uint64_t* full = bars;                // a slot's input rows (and, with the first, the weights) have come
+  uint64_t* empty = bars + kSlots;      // the MMAs that read it are done
+  uint64_t* tfull = bars + 2 * kSlots;  // an accumulator is ready
+  uint64_t* tempty = tfull + 2;         // and read
+  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(tempty + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int q = 0; q < kStages; q++) {
+    for (int q = 0; q < kSlots; q++) {
       tc::mbar_init(&full[q], 1);
       tc::mbar_init(&empty[q], 1);
+    }
+    for (int q = 0; q < 2; q++) {
       tc::mbar_init(&tfull[q], 1);
       tc::mbar_init(&tempty[q], 4);
     }
@@ -199,68 +250,104 @@ __global__ void __launch_bounds__(kConvThreads) conv3_tc_kernel(const __nv_bfloa
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tbase = *s_tmem;
+  const int64_t t0 = T.first(blockIdx.x, gridDim.x), t1 = T.first(blockIdx.x + 1, gridDim.x);
 
-  if (warp == 5) {  // loads
+  if (warp == 5) {  // loads: a tile's three planes, or its third where the tile before had the others
     int64_t i = 0;
-    for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
-      const int q = (int)(i % kStages);
-      const bool ok = i < kStages || tc::mbar_wait(&empty[q], (uint32_t)(i / kStages - 1) & 1u);
-      if (!__all_sync(0xffffffffu, ok)) {
-        if (lane == 0) atomicOr(err, 1);
-        break;
-      }
+    bool ok = true;
+    for (int64_t t = t0; t < t1 && ok; t++) {
       int x0, y0, z;
       T.at(t, x0, y0, z);
-      if (i == 0 && lane == 0) bulk_load(s_w, wblob, (uint32_t)kWeightB, &full[q]);
-      stage_rows<kInX, kInY, kInZ>(s_in + q * kStageB, in_act, D, x0 - 1, y0 - 1, z - 1,
+      for (int dz = (t == t0 || z == 0) ? -1 : 1; dz <= 1 && ok; dz++, i++) {
+        const int q = (int)(i % kSlots);
+        ok = i < kSlots || tc::mbar_wait(&empty[q], (uint32_t)(i / kSlots - 1) & 1u);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) {
+          if (lane == 0) atomicOr(err, 1);
+          break;
+        }
+        if (i == 0 && lane == 0) bulk_load(s_w, wblob, (uint32_t)kWeightB, &full[q]);
+        stage_rows<kInX, kCInY, 1>(s_in + q * kSlotB, in_act, D, x0 - 1, y0 - 1, z + dz,
                                    i == 0 ? (uint32_t)kWeightB : 0u, &full[q]);
+      }
     }
     // every load has landed before the block ends, also where the MMAs gave up on it
-    for (int64_t k = i > kStages ? i - kStages : 0; k < i; k++)
-      if (!tc::mbar_wait(&full[k % kStages], (uint32_t)(k / kStages) & 1u) && lane == 0) atomicOr(err, 1);
+    for (int64_t k = i > kSlots ? i - kSlots : 0; k < i; k++)
+      if (!tc::mbar_wait(&full[k % kSlots], (uint32_t)(k / kSlots) & 1u) && lane == 0) atomicOr(err, 1);
   } else if (warp == 4) {  // MMAs
     if (lane == 0) {
-      constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 16);
-      const uint32_t b0 = tc::smem_u32(s_w);
-      int64_t i = 0;
-      for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
-        const int q = (int)(i % kStages);
-        if (!tc::mbar_wait(&full[q], (uint32_t)(i / kStages) & 1u) ||
-            (i >= kStages && !tc::mbar_wait(&tempty[q], (uint32_t)(i / kStages - 1) & 1u))) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(128, kBX);
+      const uint32_t w0 = tc::smem_u32(s_w), i0 = tc::smem_u32(s_in);
+      int64_t s = 0, have = 0;  // the tile's first plane, planes that have come
+      for (int64_t t = t0; t < t1; t++) {
+        int x0, y0, z;
+        T.at(t, x0, y0, z);
+        const int q = (int)((t - t0) & 1);
+        const uint32_t use = (uint32_t)((t - t0) >> 1);
+        bool ok = use == 0 || tc::mbar_wait(&tempty[q], (use - 1) & 1u);
+        for (; have < s + 3 && ok; have++) ok = tc::mbar_wait(&full[have % kSlots], (uint32_t)(have / kSlots) & 1u);
+        if (!ok) {
           atomicOr(err, 1);
           break;
         }
         tc::fence_after_sync();
-        const uint32_t a0 = tc::smem_u32(s_in + q * kStageB), d0 = tbase + q * kSetCols;
+        const uint32_t d = tbase + q * kSetCols;
 #pragma unroll 1
-        for (int tap = 0; tap < 27; tap++) {
-          const int dx = tap % 3, dy = (tap / 3) % 3, dz = tap / 9;  // 0..2 = offset -1..+1
-          const uint64_t bd = tc::smem_desc(b0 + tap * kTapB, 256, 128);
+        for (int dz = 0; dz < 3; dz++) {
+          const uint32_t rows = i0 + (uint32_t)((s + dz) % kSlots) * kSlotB;
 #pragma unroll
-          for (int j = 0; j < kBY; j++) {  // (four accumulators in turn: no MMA waits for the one before)
-            const uint32_t a = a0 + (uint32_t)((dz * kInY + j + dy) * kRowB + dx * 16);
-            tc::mma_bf16(d0 + 16 * j, tc::smem_desc(a, kPlaneB, 128), bd, idesc, tap > 0);
+          for (int yy = 0; yy < kCInY; yy++) {
+            // output rows lo .. hi take this input row, at dy = yy - j
+            const int lo = yy > 2 ? yy - 2 : 0, hi = yy < kCY ? yy : kCY - 1;
+            uint32_t off[4], old[4], fresh[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              off[k] = old[k] = fresh[k] = 0;
+              for (int j = 2 * k; j < 2 * k + 2; j++) {
+                const uint32_t m = 0xFFFFu << (16 * (j & 1));
+                if (j < lo || j > hi) off[k] |= m;
+                if (j < lo || j >= yy) old[k] |= m;
+                if (j != yy) fresh[k] |= m;
+              }
+            }
+#pragma unroll
+            for (int dx = 0; dx < 3; dx++) {
+              const uint64_t a =
+                  tc::smem_desc(w0 + (uint32_t)(((dz * 3 + dx) * 3 + 2 - yy) * kTapB), kHalfB, 128);
+              const uint64_t b = tc::smem_desc(rows + (uint32_t)(yy * kRowB + dx * 16), kPlaneB, 128);
+              if (dx == 0 && yy < kCY && dz == 0) {  // output row yy starts here
+                if (yy > 0) tc::mma_bf16_lanes(d, a, b, idesc, old, true);
+                tc::mma_bf16_lanes(d, a, b, idesc, fresh, false);
+              } else {
+                tc::mma_bf16_lanes(d, a, b, idesc, off, true);
+              }
+            }
           }
         }
-        tc::mma_commit(&empty[q]);
+        // planes that no further tile reads: one, or all at the end of a column
+        const int last = (z == D.Z - 1 || t == t1 - 1) ? 3 : 1;
+        for (int k = 0; k < last; k++) tc::mma_commit(&empty[(s + k) % kSlots]);
         tc::mma_commit(&tfull[q]);
+        s += last;
       }
     }
   } else {  // epilogue
-    int64_t i = 0;
-    for (int64_t t = blockIdx.x; t < T.n; t += gridDim.x, i++) {
-      const int q = (int)(i % kStages);
-      const bool ok = tc::mbar_wait(&tfull[q], (uint32_t)(i / kStages) & 1u);
+    const int ch = lane & 15;
+    const float b = EPI == kEpiMaskBf16 ? 0.f : (EPI == kEpiLogits && ch >= 2 ? 0.f : bias[ch]);
+    for (int64_t t = t0; t < t1; t++) {
+      const int q = (int)((t - t0) & 1);
+      int x0, y0, z;
+      T.at(t, x0, y0, z);
+      uint4 mask[16];
+      if (EPI == kEpiMaskBf16) load_mask(mask, mask_act, x0, y0 + 2 * warp, z, D);
+      const bool ok = tc::mbar_wait(&tfull[q], (uint32_t)((t - t0) >> 1) & 1u);
       if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) atomicOr(err, 2);
         break;
       }
       tc::fence_after_sync();
-      int x0, y0, z;
-      T.at(t, x0, y0, z);
-      // TMEM lane = output vertex
-      conv_epilogue<EPI>(tbase + q * kSetCols + ((uint32_t)(32 * warp) << 16), x0 + 32 * warp + lane, y0, z, bias, D,
-                         out_act, out_logits, mask_act, &tempty[q]);
+      conv_epilogue<EPI>(tbase + q * kSetCols + ((uint32_t)(32 * warp) << 16), s_out + warp * kOutB, x0, y0 + 2 * warp,
+                         z, b, D, out_act, out_logits, mask, &tempty[q]);
     }
   }
   __syncwarp();
@@ -287,6 +374,18 @@ __global__ void __launch_bounds__(kConvThreads) conv3_tc_kernel(const __nv_bfloa
 // accumulators kept in TMEM over all tiles).
 // The CUDA-core form (27 x 2 accumulators per thread, X and dY staged as FP32) took 1.0 ms
 // a layer at 128^3; this one 197-211 us.
+constexpr int kBY = 4, kInY = kBY + 2;              // output rows of a tile, input rows per z
+constexpr int kStageB = kRowB * kInY * kInZ;
+struct ConvTiles {
+  int nx, ny;
+  int64_t n;
+  __device__ __forceinline__ void at(int64_t t, int& x0, int& y0, int& z) const {
+    const int64_t r = t / nx;
+    x0 = (int)(t - r * nx) * kBX;
+    y0 = (int)(r % ny) * kBY;
+    z = (int)(r / ny);
+  }
+};
 constexpr int kDyB = kBY * 2 * kBX * 16;  // staged dY rows
 constexpr int kSmemWgrad = 1024 + kStageB + kDyB + 64;
 constexpr uint32_t kWgradSet = 96;        // 6 x 16 columns
@@ -437,7 +536,11 @@ template <int EPI>
 static cudaError_t launch_conv(const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias, const ConvDims& D,
                                __nv_bfloat16* out_act, float* out_logits, const __nv_bfloat16* mask_act, int* err,
                                int num_sms, cudaStream_t st) {
-  const ConvTiles T = conv_tiles(D);
+  ConvColumns T;
+  T.nx = (int)((D.X + kBX - 1) / kBX);
+  T.ny = (int)((D.Y + kCY - 1) / kCY);
+  T.Z = D.Z;
+  T.n = (int64_t)T.nx * T.ny * D.Z;
   cudaError_t e = cudaFuncSetAttribute(conv3_tc_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemConv);
   if (e != cudaSuccess) return e;
   ::msc::count_launch();

@@ -208,7 +208,10 @@ __global__ void pack_weights_kernel(const float* __restrict__ params, uint8_t* _
       const int l = b - 2;  // layer 2 or 3 (0-based 1, 2)
       w = params[l * kTriageW + (26 - t) * 256 + n * 16 + k];  // cin = n, cout = k
     }
-    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(blobs + (size_t)b * 27 * 512 + t * 512 + (k / 8) * 256 + n * 16);
+    // per 8-channel half of K and (dz, dx) the taps dy = +1, 0, -1, 16 rows (n) of 16 bytes each
+    const int dx = t % 3, dy = (t / 3) % 3, dz = t / 9;
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(blobs + (size_t)b * 27 * 512 + (k / 8) * 27 * 256 +
+                                                          ((dz * 3 + dx) * 3 + 2 - dy) * 256 + n * 16);
     dst[k % 8] = __float2bfloat16_rn(w);
   }
 }

@@ -183,3 +183,24 @@ def test_trained_network_saves_redecisions(gpu):
         print(d, "re-decisions saved", saved, "label difference", mism)
         assert saved > 0.05, saved
         assert mism <= 1e-3, mism
+
+
+@pytest.mark.parametrize("shape", [(67, 17, 129), (160, 8, 128), (2, 1, 1), (310, 1, 3), (1, 40, 257)],
+                         ids=lambda s: "x".join(map(str, s)))
+def test_convolution_tiles(gpu, shape):
+    """Runs of tiles along z that start and end inside a column, volumes of fewer tiles than
+    SMs, tiles with rows and vertices past the volume: the forward pass as above, and
+    the input gradients through the parameter gradients of the first two layers."""
+    import torch
+    from msceer_gb300 import triage
+    test_forward_matches_oracle(gpu, shape)
+    feat, w, y, raw = random_problem(shape, 5)
+    wt = torch.from_numpy(w).cuda()
+    a1, a2, logits = triage.forward(raw, shape, wt)
+    loss, g = triage.backward(raw, a1, a2, logits, torch.from_numpy(y.reshape(2, -1)).cuda(), shape, wt, 3.0)
+    want_loss, want_g = T.loss_and_grads(feat, w, y, 3.0)
+    g = g.cpu().numpy().astype(np.float64)
+    assert abs(loss - want_loss) <= 1e-3 * abs(want_loss)
+    for name, sl in (("W1", slice(0, T.NW)), ("W2", slice(T.NW, 2 * T.NW)), ("W3", slice(2 * T.NW, 3 * T.NW))):
+        err = np.linalg.norm(g[sl] - want_g[sl]) / max(np.linalg.norm(want_g[sl]), 1e-30)
+        assert err < 0.02, (name, err)

@@ -37,7 +37,7 @@ namespace msc {
 
 namespace {
 constexpr int kBX = 128;                            // vertices of a tile along x
-constexpr int kInX = kBX + 2, kInZ = 3;
+constexpr int kInX = kBX + 2;
 constexpr int kPlaneB = kInX * 16;                  // one staged 8-channel plane of a row
 constexpr int kRowB = 2 * kPlaneB;                  // one staged row
 // convolution
@@ -361,176 +361,180 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3_tc_kernel(const __nv_bf
 //
 // dW[tap][cin][cout] = sum over the vertices v of X[v + tap][cin] * dY[v][cout], db[cout] =
 // sum dY[v][cout]: the vertices are the MMA's K, so both operands are MN-major as the
-// row-planar rows lie (a core matrix is 8 channels x 8 vertices).  A tile's staged X is 18
-// rows (3 z x 6 y) of two 8-channel planes, all planes kPlaneB apart, so one M = 128
-// operand spans eight consecutive rows: for output row j the rows from j on hold the taps
-// (dy, dz) = (0..2, 0) and, six rows on, (0..1, 1); the rows from j + 8 on (2, 1) and, four
-// rows on, (0..2, 2).  With dx as a shift of 16 bytes, two MMAs per dx and 16 vertices
-// cover all 27 taps; the products of the other rows are not read.  The tensor core's FP32
-// accumulation loses up to an ulp per MMA, so its six accumulators (dx, which of the two)
-// run over one output row only, eight MMAs, and are added to FP32 registers; two sets take
-// turns, so that a row's MMAs run while the one before is read.  Against 64 bits the
-// layer-3 gradient at 128^3 is off by 2.9e-7 (4.4e-7 with FP32 FMAs, 4.3e-6 with the
-// accumulators kept in TMEM over all tiles).
+// row-planar rows lie (a core matrix is 8 channels x 8 vertices).  A tile is 128 (x) x 2 (y)
+// x 2 (z) vertices; its staged X is the 4 x 4 rows around, all 8-channel planes kPlaneB
+// apart, so M = 128 spans eight rows, and its dY the four rows, N = 64.  With dx as a shift
+// of 16 bytes, six MMAs per 16 vertices (three dx, two halves of the rows) give the products
+// of every input row with every output row; those with -1 <= dy, dz <= 1 are read.  An MMA
+// takes some 95 cycles whatever its N up to 128, so few and wide ones bound it least: with
+// one output row (N = 16) it took four times as many.
+// The tensor core's FP32 accumulation loses up to an ulp per MMA, so an accumulator runs
+// over one tile only, eight MMAs, and is added to FP32 registers: 16 warps, each with the
+// lanes of its quarter, one half of the rows and one z of dY.  Against 64 bits the layer-3
+// gradient at 128^3 is off by 2.5e-7 (4.4e-7 with FP32 FMAs, 4.3e-6 with the accumulators kept
+// in TMEM over all tiles).
 // The CUDA-core form (27 x 2 accumulators per thread, X and dY staged as FP32) took 1.0 ms
-// a layer at 128^3; this one 197-211 us.
-constexpr int kBY = 4, kInY = kBY + 2;              // output rows of a tile, input rows per z
-constexpr int kStageB = kRowB * kInY * kInZ;
-struct ConvTiles {
+// a layer at 128^3, one output row to an MMA 197-211 us; so 95 us.
+constexpr int kGY = 2, kGZ = 2;                     // output rows of a tile
+constexpr int kGRows = (kGY + 2) * (kGZ + 2);       // its input rows
+constexpr int kXB = kGRows * kRowB, kDyB = kGY * kGZ * 2 * kBX * 16;
+constexpr int kGStageB = kXB + kDyB;
+constexpr int kSmemWgrad = 1024 + 2 * kGStageB + 64;
+constexpr int kWgradThreads = 512;
+constexpr uint32_t kAccCols = 16 * kGY * kGZ;       // columns of one of the six accumulators
+constexpr uint32_t kWgradCols = 512;
+static_assert(kGRows == 16 && 6 * kAccCols <= kWgradCols, "two operands of eight rows");
+static_assert(27 * 256 * 4 + 16 * 8 * 4 <= kGStageB, "the final sums fit a stage");
+struct WgradTiles {
   int nx, ny;
   int64_t n;
-  __device__ __forceinline__ void at(int64_t t, int& x0, int& y0, int& z) const {
+  __device__ __forceinline__ void at(int64_t t, int& x0, int& y0, int& z0) const {
     const int64_t r = t / nx;
     x0 = (int)(t - r * nx) * kBX;
-    y0 = (int)(r % ny) * kBY;
-    z = (int)(r / ny);
+    y0 = (int)(r % ny) * kGY;
+    z0 = (int)(r / ny) * kGZ;
   }
 };
-constexpr int kDyB = kBY * 2 * kBX * 16;  // staged dY rows
-constexpr int kSmemWgrad = 1024 + kStageB + kDyB + 64;
-constexpr uint32_t kWgradSet = 96;        // 6 x 16 columns
-constexpr uint32_t kWgradCols = 256;      // two sets
-static_assert(18 * kRowB == kStageB && kRowB <= kDyB, "the row after the last staged one lies in shared memory");
 
-__global__ void __launch_bounds__(128, 2) conv_wgrad_tc_kernel(const __nv_bfloat16* __restrict__ X,
-                                                               const __nv_bfloat16* __restrict__ dY, const ConvDims D,
-                                                               const ConvTiles T, float* __restrict__ dW,
-                                                               float* __restrict__ db, int* __restrict__ err) {
+__global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_tc_kernel(const __nv_bfloat16* __restrict__ X,
+                                                                         const __nv_bfloat16* __restrict__ dY,
+                                                                         const ConvDims D, const WgradTiles T,
+                                                                         float* __restrict__ dW,
+                                                                         float* __restrict__ db,
+                                                                         int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* s_x = sm;
-  unsigned char* s_dy = sm + kStageB;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_dy + kDyB);  // [0] loads, [1] [2] the MMAs of a set
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + 2 * kGStageB);  // [0], [1] a stage's loads, [2] the MMAs
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 3);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int q = 0; q < 3; q++) tc::mbar_init(&bars[q], q == 0 ? 2 : 1);
+    tc::mbar_init(&bars[0], 2);
+    tc::mbar_init(&bars[1], 2);
+    tc::mbar_init(&bars[2], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) tc::tmem_alloc<kWgradCols>(s_tmem);
-  // the row after the last staged one is read for products that are not used
-  for (int i = tid; i < kDyB / 16; i += 128) reinterpret_cast<uint4*>(s_dy)[i] = make_uint4(0u, 0u, 0u, 0u);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  const uint32_t tbase = *s_tmem, tlane = tbase + ((uint32_t)(32 * warp) << 16);
-  constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 16, true);
-  const uint32_t a0 = tc::smem_u32(s_x), b0 = tc::smem_u32(s_dy);
+  const uint32_t tbase = *s_tmem;
+  // this warp's part of the accumulators: TMEM lane = 16 r + channel of the r-th of eight
+  // input rows; columns by output row jz, jy
+  const int half = (warp >> 2) & 1, jz = warp >> 3;
+  const int zz = 2 * half + ((warp & 3) >> 1), yy = 2 * (warp & 1) + (lane >> 4);  // input row
+  const int dz = zz - jz;                                                          // warp-uniform
+  const uint32_t tl = tbase + ((uint32_t)(32 * (warp & 3)) << 16) + 3 * kAccCols * half + 16 * kGY * jz;
+  constexpr uint32_t idesc = tc::idesc_bf16_f32(128, kAccCols, true);
 
-  float acc[6][16], bsum[16];
+  float acc[3][kGY][16];  // [dx][jy][cout] of the thread's input row and channel
+  float bsum[2] = {0.f, 0.f};
 #pragma unroll
-  for (int c = 0; c < 16; c++) bsum[c] = 0.f;
+  for (int q = 0; q < 3 * kGY; q++)
 #pragma unroll
-  for (int q = 0; q < 6; q++)
-#pragma unroll
-    for (int c = 0; c < 16; c++) acc[q][c] = 0.f;
-  uint32_t parity = 0;
+    for (int c = 0; c < 16; c++) acc[q / kGY][q % kGY][c] = 0.f;
+
+  auto stage = [&](int64_t t, int64_t i) {  // warps 1 and 2
+    int x0, y0, z0;
+    T.at(t, x0, y0, z0);
+    unsigned char* s = sm + (i & 1) * kGStageB;
+    if (warp == 1) stage_rows<kInX, kGY + 2, kGZ + 2>(s, X, D, x0 - 1, y0 - 1, z0 - 1, 0u, &bars[i & 1]);
+    if (warp == 2) stage_rows<kBX, kGY, kGZ>(s + kXB, dY, D, x0, y0, z0, 0u, &bars[i & 1]);
+  };
+  int64_t t = blockIdx.x, i = 0;
   bool ok = true;
-  for (int64_t t = blockIdx.x; t < T.n && ok; t += gridDim.x, parity ^= 1u) {
-    int x0, y0, z;
-    T.at(t, x0, y0, z);
-    if (warp == 0) {
-      stage_rows<kBX, kBY, 1>(s_dy, dY, D, x0, y0, z, 0u, &bars[0]);
-      stage_rows<kInX, kInY, kInZ>(s_x, X, D, x0 - 1, y0 - 1, z - 1, 0u, &bars[0]);
-    }
-    ok = tc::mbar_wait(&bars[0], parity);
+  if (t < T.n) stage(t, 0);
+  for (; t < T.n && ok; t += gridDim.x, i++) {
+    const unsigned char* s_dy = sm + (i & 1) * kGStageB + kXB;
+    // (the other stage's MMAs ended with the tile before)
+    const bool more = t + gridDim.x < T.n;
+    if (more) stage(t + gridDim.x, i + 1);
+    ok = tc::mbar_wait(&bars[i & 1], (uint32_t)(i >> 1) & 1u);
     if (!ok && lane == 0) atomicOr(err, 1);
-    ok = __syncthreads_and(ok);
-    // row j's MMAs go out, then row j - 1's accumulators are read; a set's barrier
-    // completes twice a tile
-#pragma unroll 1
-    for (int j = 0; j <= kBY && ok; j++) {
-      if (tid == 0 && j < kBY) {
+    if (warp == 0) {
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok && lane == 0) {
         tc::fence_after_sync();
-        const uint32_t d0 = tbase + (j & 1) * kWgradSet;
+        const uint32_t a0 = tc::smem_u32(sm + (i & 1) * kGStageB), b0 = a0 + kXB;
 #pragma unroll 1
         for (int k = 0; k < kBX; k += 16) {
-          const uint64_t bd = tc::smem_desc(b0 + (uint32_t)(j * 2 * kBX * 16 + k * 16), 128, kBX * 16);
+          // N groups of 8 channels: (row, plane), kBX x 16 bytes apart
+          const uint64_t bd = tc::smem_desc(b0 + (uint32_t)(k * 16), 128, kBX * 16);
 #pragma unroll
           for (int q = 0; q < 6; q++) {
-            const uint32_t a = a0 + (uint32_t)((j + 8 * (q & 1)) * kRowB + (k + (q >> 1)) * 16);
-            tc::mma_bf16(d0 + 16 * q, tc::smem_desc(a, 128, kPlaneB), bd, idesc, k > 0);
+            const uint32_t a = a0 + (uint32_t)((8 * (q / 3)) * kRowB + (k + q % 3) * 16);
+            tc::mma_bf16(tbase + kAccCols * q, tc::smem_desc(a, 128, kPlaneB), bd, idesc, k > 0);
           }
         }
-        tc::mma_commit(&bars[1 + (j & 1)]);
-      }
-      if (j < kBY) {  // the bias gradient while the MMAs run: thread = vertex along x
-#pragma unroll
-        for (int p = 0; p < 2; p++) {
-          const uint4 q = *reinterpret_cast<const uint4*>(s_dy + ((j * 2 + p) * kBX + tid) * 16);
-          const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&q);
-#pragma unroll
-          for (int c = 0; c < 8; c++) bsum[8 * p + c] += __bfloat162float(h[c]);
-        }
+        tc::mma_commit(&bars[2]);
       }
       __syncwarp();
-      if (j > 0) {
-        const int i = j - 1;
-        ok = tc::mbar_wait(&bars[1 + (i & 1)], (uint32_t)(i >> 1) & 1u);
-        if (!ok && lane == 0) atomicOr(err, 2);
-        if (__all_sync(0xffffffffu, ok)) {
-          tc::fence_after_sync();
+    }
+    // the bias gradient while the MMAs run: a warp has 64 vertices of an output row's plane,
+    // a thread two channels of every eighth
+    if (ok) {
+      const unsigned char* p = s_dy + (((warp >> 1) & 3) * 2 + (warp & 1)) * (kBX * 16) + (warp >> 3) * 64 * 16 + lane * 4;
 #pragma unroll
-          for (int q = 0; q < 6; q++) {
-            float v[16];
-            tc::tmem_ld16(tlane + (i & 1) * kWgradSet + 16 * q, v);
-#pragma unroll
-            for (int c = 0; c < 16; c++) acc[q][c] += v[c];
-          }
-        }
-        tc::fence_before_sync();
-        ok = __syncthreads_and(ok);  // the set is free, and after the last row the buffers
+      for (int k = 0; k < 8; k++) {
+        const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(p + k * 128);
+        bsum[0] += __low2float(h);
+        bsum[1] += __high2float(h);
       }
     }
-    if (!ok && tid == 0) {  // nothing in flight when the block ends
-      tc::mbar_wait(&bars[0], parity);
-      tc::mbar_wait(&bars[1], 1);
-      tc::mbar_wait(&bars[2], 1);
+    const bool done = tc::mbar_wait(&bars[2], (uint32_t)i & 1u);
+    if (!done && lane == 0) atomicOr(err, 2);
+    ok = __all_sync(0xffffffffu, ok && done);
+    if (ok && dz >= 0 && dz <= 2) {
+      tc::fence_after_sync();
+#pragma unroll
+      for (int q = 0; q < 3 * kGY; q++) {
+        float v[16];
+        tc::tmem_ld16(tl + kAccCols * (q / kGY) + 16 * (q % kGY), v);
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[q / kGY][q % kGY][c] += v[c];
+      }
     }
+    tc::fence_before_sync();
+    ok = __syncthreads_and(ok);  // the accumulators and this stage are free
+    tc::fence_after_sync();
+    if (!ok && more && tid == 0) tc::mbar_wait(&bars[(i + 1) & 1], (uint32_t)((i + 1) >> 1) & 1u);  // nothing in flight
   }
   if (ok) {
-    // TMEM lane = row of the operand: 16 r + channel of the r-th of its eight rows
-    const int r = 2 * warp + (lane >> 4), ci = lane & 15;
+    // the block's sums in shared memory, an output row at a time: within one, every weight
+    // has one writer
+    float* s_w = reinterpret_cast<float*>(sm);  // [tap][cout][cin]
+    float* s_b = s_w + 27 * 256;                // [warp][channel of the plane]
+    for (int k = tid; k < 27 * 256; k += kWgradThreads) s_w[k] = 0.f;
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-      const int dx = q >> 1;
-      int dy, dz;
-      if ((q & 1) == 0) {
-        dz = r >= 6 ? 1 : 0;
-        dy = r >= 6 ? r - 6 : r;
-      } else {
-        dz = r >= 4 ? 2 : 1;
-        dy = r >= 4 ? r - 4 : (r == 0 ? 2 : 3);
-      }
-      if (dy > 2) continue;
-      float* w = dW + (dx + 3 * dy + 9 * dz) * 256 + ci * 16;
+    for (int c = 0; c < 2; c++) {
+      float v = bsum[c];
 #pragma unroll
-      for (int c = 0; c < 16; c++) atomicAdd(&w[c], acc[q][c]);
+      for (int o = 16; o >= 4; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < 4) s_b[warp * 8 + 2 * lane + c] = v;
     }
+    __syncthreads();
 #pragma unroll
-    for (int c = 0; c < 16; c++) {
-      float b = bsum[c];
+    for (int j = 0; j < kGY * kGZ; j++) {
+      const int dy = yy - j % kGY;
+      if (jz == j / kGY && dz >= 0 && dz <= 2 && dy >= 0 && dy <= 2)
 #pragma unroll
-      for (int o = 16; o; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-      if (lane == 0) atomicAdd(&db[c], b);
+        for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+          for (int c = 0; c < 16; c++) s_w[((dx + 3 * dy + 9 * dz) * 16 + c) * 16 + (lane & 15)] += acc[dx][j % kGY][c];
+      __syncthreads();
+    }
+    for (int k = tid; k < 27 * 256; k += kWgradThreads)
+      atomicAdd(&dW[(k & ~255) + (k & 15) * 16 + ((k >> 4) & 15)], s_w[k]);
+    if (tid < 16) {
+      float v = 0.f;
+      for (int w = tid >> 3; w < 16; w += 2) v += s_b[w * 8 + (tid & 7)];
+      atomicAdd(&db[tid], v);
     }
   }
-  __syncwarp();
-  tc::fence_before_sync();
   __syncthreads();
-  tc::fence_after_sync();
   if (warp == 0) tc::tmem_dealloc<kWgradCols>(tbase);
 }
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
-static ConvTiles conv_tiles(const ConvDims& D) {
-  ConvTiles T;
-  T.nx = (int)((D.X + kBX - 1) / kBX);
-  T.ny = (int)((D.Y + kBY - 1) / kBY);
-  T.n = (int64_t)T.nx * T.ny * D.Z;
-  return T;
-}
 
 template <int EPI>
 static cudaError_t launch_conv(const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias, const ConvDims& D,
@@ -563,12 +567,15 @@ cudaError_t launch_conv3_tc(int epi, const __nv_bfloat16* in_act, const uint8_t*
 cudaError_t launch_conv_wgrad(const __nv_bfloat16* X, const __nv_bfloat16* dY, const ConvDims& D, float* dW, float* db,
                               int* err, int num_sms, cudaStream_t st) {
   if (!aligned16(X) || !aligned16(dY)) return cudaErrorInvalidValue;  // bulk copies
-  const ConvTiles T = conv_tiles(D);
+  WgradTiles T;
+  T.nx = (int)((D.X + kBX - 1) / kBX);
+  T.ny = (int)((D.Y + kGY - 1) / kGY);
+  T.n = (int64_t)T.nx * T.ny * ((D.Z + kGZ - 1) / kGZ);
   cudaError_t e = cudaFuncSetAttribute(conv_wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemWgrad);
   if (e != cudaSuccess) return e;
   ::msc::count_launch();
-  conv_wgrad_tc_kernel<<<(unsigned)(T.n < 2 * num_sms ? T.n : 2 * num_sms), 128, kSmemWgrad, st>>>(X, dY, D, T, dW, db,
-                                                                                                   err);
+  conv_wgrad_tc_kernel<<<(unsigned)(T.n < num_sms ? T.n : num_sms), kWgradThreads, kSmemWgrad, st>>>(X, dY, D, T, dW, db,
+                                                                                                     err);
   return cudaGetLastError();
 }
 

@@ -338,7 +338,7 @@ def grad_kernels(V, C, t_pairs, t_ldir, nlaunch, reps, n, peak, peak_kind):
                          "algorithmic_bytes": alg_pairs, "gbs": alg_pairs / (t_pairs * 1e-3) / 1e9},
         "ldir_stage": {"launches_per_step": nlaunch / reps, "ms_per_stage": t_ldir,
                        "algorithmic_bytes": alg_ldir, "gbs": alg_ldir / (t_ldir * 1e-3) / 1e9,
-                       "kernels": "ldir_tile_kernel + ldir_check_kernel + ldir_walk_kernel"},
+                       "kernels": "ldir_tile3_kernel (2D: ldir_tile2_kernel) + ldir_check_kernel + ldir_walk_kernel"},
     }
     dom = "lstar_kernel" if t_pairs >= t_ldir else "ldir_stage"
     kd = kernels[dom]
@@ -346,6 +346,8 @@ def grad_kernels(V, C, t_pairs, t_ldir, nlaunch, reps, n, peak, peak_kind):
                 "frac": kd["gbs"] / peak, "peak_kind": f"{peak_kind} hbm_gbs", "traffic": TRAFFIC_PER_LAUNCH.get((dom, n)),
                 "scope": "dominant kernel of the .grad; the label integration that dominates the full step is "
                          "FP32/FP64 issue-bound, neither HBM nor tensor bound"}
+    if n is None:  # 2D
+        return kernels, roofline
     # the bound these kernels actually meet: instruction issue (per-unit counts from ncu)
     per, unit = WARP_INST_PER_UNIT[dom]
     units = V if unit == "vertex" else C
@@ -578,7 +580,8 @@ def run_ours(args, ws, rank, local):
         del vols, outs, singles, lab_b, lab_l
 
     peak, peak_kind = load_peaks()
-    kernels, roofline = grad_kernels(V, C, t_pairs, t_ldir, nlaunch, reps, n, peak, peak_kind)
+    kernels, roofline = grad_kernels(V, C, t_pairs, t_ldir, nlaunch, reps, n if len(dims) == 3 else None, peak,
+                                     peak_kind)
 
     # the 2D scale workload: the .grad of the 8192^2 k^-3 field
     grad_2d = None
@@ -590,7 +593,7 @@ def run_ours(args, ws, rank, local):
             lower_star_grad(f2, out=g2)
         p2, l2, t2, nl2 = grad_stage_times(f2, g2, (8192, 8192), reps, stream, dev)
         V2, C2 = 8192 * 8192, num_cells((8192, 8192))
-        k2, r2 = grad_kernels(V2, C2, p2, l2, nl2, reps, 8192, peak, peak_kind)
+        k2, r2 = grad_kernels(V2, C2, p2, l2, nl2, reps, None, peak, peak_kind)
         grad_2d = {"workload": "8192^2 float32 k^-3 Gaussian random field, seed = rank", "vertices": V2, "cells": C2,
                    "value": V2 / (t2 * 1e-3) / 1e9, "unit": UNIT, "ms_per_step": t2, "kernels": k2, "roofline": r2}
         del f2, g2
@@ -709,8 +712,8 @@ def run_ours(args, ws, rank, local):
 # --set full capture of each kernel at 256^3 (f and .grad together 201 MB, above the
 # L2), scaled to 512^3 by the vertex count (x 8): the traffic grows with the volume.
 # ldir_stage = tile + check kernels (the walk is below 5% of the stage's time).
-_T_LSTAR = 67.342e6 + 78.792e6
-_T_LDIR = 133.928e6 + 96.585e6 + 147.920e6 + 9.383e6
+_T_LSTAR = 67.332e6 + 77.410e6
+_T_LDIR = 133.517e6 + 96.392e6 + 155.732e6 + 8.012e6
 TRAFFIC_PER_LAUNCH: dict = {
     ("lstar_kernel", 256): _T_LSTAR,
     ("ldir_stage", 256): _T_LDIR,
@@ -719,11 +722,11 @@ TRAFFIC_PER_LAUNCH: dict = {
 }
 # Warp instructions per unit from the same captures (smsp__inst_executed.sum): the .grad
 # kernels are integer-issue bound, so their ceiling is the SMs' issue rate (152 SMs x 4
-# schedulers x clock), not HBM.  lstar_kernel: 1.320 G per 256^3 launch (per vertex);
-# ldir stage: tile 1.806 G + check 0.111 G per 256^3 (per cell).
+# schedulers x clock), not HBM.  lstar_kernel: 0.869 G per 256^3 launch (per vertex);
+# ldir stage: tile 0.314 G + check 0.072 G per 256^3 (per cell).  3D only.
 WARP_INST_PER_UNIT: dict = {
-    "lstar_kernel": (1.320036e9 / 256 ** 3, "vertex"),
-    "ldir_stage": ((1.805696e9 + 0.110793e9) / 511 ** 3, "cell"),
+    "lstar_kernel": (0.868808e9 / 256 ** 3, "vertex"),
+    "ldir_stage": ((0.314411e9 + 0.072291e9) / 511 ** 3, "cell"),
 }
 SCHEDULERS_PER_SM = 4
 SMS = 152

@@ -713,7 +713,7 @@ def run_ours(args, ws, rank, local):
 # L2), scaled to 512^3 by the vertex count (x 8): the traffic grows with the volume.
 # ldir_stage = tile + check kernels (the walk is below 5% of the stage's time).
 _T_LSTAR = 67.332e6 + 77.410e6
-_T_LDIR = 133.517e6 + 96.392e6 + 155.732e6 + 8.012e6
+_T_LDIR = 133.5e6 + 115.1e6 + 155.7e6 + 8.2e6
 TRAFFIC_PER_LAUNCH: dict = {
     ("lstar_kernel", 256): _T_LSTAR,
     ("ldir_stage", 256): _T_LDIR,
@@ -726,7 +726,7 @@ TRAFFIC_PER_LAUNCH: dict = {
 # ldir stage: tile 0.314 G + check 0.072 G per 256^3 (per cell).  3D only.
 WARP_INST_PER_UNIT: dict = {
     "lstar_kernel": (0.868808e9 / 256 ** 3, "vertex"),
-    "ldir_stage": ((0.314411e9 + 0.072291e9) / 511 ** 3, "cell"),
+    "ldir_stage": ((0.313797e9 + 0.072406e9) / 511 ** 3, "cell"),
 }
 SCHEDULERS_PER_SM = 4
 SMS = 152

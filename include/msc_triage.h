@@ -21,6 +21,7 @@
  *   weights                  FP32 [MSC_TRIAGE_PARAMS]: W1, W2, W3 as [27 taps][16 cin][16 cout]
  *                            (tap = dx + 3 dy + 9 dz, offsets -1..1), then b1, b2, b3 [16];
  *                            channels beyond 10 inputs / 2 outputs must be zero
+ * Features and activations are 16-byte aligned (anything else is refused).
  * All pointers are device memory; every call runs on `stream`, synchronises it, and
  * returns MSC_OK or a negative MSC_ERR_* code (text: msc_triage_last_error_string()
  * for the network entries, msc_labels_last_error_string() for the labeling ones). */

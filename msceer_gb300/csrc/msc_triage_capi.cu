@@ -79,6 +79,13 @@ struct Scratch {
   }
 };
 
+// The kernels copy and store the activations 16 bytes at a time: refused here, before any
+// device work, since a first layer that ran would store to the second's misaligned input.
+bool aligned(const void* a, const void* b, const void* c) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) == 0;
+}
+constexpr const char* kMisaligned = "features and activations must be 16-byte aligned";
+
 int read_err(const int* d, cudaStream_t st) {
   int h = 0;
   TCUDA(cudaMemcpyAsync(&h, d, sizeof(int), cudaMemcpyDeviceToHost, st), "read status");
@@ -111,6 +118,7 @@ int msc_triage_forward_3d(const uint16_t* features, const int64_t dims[3], const
   msc::ConvDims D;
   if (!conv_dims(dims, &D)) return fail(MSC_ERR_BAD_DIMS, "invalid dims");
   if (!features || !weights || !logits) return fail(MSC_ERR_NULL_POINTER, "null argument");
+  if (!aligned(features, act1, act2)) return fail(MSC_ERR_CUDA, kMisaligned);
   cudaStream_t st = (cudaStream_t)stream;
   Scratch s(st);
   uint8_t* blobs;
@@ -134,6 +142,7 @@ int msc_triage_backward_3d(const uint16_t* features, const uint16_t* act1, const
   if (!conv_dims(dims, &D)) return fail(MSC_ERR_BAD_DIMS, "invalid dims");
   if (!features || !act1 || !act2 || !logits || !targets || !weights || !grads || !loss)
     return fail(MSC_ERR_NULL_POINTER, "null argument");
+  if (!aligned(features, act1, act2)) return fail(MSC_ERR_CUDA, kMisaligned);
   cudaStream_t st = (cudaStream_t)stream;
   const int sms = sm_count();
   Scratch s(st);

@@ -556,7 +556,9 @@ static cudaError_t launch_conv(const __nv_bfloat16* in_act, const uint8_t* wblob
 cudaError_t launch_conv3_tc(int epi, const __nv_bfloat16* in_act, const uint8_t* wblob, const float* bias,
                             const ConvDims& D, __nv_bfloat16* out_act, float* out_logits,
                             const __nv_bfloat16* mask_act, int* err, int num_sms, cudaStream_t st) {
-  if (!aligned16(in_act) || !aligned16(wblob)) return cudaErrorInvalidValue;  // bulk copies
+  // bulk copies in, 16-byte loads of the mask, 16-byte stores out
+  if (!aligned16(in_act) || !aligned16(wblob) || !aligned16(out_act) || !aligned16(mask_act))
+    return cudaErrorInvalidValue;
   if (epi == kEpiReluBf16)
     return launch_conv<kEpiReluBf16>(in_act, wblob, bias, D, out_act, out_logits, mask_act, err, num_sms, st);
   if (epi == kEpiLogits)

@@ -144,6 +144,12 @@ __device__ __forceinline__ void load_mask(uint4 (&m)[16], const __nv_bfloat16* _
   }
 }
 
+// The mask multiplies the FP32 gradient, but meets it only after it has been rounded: one
+// that is finite and rounds to infinity waits in the staging under this mark (a NaN that no
+// conversion makes), so that masked it is zero, while an infinite or NaN gradient stays NaN.
+constexpr uint32_t kOverflowMark = 0x7F81u;
+constexpr float kRoundsToInf = 0x1.FFp127f;
+
 // One warp's share of a tile: the accumulator lanes of output rows 2 w and 2 w + 1.
 // `done` gets an arrival when they have been read.
 template <int EPI>
@@ -154,32 +160,48 @@ __device__ __forceinline__ void conv_epilogue(uint32_t tl, unsigned char* s_out,
   const int lane = threadIdx.x & 31, row = lane >> 4, ch = lane & 15;
   const bool odd = lane & 1;
   unsigned char* mine = s_out + (2 * row + (ch >> 3)) * kOutPlaneB + (odd ? 16 : 0) + (ch & 6) * 2;
+  bool marked = false;
   __syncwarp();  // the tile before has left the staging
+  while (true) {
+    float most[4] = {0.f, 0.f, 0.f, 0.f};  // largest magnitudes, four chains of them
 #pragma unroll 1
-  for (int c = 0; c < kBX; c += 16) {
-    float v[16];
-    tc::tmem_ld16(tl + c, v);
-    if (EPI == kEpiLogits) {
-      if (ch < 2) {
-        float4* o = reinterpret_cast<float4*>(s_out + (2 * row + ch) * kBX * 4 + c * 4);
+    for (int c = 0; c < kBX; c += 16) {
+      float v[16];
+      tc::tmem_ld16(tl + c, v);
+      if (EPI == kEpiLogits) {
+        if (ch < 2) {
+          float4* o = reinterpret_cast<float4*>(s_out + (2 * row + ch) * kBX * 4 + c * 4);
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-          o[k] = make_float4(v[4 * k] + bias, v[4 * k + 1] + bias, v[4 * k + 2] + bias, v[4 * k + 3] + bias);
-      }
-    } else {
-      uint32_t h[16];
+          for (int k = 0; k < 4; k++)
+            o[k] = make_float4(v[4 * k] + bias, v[4 * k + 1] + bias, v[4 * k + 2] + bias, v[4 * k + 3] + bias);
+        }
+      } else {
+        uint32_t h[16];
 #pragma unroll
-      for (int k = 0; k < 16; k++) {
-        const float a = EPI == kEpiReluBf16 ? fmaxf(v[k] + bias, 0.f) : v[k];
-        h[k] = __bfloat16_as_ushort(__float2bfloat16_rn(a));
-      }
-      // two channels to a word: the even lane of a pair takes the even vertices
+        for (int k = 0; k < 16; k++) {
+          const float a = EPI == kEpiReluBf16 ? fmaxf(v[k] + bias, 0.f) : v[k];
+          h[k] = __bfloat16_as_ushort(__float2bfloat16_rn(a));
+        }
+        if (EPI == kEpiMaskBf16) {
 #pragma unroll
-      for (int k = 0; k < 16; k += 2) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? h[k] : h[k + 1], 1);
-        *reinterpret_cast<uint32_t*>(mine + (c + k) * 16) = odd ? (got | (h[k + 1] << 16)) : (h[k] | (got << 16));
+          for (int k = 0; k < 16; k++) most[k & 3] = fmaxf(most[k & 3], fabsf(v[k]));
+          if (marked)
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+              if (isfinite(v[k]) && fabsf(v[k]) >= kRoundsToInf) h[k] = (h[k] & 0x8000u) | kOverflowMark;
+        }
+        // two channels to a word: the even lane of a pair takes the even vertices
+#pragma unroll
+        for (int k = 0; k < 16; k += 2) {
+          const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? h[k] : h[k + 1], 1);
+          *reinterpret_cast<uint32_t*>(mine + (c + k) * 16) = odd ? (got | (h[k + 1] << 16)) : (h[k] | (got << 16));
+        }
       }
     }
+    if (EPI != kEpiMaskBf16 || marked) break;
+    marked = __any_sync(0xffffffffu, fmaxf(fmaxf(most[0], most[1]), fmaxf(most[2], most[3])) >= kRoundsToInf);
+    if (!marked) break;
+    __syncwarp();  // once more, with the marks
   }
   tc::fence_before_sync();
   __syncwarp();
@@ -193,6 +215,16 @@ __device__ __forceinline__ void conv_epilogue(uint32_t tl, unsigned char* s_out,
       for (int x = lane; x < kBX && x0 + x < D.X; x += 32) o[x] = sv[x];
     }
   } else {
+    if (marked)  // apart from the loop below, whose loads go out together
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        unsigned short* r = reinterpret_cast<unsigned short*>(s_out + (i >> 2) * kOutPlaneB + (lane + 32 * (i & 3)) * 16);
+        const __nv_bfloat16* mh = reinterpret_cast<const __nv_bfloat16*>(&mask[i]);
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+          if ((r[c] & 0x7FFFu) == kOverflowMark)
+            r[c] = (unsigned short)((r[c] & 0x8000u) | (__bfloat162float(mh[c]) > 0.f ? 0x7F80u : 0u));
+      }
 #pragma unroll
     for (int i = 0; i < 16; i++) {
       const int q = i >> 2, x = lane + 32 * (i & 3);  // q: row, plane

@@ -417,6 +417,11 @@ constexpr uint32_t kAccCols = 16 * kGY * kGZ;       // columns of one of the six
 constexpr uint32_t kWgradCols = 512;
 static_assert(kGRows == 16 && 6 * kAccCols <= kWgradCols, "two operands of eight rows");
 static_assert(27 * 256 * 4 + 16 * 8 * 4 <= kGStageB, "the final sums fit a stage");
+// A tile's vertices along x (what lies past the volume is not multiplied), and whether its
+// second output row along y or z lies past the volume: their products are not read, since a
+// zero times an infinite input is none.
+constexpr int kEdgeY = 1 << 8, kEdgeZ = 1 << 9;
+static_assert(kGY == 2 && kGZ == 2 && kBX <= 0xFF, "the edge word");
 struct WgradTiles {
   int nx, ny;
   int64_t n;
@@ -438,6 +443,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_tc_kernel(const _
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(sm + 2 * kGStageB);  // [0], [1] a stage's loads, [2] the MMAs
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(bars + 3);
+  int* s_edge = reinterpret_cast<int*>(s_tmem + 1);  // of a stage's tile
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     tc::mbar_init(&bars[0], 2);
@@ -469,6 +475,8 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_tc_kernel(const _
     int x0, y0, z0;
     T.at(t, x0, y0, z0);
     unsigned char* s = sm + (i & 1) * kGStageB;
+    if (warp == 1 && lane == 0)  // (what this thread's arrival below makes visible)
+      s_edge[i & 1] = (int)min((int64_t)kBX, D.X - x0) | (y0 + 1 < D.Y ? 0 : kEdgeY) | (z0 + 1 < D.Z ? 0 : kEdgeZ);
     if (warp == 1) stage_rows<kInX, kGY + 2, kGZ + 2>(s, X, D, x0 - 1, y0 - 1, z0 - 1, 0u, &bars[i & 1]);
     if (warp == 2) stage_rows<kBX, kGY, kGZ>(s + kXB, dY, D, x0, y0, z0, 0u, &bars[i & 1]);
   };
@@ -482,13 +490,14 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_tc_kernel(const _
     if (more) stage(t + gridDim.x, i + 1);
     ok = tc::mbar_wait(&bars[i & 1], (uint32_t)(i >> 1) & 1u);
     if (!ok && lane == 0) atomicOr(err, 1);
+    const int edge = s_edge[i & 1];
     if (warp == 0) {
       ok = __all_sync(0xffffffffu, ok);
       if (ok && lane == 0) {
         tc::fence_after_sync();
         const uint32_t a0 = tc::smem_u32(sm + (i & 1) * kGStageB), b0 = a0 + kXB;
 #pragma unroll 1
-        for (int k = 0; k < kBX; k += 16) {
+        for (int k = 0; k < (edge & 0xFF); k += 16) {
           // N groups of 8 channels: (row, plane), kBX x 16 bytes apart
           const uint64_t bd = tc::smem_desc(b0 + (uint32_t)(k * 16), 128, kBX * 16);
 #pragma unroll
@@ -515,14 +524,18 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_tc_kernel(const _
     const bool done = tc::mbar_wait(&bars[2], (uint32_t)i & 1u);
     if (!done && lane == 0) atomicOr(err, 2);
     ok = __all_sync(0xffffffffu, ok && done);
-    if (ok && dz >= 0 && dz <= 2) {
+    if (ok && dz >= 0 && dz <= 2 && !(jz == 1 && (edge & kEdgeZ))) {
       tc::fence_after_sync();
 #pragma unroll
-      for (int q = 0; q < 3 * kGY; q++) {
-        float v[16];
-        tc::tmem_ld16(tl + kAccCols * (q / kGY) + 16 * (q % kGY), v);
+      for (int jy = 0; jy < kGY; jy++) {
+        if (jy == 1 && (edge & kEdgeY)) break;
 #pragma unroll
-        for (int c = 0; c < 16; c++) acc[q / kGY][q % kGY][c] += v[c];
+        for (int dx = 0; dx < 3; dx++) {
+          float v[16];
+          tc::tmem_ld16(tl + kAccCols * dx + 16 * jy, v);
+#pragma unroll
+          for (int c = 0; c < 16; c++) acc[dx][jy][c] += v[c];
+        }
       }
     }
     tc::fence_before_sync();

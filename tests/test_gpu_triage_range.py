@@ -32,3 +32,30 @@ def test_masked_gradient_that_rounds_to_infinity(gpu, w_exp, masked, want):
     _, g = triage.backward(_bits(np.zeros(16)), a, a, logits, target, (1, 1, 1), w, 2.0 * 129 / 128 * 2.0 ** 63)
     db2 = g[3 * NW + 16: 3 * NW + 32].cpu().numpy()
     assert np.array_equal(db2, np.full(16, want, dtype=np.float32), equal_nan=True), db2
+
+
+@pytest.mark.parametrize("at", [(0, 3, 31), (0, 0, 0), (0, 3, 17)], ids=str)
+def test_weight_gradient_of_an_infinite_feature(gpu, at):
+    """A 32 x 4 x 1 volume with one infinite feature: the weight gradients that a vertex of the
+    volume gives it are infinite, all others finite, whatever lies past the volume in its tile."""
+    import torch
+    from msceer_gb300 import triage
+    shape = (1, 4, 32)
+    rng = np.random.default_rng(4)
+    feat = np.ones(shape + (16,), dtype=np.float32)
+    feat[at + (0,)] = np.inf
+    rows = _bits(np.stack([feat[..., :8], feat[..., 8:]], 2))
+    w = torch.from_numpy(rng.uniform(0.5, 1.0, triage.PARAMS).astype(np.float32)).cuda()
+    a = _bits(np.ones(16 * feat[..., 0].size))
+    logits = torch.zeros((2, feat[..., 0].size), device="cuda")
+    target = torch.zeros((2, feat[..., 0].size), dtype=torch.uint8, device="cuda")
+    _, g = triage.backward(rows.reshape(-1), a, a, logits, target, shape, w, 1.0)
+    g = g.cpu().numpy()
+    dw1 = g[:NW].reshape(3, 3, 3, 16, 16)  # dz, dy, dx, cin, cout
+    for dz in range(3):
+        for dy in range(3):
+            for dx in range(3):
+                v = (at[0] - dz + 1, at[1] - dy + 1, at[2] - dx + 1)  # the vertex that sees the feature there
+                inside = all(0 <= c < n for c, n in zip(v, shape))
+                assert np.all(dw1[dz, dy, dx, 0] == np.inf) if inside else np.all(np.isfinite(dw1[dz, dy, dx, 0]))
+    assert np.isfinite(dw1[..., 1:, :]).all() and np.isfinite(g[NW:]).all()

@@ -74,9 +74,10 @@ struct Lane32 {
 // kShortStep: an accepted step differs from the full Euler step, of length max_step at
 // most, by less than sqrt(ethresh)).  Then the nearest vertex of a position in a voxel, or
 // just stepped out of it, is one of the voxel's corners, and whether it stops the
-// streamline was read with the corner gradients, from their fourth component
-// (kStopTerminal / kStopLabelled): a step reads no memory and converts nothing to an
-// integer.  The longer steps that a caller may ask for read the vertex's state.
+// streamline was read where the voxel was entered -- in the fix-up from the corner gradients'
+// fourth component (kStopTerminal), in the first pass from the voxel's byte of corners
+// (stop_corners_kernel): a step reads no memory and converts nothing to an integer.  The
+// longer steps that a caller may ask for read the vertex's state.
 constexpr float kShortStep = 0.45f;
 constexpr float kShortThresh = 1e-3f;  // sqrt: 0.032
 
@@ -88,6 +89,7 @@ struct Adv32 {
   const uint8_t* lvl;    // pass-1 stop (when set): nearest vertex labelled in an earlier level
   int level;
   const uint8_t* state;  // fix-up stop (when set): nearest vertex certain terminal
+  const uint8_t* stops;  // pass-1 stop of short steps: a voxel's corners labelled in an earlier level
   // Converted once on the host: (float)P.max_step, (float)P.step_mult, the extents
   // (float)V.X .. and (float)(V.X - 2) ..  (a double-to-float or 64-bit integer
   // conversion per iteration would run on the slow FP64 pipe)
@@ -96,8 +98,8 @@ struct Adv32 {
   int32_t X = 0, XY = 0;  // vertices per row and z-plane (fewer than 2^31 vertices)
 
   static Adv32 make(const float4* G, const VolDims& V, const IntegParams& P, const uint8_t* lvl, int level,
-                    const uint8_t* state) {
-    Adv32 A{G, V, P, lvl, level, state};
+                    const uint8_t* state, const uint8_t* stops) {
+    Adv32 A{G, V, P, lvl, level, state, stops};
     A.ms = (float)P.max_step;
     A.sgn = (float)P.step_mult;
     const int64_t e[3] = {V.X, V.Y, V.Z};
@@ -133,13 +135,14 @@ struct Adv32 {
     }
     L.base = index(b[0], b[1], b[2]);
     uint32_t stop = 0;
+    if (SHORT && !state) stop = __ldg(stops + L.base);
 #pragma unroll
     for (int n = 0; n < 8; n++) {
       const float4 v = __ldg(G + (L.base + ((n & 1) ? o[0] : 0) + ((n & 2) ? o[1] : 0) + ((n & 4) ? o[2] : 0)));
       L.c[n] = {v.x, v.y, v.z};
-      if (SHORT) stop |= __float_as_uint(v.w) & ((state ? 1u : 0x100u) << n);
+      if (SHORT && state) stop |= __float_as_uint(v.w) & (1u << n);
     }
-    if (SHORT) L.stop = state ? stop : stop >> 8;
+    if (SHORT) L.stop = stop;
 #pragma unroll
     for (int n = 1; n < 8; n += 2) L.c[n] = {L.c[n].x - L.c[n - 1].x, L.c[n].y - L.c[n - 1].y, L.c[n].z - L.c[n - 1].z};
   }
@@ -1056,12 +1059,11 @@ __global__ void spec_jump_kernel(const SpecSet Q, int64_t k0, int64_t k1) {
 constexpr int kChainSteps = 64;
 __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8_t* __restrict__ lvl, int level,
                                   const uint32_t* __restrict__ claim, int32_t* __restrict__ lab,
-                                  float4* __restrict__ g32, int* __restrict__ long_chain) {
+                                  int* __restrict__ long_chain) {
   const int lane = threadIdx.x & 31;
   auto put = [&](uint32_t v, int32_t l) {
     lab[v] = l;
     lvl[v] = (uint8_t)level;
-    reinterpret_cast<uint32_t*>(g32 + v)[3] = kStopLabelled;
   };
   for (int64_t b0 = k0 + blockIdx.x * (int64_t)blockDim.x; b0 < k1; b0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t k = b0 + threadIdx.x;  // (warp-uniform trips)
@@ -1114,8 +1116,8 @@ __global__ void spec_write_kernel(const SpecSet Q, int64_t k0, int64_t k1, uint8
 // The gradient of every vertex for the FP32 passes (central differences as
 // central_diff_kernel's xyzw form; zero where a bit of `zeroed` is set), with what stops a
 // streamline there as the fourth component, and the vertex's state, from the certain
-// terminal regions.  (The first pass adds kStopLabelled to the vertices it labels while
-// the ends beside it run; those look at kStopTerminal's bits alone, which stay.)
+// terminal regions.  (Nothing writes the gradient after the first pass and the ends beside
+// it have started: both read it through the read-only path.)
 __global__ void __launch_bounds__(256) label_gradient_kernel(const float* __restrict__ f,
                                                              const int32_t* __restrict__ lab,
                                                              const uint32_t* __restrict__ zeroed, const VolDims V,
@@ -1133,7 +1135,43 @@ __global__ void __launch_bounds__(256) label_gradient_kernel(const float* __rest
     uint8_t st = state[v];
     const bool seed = st == kStSeed;
     if (!seed) state[v] = st = lab[v] >= 0 ? kStTerminal : kStUnassigned;
-    g32[v] = make_float4(gx, gy, gz, __uint_as_float(st == kStUnassigned ? 0u : kStopTerminal | kStopLabelled));
+    g32[v] = make_float4(gx, gy, gz, __uint_as_float(st == kStUnassigned ? 0u : kStopTerminal));
+  }
+}
+
+// For every voxel, named by its base vertex, the corners (bit x + 2y + 4z) labelled before
+// the batch, for the batch's speculative streamlines.  On the grid's last plane along an axis
+// a voxel repeats that plane's corners, as Adv32::load_voxel does.  A thread takes four voxels
+// of a row, their levels eight bytes a row of corners (lvl has kLevelPad bytes to spare).  A
+// voxel a lane, a byte at a time, took 0.67 ms a batch at 512^3; so 0.20.
+__global__ void __launch_bounds__(256) stop_corners_kernel(const uint8_t* __restrict__ lvl, int level, const VolDims V,
+                                                           uint8_t* __restrict__ stops) {
+  const uint32_t X = (uint32_t)V.X, Y = (uint32_t)V.Y, Z = (uint32_t)V.Z;  // (fewer than 2^31 vertices)
+  const uint32_t per_row = (X + 3) / 4, n = per_row * Y * Z, below = 0x01010101u * (uint32_t)level;
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    const uint32_t row = t / per_row, x0 = 4 * (t - row * per_row), z = row / Y, y = row - z * Y;
+    const uint32_t v = row * X + x0, oy = y < Y - 1 ? X : 0u, oz = z < Z - 1 ? X * Y : 0u;
+    uint32_t here = 0, next = 0;  // a byte per voxel: bits 0, 2, 4, 6 the corners at its x, at x + 1
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t at = v + ((k & 1) ? oy : 0u) + ((k & 2) ? oz : 0u), sh = 8 * (at & 3u);
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(lvl + (at & ~3u));
+      const uint32_t a = __vcmpltu4(w[0], below) & 0x01010101u, b = __vcmpltu4(w[1], below) & 0x01010101u;
+      const uint32_t h = __funnelshift_r(a, b, sh);
+      here |= h << (2 * k);
+      next |= ((h >> 8) | (((b >> sh) & 0xFFu) << 24)) << (2 * k);
+    }
+    const uint32_t left = X - x0;  // voxels of the row from here on
+    if (left <= 4) {
+      const uint32_t last = 0xFFu << (8 * (left - 1));
+      next = (next & ~last) | (here & last);
+    }
+    const uint32_t m = here | (next << 1);
+    if (left >= 4 && (X & 3u) == 0) {
+      *reinterpret_cast<uint32_t*>(stops + v) = m;
+    } else {
+      for (uint32_t j = 0; j < 4 && j < left; j++) stops[v + j] = (uint8_t)(m >> (8 * j));
+    }
   }
 }
 
@@ -1894,19 +1932,28 @@ cudaError_t launch_spread_compact(const SpreadOrder& S, int64_t u0, int64_t u1, 
   return cudaGetLastError();
 }
 
+cudaError_t launch_stop_corners(const uint8_t* lvl, int stamp, const VolDims& V, const IntegParams& P, uint8_t* stops,
+                                int num_sms, cudaStream_t stream) {
+  if (!short_steps(P)) return cudaSuccess;  // the longer steps read the levels
+  ::msc::count_launch();
+  stop_corners_kernel<<<grid_for((V.X + 3) / 4 * V.Y * V.Z, num_sms), 256, 0, stream>>>(lvl, stamp, V, stops);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParams& P, const SpecSet& Q, int64_t k0,
-                             int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, uint32_t* claim,
-                             unsigned long long* work, unsigned long long* trips, int num_sms, cudaStream_t stream) {
+                             int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, const uint8_t* stops,
+                             uint32_t* claim, unsigned long long* work, unsigned long long* trips, int num_sms,
+                             cudaStream_t stream) {
   if (k1 <= k0) return cudaSuccess;
   const int64_t blocks = (k1 - k0 + 127) / 128;
   const int cap = num_sms * lane_ctas_per_sm();
   const int grid = (int)(blocks < cap ? blocks : cap);
   ::msc::count_launch();
   if (short_steps(P))
-    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr), Q, k0, k1, lab,
+    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr, stops), Q, k0, k1, lab,
                                                      claim, work, trips);
   else
-    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr), Q, k0, k1, lab,
+    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr, stops), Q, k0, k1, lab,
                                                       claim, work, trips);
   return cudaGetLastError();
 }
@@ -1968,10 +2015,9 @@ cudaError_t launch_spec_jumps(const SpecSet& Q, int64_t k0, int64_t k1, int num_
 }
 
 cudaError_t launch_spec_write(const SpecSet& Q, int64_t k0, int64_t k1, uint8_t* lvl, int stamp, const uint32_t* claim,
-                              int32_t* lab, float4* g32, int* long_chain, int num_sms, cudaStream_t stream) {
+                              int32_t* lab, int* long_chain, int num_sms, cudaStream_t stream) {
   ::msc::count_launch();
-  spec_write_kernel<<<grid_for(k1 - k0, num_sms), 256, 0, stream>>>(Q, k0, k1, lvl, stamp, claim, lab, g32,
-                                                                    long_chain);
+  spec_write_kernel<<<grid_for(k1 - k0, num_sms), 256, 0, stream>>>(Q, k0, k1, lvl, stamp, claim, lab, long_chain);
   return cudaGetLastError();
 }
 
@@ -2040,10 +2086,10 @@ cudaError_t launch_fixup_end32(const float4* G, const VolDims& V, const IntegPar
   const int cap = num_sms * (n_dev ? early_ctas : lane_ctas_per_sm());
   const int grid = blocks < cap ? blocks : cap;
   if (short_steps(P))
-    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state), lab, state, list,
+    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state, nullptr), lab, state, list,
                                                        n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
   else
-    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state), lab, state,
+    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state, nullptr), lab, state,
                                                         list, n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
   return cudaGetLastError();
 }

@@ -33,10 +33,10 @@ enum : uint8_t {
   kStNonterminal = 4,
 };
 
-// What stops a streamline at a vertex, in the fourth component of the FP32 gradient (a byte
-// of ones each, so that a voxel's eight corners make a mask by one AND and OR apiece): a
-// certain terminal region stops the fix-up's, any label of an earlier batch the first pass's.
-constexpr uint32_t kStopTerminal = 0x00FFu, kStopLabelled = 0xFF00u;
+// A certain terminal region, which stops the fix-up's streamlines, in the fourth component of
+// the FP32 gradient (a byte of ones, so that a voxel's eight corners make a mask by one AND
+// and OR apiece).
+constexpr uint32_t kStopTerminal = 0x00FFu;
 
 // Label of a vertex that a first-pass streamline reached without finding a region.
 constexpr int32_t kLabelNone = -2;
@@ -168,14 +168,22 @@ cudaError_t launch_spread_compact(const SpreadOrder& S, int64_t u0, int64_t u1, 
                                   int* counts, int32_t* items, unsigned long long* n_items, cudaStream_t stream);
 // Speculative streamlines of items [k0, k1) (stopping at lvl < stamp); they build the
 // holder counts (hcount all 0 at launch) and make the first resolution round's claims.
-// `work`: a device counter, zero at launch; `trips`: advection iterations are added to it.
+// `work`: a device counter, zero at launch; `trips`: advection iterations are added to it;
+// `stops`: launch_stop_corners of the same stamp.
 // The FP32 gradient with the stop flags, and the vertices' states, from the certain
 // terminal regions (label_gradient_kernel).
 cudaError_t launch_label_gradient(const float* f, const int32_t* lab, const uint32_t* zeroed, const VolDims& V,
                                   uint8_t* state, float4* g32, int num_sms, cudaStream_t stream);
+// stops[v]: the corners (bit x + 2y + 4z) of the voxel at base vertex v with lvl < stamp
+// (nothing where P's steps are too long for the corner test).  lvl has kLevelPad bytes to spare
+// and both start at a multiple of four.
+constexpr int kLevelPad = 8;
+cudaError_t launch_stop_corners(const uint8_t* lvl, int stamp, const VolDims& V, const IntegParams& P, uint8_t* stops,
+                                int num_sms, cudaStream_t stream);
 cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParams& P, const SpecSet& Q, int64_t k0,
-                             int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, uint32_t* claim,
-                             unsigned long long* work, unsigned long long* trips, int num_sms, cudaStream_t stream);
+                             int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, const uint8_t* stops,
+                             uint32_t* claim, unsigned long long* work, unsigned long long* trips, int num_sms,
+                             cudaStream_t stream);
 // After a pool overflow: drops the claims on vertices with lvl >= stamp.
 cudaError_t launch_spec_unclaim_all(const uint8_t* lvl, int stamp, uint32_t* claim, int64_t N, int num_sms,
                                     cudaStream_t stream);
@@ -207,7 +215,7 @@ cudaError_t launch_spec_ptr(const SpecSet& Q, int64_t k0, int64_t k1, const uint
                             cudaStream_t stream);
 cudaError_t launch_spec_jumps(const SpecSet& Q, int64_t k0, int64_t k1, int num_sms, cudaStream_t stream);
 cudaError_t launch_spec_write(const SpecSet& Q, int64_t k0, int64_t k1, uint8_t* lvl, int stamp, const uint32_t* claim,
-                              int32_t* lab, float4* g32, int* long_chain, int num_sms, cudaStream_t stream);
+                              int32_t* lab, int* long_chain, int num_sms, cudaStream_t stream);
 cudaError_t launch_boundary_set(const int32_t* lab, const uint8_t* state, const VolDims& V, int64_t* list, int* n,
                                 uint32_t* queued, int num_sms, cudaStream_t stream);
 // Fix-up streamline ends (FP64 / FP32): endv[v] = the final nearest vertex of v's

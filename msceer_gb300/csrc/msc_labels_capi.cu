@@ -564,7 +564,7 @@ int first_pass(LabelCtx& c, DirLabels& d) {
     S.offset[S.nlev + 1] = S.offset[S.nlev] + (N - start + stride - 1) / stride;
     S.nlev++;
   }
-  uint8_t* lvl;
+  uint8_t *lvl, *stops;
   uint32_t* claim;
   int* counts;
   int32_t* vtx;
@@ -576,7 +576,8 @@ int first_pass(LabelCtx& c, DirLabels& d) {
   const int64_t ibits_cap = max_items / 32 + 1;
   Q.pool_words = std::min<unsigned long long>(2ull * (unsigned long long)N + (1ull << 20), 0xFFFFFF00ull);
   Q.node_cap = std::min<unsigned long long>(3ull * (unsigned long long)N + (1ull << 20), 0x7FFFFF00ull);
-  LCUDA(c.pool.get(&lvl, N), "alloc");
+  LCUDA(c.pool.get(&lvl, N + msc::kLevelPad), "alloc");
+  LCUDA(c.pool.get(&stops, N), "alloc");
   LCUDA(c.pool.get(&claim, N), "alloc");
   LCUDA(c.pool.get(&counts, S.offset[S.nlev] / 1024 + 2), "alloc");
   LCUDA(c.pool.get(&vtx, max_items), "alloc");
@@ -647,14 +648,15 @@ int first_pass(LabelCtx& c, DirLabels& d) {
     for (int64_t k0 = 0; k0 < n;) {
       if (k0 > 0)
         if (int rc = next_stamp()) return rc;
+      LCUDA(msc::launch_stop_corners(lvl, stamp, c.V, P, stops, c.sms, st), "stop corners");
       int64_t k1 = n;
       for (;;) {
         LCUDA(cudaMemsetAsync(sc, 0, sizeof(unsigned long long), st), "memset");
         LCUDA(cudaMemsetAsync(sc + 3, 0, sizeof(unsigned long long), st), "memset");
         LCUDA(cudaMemsetAsync(sc + 6, 0, sizeof(unsigned long long), st), "memset");
         LCUDA(cudaMemsetAsync(Q.overflow, 0, sizeof(int), st), "memset");
-        LCUDA(msc::launch_speculate(c.g32, c.V, P, Q, k0, k1, d.lab, lvl, stamp, claim, sc + 3, c.work + 48, c.sms,
-                                    st),
+        LCUDA(msc::launch_speculate(c.g32, c.V, P, Q, k0, k1, d.lab, lvl, stamp, stops, claim, sc + 3, c.work + 48,
+                                    c.sms, st),
               "speculate");
         int ovf = 0;
         if (int rc = read_dev(c, Q.overflow, 1, &ovf)) return rc;
@@ -686,12 +688,12 @@ int first_pass(LabelCtx& c, DirLabels& d) {
       trace_mark(st, d.dir, "  resolved");
       LCUDA(msc::launch_spec_ptr(Q, k0, k1, claim, c.sms, st), "label");
       LCUDA(cudaMemsetAsync(Q.overflow, 0, sizeof(int), st), "memset");
-      LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, c.g32, Q.overflow, c.sms, st), "label");
+      LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, Q.overflow, c.sms, st), "label");
       int long_chain = 0;
       if (int rc = read_dev(c, Q.overflow, 1, &long_chain)) return rc;
       if (long_chain) {  // a few long chains of cut items: jump, then write again
         LCUDA(msc::launch_spec_jumps(Q, k0, k1, c.sms, st), "label");
-        LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, c.g32, Q.overflow, c.sms, st), "label");
+        LCUDA(msc::launch_spec_write(Q, k0, k1, lvl, stamp, claim, d.lab, Q.overflow, c.sms, st), "label");
       }
       batches++;
       trace_mark(st, d.dir, "batch " + std::to_string(g0) + "-" + std::to_string(L1 - 1) + " items " +

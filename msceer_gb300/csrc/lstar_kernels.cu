@@ -247,7 +247,8 @@ template <int ND>
 cudaError_t launch_lstar_nd(const float* f, uint8_t* g, const GradDims& D, int* err, cudaStream_t stream) {
   using T = LstarTile<ND>;
   const int64_t gy = (D.v[1] + T::BY - 1) / T::BY, gz = (D.v[2] + T::BZ - 1) / T::BZ;
-  if (gy > 65535) return cudaErrorInvalidValue;
+  // (262,140 rows in either dimension: what a grid of four rows a block along y takes)
+  if ((D.v[1] + 3) / 4 > 65535) return cudaErrorInvalidValue;
   const dim3 grid((unsigned)((D.v[0] + T::BX - 1) / T::BX), (unsigned)gy, (unsigned)(gz < 65535 ? gz : 65535));
   if (cudaError_t e = allow_smem(lstar_kernel<ND>, sizeof(LstarSmem<ND>))) return e;
   ::msc::count_launch();

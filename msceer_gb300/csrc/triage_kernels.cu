@@ -604,6 +604,8 @@ cudaError_t launch_conv3_tc(int epi, const __nv_bfloat16* in_act, const uint8_t*
   // bulk copies in, 16-byte loads of the mask, 16-byte stores out
   if (!aligned16(in_act) || !aligned16(wblob) || !aligned16(out_act) || !aligned16(mask_act))
     return cudaErrorInvalidValue;
+  // (262,140 rows: what a grid of four rows a block along y takes)
+  if ((D.Y + 3) / 4 > 65535) return cudaErrorInvalidConfiguration;
   if (epi == kEpiReluBf16)
     return launch_conv<kEpiReluBf16>(in_act, wblob, bias, D, out_act, out_logits, mask_act, err, num_sms, st);
   if (epi == kEpiLogits)

@@ -90,6 +90,7 @@ struct Adv32 {
   int level;
   const uint8_t* state;  // fix-up stop (when set): nearest vertex certain terminal
   const uint8_t* stops;  // pass-1 stop of short steps: a voxel's corners labelled in an earlier level
+  int rounds;            // per turn, at most kRoundsPerTurn
   // Converted once on the host: (float)P.max_step, (float)P.step_mult, the extents
   // (float)V.X .. and (float)(V.X - 2) ..  (a double-to-float or 64-bit integer
   // conversion per iteration would run on the slow FP64 pipe)
@@ -98,8 +99,8 @@ struct Adv32 {
   int32_t X = 0, XY = 0;  // vertices per row and z-plane (fewer than 2^31 vertices)
 
   static Adv32 make(const float4* G, const VolDims& V, const IntegParams& P, const uint8_t* lvl, int level,
-                    const uint8_t* state, const uint8_t* stops) {
-    Adv32 A{G, V, P, lvl, level, state, stops};
+                    const uint8_t* state, const uint8_t* stops, int rounds) {
+    Adv32 A{G, V, P, lvl, level, state, stops, rounds};
     A.ms = (float)P.max_step;
     A.sgn = (float)P.step_mult;
     const int64_t e[3] = {V.X, V.Y, V.Z};
@@ -311,8 +312,10 @@ __device__ __forceinline__ void split_index(const VolDims& V, int64_t v, int& x,
 
 // Rounds between the hand-outs of new work items: a hand-out costs about half a round, a
 // lane whose streamline ends waits for it (512^3 k^-3 / 256^3 Gaussian labels: 368 / 97 ms
-// with 4, 342 / 91 with 8, 336 / 90 with 16, 361 / 91 with 32).
-constexpr int kRoundsPerTurn = 16;
+// with 4, 342 / 91 with 8, 336 / 90 with 16, 361 / 91 with 32).  MSC_TRIPS_PER_TURN (2, 4, 8
+// or 16) overrides it for tuning, MSC_TRIPS_PER_TURN_PASS1 the first pass's apart from the
+// fix-up's.
+constexpr int kRoundsPerTurn = 16;  // at most
 constexpr unsigned kFullMask = 0xffffffffu;
 
 // CTAs of 128 threads per SM launched for the lane-refilling FP32 kernels (their
@@ -593,7 +596,6 @@ __global__ void __launch_bounds__(128, 6) speculate_kernel(const Adv32<SHORT> A,
                                                            uint32_t* __restrict__ claim,
                                                            unsigned long long* __restrict__ work,
                                                            unsigned long long* __restrict__ trips) {
-  constexpr int K = kRoundsPerTurn;
   const VolDims& V = A.V;
   const int level = A.level;
   const int lane = threadIdx.x & 31;
@@ -646,7 +648,7 @@ __global__ void __launch_bounds__(128, 6) speculate_kernel(const Adv32<SHORT> A,
       add_trips(ntrips, trips);
       break;
     }
-    for (int r = 0; r < K; r++) {
+    for (int r = 0; r < A.rounds; r++) {
       if (phase != kLaneEnter && phase != kLaneStep) continue;
       const int32_t seen = L.nv;
       bool out;
@@ -1479,7 +1481,6 @@ __global__ void __launch_bounds__(128, 6) fixup_end32_kernel(const Adv32<SHORT> 
                                                           int* __restrict__ n_amb, int amb_mode,
                                                           unsigned long long* __restrict__ work,
                                                           unsigned long long* __restrict__ trips) {
-  constexpr int K = kRoundsPerTurn;
   const VolDims& V = A.V;
   if (n_dev) n = *n_dev;  // a list whose length the stream wrote before this launch
   int phase = kLaneIdle;
@@ -1508,7 +1509,7 @@ __global__ void __launch_bounds__(128, 6) fixup_end32_kernel(const Adv32<SHORT> 
       add_trips(ntrips, trips);
       break;
     }
-    for (int r = 0; r < K; r++) {
+    for (int r = 0; r < A.rounds; r++) {
       if (phase != kLaneEnter && phase != kLaneStep) continue;
       bool out;
       ev = A.advance(phase, L, out);
@@ -1867,12 +1868,16 @@ __global__ void clean_resolve_kernel(const int32_t* __restrict__ lab, const VolD
 
 // ---- launchers ---------------------------------------------------------------------------
 
-// MSC_TRIPS_PER_TURN_FP64 (2, 4, 8 or 16): stepping iterations per turn of the FP64 loop,
-// for tuning.
+// MSC_TRIPS_PER_TURN, _PASS1, _FP64 (2, 4, 8 or 16): rounds per turn of the fix-up's and the
+// first pass's FP32 loops and of the FP64 loop, for tuning.
 static int trips_env(const char* name, int dflt) {
   const char* e = std::getenv(name);
   const int v = e ? std::atoi(e) : dflt;
   return (v == 2 || v == 4 || v == 8 || v == 16) ? v : dflt;
+}
+static int rounds_per_turn() {
+  static const int k = trips_env("MSC_TRIPS_PER_TURN", kRoundsPerTurn);
+  return k;
 }
 int lane_ctas_per_sm() {
   static const int k = [] {
@@ -1945,15 +1950,16 @@ cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParam
                              uint32_t* claim, unsigned long long* work, unsigned long long* trips, int num_sms,
                              cudaStream_t stream) {
   if (k1 <= k0) return cudaSuccess;
+  static const int rounds = trips_env("MSC_TRIPS_PER_TURN_PASS1", rounds_per_turn());
   const int64_t blocks = (k1 - k0 + 127) / 128;
   const int cap = num_sms * lane_ctas_per_sm();
   const int grid = (int)(blocks < cap ? blocks : cap);
   ::msc::count_launch();
   if (short_steps(P))
-    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr, stops), Q, k0, k1, lab,
+    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab,
                                                      claim, work, trips);
   else
-    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr, stops), Q, k0, k1, lab,
+    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab,
                                                       claim, work, trips);
   return cudaGetLastError();
 }
@@ -2083,13 +2089,14 @@ cudaError_t launch_fixup_end32(const float4* G, const VolDims& V, const IntegPar
     const int v = e ? std::atoi(e) : 2;
     return v >= 1 && v <= 16 ? v : 2;
   }();
+  const int rounds = rounds_per_turn();
   const int cap = num_sms * (n_dev ? early_ctas : lane_ctas_per_sm());
   const int grid = blocks < cap ? blocks : cap;
   if (short_steps(P))
-    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state, nullptr), lab, state, list,
+    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state, list,
                                                        n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
   else
-    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state, nullptr), lab, state,
+    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state,
                                                         list, n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
   return cudaGetLastError();
 }

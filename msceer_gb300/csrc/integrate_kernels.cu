@@ -81,15 +81,17 @@ struct Lane32 {
 constexpr float kShortStep = 0.45f;
 constexpr float kShortThresh = 1e-3f;  // sqrt: 0.032
 
-template <bool SHORT>
+// ENDS: the fix-up's streamlines, which a certain terminal region stops; else the first
+// pass's, which a vertex labelled in an earlier level stops.
+template <bool SHORT, bool ENDS>
 struct Adv32 {
   const float4* G;
   VolDims V;
   IntegParams P;
-  const uint8_t* lvl;    // pass-1 stop (when set): nearest vertex labelled in an earlier level
+  const uint8_t* lvl;    // pass 1: labelled in an earlier level if below `level`
   int level;
-  const uint8_t* state;  // fix-up stop (when set): nearest vertex certain terminal
-  const uint8_t* stops;  // pass-1 stop of short steps: a voxel's corners labelled in an earlier level
+  const uint8_t* state;  // fix-up: certain terminal or not
+  const uint8_t* stops;  // pass 1, short steps: a voxel's corners labelled in an earlier level
   int rounds;            // per turn, at most kRoundsPerTurn
   // Converted once on the host: (float)P.max_step, (float)P.step_mult, the extents
   // (float)V.X .. and (float)(V.X - 2) ..  (a double-to-float or 64-bit integer
@@ -136,12 +138,12 @@ struct Adv32 {
     }
     L.base = index(b[0], b[1], b[2]);
     uint32_t stop = 0;
-    if (SHORT && !state) stop = __ldg(stops + L.base);
+    if (SHORT && !ENDS) stop = __ldg(stops + L.base);
 #pragma unroll
     for (int n = 0; n < 8; n++) {
       const float4 v = __ldg(G + (L.base + ((n & 1) ? o[0] : 0) + ((n & 2) ? o[1] : 0) + ((n & 4) ? o[2] : 0)));
       L.c[n] = {v.x, v.y, v.z};
-      if (SHORT && state) stop |= __float_as_uint(v.w) & (1u << n);
+      if (SHORT && ENDS) stop |= __float_as_uint(v.w) & (1u << n);
     }
     if (SHORT) L.stop = stop;
 #pragma unroll
@@ -269,8 +271,8 @@ struct Adv32 {
       nearest3(np, ix, iy, iz);
       const int32_t nv = index(ix, iy, iz);
       if (acc && nv != L.nv) {
-        const uint8_t st = state ? state[nv] : lvl[nv];
-        const bool hit = state ? (st == kStSeed || st == kStTerminal) : st < level;
+        const uint8_t st = ENDS ? state[nv] : lvl[nv];
+        const bool hit = ENDS ? (st == kStSeed || st == kStTerminal) : st < level;
         if (hit) return EV_HIT_PREASSIGNED;
         L.nv = nv;
       }
@@ -591,7 +593,7 @@ __device__ __forceinline__ uint32_t entry_of(const SpecSet& Q, int64_t k, int e)
 // at their vertices, and make the first round's claims (every item alive, its whole path
 // effective).
 template <bool SHORT>
-__global__ void __launch_bounds__(128, 6) speculate_kernel(const Adv32<SHORT> A, const SpecSet Q, int64_t k0,
+__global__ void __launch_bounds__(128, 6) speculate_kernel(const Adv32<SHORT, false> A, const SpecSet Q, int64_t k0,
                                                            int64_t k1, const int32_t* __restrict__ lab,
                                                            uint32_t* __restrict__ claim,
                                                            unsigned long long* __restrict__ work,
@@ -1473,7 +1475,7 @@ __global__ void __launch_bounds__(32) fixup_end64_kernel(const Adv64 A64, const 
 //   amb_mode 2: its final voxel touches two different certain regions (any ending
 //     within half a voxel of a basin boundary).
 template <bool SHORT>
-__global__ void __launch_bounds__(128, 6) fixup_end32_kernel(const Adv32<SHORT> A, const int32_t* __restrict__ lab,
+__global__ void __launch_bounds__(128, 6) fixup_end32_kernel(const Adv32<SHORT, true> A, const int32_t* __restrict__ lab,
                                                           const uint8_t* __restrict__ state,
                                                           const int64_t* __restrict__ list, int n,
                                                           const int* __restrict__ n_dev,
@@ -1887,7 +1889,7 @@ int lane_ctas_per_sm() {
   }();
   return k;
 }
-// The corner test of Adv32<true> holds for these parameters (MSC_STOP_TEST=memory: the
+// The corner test of short steps (Adv32) holds for these parameters (MSC_STOP_TEST=memory: the
 // general path all the same, for the test that compares the two).
 static bool short_steps(const IntegParams& P) {
   static const bool memory = [] {
@@ -1956,11 +1958,11 @@ cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParam
   const int grid = (int)(blocks < cap ? blocks : cap);
   ::msc::count_launch();
   if (short_steps(P))
-    speculate_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab,
-                                                     claim, work, trips);
+    speculate_kernel<true><<<grid, 128, 0, stream>>>(
+        Adv32<true, false>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab, claim, work, trips);
   else
-    speculate_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab,
-                                                      claim, work, trips);
+    speculate_kernel<false><<<grid, 128, 0, stream>>>(
+        Adv32<false, false>::make(G, V, P, lvl, stamp, nullptr, stops, rounds), Q, k0, k1, lab, claim, work, trips);
   return cudaGetLastError();
 }
 
@@ -2093,11 +2095,13 @@ cudaError_t launch_fixup_end32(const float4* G, const VolDims& V, const IntegPar
   const int cap = num_sms * (n_dev ? early_ctas : lane_ctas_per_sm());
   const int grid = blocks < cap ? blocks : cap;
   if (short_steps(P))
-    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(Adv32<true>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state, list,
-                                                       n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
+    fixup_end32_kernel<true><<<grid, 128, 0, stream>>>(
+        Adv32<true, true>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state, list, n, n_dev, endv, amb,
+        n_amb, amb_mode, work, trips);
   else
-    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(Adv32<false>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state,
-                                                        list, n, n_dev, endv, amb, n_amb, amb_mode, work, trips);
+    fixup_end32_kernel<false><<<grid, 128, 0, stream>>>(
+        Adv32<false, true>::make(G, V, P, nullptr, 0, state, nullptr, rounds), lab, state, list, n, n_dev, endv, amb,
+        n_amb, amb_mode, work, trips);
   return cudaGetLastError();
 }
 

@@ -631,6 +631,7 @@ int first_pass(LabelCtx& c, DirLabels& d) {
       stamp = 0;
     }
     ++stamp;
+    LCUDA(msc::launch_stop_corners(lvl, stamp, c.V, P, stops, c.sms, st), "stop corners");
     return MSC_OK;
   };
   for (int L0 = 0; L0 < S.nlev;) {
@@ -648,7 +649,6 @@ int first_pass(LabelCtx& c, DirLabels& d) {
     for (int64_t k0 = 0; k0 < n;) {
       if (k0 > 0)
         if (int rc = next_stamp()) return rc;
-      LCUDA(msc::launch_stop_corners(lvl, stamp, c.V, P, stops, c.sms, st), "stop corners");
       int64_t k1 = n;
       for (;;) {
         LCUDA(cudaMemsetAsync(sc, 0, sizeof(unsigned long long), st), "memset");

@@ -291,12 +291,6 @@ struct Adv32 {
   }
 };
 
-// Distance of vertex (x, y, z) to the grid's nearest face, in vertices
-__device__ __forceinline__ int dist_to_boundary(const VolDims& V, int x, int y, int z) {
-  const int X = (int)V.X, Y = (int)V.Y, Z = (int)V.Z;
-  return min(min(min(x, X - 1 - x), min(y, Y - 1 - y)), min(z, Z - 1 - z));
-}
-
 // Vertex coordinates of index v; 32-bit division while the grid's indices fit 32 bits.
 __device__ __forceinline__ void split_index(const VolDims& V, int64_t v, int& x, int& y, int& z) {
   if (V.X * V.Y * V.Z <= (int64_t)0xFFFFFFFF) {

@@ -166,11 +166,7 @@ cudaError_t launch_count_unlabelled(const uint8_t* lvl, int64_t N, unsigned long
 // their number to *n_items.  counts: (u1 - u0) / 1024 + 1 ints of scratch.
 cudaError_t launch_spread_compact(const SpreadOrder& S, int64_t u0, int64_t u1, const uint8_t* lvl, int stamp,
                                   int* counts, int32_t* items, unsigned long long* n_items, cudaStream_t stream);
-// Speculative streamlines of items [k0, k1) (stopping at lvl < stamp); they build the
-// holder counts (hcount all 0 at launch) and make the first resolution round's claims.
-// `work`: a device counter, zero at launch; `trips`: advection iterations are added to it;
-// `stops`: launch_stop_corners of the same stamp.
-// The FP32 gradient with the stop flags, and the vertices' states, from the certain
+// The FP32 gradient with the ends' stop flags, and the vertices' states, from the certain
 // terminal regions (label_gradient_kernel).
 cudaError_t launch_label_gradient(const float* f, const int32_t* lab, const uint32_t* zeroed, const VolDims& V,
                                   uint8_t* state, float4* g32, int num_sms, cudaStream_t stream);
@@ -180,6 +176,10 @@ cudaError_t launch_label_gradient(const float* f, const int32_t* lab, const uint
 constexpr int kLevelPad = 8;
 cudaError_t launch_stop_corners(const uint8_t* lvl, int stamp, const VolDims& V, const IntegParams& P, uint8_t* stops,
                                 int num_sms, cudaStream_t stream);
+// Speculative streamlines of items [k0, k1) (stopping at lvl < stamp); they build the
+// holder counts (hcount all 0 at launch) and make the first resolution round's claims.
+// `work`: a device counter, zero at launch; `trips`: advection iterations are added to it;
+// `stops`: launch_stop_corners of the same stamp.
 cudaError_t launch_speculate(const float4* G, const VolDims& V, const IntegParams& P, const SpecSet& Q, int64_t k0,
                              int64_t k1, const int32_t* lab, const uint8_t* lvl, int stamp, const uint8_t* stops,
                              uint32_t* claim, unsigned long long* work, unsigned long long* trips, int num_sms,
@@ -195,6 +195,9 @@ struct SpecDirty {
   uint32_t* list;
   unsigned long long* n;
 };
+// The holder lists of the batch's recorded entries (hcount goes back to 0).
+cudaError_t launch_spec_holders(const SpecSet& Q, int64_t k0, int64_t k1, int64_t N, int* cursor, int num_sms,
+                                cudaStream_t stream);
 // Resolution rounds of items [k0, k1), three stream operations each.  The first (cur ==
 // nullptr) looks at every item (the speculation made its claims); a later one
 // recomputes the claims of cur's vertices from their holders and looks at the items
@@ -202,9 +205,6 @@ struct SpecDirty {
 // between rounds).  An item whose alive / cut changed marks the path vertices between
 // its old and new extent in nxt (whose bitmap must be clear).  The rounds end when a
 // round marks nothing; a round after that one finds no items and marks nothing.
-// The holder lists of the batch's recorded entries (hcount goes back to 0).
-cudaError_t launch_spec_holders(const SpecSet& Q, int64_t k0, int64_t k1, int64_t N, int* cursor, int num_sms,
-                                cudaStream_t stream);
 cudaError_t launch_spec_round(const SpecSet& Q, int64_t k0, int64_t k1, uint32_t* claim, const SpecDirty* cur,
                               const SpecDirty& nxt, uint32_t* ibits, int64_t ibits_words, int num_sms,
                               cudaStream_t stream);

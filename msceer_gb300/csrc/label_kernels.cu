@@ -512,7 +512,8 @@ __global__ void __launch_bounds__(BS) terminal_pass_kernel(const float* __restri
 constexpr int kWalkThreads = 384;
 constexpr int kWalkItems = 128;   // vertices a turn at most: the 64 of a long chain's turn are one pass
 constexpr int kWalkStack = 2048;  // vertices on the block's stack
-constexpr int kWalkTail = 16;
+constexpr int kWalkTail = 16;     // (4 / 16 / 64: labels of a 64^3 Gaussian sum 24.4 / 24.6 / 25.0 ms, of a
+                                  // 256^3 one 85 ms with each)
 
 // Comparer::Compare(a, b), "a comes before b", on the vertices' values and indices
 // (ascending labels: the lower value; descending: the higher)

@@ -1,5 +1,5 @@
 // Learned triage: shared declarations of the network kernels (triage_kernels.cu,
-// triage_train.cu) and the labeling glue (msc_triage_capi.cu).
+// triage_prep.cu) and their host sequences (msc_triage_capi.cu, msc_labels_capi.cu).
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

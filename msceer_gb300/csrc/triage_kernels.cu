@@ -17,8 +17,9 @@
 // (M = eight rows x 16 channels, N = 128 vertices, K = 16 input channels) takes it to all of
 // them: the weights of dy = +1, 0, -1 lie one after the other, so that the operand of input
 // row yy, at the block of dy = yy, holds for output row j the weights of dy = yy - j; the
-// lanes of the other rows are switched off.  90 MMAs for a tile's 8 x 27 taps, each output
-// row's in the order dz, dy, dx, all of one shape on one accumulator and so in order.
+// lanes of the other rows are switched off.  97 MMAs for a tile's 8 x 27 taps (3 x 10 x 3, and
+// seven output rows start with one of their own), each output row's in the order dz, dy, dx,
+// all of one shape on one accumulator and so in order.
 // One CTA per SM keeps the weights in shared memory and works through a run of tiles along
 // z, each with one new plane of input rows (10 x 130, staged by bulk copies, one per
 // 8-channel plane of a row, zeros outside the volume) in a ring of four, and two
@@ -27,7 +28,7 @@
 // shared memory.
 // (One MMA per tap and output row, M = 128 vertices and N = 16 channels, took the same 95
 // cycles, 108 of them for 4 x 128 vertices: 152-159 us a layer at 128^3, and with a CTA per
-// tile 181-217 us; so 80-87 us.  A layer's activations in and out take 20 us of HBM time.)
+// tile 181-217 us; so 79-89 us.  A layer's activations in and out take 20 us of HBM time.)
 #include <cuda_bf16.h>
 
 #include "tc_sm100.cuh"
@@ -130,7 +131,7 @@ struct ConvColumns {
 
 // The mask's values for one warp's share of a tile, as conv_epilogue writes it.  They are
 // asked for before the wait for the tile's MMAs: loaded where they are used, the mask held
-// up the epilogue (164 us a layer at 128^3 instead of 87).
+// up the epilogue (164 us a layer at 128^3 instead of 87; 89 with the marks below).
 __device__ __forceinline__ void load_mask(uint4 (&m)[16], const __nv_bfloat16* __restrict__ mask_act, int x0, int y,
                                           int z, const ConvDims& D) {
   const int lane = threadIdx.x & 31;

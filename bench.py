@@ -345,7 +345,7 @@ def grad_kernels(V, C, t_pairs, t_ldir, nlaunch, reps, n, peak, peak_kind):
     roofline = {"kernel": dom, "bound": "hbm", "achieved": kd["gbs"], "peak": peak, "unit": "GB/s",
                 "frac": kd["gbs"] / peak, "peak_kind": f"{peak_kind} hbm_gbs", "traffic": TRAFFIC_PER_LAUNCH.get((dom, n)),
                 "scope": "dominant kernel of the .grad; the label integration that dominates the full step is "
-                         "FP32/FP64 issue-bound, neither HBM nor tensor bound"}
+                         "bound by instruction issue and by SMs short of warps, neither HBM nor tensor bound"}
     if n is None:  # 2D
         return kernels, roofline
     # the bound these kernels actually meet: instruction issue (per-unit counts from ncu)
@@ -510,8 +510,8 @@ def run_ours(args, ws, rank, local):
                 "speedup_vs_plain": ms_plain / ms_learned,
                 "mismatch_vs_plain": {k: float((learned[k] != plain[k]).float().mean().item()) for k in ("asc", "dsc")},
                 "stats": learned["stats"], "thresholds": [net.threshold_asc, net.threshold_dsc]}
-        # the labeling's kernels are FP32 issue-bound streamline integrations: their
-        # roofline is the FP32 rate.  Operations per advection iteration: two trilinear
+        # the labeling's kernels are FP32 streamline integrations: their roofline is the
+        # FP32 rate.  Operations per advection iteration: two trilinear
         # interpolations of the 3-vector gradient (73 each) plus step control (~37).
         st = res["stats"]
         it32 = sum(st.get(f"{d}_iterations_{k}", 0) for d in ("asc", "dsc") for k in ("first_pass", "fp32"))
@@ -712,8 +712,8 @@ def run_ours(args, ws, rank, local):
 # --set full capture of each kernel at 256^3 (f and .grad together 201 MB, above the
 # L2), scaled to 512^3 by the vertex count (x 8): the traffic grows with the volume.
 # ldir_stage = tile + check kernels (the walk is below 5% of the stage's time).
-_T_LSTAR = 67.332e6 + 77.410e6
-_T_LDIR = 133.5e6 + 115.1e6 + 155.7e6 + 8.2e6
+_T_LSTAR = 67.2e6 + 77.0e6
+_T_LDIR = 133.5e6 + 114.3e6 + 156.4e6 + 8.2e6
 TRAFFIC_PER_LAUNCH: dict = {
     ("lstar_kernel", 256): _T_LSTAR,
     ("ldir_stage", 256): _T_LDIR,
@@ -725,8 +725,8 @@ TRAFFIC_PER_LAUNCH: dict = {
 # schedulers x clock), not HBM.  lstar_kernel: 0.869 G per 256^3 launch (per vertex);
 # ldir stage: tile 0.314 G + check 0.072 G per 256^3 (per cell).  3D only.
 WARP_INST_PER_UNIT: dict = {
-    "lstar_kernel": (0.868808e9 / 256 ** 3, "vertex"),
-    "ldir_stage": ((0.313797e9 + 0.072406e9) / 511 ** 3, "cell"),
+    "lstar_kernel": (0.868858e9 / 256 ** 3, "vertex"),
+    "ldir_stage": ((0.313628e9 + 0.072496e9) / 511 ** 3, "cell"),
 }
 SCHEDULERS_PER_SM = 4
 SMS = 152

@@ -75,7 +75,8 @@ int64_t msc_num_cells_2d(const int64_t dims[2]);
 int msc_lower_star_grad_3d(const float* f, const int64_t dims[3], uint8_t* grad_out, msc_stream_t stream);
 
 /* 2D counterpart: Accurate2D::DiscreteGradientBuilder::ComputeDiscreteGradient with
- * no saddle streamlines (gi_discrete_gradient_computer.h:561-583, 681-689). */
+ * no saddle streamlines (gi_discrete_gradient_computer.h:561-583, 681-689).  Images and
+ * volumes of more than 262,140 rows along y are refused. */
 int msc_lower_star_grad_2d(const float* f, const int64_t dims[2], uint8_t* grad_out, msc_stream_t stream);
 
 /* Many 3D volumes of different sizes in one call (no counterpart in the reference,
@@ -248,9 +249,9 @@ void msc_labels_last_stats(int64_t out[4]);
  * the calling thread: first pass, FP32 boundary re-decisions, FP64 re-decisions;
  * ascending, then descending. */
 void msc_labels_last_iterations(int64_t out[6]);
-/* The labeling keeps its device scratch (about 240 bytes per vertex and direction) in a
- * memory pool of its own that holds on to the memory between calls; this returns the
- * unused part to the device (call it before the application needs that memory
+/* The library keeps its device scratch (the labeling's about 240 bytes per vertex and
+ * direction) in a memory pool of its own that holds on to the memory between calls; this
+ * returns the unused part to the device (call it before the application needs that memory
  * elsewhere).  No counterpart in the reference. */
 void msc_trim_scratch(void);
 
